@@ -44,7 +44,8 @@ class ConvCL:
     """One convolution with repacked weights. ``taps``: (dt, dh, dw) offsets added to an output coordinate to get the input
     coordinate; ``weight_taps``: [C_out, n_taps, C_in] fp32/bf16 in the same order."""
 
-    def __init__(self, weight_taps: torch.Tensor, bias: Optional[torch.Tensor], taps: Sequence[Tuple[int, int, int]], device):
+    def __init__(self, weight_taps: torch.Tensor, bias: Optional[torch.Tensor], taps: Sequence[Tuple[int, int, int]], device,
+                 t_stride: int = 1, hw_stride: int = 1):
         cout, ntaps, cin = weight_taps.shape
         assert ntaps == len(taps) and cin % 16 == 0, (weight_taps.shape, len(taps))
         self.cout, self.cin, self.n_tile = cout, cin, _n_tile(cout)
@@ -57,6 +58,7 @@ class ConvCL:
         self.taps = [int(v) for t in taps for v in t]
         self.spatial = any(t[1] != 0 for t in taps)            # reads neighbouring rows: needs halo rows under row sharding
         self.taps_halo = [int(v) for t in taps for v in (t[0], t[1] + 1, t[2])]
+        self.t_stride, self.hw_stride = t_stride, hw_stride
 
     def __call__(self, x: torch.Tensor, t_out: int, out: Optional[torch.Tensor] = None, out_map: Optional[List[int]] = None,
                  resid: Optional[torch.Tensor] = None, h_out: Optional[int] = None, w_out: Optional[int] = None) -> torch.Tensor:
@@ -64,18 +66,52 @@ class ConvCL:
         decoding (``vae_parallel.row_sharded``) a convolution that reads neighbouring rows first receives one boundary row from
         each neighbouring rank (zeros at the frame border) and reads its input shifted by that row."""
         _, H, W, _ = x.shape
-        h_out, w_out = h_out or H, w_out or W
-        taps = self.taps
+        x, taps = self._halo(x)
+        return self._launch(x, taps, t_out, h_out or H, w_out or W, out, out_map, resid)
+
+    def _halo(self, x):
         if self.spatial and vae_parallel.active() is not None:
-            x = vae_parallel.exchange_rows(x, 1, 1)
-            taps = self.taps_halo
+            return vae_parallel.exchange_rows(x, 1, 1), self.taps_halo
+        return x, self.taps
+
+    def _launch(self, x, taps, t_out, h_out, w_out, out, out_map, resid, cache=None, pad=0):
         if out is None:
             out = torch.empty(t_out, h_out, w_out, self.cout, dtype=torch.bfloat16, device=x.device)
         if out_map is None:
             out_map = [1, 0, 1, 0, 1, 0, out.shape[1], out.shape[2], out.shape[3], 0]
-        native.load().conv_cl(x, self.w, self.n_tile, self.cout, taps, t_out, h_out, w_out, out_map, out, resid, self.bias)
+        native.load().conv_cl(x, self.w, self.n_tile, self.cout, taps, t_out, h_out, w_out, out_map, out, resid, self.bias, cache, pad,
+                              self.t_stride, self.hw_stride)
         native.count_launch()
         return out
+
+    def strided(self, x: torch.Tensor) -> torch.Tensor:
+        """The spatially strided convolution of every frame of ``x``; pixels past the bottom / right edge are zeros."""
+        T, H, W, _ = x.shape
+        if not x.is_cuda:                                      # plain definition: stride 1, every second pixel
+            return self(x, T)[:, ::self.hw_stride, ::self.hw_stride].contiguous()
+        return self._launch(x, self.taps, T, H // self.hw_stride, W // self.hw_stride, None, None, None)
+
+    def causal(self, x: torch.Tensor, state: "_Stream", pad_frames: int = CACHE_T, resid: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """The causal convolution of the chunk ``x`` with the ``pad_frames`` input frames before it, which the stream carries (zeros
+        before the first chunk); leaves this chunk's last frames in the stream."""
+        T, H, W, _ = x.shape
+        t_out = T // self.t_stride
+        if not x.is_cuda:
+            full = _with_cache(self, x, state, pad_frames)
+            return self(full, T, resid=resid)[:t_out * self.t_stride:self.t_stride].contiguous()
+        x, taps = self._halo(x)
+        prev = state.store.get(id(self))
+        out = self._launch(x, taps, t_out, H, W, None, None, resid, prev, pad_frames)
+        state.store[id(self)] = _last_frames(prev, x, pad_frames)
+        return out
+
+
+def _last_frames(prev: Optional[torch.Tensor], x: torch.Tensor, n: int) -> torch.Tensor:
+    """The last ``n`` frames of [prev | x], or fewer when the stream has not seen as many. A view of ``x`` where that is enough: the
+    stream keeps the chunk's tensor alive instead of copying frames out of it."""
+    if x.shape[0] >= n or prev is None:
+        return x[-n:]
+    return torch.cat([prev, x], 0)[-n:]
 
 
 def _causal3_taps(kt: int, kh: int, kw: int):
@@ -117,7 +153,8 @@ class _Stream:
 
 
 def _with_cache(conv: ConvCL, x: torch.Tensor, state: _Stream, pad_frames: int = CACHE_T) -> torch.Tensor:
-    """[cache | x] along time and the cache update: the convolution's input tensor with its causal padding in front."""
+    """[cache | x] along time and the cache update: the convolution's input tensor with its causal padding in front (tensors that the
+    kernel does not serve; it reads the cache where it lies)."""
     prev = state.store.get(id(conv))
     if prev is None:
         prev = x.new_zeros(pad_frames, *x.shape[1:])
@@ -140,10 +177,10 @@ class _ResBlockCL:
         T = x.shape[0]
         h = self.short(x, T) if self.short is not None else x
         y = ops.rmsnorm_silu_cl(x, self.g1, True)
-        y = self.c1(_with_cache(self.c1, y, state), T)
+        y = self.c1.causal(y, state)
         y = ops.rmsnorm_silu_cl(y, self.g2, True)
         native.count_launch(2)
-        return self.c2(_with_cache(self.c2, y, state), T, resid=h)
+        return self.c2.causal(y, state, resid=h)
 
 
 class _AttnCL:
@@ -192,16 +229,11 @@ class _UpsampleCL:
             if prev is None:
                 state.store[id(self._key)] = "first"          # first step: no temporal up-sampling
             else:
-                cache = x[-CACHE_T:].clone()
-                if cache.shape[0] < CACHE_T:
-                    head = prev[-1:] if isinstance(prev, torch.Tensor) else torch.zeros_like(cache[:1])
-                    cache = torch.cat([head, cache], 0)
-                pad = prev if isinstance(prev, torch.Tensor) else x.new_zeros(CACHE_T, H, W, C)
-                full = torch.cat([pad[-CACHE_T:], x], 0)
+                cache = prev if isinstance(prev, torch.Tensor) else None      # nothing before the second step: zeros
                 out = torch.empty(2 * T, H, W, C, dtype=x.dtype, device=x.device)
                 for s, conv in enumerate(self.time):
-                    conv(full, T, out=out, out_map=[2, s, 1, 0, 1, 0, H, W, C, 0])
-                state.store[id(self._key)] = cache
+                    conv._launch(x, conv.taps, T, H, W, out, [2, s, 1, 0, 1, 0, H, W, C, 0], None, cache, CACHE_T)
+                state.store[id(self._key)] = _last_frames(cache, x, CACHE_T)
                 x = out
                 T = 2 * T
         cout = self.phases[0][0].cout
@@ -252,12 +284,12 @@ class DecoderCL:
         T, h, w = x.shape[2:]
         xin = torch.zeros(T, h, w, self.z_pad, dtype=torch.bfloat16, device=self.device)
         xin[..., : self.z_dim] = x[0].permute(1, 2, 3, 0)
-        y = self.conv1(_with_cache(self.conv1, xin, st), T)
+        y = self.conv1.causal(xin, st)
         for layer in self.layers:
             y = layer(y, st)
         y = native.load().rmsnorm_silu_cl(y, self.head_gamma, True)
         native.count_launch()
-        y = self.head(_with_cache(self.head, y, st), y.shape[0])
+        y = self.head.causal(y, st)
         return y.permute(3, 0, 1, 2).unsqueeze(0)
 
 
@@ -270,55 +302,28 @@ def supported(decoder, z: torch.Tensor) -> bool:
 # ------------------------------------------------------------------------------------------------------------------ encoder
 class _DownsampleCL:
     """``ZeroPad2d((0, 1, 0, 1)) + Conv2d(3 x 3, stride 2)`` and, for the 3-D mode, the causal ``(3, 1, 1)`` convolution with
-    temporal stride 2 (wan2pt1.py:84-137), both restated as stride-1 convolutions the kernel can run:
-
-      * space: the frame is regrouped into 2 x 2 pixel blocks ([T, H/2, W/2, 4C], channel = (row in block, column in block, c));
-        output pixel (y, x) reads input pixels (2y + i, 2x + j), i, j in 0..2, which live in blocks (y, x), (y, x + 1), (y + 1, x),
-        (y + 1, x + 1): a 2 x 2-tap convolution whose weights are the 3 x 3 kernel scattered over the block positions (the rest
-        zero); blocks past the bottom / right edge read the kernel's out-of-range fill, which is the zero padding;
-      * time: [previous last frame | chunk] is regrouped into frame pairs ([T/2 + 1, H, W, 2C]); output frame t reads input frames
-        2t, 2t + 1 (pair t) and 2t + 2 (first half of pair t + 1): two taps."""
+    temporal stride 2 (wan2pt1.py:84-137): strided launches of the convolution kernel. Pixels past the bottom / right edge read its
+    out-of-range fill, which is the zero padding; the time convolution's input is [last frame of the previous chunk | chunk]."""
 
     def __init__(self, mod, device):
         conv = mod.resample[1]
-        w = conv.weight.detach().float().cpu()               # [Cout, C, 3, 3]
+        w = conv.weight.detach().float()                     # [Cout, C, 3, 3]
         cout, C = w.shape[:2]
-        taps, mats = [], []
-        for dy in (0, 1):
-            for dx in (0, 1):
-                m = torch.zeros(cout, 2, 2, C)
-                for a in (0, 1):
-                    for b in (0, 1):
-                        if 2 * dy + a < 3 and 2 * dx + b < 3:
-                            m[:, a, b] = w[:, :, 2 * dy + a, 2 * dx + b]
-                mats.append(m.reshape(cout, 4 * C))
-                taps.append((0, dy, dx))
-        self.space = ConvCL(torch.stack(mats, 1), conv.bias, taps, device)
+        self.space = ConvCL(w.permute(0, 2, 3, 1).reshape(cout, 9, C), conv.bias, [(0, i, j) for i in range(3) for j in range(3)], device,
+                            hw_stride=2)
         self.time = None
         if mod.mode == "downsample3d":
-            wt = mod.time_conv.weight.detach().float().cpu()[:, :, :, 0, 0]     # [C, C, 3]
-            c2 = wt.shape[0]
-            m0 = torch.cat([wt[:, :, 0], wt[:, :, 1]], 1)                   # pair t: frames 2t, 2t + 1
-            m1 = torch.cat([wt[:, :, 2], torch.zeros(c2, c2)], 1)          # pair t + 1: frame 2t + 2
-            self.time = ConvCL(torch.stack([m0, m1], 1), mod.time_conv.bias, [(0, 0, 0), (1, 0, 0)], device)
-        self._key = object()
+            wt = mod.time_conv.weight.detach().float()[:, :, :, 0, 0].permute(0, 2, 1)          # [C, 3, C]
+            self.time = ConvCL(wt, mod.time_conv.bias, _causal3_taps(3, 1, 1), device, t_stride=2)
 
     def __call__(self, x, state):
-        T, H, W, C = x.shape
-        blocks = x.view(T, H // 2, 2, W // 2, 2, C).permute(0, 1, 3, 2, 4, 5).reshape(T, H // 2, W // 2, 4 * C)
-        y = self.space(blocks, T)
+        y = self.space.strided(x)
         if self.time is None:
             return y
-        prev = state.store.get(id(self._key))
-        state.store[id(self._key)] = y[-1:].clone()
-        if prev is None:                                                 # first chunk: no temporal down-sampling
+        if id(self.time) not in state.store:                             # first chunk: no temporal down-sampling
+            state.store[id(self.time)] = y[-1:]
             return y
-        full = torch.cat([prev, y], 0)                                   # T + 1 frames
-        if full.shape[0] % 2:
-            full = torch.cat([full, torch.zeros_like(full[:1])], 0)
-        n_p, (_, h, w, c) = full.shape[0] // 2, full.shape
-        pairs = full.view(n_p, 2, h, w, c).permute(0, 2, 3, 1, 4).reshape(n_p, h, w, 2 * c)
-        return self.time(pairs, T // 2)
+        return self.time.causal(y, state, pad_frames=1)
 
 
 class EncoderCL:
@@ -364,18 +369,19 @@ class EncoderCL:
         T, H, W = x.shape[2:]
         xin = torch.zeros(T, H, W, self.in_pad, dtype=torch.bfloat16, device=self.device)
         xin[..., : self.cin] = x[0].permute(1, 2, 3, 0)
-        y = self.conv1(_with_cache(self.conv1, xin, st), T)
+        y = self.conv1.causal(xin, st)
         for layer in self.layers:
             y = layer(y, st)
         y = native.load().rmsnorm_silu_cl(y, self.head_gamma, True)
         native.count_launch()
-        y = self.head(_with_cache(self.head, y, st), y.shape[0])
+        y = self.head.causal(y, st)
         return y.permute(3, 0, 1, 2).unsqueeze(0)
 
 
 def encoder_supported(x: torch.Tensor) -> bool:
     """The kernel encoder serves bf16 CUDA videos, one at a time, whole frames (row-sharded encoding stays on the torch path),
-    with frame sizes that survive three halvings as whole 16 x 8 pixel tiles."""
-    return (x.is_cuda and x.dtype == torch.bfloat16 and x.shape[0] == 1 and x.shape[-2] % 64 == 0 and x.shape[-1] % 128 == 0
+    whose frames halve three times without a remainder (the kernel serves ragged tiles; 29 frames of 768 x 432, which are not whole
+    16 x 8 pixel tiles at the last level: 218 ms on torch convolutions, 69 ms here)."""
+    return (x.is_cuda and x.dtype == torch.bfloat16 and x.shape[0] == 1 and x.shape[-2] % 8 == 0 and x.shape[-1] % 8 == 0
             and vae_parallel.active() is None and native.available() and hasattr(native.load(), "conv_cl")
             and not native.forward_mode())

@@ -22,10 +22,11 @@ int sm_count(int device) {
 }
 
 // x [T_in, H_in, W_in, Cin] bf16; w [n_rows, ntaps * ceil(Cin / 64) * 64] bf16 (tap-major, channels zero-padded to 64);
-// taps: ntaps * 3 ints (dt, dh, dw) added to the output coordinate; out_map: 10 ints (see ConvParams); y is written in place.
+// taps: ntaps * 3 ints (dt, dh, dw) added to the (strided) output coordinate, dt counted from the first of `pad` frames in front of
+// x: the frames of `cache` are the last of these, frames before them are zeros; out_map: 10 ints (see ConvParams); y is written in place.
 void conv_cl(const Tensor& x, const Tensor& w, int64_t n_tile, int64_t Cout, c10::ArrayRef<int64_t> taps, int64_t T_out, int64_t H_out,
              int64_t W_out, c10::ArrayRef<int64_t> out_map, Tensor y, const c10::optional<Tensor>& resid,
-             const c10::optional<Tensor>& bias) {
+             const c10::optional<Tensor>& bias, const c10::optional<Tensor>& cache, int64_t pad, int64_t t_stride, int64_t hw_stride) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.is_contiguous() && x.dim() == 4, "x must be contiguous CUDA bf16 [T, H, W, C]");
   TORCH_CHECK(w.is_cuda() && w.scalar_type() == at::kBFloat16 && w.is_contiguous() && w.dim() == 2 && w.device() == x.device(),
               "w must be contiguous CUDA bf16 [rows, K] on the device of x");
@@ -36,6 +37,11 @@ void conv_cl(const Tensor& x, const Tensor& w, int64_t n_tile, int64_t Cout, c10
   TORCH_CHECK(Cin % 16 == 0, "input channels must be a multiple of 16");
   TORCH_CHECK(n_tile % 16 == 0 && n_tile >= 16 && n_tile <= 256 && w.size(0) % n_tile == 0 && Cout >= 1 && Cout <= w.size(0), "bad N tiling");
   TORCH_CHECK(w.size(1) == ntaps * kblocks * 64, "weight K extent must be taps * ceil(Cin / 64) * 64");
+  TORCH_CHECK(pad >= 0 && pad <= 64 && t_stride >= 1 && t_stride <= 8 && (hw_stride == 1 || hw_stride == 2), "pad 0..64, time stride 1..8, spatial stride 1 or 2");
+  if (cache.has_value())
+    TORCH_CHECK(cache->is_cuda() && cache->scalar_type() == at::kBFloat16 && cache->is_contiguous() && cache->device() == x.device() && cache->dim() == 4 &&
+                    cache->size(0) >= 1 && cache->size(0) <= pad && cache->sizes().slice(1) == x.sizes().slice(1),
+                "cache must be contiguous CUDA bf16 [1..pad, H, W, C] like x");
   TORCH_CHECK(T_out >= 1 && H_out >= 1 && W_out >= 1, "empty output grid");
   // the largest output element the kernel can touch must lie inside y (and inside resid)
   const int64_t ot_mul = out_map[0], ot_add = out_map[1], oh_mul = out_map[2], oh_add = out_map[3], ow_mul = out_map[4], ow_add = out_map[5],
@@ -53,8 +59,9 @@ void conv_cl(const Tensor& x, const Tensor& w, int64_t n_tile, int64_t Cout, c10
   c10::cuda::CUDAGuard g(x.device());
   std::vector<int> tp(taps.begin(), taps.end()), om(out_map.begin(), out_map.end());
   const int dev = x.get_device();
-  const int rc = cb200_conv_cl(x.data_ptr(), (int)x.size(0), (int)x.size(1), (int)x.size(2), (int)Cin, w.data_ptr(), (int)w.size(0),
-                               (int)n_tile, (int)Cout, tp.data(), (int)ntaps, (int)T_out, (int)H_out, (int)W_out, om.data(), y.data_ptr(),
+  const int rc = cb200_conv_cl(x.data_ptr(), (int)x.size(0), (int)x.size(1), (int)x.size(2), (int)Cin,
+                               cache.has_value() ? cache->data_ptr() : nullptr, cache.has_value() ? (int)cache->size(0) : 0, (int)pad,
+                               (int)t_stride, (int)hw_stride, w.data_ptr(), (int)w.size(0), (int)n_tile, (int)Cout, tp.data(), (int)ntaps, (int)T_out, (int)H_out, (int)W_out, om.data(), y.data_ptr(),
                                resid.has_value() ? resid->data_ptr() : nullptr, bias.has_value() ? bias->data_ptr<float>() : nullptr,
                                cb200_error_word(dev), sm_count(dev), at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(rc == 0, "conv_cl launch failed with code ", rc);
@@ -69,7 +76,8 @@ Tensor rmsnorm_silu_cl(const Tensor& x, const Tensor& gamma, bool silu) {
   TORCH_CHECK(C % 8 == 0 && C <= 1024, "channels must be a multiple of 8, at most 1024");
   c10::cuda::CUDAGuard g(x.device());
   Tensor y = at::empty_like(x);
-  const int rc = cb200_rmsnorm_silu_cl(x.data_ptr(), gamma.data_ptr<float>(), y.data_ptr(), x.numel() / C, (int)C, silu ? 1 : 0,
+  const Tensor gm = reinterpret_cast<uintptr_t>(gamma.data_ptr()) % 16 == 0 ? gamma : gamma.clone();   // read as float4
+  const int rc = cb200_rmsnorm_silu_cl(x.data_ptr(), gm.data_ptr<float>(), y.data_ptr(), x.numel() / C, (int)C, silu ? 1 : 0,
                                        at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(rc == 0, "rmsnorm_silu_cl launch failed with code ", rc);
   return y;
@@ -78,6 +86,6 @@ Tensor rmsnorm_silu_cl(const Tensor& x, const Tensor& gamma, bool silu) {
 
 void register_conv_ops(torch::Library& m) {
   m.def("conv_cl(Tensor x, Tensor w, int n_tile, int Cout, int[] taps, int T_out, int H_out, int W_out, int[] out_map, Tensor(a!) y, "
-        "Tensor? resid, Tensor? bias) -> ()", &conv_cl);
+        "Tensor? resid, Tensor? bias, Tensor? cache=None, int pad=0, int t_stride=1, int hw_stride=1) -> ()", &conv_cl);
   m.def("rmsnorm_silu_cl(Tensor x, Tensor gamma, bool silu) -> Tensor", &rmsnorm_silu_cl);
 }

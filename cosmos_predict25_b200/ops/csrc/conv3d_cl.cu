@@ -8,19 +8,32 @@
 //   weights    W [N_pad, taps, C_pad]        (K-major; C_pad = C_in rounded up to 64, N_pad = C_out rounded up to the N tile)
 //   output     Y[t, h, w, n] = bias[n] + sum_{tap, c} X[t + dt(tap), h + dh(tap), w + dw(tap), c] * W[n, tap, c]  (+ residual)
 //
-// There is no im2col buffer: an output tile is 128 voxels = 8 rows x 16 columns of one frame, and the A operand of tap
-// (dt, dh, dw), channel block kb is the TMA box {64 channels, 16 w, 8 h, 1 t} at coordinates (64 kb, w0 + dw, h0 + dh, t + dt) of
-// the activation tensor itself. It lands in shared memory as a [128 rows][64 channels] 128-byte-swizzled K-major tile, which is
-// what the MMA wants. Coordinates outside the tensor read zeros: that IS the zero padding of the convolution (the channel
-// coordinate stays a multiple of 64, so the 16-byte alignment rule of TMA holds for every tap). The causal time padding is
-// two leading frames of the input tensor (the stream cache of the previous chunk, or zeros).
+// There is no im2col buffer: an output tile is 128 voxels = 8 rows x 16 columns of one frame, and the A operand of taps
+// (dt, dh .. dh + n - 1, dw), channel block kb is ONE TMA box {64 channels, 16 w, 7 + n h, 1 t} at coordinates
+// (64 kb, w0 + dw, h0 + dh, t + dt) of the activation tensor itself. It lands in shared memory as rows of 64 channels with 128-byte
+// swizzle, K-major, which is what the MMA wants; a step of one tap down is 16 rows = 2,048 bytes, a whole number of swizzle atoms,
+// so the n taps of a column read the same box at shifted start addresses. Coordinates outside the tensor read zeros: that IS the
+// zero padding of the convolution (the channel coordinate stays a multiple of 64, so the 16-byte alignment rule of TMA holds).
 //
-// Persistent, warp-specialised, one CTA per SM, same skeleton as the GEMM of this package: warp 0 TMA producer (4-stage ring of
-// A box + B box), warp 1 MMA issuer (UMMA 128 x N x 16 into one of two TMEM accumulators), warps 2-9 epilogue (bias, optional
+// The causal time padding is either the leading frames of the input tensor (pad = 0), or `pad` frames in a tensor of their own
+// (the stream cache of the previous chunk) of which the oldest may be missing = zeros: taps whose frame lies in zero padding for
+// the whole tile are skipped (two thirds of a 3 x 3 x 3 convolution on a single image). Strided convolutions (the encoder's
+// down-sampling) step the frame coordinate, and the pixel coordinates through the tensor map's element strides.
+//
+// CTA pairs (tcgen05 cta_group::2): two consecutive voxel tiles share the B operand, each CTA fetches its own A box and half of
+// the B rows, the even CTA issues M = 256 MMAs. What bounds the kernel is the L2 -> shared-memory path of narrow layers: for one
+// (dt, dw) column of a 3 x 3 x 3 convolution with 96 channels a CTA now fetches 20 + 18 KB per channel block instead of
+// 3 x (16 + 12) KB. Decoding 8 latent frames of 720p: 296 ms in this kernel
+// before (one CTA per tile, a box per tap), 224 ms now; a single 640 x 640 image 5.7 -> 2.6 ms.
+//
+// Persistent, warp-specialised, one CTA per SM, same skeleton as the GEMM of this package: warp 0 TMA producer (ring of A box + B
+// boxes, as many stages as fit), warp 1 MMA issuer (two TMEM accumulators of n_tile columns), warps 2-9 epilogue (bias, optional
 // residual, bf16 store through a per-voxel output mapping that also expresses the phase interleave of the up-sampling
 // convolutions and the frame interleave of the temporal up-sampler). All waits are bounded and report through `err`.
 
 #include <math.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 #include "launchers.h"
@@ -32,21 +45,22 @@ using namespace sm100;
 
 namespace cv {
 constexpr int BM = 128, BK = 64, TH = 8, TW = 16;
-constexpr int kStages = 4;
-constexpr int kABytes = BM * BK * 2;          // 16 KB
-constexpr int kBMaxBytes = 256 * BK * 2;      // 32 KB
-constexpr int kStageBytes = kABytes + kBMaxBytes;
 constexpr int kThreads = 320;                 // TMA warp, MMA warp, 8 epilogue warps
-constexpr size_t kSmem = (size_t)kStages * kStageBytes + 1024 + 256;
-constexpr int kMaxTaps = 27;
+constexpr int kMaxTaps = 27, kMaxRun = 3;     // taps, and taps of one column that share a box
+constexpr int kMaxStages = 8;
+constexpr int kSmemMax = 227 * 1024, kSmemFixed = 1024 /*alignment slack*/ + 256 /*barriers*/;
 }  // namespace cv
 
 struct ConvParams {
   int T_out, H_out, W_out;      // output grid walked by the tiles
   int Cin, Cout;
   int n_tile, tiles_n;          // N per tile (multiple of 16, <= 256) and number of N tiles
-  int ntaps, kblocks;           // K loop: taps x 64-channel blocks
-  int8_t dt[cv::kMaxTaps], dh[cv::kMaxTaps], dw[cv::kMaxTaps];   // input coordinate = output coordinate + offset
+  int ngroups, run, kblocks;    // K loop: groups of `run` vertically adjacent taps x 64-channel blocks
+  int stages, a_bytes;          // ring depth, bytes of the A box
+  int pad, cache_frames;        // frames of causal padding in front of X; tm_c holds the last `cache_frames` of them, the rest is zero
+  int t_stride, hw_stride;      // input coordinate = output coordinate x stride + offset
+  int8_t dt[cv::kMaxTaps], dh[cv::kMaxTaps], dw[cv::kMaxTaps];   // per group: input coordinate = output coordinate + offset
+  int8_t tap[cv::kMaxTaps][cv::kMaxRun];                         // weight column block of each tap of the group
   // element offset of output voxel (t, h, w), channel n:
   //   (((t * ot_mul + ot_add) * out_H + h * oh_mul + oh_add) * out_W + w * ow_mul + ow_add) * out_C + oc_add + n
   int ot_mul, ot_add, oh_mul, oh_add, ow_mul, ow_add, out_H, out_W, out_C, oc_add;
@@ -56,80 +70,97 @@ struct ConvParams {
 };
 
 __global__ void __launch_bounds__(cv::kThreads, 1)
-conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const ConvParams p,
-               int* __restrict__ err) {
+conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_w,
+               const __grid_constant__ ConvParams p, int* __restrict__ err) {
   using namespace cv;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
-  uint64_t* full = bars;                    // [kStages]
-  uint64_t* empty = bars + kStages;         // [kStages]
-  uint64_t* acc_full = bars + 2 * kStages;  // [2]
-  uint64_t* acc_empty = acc_full + 2;       // [2]
+  const int b_half = p.n_tile * (BK * 2 / 2);                  // bytes of one tap's B rows in this CTA (half of the N tile)
+  const int stage_bytes = p.a_bytes + p.run * b_half;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + p.stages * stage_bytes);
+  uint64_t* full = bars;                      // [stages], the even CTA's count the bytes of both
+  uint64_t* empty = bars + kMaxStages;        // [stages]
+  uint64_t* acc_full = bars + 2 * kMaxStages; // [2]
+  uint64_t* acc_empty = acc_full + 2;         // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   // the shuffle makes the warp index (and every role branch below) provably warp-uniform for the compiler
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
   const int tiles_w = (p.W_out + TW - 1) / TW, tiles_h = (p.H_out + TH - 1) / TH;
-  const int n_tiles = p.T_out * tiles_h * tiles_w * p.tiles_n;
-  const int b_bytes = p.n_tile * BK * 2;
+  const int vox_tiles = p.T_out * tiles_h * tiles_w;
+  const int n_tiles = (vox_tiles + 1) / 2 * p.tiles_n;         // tiles of the pair: two voxel tiles x one N tile
+  const int first_tile = (int)(blockIdx.x >> 1), tile_step = (int)(gridDim.x >> 1);
 
-  if (threadIdx.x == 0) *abort_flag = *reinterpret_cast<volatile int*>(err);   // an earlier error: drain the grid at once
-  __syncthreads();
-  if (*abort_flag != 0) return;
-  __syncthreads();
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < p.stages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 8);
+      mbar_init(&acc_empty[a], 16);           // the even CTA hears from the epilogue warps of both
     }
     *abort_flag = 0;
     fence_barrier_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 512);
-    tmem_relinquish();
+    tmem_alloc_pair(tmem_slot, 512);
+    tmem_relinquish_pair();
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync_all();                         // the other CTA's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  // tile index -> (n tile, w tile, h tile, frame); N tiles of one voxel tile are neighbours so that they run at the same time
-  // on different SMs and share the activation boxes through L2
-  auto decode = [&](int t, int& nt, int& w0, int& h0, int& tf) {
+  // pair tile -> N tile and this CTA's voxel tile (a trailing odd tile is computed by both CTAs and stored by the even one);
+  // N tiles of one voxel pair are neighbours so that they run at the same time and share the activation boxes through L2
+  auto decode = [&](int t, int& nt, int& w0, int& h0, int& tf, bool& mine) {
     nt = t % p.tiles_n;
-    t /= p.tiles_n;
-    w0 = (t % tiles_w) * TW;
-    t /= tiles_w;
-    h0 = (t % tiles_h) * TH;
-    tf = t / tiles_h;
+    int v = t / p.tiles_n * 2 + (int)rank;
+    mine = v < vox_tiles;
+    v = min(v, vox_tiles - 1);
+    w0 = (v % tiles_w) * TW;
+    v /= tiles_w;
+    h0 = (v % tiles_h) * TH;
+    tf = v / tiles_h;
   };
+  // groups whose frame is zero padding for both tiles of the pair are left out: the later tile's frame decides
+  auto last_frame = [&](int t) { return min(t / p.tiles_n * 2 + 1, vox_tiles - 1) / (tiles_h * tiles_w); };
+  auto skipped = [&](int g, int tf_last) { return tf_last * p.t_stride + p.dt[g] < p.pad - p.cache_frames; };
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       prefetch_tmap(&tm_x);
+      prefetch_tmap(&tm_c);
       prefetch_tmap(&tm_w);
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+      for (int t = first_tile; t < n_tiles && ok; t += tile_step) {
         int nt, w0, h0, tf;
-        decode(t, nt, w0, h0, tf);
-        for (int tap = 0; tap < p.ntaps && ok; ++tap) {
+        bool mine;
+        decode(t, nt, w0, h0, tf, mine);
+        const int tl = last_frame(t), n0 = nt * p.n_tile + (int)rank * (p.n_tile / 2);
+        for (int g = 0; g < p.ngroups && ok; ++g) {
+          if (skipped(g, tl)) continue;
+          const int tx = tf * p.t_stride + p.dt[g] - p.pad;          // frame of X; negative: a cached frame or padding
+          const bool cached = tx < 0 && p.cache_frames > 0;
+          const CUtensorMap* tm = cached ? &tm_c : &tm_x;
+          const int tc = cached ? tx + p.cache_frames : tx;
+          const int xw = w0 * p.hw_stride + p.dw[g], xh = h0 * p.hw_stride + p.dh[g];
           for (int kb = 0; kb < p.kblocks; ++kb) {
             if (!mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-            uint8_t* sa = smem + s * kStageBytes;
-            mbar_arrive_expect_tx(&full[s], kABytes + b_bytes);
-            tma_load_4d(sa, &tm_x, &full[s], kb * BK, w0 + p.dw[tap], h0 + p.dh[tap], tf + p.dt[tap]);
-            tma_load_2d(sa + kABytes, &tm_w, &full[s], (tap * p.kblocks + kb) * BK, nt * p.n_tile);
-            if (++s == kStages) { s = 0; ph ^= 1; }
+            uint8_t* sa = smem + s * stage_bytes;
+            if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * stage_bytes);
+            const uint32_t bar = mapa_shared(smem_u32(&full[s]), 0);
+            tma_load_4d_pair(sa, tm, bar, kb * BK, xw, xh, tc);
+            for (int j = 0; j < p.run; ++j)
+              tma_load_2d_pair(sa + p.a_bytes + j * b_half, &tm_w, bar, (p.tap[g][j] * p.kblocks + kb) * BK, n0);
+            if (++s == p.stages) { s = 0; ph ^= 1; }
           }
         }
       }
@@ -139,35 +170,40 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     // ------------------------------------------------------------------ MMA issuer (warp-uniform; the elected lane issues)
     const uint32_t leader = elect_one() ? 1u : 0u;
     auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)); };
-    const uint32_t idesc = umma_idesc_bf16(BM, p.n_tile, 0, 0);
+    const uint32_t idesc = umma_idesc_bf16(2 * BM, p.n_tile, 0, 0);
     const uint64_t da0 = umma_desc_sw128(smem_u32(smem), 16, 1024);
-    const uint64_t db0 = umma_desc_sw128(smem_u32(smem) + kABytes, 16, 1024);
+    const uint64_t db0 = umma_desc_sw128(smem_u32(smem) + p.a_bytes, 16, 1024);
     int s = 0;
     uint32_t ph = 0;
     int acc = 0;
     uint32_t acc_ph = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+    for (int t = first_tile; t < n_tiles && ok && rank == 0; t += tile_step) {      // only the even CTA issues
       if (!wait_all(&acc_empty[acc], acc_ph ^ 1)) { ok = false; break; }
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + acc * 256;
+      const int tl = last_frame(t);
       uint32_t first = 0;
-      for (int tap = 0; tap < p.ntaps && ok; ++tap) {
+      for (int g = 0; g < p.ngroups && ok; ++g) {
+        if (skipped(g, tl)) continue;
         for (int kb = 0; kb < p.kblocks; ++kb) {
           if (!wait_all(&full[s], ph)) { ok = false; break; }
           tc_fence_after();
-          const uint64_t da_s = da0 + (uint64_t)(s * (kStageBytes >> 4)), db_s = db0 + (uint64_t)(s * (kStageBytes >> 4));
+          const uint64_t da_s = da0 + (uint64_t)(s * (stage_bytes >> 4)), db_s = db0 + (uint64_t)(s * (stage_bytes >> 4));
           const int ksteps = min(4, (p.Cin - kb * BK) / 16);   // the last channel block of C_in = 96 holds 32 real channels
-          for (int k = 0; k < ksteps; ++k) {
-            umma_ss_w(d_tmem, da_s + (uint32_t)((k * 32) >> 4), db_s + (uint32_t)((k * 32) >> 4), idesc, first, leader);
-            first = 1u;
+          for (int j = 0; j < p.run; ++j) {
+            const uint64_t da = da_s + (uint32_t)((j * TW * 128) >> 4), db = db_s + (uint32_t)((j * b_half) >> 4);
+            for (int k = 0; k < ksteps; ++k) {
+              umma_ss_pair_w(d_tmem, da + (uint32_t)((k * 32) >> 4), db + (uint32_t)((k * 32) >> 4), idesc, first, leader);
+              first = 1u;
+            }
           }
-          umma_commit_w(&empty[s], leader);  // slot reusable once these MMAs have read it
-          if (++s == kStages) { s = 0; ph ^= 1; }
+          umma_commit_pair_w(&empty[s], leader);  // slot reusable in both CTAs once these MMAs have read it
+          if (++s == p.stages) { s = 0; ph ^= 1; }
         }
       }
       if (!ok) break;
-      umma_commit_w(&acc_full[acc], leader);
+      umma_commit_pair_w(&acc_full[acc], leader);
       if (++acc == 2) { acc = 0; acc_ph ^= 1; }
     }
     if (!ok && lane == 0) { atomicCAS(err, 0, 62); *abort_flag = 1; }
@@ -182,13 +218,15 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     uint32_t acc_ph = 0;
     bool ok = true;
     const bool vec_ok = ((p.out_C | p.oc_add) & 7) == 0;
-    for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+    const uint32_t acc_empty_leader[2] = {mapa_shared(smem_u32(&acc_empty[0]), 0), mapa_shared(smem_u32(&acc_empty[1]), 0)};
+    for (int t = first_tile; t < n_tiles && ok; t += tile_step) {
       int nt, w0, h0, tf;
-      decode(t, nt, w0, h0, tf);
+      bool mine;
+      decode(t, nt, w0, h0, tf, mine);
       if (!mbar_wait(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const int h = h0 + hh, w = w0 + ww;
-      const bool valid = h < p.H_out && w < p.W_out;
+      const bool valid = mine && h < p.H_out && w < p.W_out;
       const size_t vox = ((size_t)(tf * p.ot_mul + p.ot_add) * p.out_H + (h * p.oh_mul + p.oh_add)) * p.out_W + (w * p.ow_mul + p.ow_add);
       const size_t base = vox * p.out_C + p.oc_add;
       const uint32_t t_row = tmem_base + acc * 256 + ((uint32_t)(quarter * 32) << 16);
@@ -241,7 +279,7 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[acc]);
+      if (lane == 0) mbar_arrive_cluster(acc_empty_leader[acc]);
       if (++acc == 2) { acc = 0; acc_ph ^= 1; }
     }
     if (!ok && lane == 0) { atomicCAS(err, 0, 63); *abort_flag = 1; }
@@ -254,44 +292,56 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync_all();                  // neither CTA leaves (or frees TMEM) while the other may still signal it or read its tiles
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc_pair(tmem_base, 512);
   }
 }
 
 // y[v, :] = silu(x[v, :] / max(||x[v, :]||_2, 1e-12) * sqrt(C) * gamma): the RMS-norm + SiLU in front of every convolution of a
-// residual block, on channels-last rows (one warp per voxel, 16-byte accesses; C a multiple of 8, at most 1024).
+// residual block, on channels-last rows. Bound by memory (one read, one write). G lanes share a voxel and each holds NV 16-byte
+// pieces of it, so that every lane of a warp loads whatever C is: one warp per voxel left 20 of 32 lanes idle at C = 96 and had
+// one load in flight per lane (4 frames of 704 x 1280 x 96, read and written: 1.36 ms; now 0.37 ms, 3.8 TB/s). G * NV * 8 >= C; pieces past C are skipped.
+template <int G, int NV>
 __global__ void __launch_bounds__(256) rmsnorm_silu_cl_kernel(const bf16* __restrict__ x, const float* __restrict__ gamma,
                                                                 bf16* __restrict__ y, long n_vox, int C, float scale, int silu) {
-  const int lane = threadIdx.x & 31;
-  const long v = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (v >= n_vox) return;
-  const bf16* row = x + v * C;
-  bf16* out = y + v * C;
+  const int sub = threadIdx.x % G;
+  const long v = (long)blockIdx.x * (256 / G) + threadIdx.x / G;
+  const bool live = v < n_vox;                         // no early return: the reduction below is warp-wide
+  const bf16* row = x + (live ? v : 0) * C;
   const int nvec = C >> 3;
-  float vals[4][8];
+  float vals[NV][8];
   float ss = 0.f;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int idx = lane + i * 32;
+  for (int i = 0; i < NV; ++i) {
+    const int idx = sub + i * G;
     if (idx < nvec) {
-      const bf16x8 pk = *reinterpret_cast<const bf16x8*>(row + idx * 8);
-      unpack8(pk, vals[i]);
+      unpack8(*reinterpret_cast<const bf16x8*>(row + idx * 8), vals[i]);
+    } else {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) ss = fmaf(vals[i][j], vals[i][j], ss);
+      for (int j = 0; j < 8; ++j) vals[i][j] = 0.f;
     }
   }
-  ss = warp_sum(ss);
-  const float inv = scale / fmaxf(sqrtf(ss), 1e-12f);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int idx = lane + i * 32;
+  for (int i = 0; i < NV; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss = fmaf(vals[i][j], vals[i][j], ss);
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (!live) return;
+  const float inv = scale / fmaxf(sqrtf(ss), 1e-12f);
+  bf16* out = y + v * C;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int idx = sub + i * G;
     if (idx < nvec) {
+      const float4 g0 = *reinterpret_cast<const float4*>(gamma + idx * 8), g1 = *reinterpret_cast<const float4*>(gamma + idx * 8 + 4);
+      const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
       float o[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float z = vals[i][j] * inv * gamma[idx * 8 + j];
+        const float z = vals[i][j] * inv * g[j];
         o[j] = silu ? z / (1.f + __expf(-z)) : z;
       }
       *reinterpret_cast<bf16x8*>(out + idx * 8) = pack8(o);
@@ -303,14 +353,15 @@ __global__ void __launch_bounds__(256) rmsnorm_silu_cl_kernel(const bf16* __rest
 
 using namespace cb200;
 
-// x [T_in, H_in, W_in, Cin] bf16; w [n_rows, ntaps * kblocks * 64] bf16 with n_rows = tiles_n * n_tile; taps: ntaps x (dt, dh, dw).
+// x [T_in, H_in, W_in, Cin] bf16; cache [cache_frames <= pad, H_in, W_in, Cin] or null; w [n_rows, ntaps * kblocks * 64] bf16 with
+// n_rows = tiles_n * n_tile; taps: ntaps x (dt, dh, dw), dt counted from the first of the `pad` frames in front of x.
 // out_map: {ot_mul, ot_add, oh_mul, oh_add, ow_mul, ow_add, out_H, out_W, out_C, oc_add}.
-extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Cin, const void* w, int n_rows, int n_tile, int Cout,
-                             const int* taps, int ntaps, int T_out, int H_out, int W_out, const int* out_map, void* y,
-                             const void* resid, const float* bias, int* err, int sms, cudaStream_t st) {
+extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Cin, const void* cache, int cache_frames, int pad, int t_stride,
+                             int hw_stride, const void* w, int n_rows, int n_tile, int Cout, const int* taps, int ntaps, int T_out, int H_out, int W_out, const int* out_map,
+                             void* y, const void* resid, const float* bias, int* err, int sms, cudaStream_t st) {
   using namespace cv;
   if (Cin % 16 != 0 || Cin < 16 || ntaps < 1 || ntaps > kMaxTaps || n_tile % 16 != 0 || n_tile < 16 || n_tile > 256 ||
-      n_rows % n_tile != 0 || Cout > n_rows || Cout < 1)
+      n_rows % n_tile != 0 || Cout > n_rows || Cout < 1 || pad < 0 || pad > 64 || cache_frames < 0 || cache_frames > pad || t_stride < 1 || t_stride > 8 || hw_stride < 1 || hw_stride > 2)
     return -51;
   ConvParams p{};
   p.T_out = T_out;
@@ -320,15 +371,55 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
   p.Cout = Cout;
   p.n_tile = n_tile;
   p.tiles_n = (Cout + n_tile - 1) / n_tile;
-  p.ntaps = ntaps;
   p.kblocks = (Cin + BK - 1) / BK;
+  p.pad = pad;
+  p.cache_frames = cache != nullptr ? cache_frames : 0;
+  p.t_stride = t_stride;
+  p.hw_stride = hw_stride;
+  int max_dt = -128;
   for (int i = 0; i < ntaps; ++i) {
     const int dt = taps[3 * i], dh = taps[3 * i + 1], dw = taps[3 * i + 2];
     if (dt < -64 || dt > 64 || dh < -64 || dh > 64 || dw < -64 || dw > 64) return -52;
-    p.dt[i] = (int8_t)dt;
-    p.dh[i] = (int8_t)dh;
-    p.dw[i] = (int8_t)dw;
+    max_dt = std::max(max_dt, dt);
   }
+  if (pad > 0 && max_dt < pad) return -52;      // the newest tap has to read X itself: otherwise a frame could be all padding
+  // Columns of taps: for `run` = 3, 2 the whole list has to fall into (dt, dw) columns of exactly `run` adjacent rows, else 1.
+  // (with a spatial stride neighbouring taps do not share rows of a strided box)
+  for (int run = hw_stride == 1 ? kMaxRun : 1; run >= 1; --run) {
+    bool used[kMaxTaps] = {};
+    int ng = 0;
+    bool fits = ntaps % run == 0;
+    for (int i = 0; i < ntaps && fits; ++i) {
+      if (used[i]) continue;
+      const int dt = taps[3 * i], dw = taps[3 * i + 2];
+      int dh0 = taps[3 * i + 1];
+      if (run > 1)
+        for (int k = 0; k < ntaps; ++k)
+          if (!used[k] && taps[3 * k] == dt && taps[3 * k + 2] == dw) dh0 = std::min(dh0, taps[3 * k + 1]);
+      for (int j = 0; j < run && fits; ++j) {
+        int found = -1;
+        for (int k = run > 1 ? 0 : i; k < ntaps && found < 0; ++k)
+          if (!used[k] && taps[3 * k] == dt && taps[3 * k + 2] == dw && taps[3 * k + 1] == dh0 + j) found = k;
+        fits = found >= 0;
+        if (fits) {
+          used[found] = true;
+          p.tap[ng][j] = (int8_t)found;
+        }
+      }
+      p.dt[ng] = (int8_t)dt;
+      p.dh[ng] = (int8_t)dh0;
+      p.dw[ng] = (int8_t)dw;
+      ++ng;
+    }
+    if (fits) {
+      p.run = run;
+      p.ngroups = ng;
+      break;
+    }
+  }
+  p.a_bytes = (TH + p.run - 1) * TW * BK * 2;
+  const int stage_bytes = p.a_bytes + p.run * n_tile * BK;
+  p.stages = std::min(kMaxStages, (kSmemMax - kSmemFixed) / stage_bytes);
   p.ot_mul = out_map[0];
   p.ot_add = out_map[1];
   p.oh_mul = out_map[2];
@@ -342,34 +433,73 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
   p.Y = (bf16*)y;
   p.resid = (const bf16*)resid;
   p.bias = bias;
-  CUtensorMap tx, tw;
+  CUtensorMap tx, tc, tw;
+  const uint64_t strides[3] = {(uint64_t)Cin * 2, (uint64_t)W_in * Cin * 2, (uint64_t)H_in * W_in * Cin * 2};
+  const uint32_t hw = (uint32_t)hw_stride, box[4] = {BK, TW * hw, (uint32_t)(TH + p.run - 1) * hw, 1}, step[4] = {1, hw, hw, 1};
   {
     const uint64_t dims[4] = {(uint64_t)Cin, (uint64_t)W_in, (uint64_t)H_in, (uint64_t)T_in};
-    const uint64_t strides[3] = {(uint64_t)Cin * 2, (uint64_t)W_in * Cin * 2, (uint64_t)H_in * W_in * Cin * 2};
-    const uint32_t box[4] = {BK, TW, TH, 1};
-    const int rc = make_tmap_bf16(&tx, x, 4, dims, strides, box);
+    const int rc = make_tmap_bf16(&tx, x, 4, dims, strides, box, 1, step);
+    if (rc) return rc;
+  }
+  tc = tx;
+  if (p.cache_frames > 0) {
+    const uint64_t dims[4] = {(uint64_t)Cin, (uint64_t)W_in, (uint64_t)H_in, (uint64_t)p.cache_frames};
+    const int rc = make_tmap_bf16(&tc, cache, 4, dims, strides, box, 1, step);
     if (rc) return rc;
   }
   {
     const uint64_t kdim = (uint64_t)ntaps * p.kblocks * BK;
-    const int rc = make_tmap_2d_bf16(&tw, w, kdim, (uint64_t)n_rows, kdim * 2, BK, (uint32_t)n_tile);
+    const int rc = make_tmap_2d_bf16(&tw, w, kdim, (uint64_t)n_rows, kdim * 2, BK, (uint32_t)(n_tile / 2));
     if (rc) return rc;
   }
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(conv_cl_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    cudaError_t e = cudaFuncSetAttribute(conv_cl_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
     if (e != cudaSuccess) return 100 + (int)e;
     attr = true;
   }
-  const long tiles = (long)T_out * ((H_out + TH - 1) / TH) * ((W_out + TW - 1) / TW) * p.tiles_n;
-  if (tiles <= 0 || tiles > 0x7fffffffL) return -53;
-  const int grid = tiles < sms ? (int)tiles : sms;
-  conv_cl_kernel<<<grid, kThreads, kSmem, st>>>(tx, tw, p, err);
-  return (int)cudaGetLastError();
+  const long vox = (long)T_out * ((H_out + TH - 1) / TH) * ((W_out + TW - 1) / TW);
+  const long tiles = (vox + 1) / 2 * p.tiles_n;
+  if (tiles <= 0 || 2 * tiles > 0x7fffffffL) return -53;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * (sms / 2));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = (size_t)p.stages * stage_bytes + kSmemFixed;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  // as in the GEMM: the persistent grid is bounded by the pairs that the GPU can hold at once. One CTA per SM whatever the ring
+  // depth (TMEM is allocated whole), so the figure for the largest shared-memory size holds for all
+  static int max_pairs = 0;
+  if (max_pairs == 0) {
+    int n = 0;
+    cudaLaunchConfig_t c = cfg;
+    c.dynamicSmemBytes = kSmemMax;
+    if (cudaOccupancyMaxActiveClusters(&n, conv_cl_kernel, &c) != cudaSuccess || n < 1) return 600;
+    max_pairs = n;
+  }
+  cfg.gridDim = dim3(2 * (unsigned)std::min<long>(tiles, std::min(max_pairs, sms / 2)));
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, conv_cl_kernel, tx, tc, tw, p, err);
+  return e == cudaSuccess ? 0 : 500 + (int)e;
 }
 
 extern "C" int cb200_rmsnorm_silu_cl(const void* x, const float* gamma, void* y, long n_vox, int C, int silu, cudaStream_t st) {
   if (C % 8 != 0 || C > 1024 || n_vox <= 0) return -54;
-  rmsnorm_silu_cl_kernel<<<(unsigned)((n_vox + 7) / 8), 256, 0, st>>>((const bf16*)x, gamma, (bf16*)y, n_vox, C, sqrtf((float)C), silu);
+  const float scale = sqrtf((float)C);
+  auto run = [&](auto kern, int lanes) {
+    const int per_block = 256 / lanes;
+    kern<<<(unsigned)((n_vox + per_block - 1) / per_block), 256, 0, st>>>((const bf16*)x, gamma, (bf16*)y, n_vox, C, scale, silu);
+  };
+  // three pieces per lane while that fills the lanes (C = 96, 192, 384: no idle lane); the widest rows take four
+  if (C <= 48) run(rmsnorm_silu_cl_kernel<2, 3>, 2);
+  else if (C <= 96) run(rmsnorm_silu_cl_kernel<4, 3>, 4);
+  else if (C <= 192) run(rmsnorm_silu_cl_kernel<8, 3>, 8);
+  else if (C <= 384) run(rmsnorm_silu_cl_kernel<16, 3>, 16);
+  else run(rmsnorm_silu_cl_kernel<32, 4>, 32);
   return (int)cudaGetLastError();
 }

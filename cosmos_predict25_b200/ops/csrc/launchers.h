@@ -112,8 +112,8 @@ int cb200_fa_bwd(const void* d_o, const void* q, const void* k, const void* v, c
 
 extern "C" {
 // conv3d_cl.cu
-int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Cin, const void* w, int n_rows, int n_tile, int Cout,
-                  const int* taps, int ntaps, int T_out, int H_out, int W_out, const int* out_map, void* y, const void* resid,
+int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Cin, const void* cache, int cache_frames, int pad, int t_stride,
+                  int hw_stride, const void* w, int n_rows, int n_tile, int Cout, const int* taps, int ntaps, int T_out, int H_out, int W_out, const int* out_map, void* y, const void* resid,
                   const float* bias, int* err, int sms, cudaStream_t st);
 int cb200_rmsnorm_silu_cl(const void* x, const float* gamma, void* y, long n_vox, int C, int silu, cudaStream_t st);
 }

@@ -45,7 +45,7 @@ static EncodeTiledFn resolve_encode() {
 }
 
 int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
-                   const uint32_t* box, int swizzle_128) {
+                   const uint32_t* box, int swizzle_128, const uint32_t* elem_strides) {
   EncodeTiledFn fn = resolve_encode();
   if (fn == nullptr) return 901;
   if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) return 902;
@@ -58,6 +58,7 @@ int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t*
     key.v[2 + i] = dims[i];
     key.v[7 + i] = box[i];
     if (i > 0) key.v[12 + i - 1] = strides_bytes[i - 1];
+    key.v[1] |= (uint64_t)(elem_strides != nullptr ? elem_strides[i] : 1) << (8 + 4 * i);
   }
   {
     std::lock_guard<std::mutex> lk(g_tmap_mu);
@@ -88,7 +89,7 @@ int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t*
   for (int i = 0; i < rank; ++i) {
     gdim[i] = dims[i];
     bx[i] = box[i];
-    estr[i] = 1;
+    estr[i] = elem_strides != nullptr ? elem_strides[i] : 1;
     if (i > 0) {
       gstr[i - 1] = strides_bytes[i - 1];
       if (gstr[i - 1] % 16 != 0) return 903;

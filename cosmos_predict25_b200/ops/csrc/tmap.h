@@ -9,7 +9,7 @@ namespace cb200 {
 // rank-N bf16 tensor map with 128-byte swizzle. dims/box innermost first; strides_bytes has rank-1
 // entries (stride of dims 1..rank-1). Returns 0 on success, a positive error code otherwise.
 int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
-                   const uint32_t* box, int swizzle_128 = 1);
+                   const uint32_t* box, int swizzle_128 = 1, const uint32_t* elem_strides = nullptr);
 
 inline int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t dim0, uint64_t dim1, uint64_t stride1_bytes,
                              uint32_t box0, uint32_t box1) {

@@ -65,6 +65,58 @@ def test_upsample_phase_convolutions_match_nearest_then_conv():
     _close(got, want, 6e-2, 3e-2, "upsample + conv2d")
 
 
+# chunk lengths x kernel shape: one image (all but one frame of taps is padding), a one-frame first chunk (its cache is shorter than
+# the padding), one-frame chunks, longer ones; an odd number of voxel tiles; 3, 2 and 1 taps per box; an N tile of 16
+@pytest.mark.parametrize("chunks", [(1,), (1, 1, 1), (1, 4, 2), (3,), (2, 3)])
+@pytest.mark.parametrize("ksize,H,W,Cin,Cout", [((3, 3, 3), 9, 17, 96, 96), ((3, 1, 1), 24, 16, 32, 64), ((3, 3, 3), 8, 16, 64, 3),
+                                                ((3, 2, 2), 13, 40, 160, 384)])
+def test_streamed_causal_convolution_reads_cached_frames(chunks, ksize, H, W, Cin, Cout):
+    from cosmos_predict25_b200.models import vae_wan_cl
+    torch.manual_seed(5)
+    kt, kh, kw = ksize
+    w = (torch.randn(Cout, Cin, kt, kh, kw, device=DEV) / (Cin * kt * kh * kw) ** 0.5).bfloat16().float()
+    b = torch.randn(Cout, device=DEV)
+    x = torch.randn(1, Cin, sum(chunks), H, W, device=DEV).bfloat16()
+    want = F.conv3d(F.pad(x.float(), (kw // 2, (kw - 1) // 2, kh // 2, (kh - 1) // 2, kt - 1, 0)), w, b)[0].permute(1, 2, 3, 0)
+    cl = vae_wan_cl.ConvCL(w.permute(0, 2, 3, 4, 1).reshape(Cout, -1, Cin), b, vae_wan_cl._causal3_taps(kt, kh, kw), DEV)
+    st, got, lo = vae_wan_cl._Stream(), [], 0
+    for n in chunks:
+        got.append(cl.causal(x[0, :, lo:lo + n].permute(1, 2, 3, 0).contiguous(), st))
+        lo += n
+    _no_kernel_error()
+    # unit-variance products summed in fp32, stored in bf16: half an ulp relative, plus the order of the sums
+    _close(torch.cat(got, 0), want, 4e-3, 1e-2, "streamed conv")
+
+
+@pytest.mark.parametrize("H,W,C", [(16, 32, 96), (22, 50, 32), (54, 96, 192), (2, 4, 384)])
+def test_strided_convolutions_match_torch_resample(H, W, C):
+    """The encoder's down-sampling (spatial stride 2 with bottom / right padding, causal temporal stride 2) chunk by chunk."""
+    from cosmos_predict25_b200.models import vae_wan, vae_wan_cl
+    torch.manual_seed(6)
+    mod = vae_wan.Resample(C, "downsample3d").to(DEV)
+    for p in mod.parameters():
+        p.data = p.data.bfloat16().float()
+    cl, st, st_t = vae_wan_cl._DownsampleCL(mod, DEV), vae_wan_cl._Stream(), vae_wan.StreamState()
+    for T in (1, 4, 8, 2):
+        x = torch.randn(1, C, T, H, W, device=DEV).bfloat16()
+        with torch.no_grad():
+            want = mod(x.float(), st_t)[0].permute(1, 2, 3, 0)
+        got = cl(x[0].permute(1, 2, 3, 0).contiguous(), st)
+        _no_kernel_error()
+        _close(got, want, 3e-2, 2e-2, f"down-sampling, chunk of {T}")
+
+
+@pytest.mark.parametrize("C", [8, 32, 48, 56, 96, 160, 192, 384, 392, 1024])
+def test_rmsnorm_silu_widths(C):
+    torch.manual_seed(7)
+    x = torch.randn(3, 5, 7, C, device=DEV).bfloat16()
+    x[0, 0, 0] = 0
+    g = (1 + 0.1 * torch.randn(C + 1, device=DEV)).float()[1:]             # four bytes off a 16-byte boundary
+    for silu in (True, False):
+        want = F.normalize(x.float(), dim=-1) * C ** 0.5 * g
+        _close(native.load().rmsnorm_silu_cl(x, g, silu), F.silu(want) if silu else want, 4e-3, 8e-3, f"rmsnorm {C}")
+
+
 def test_rmsnorm_silu_channels_last():
     torch.manual_seed(2)
     x = torch.randn(5, 7, 9, 96, device=DEV).bfloat16()
