@@ -48,15 +48,17 @@ constexpr int BM = 128, BK = 64, TH = 8, TW = 16;
 constexpr int kThreads = 320;                 // TMA warp, MMA warp, 8 epilogue warps
 constexpr int kMaxTaps = 27, kMaxRun = 3;     // taps, and taps of one column that share a box
 constexpr int kMaxStages = 8;
-constexpr int kSmemMax = 227 * 1024, kSmemFixed = 1024 /*alignment slack*/ + 256 /*barriers*/;
+constexpr int kStageOut = 32 * 64;            // staging block of an epilogue warp: 32 voxels x 32 channels
+constexpr int kBiasMax = 1024;                // channels whose bias is kept in shared memory
+constexpr int kSmemMax = 227 * 1024, kSmemFixed = 1024 /*alignment slack*/ + 256 /*barriers*/ + 8 * kStageOut;
 }  // namespace cv
 
 struct ConvParams {
   int T_out, H_out, W_out;      // output grid walked by the tiles
   int Cin, Cout;
   int n_tile, tiles_n;          // N per tile (multiple of 16, <= 256) and number of N tiles
-  int ngroups, run, kblocks;    // K loop: groups of `run` vertically adjacent taps x 64-channel blocks
-  int stages, a_bytes;          // ring depth, bytes of the A box
+  int ngroups, kblocks;         // K loop: groups of RUN vertically adjacent taps (by ascending dt) x 64-channel blocks
+  int stages;                   // ring depth
   int pad, cache_frames;        // frames of causal padding in front of X; tm_c holds the last `cache_frames` of them, the rest is zero
   int t_stride, hw_stride;      // input coordinate = output coordinate x stride + offset
   int8_t dt[cv::kMaxTaps], dh[cv::kMaxTaps], dw[cv::kMaxTaps];   // per group: input coordinate = output coordinate + offset
@@ -69,6 +71,7 @@ struct ConvParams {
   const float* bias;            // optional [Cout]
 };
 
+template <int RUN>
 __global__ void __launch_bounds__(cv::kThreads, 1)
 conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_w,
                const __grid_constant__ ConvParams p, int* __restrict__ err) {
@@ -76,7 +79,8 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int b_half = p.n_tile * (BK * 2 / 2);                  // bytes of one tap's B rows in this CTA (half of the N tile)
-  const int stage_bytes = p.a_bytes + p.run * b_half;
+  constexpr int a_bytes = (TH + RUN - 1) * TW * BK * 2;
+  const int stage_bytes = a_bytes + RUN * b_half;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + p.stages * stage_bytes);
   uint64_t* full = bars;                      // [stages], the even CTA's count the bytes of both
   uint64_t* empty = bars + kMaxStages;        // [stages]
@@ -84,6 +88,8 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   uint64_t* acc_empty = acc_full + 2;         // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint8_t* stage_out = smem + p.stages * stage_bytes + 256;
+  float* bias_s = reinterpret_cast<float*>(stage_out + 8 * kStageOut);   // [Cout] when Cout <= kBiasMax
 
   // the shuffle makes the warp index (and every role branch below) provably warp-uniform for the compiler
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -105,6 +111,8 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     *abort_flag = 0;
     fence_barrier_init();
   }
+  if (p.bias != nullptr && p.Cout <= kBiasMax)
+    for (int i = threadIdx.x; i < p.Cout; i += kThreads) bias_s[i] = p.bias[i];
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, 512);
     tmem_relinquish_pair();
@@ -127,9 +135,14 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     h0 = (v % tiles_h) * TH;
     tf = v / tiles_h;
   };
-  // groups whose frame is zero padding for both tiles of the pair are left out: the later tile's frame decides
-  auto last_frame = [&](int t) { return min(t / p.tiles_n * 2 + 1, vox_tiles - 1) / (tiles_h * tiles_w); };
-  auto skipped = [&](int g, int tf_last) { return tf_last * p.t_stride + p.dt[g] < p.pad - p.cache_frames; };
+  // groups whose frame is zero padding for both tiles of the pair are left out: the later tile's frame decides, and the groups
+  // are in the order of their frames
+  auto first_group = [&](int t) {
+    const int tf_last = min(t / p.tiles_n * 2 + 1, vox_tiles - 1) / (tiles_h * tiles_w);
+    int g = 0;
+    while (g < p.ngroups - 1 && tf_last * p.t_stride + p.dt[g] < p.pad - p.cache_frames) ++g;
+    return g;
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -144,9 +157,8 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         int nt, w0, h0, tf;
         bool mine;
         decode(t, nt, w0, h0, tf, mine);
-        const int tl = last_frame(t), n0 = nt * p.n_tile + (int)rank * (p.n_tile / 2);
-        for (int g = 0; g < p.ngroups && ok; ++g) {
-          if (skipped(g, tl)) continue;
+        const int n0 = nt * p.n_tile + (int)rank * (p.n_tile / 2);
+        for (int g = first_group(t); g < p.ngroups && ok; ++g) {
           const int tx = tf * p.t_stride + p.dt[g] - p.pad;          // frame of X; negative: a cached frame or padding
           const bool cached = tx < 0 && p.cache_frames > 0;
           const CUtensorMap* tm = cached ? &tm_c : &tm_x;
@@ -158,8 +170,9 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
             if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * stage_bytes);
             const uint32_t bar = mapa_shared(smem_u32(&full[s]), 0);
             tma_load_4d_pair(sa, tm, bar, kb * BK, xw, xh, tc);
-            for (int j = 0; j < p.run; ++j)
-              tma_load_2d_pair(sa + p.a_bytes + j * b_half, &tm_w, bar, (p.tap[g][j] * p.kblocks + kb) * BK, n0);
+#pragma unroll
+            for (int j = 0; j < RUN; ++j)
+              tma_load_2d_pair(sa + a_bytes + j * b_half, &tm_w, bar, (p.tap[g][j] * p.kblocks + kb) * BK, n0);
             if (++s == p.stages) { s = 0; ph ^= 1; }
           }
         }
@@ -172,7 +185,7 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)); };
     const uint32_t idesc = umma_idesc_bf16(2 * BM, p.n_tile, 0, 0);
     const uint64_t da0 = umma_desc_sw128(smem_u32(smem), 16, 1024);
-    const uint64_t db0 = umma_desc_sw128(smem_u32(smem) + p.a_bytes, 16, 1024);
+    const uint64_t db0 = umma_desc_sw128(smem_u32(smem) + a_bytes, 16, 1024);
     int s = 0;
     uint32_t ph = 0;
     int acc = 0;
@@ -182,22 +195,36 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       if (!wait_all(&acc_empty[acc], acc_ph ^ 1)) { ok = false; break; }
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + acc * 256;
-      const int tl = last_frame(t);
       uint32_t first = 0;
-      for (int g = 0; g < p.ngroups && ok; ++g) {
-        if (skipped(g, tl)) continue;
+      for (int g = first_group(t); g < p.ngroups && ok; ++g) {
         for (int kb = 0; kb < p.kblocks; ++kb) {
           if (!wait_all(&full[s], ph)) { ok = false; break; }
           tc_fence_after();
           const uint64_t da_s = da0 + (uint64_t)(s * (stage_bytes >> 4)), db_s = db0 + (uint64_t)(s * (stage_bytes >> 4));
-          const int ksteps = min(4, (p.Cin - kb * BK) / 16);   // the last channel block of C_in = 96 holds 32 real channels
-          for (int j = 0; j < p.run; ++j) {
-            const uint64_t da = da_s + (uint32_t)((j * TW * 128) >> 4), db = db_s + (uint32_t)((j * b_half) >> 4);
-            for (int k = 0; k < ksteps; ++k) {
-              umma_ss_pair_w(d_tmem, da + (uint32_t)((k * 32) >> 4), db + (uint32_t)((k * 32) >> 4), idesc, first, leader);
-              first = 1u;
-            }
+          const int ksteps = (p.Cin - kb * BK) / 16;   // below 4 in the last block of, e.g., C_in = 96: 32 real channels
+          // straight-line issue: one warp issues every MMA of the pair, and a narrow MMA (N = 96: 48 clocks) is over before a
+          // loop with descriptor arithmetic gets to the next one (64 -> 16 channels, 27 taps: 6.8 us a tile as loops, 4.4 us)
+          if (ksteps >= 4) {
+#pragma unroll
+            for (int j = 0; j < RUN; ++j)
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                umma_ss_pair_w(d_tmem, da_s + (uint32_t)((j * TW * 128 + k * 32) >> 4),
+                               db_s + (uint32_t)(j * (b_half >> 4) + k * 2), idesc, (j | k) ? 1u : first, leader);
+          } else if (ksteps == 2) {
+#pragma unroll
+            for (int j = 0; j < RUN; ++j)
+#pragma unroll
+              for (int k = 0; k < 2; ++k)
+                umma_ss_pair_w(d_tmem, da_s + (uint32_t)((j * TW * 128 + k * 32) >> 4),
+                               db_s + (uint32_t)(j * (b_half >> 4) + k * 2), idesc, (j | k) ? 1u : first, leader);
+          } else {
+            for (int j = 0; j < RUN; ++j)
+              for (int k = 0; k < ksteps; ++k)
+                umma_ss_pair_w(d_tmem, da_s + (uint32_t)((j * TW * 128 + k * 32) >> 4),
+                               db_s + (uint32_t)(j * (b_half >> 4) + k * 2), idesc, (j | k) ? 1u : first, leader);
           }
+          first = 1u;
           umma_commit_pair_w(&empty[s], leader);  // slot reusable in both CTAs once these MMAs have read it
           if (++s == p.stages) { s = 0; ph ^= 1; }
         }
@@ -208,72 +235,113 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     }
     if (!ok && lane == 0) { atomicCAS(err, 0, 62); *abort_flag = 1; }
   } else {
-    // ------------------------------------------------------------------ epilogue warps: a thread owns one output voxel
+    // ------------------------------------------------------------------ epilogue warps
+    // A thread owns one output voxel of the accumulator and stages 32 channels of it; then 4 lanes cover the 64 contiguous bytes
+    // of a voxel. Storing (and reading the residual) per thread made 32 partly filled requests per instruction and bound every
+    // convolution with a short K loop (1 x 1, 64 -> 192 channels with residual: 13.5 us a tile, now 5.1 us).
     const int quarter = warp & 3;      // TMEM lanes [32 quarter, +32)
-    const int part = (warp - 2) >> 2;  // which half of the tile's 16-column chunks
-    const int r = quarter * 32 + lane; // row of the tile = (h, w) of the voxel inside the 8 x 16 patch
-    const int hh = r >> 4, ww = r & 15;
-    const int nch = p.n_tile >> 4, c_lo = part == 0 ? 0 : (nch + 1) / 2, c_hi = part == 0 ? (nch + 1) / 2 : nch;
+    const int part = (warp - 2) >> 2;  // which half of the tile's 32-column chunks
+    const int nch = (p.n_tile + 31) >> 5, c_lo = part == 0 ? 0 : (nch + 1) / 2, c_hi = part == 0 ? (nch + 1) / 2 : nch;
+    uint8_t* stage_warp = stage_out + (warp - 2) * kStageOut;
     int acc = 0;
     uint32_t acc_ph = 0;
     bool ok = true;
-    const bool vec_ok = ((p.out_C | p.oc_add) & 7) == 0;
+    const bool vec_ok = ((p.out_C | p.oc_add | p.Cout) & 7) == 0;
+    const float* bias = p.bias != nullptr && p.Cout <= kBiasMax ? bias_s : p.bias;
     const uint32_t acc_empty_leader[2] = {mapa_shared(smem_u32(&acc_empty[0]), 0), mapa_shared(smem_u32(&acc_empty[1]), 0)};
     for (int t = first_tile; t < n_tiles && ok; t += tile_step) {
       int nt, w0, h0, tf;
       bool mine;
       decode(t, nt, w0, h0, tf, mine);
-      if (!mbar_wait(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
-      tc_fence_after();
-      const int h = h0 + hh, w = w0 + ww;
-      const bool valid = mine && h < p.H_out && w < p.W_out;
-      const size_t vox = ((size_t)(tf * p.ot_mul + p.ot_add) * p.out_H + (h * p.oh_mul + p.oh_add)) * p.out_W + (w * p.ow_mul + p.ow_add);
-      const size_t base = vox * p.out_C + p.oc_add;
+      // element offset of a voxel of the tile (row r = 16 h + w), or -1 outside the frame
+      auto offset = [&](int r) -> long {
+        const int h = h0 + (r >> 4), w = w0 + (r & 15);
+        if (!mine || h >= p.H_out || w >= p.W_out) return -1;
+        return (((long)(tf * p.ot_mul + p.ot_add) * p.out_H + (h * p.oh_mul + p.oh_add)) * p.out_W + (w * p.ow_mul + p.ow_add)) * p.out_C + p.oc_add;
+      };
       const uint32_t t_row = tmem_base + acc * 256 + ((uint32_t)(quarter * 32) << 16);
+      if (vec_ok) {
+        const int piece = lane & 3;                       // 16-byte piece of the 64-byte run that this lane moves
+        long off[4];                                      // voxels quarter * 32 + 8 it + lane / 4
+#pragma unroll
+        for (int it = 0; it < 4; ++it) off[it] = offset(quarter * 32 + it * 8 + (lane >> 2));
+        auto slot = [&](int row, int pc) { return stage_warp + row * 64 + ((pc ^ ((row >> 1) & 3)) << 4); };   // no bank conflicts
+        // residual of the first chunk: on its way while the accumulator is still being computed
+        uint4 res[4];
+        auto fetch = [&](int c) {
+          const int n = nt * p.n_tile + c * 32 + piece * 8;
+#pragma unroll
+          for (int it = 0; it < 4; ++it)
+            if (off[it] >= 0 && n < p.Cout) res[it] = *reinterpret_cast<const uint4*>(p.resid + off[it] + n);
+        };
+        if (p.resid != nullptr && c_lo < c_hi) fetch(c_lo);
+        if (!mbar_wait(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
+        tc_fence_after();
 #pragma unroll 1
-      for (int c = c_lo; c < c_hi; ++c) {
-        uint32_t a[16];
-        tmem_ld16(t_row + c * 16, a);      // warp-collective: every lane runs it, invalid voxels only skip their stores
-        tmem_ld_wait();
-        const int n0 = nt * p.n_tile + c * 16;
-        if (valid && n0 < p.Cout) {
-          float v[16];
+        for (int c = c_lo; c < c_hi; ++c) {
+          const int n0 = nt * p.n_tile + c * 32;
+          uint32_t a[32];
+          tmem_ld32(t_row + c * 32, a);                   // warp-collective; columns past the tile are loaded and not stored
+          tmem_ld_wait();
+          if (bias != nullptr) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(a[j]);
-          const bool full_chunk = vec_ok && n0 + 16 <= p.Cout;
-          if (p.bias != nullptr) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              if (full_chunk || n0 + j < p.Cout) v[j] += p.bias[n0 + j];
+            for (int j = 0; j < 32; ++j)
+              if (n0 + j < p.Cout) a[j] = __float_as_uint(__uint_as_float(a[j]) + bias[n0 + j]);
           }
-          if (full_chunk) {
-            if (p.resid != nullptr) {
+          if (p.resid != nullptr) {
+            // the sum is rounded once: the residual comes through the staging block to the thread that owns the voxel
 #pragma unroll
-              for (int q = 0; q < 2; ++q) {
-                const uint4 rr = *reinterpret_cast<const uint4*>(p.resid + base + n0 + q * 8);
-                const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rr);
+            for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(slot(it * 8 + (lane >> 2), piece)) = res[it];
+            if (c + 1 < c_hi) fetch(c + 1);
+            __syncwarp();
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const float2 rf = __bfloat1622float2(r2[j]);
-                  v[q * 8 + 2 * j] += rf.x;
-                  v[q * 8 + 2 * j + 1] += rf.y;
-                }
+            for (int q = 0; q < 4; ++q) {
+              const uint4 rr = *reinterpret_cast<const uint4*>(slot(lane, q));
+              const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rr);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float2 rf = __bfloat1622float2(r2[j]);
+                a[q * 8 + 2 * j] = __float_as_uint(__uint_as_float(a[q * 8 + 2 * j]) + rf.x);
+                a[q * 8 + 2 * j + 1] = __float_as_uint(__uint_as_float(a[q * 8 + 2 * j + 1]) + rf.y);
               }
             }
+          }
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              uint4 o;
-              __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
+          for (int q = 0; q < 4; ++q) {
+            uint4 o;
+            __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-              for (int j = 0; j < 4; ++j) o2[j] = __floats2bfloat162_rn(v[q * 8 + 2 * j], v[q * 8 + 2 * j + 1]);
-              *reinterpret_cast<uint4*>(p.Y + base + n0 + q * 8) = o;
-            }
-          } else {
-            for (int j = 0; j < 16 && n0 + j < p.Cout; ++j) {
-              float o = v[j];
-              if (p.resid != nullptr) o += __bfloat162float(p.resid[base + n0 + j]);
-              p.Y[base + n0 + j] = __float2bfloat16(o);
-            }
+            for (int j = 0; j < 4; ++j)
+              o2[j] = __floats2bfloat162_rn(__uint_as_float(a[q * 8 + 2 * j]), __uint_as_float(a[q * 8 + 2 * j + 1]));
+            *reinterpret_cast<uint4*>(slot(lane, q)) = o;
+          }
+          __syncwarp();
+          const int n = n0 + piece * 8;
+#pragma unroll
+          for (int it = 0; it < 4; ++it)
+            if (off[it] >= 0 && n < p.Cout && c * 32 + piece * 8 < p.n_tile)
+              *reinterpret_cast<uint4*>(p.Y + off[it] + n) = *reinterpret_cast<const uint4*>(slot(it * 8 + (lane >> 2), piece));
+          __syncwarp();
+        }
+      } else {
+        const long base = offset(quarter * 32 + lane);
+        if (!mbar_wait(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+#pragma unroll 1
+        for (int c = c_lo; c < c_hi; ++c) {
+          uint32_t a[32];
+          tmem_ld32(t_row + c * 32, a);
+          tmem_ld_wait();
+          const int n0 = nt * p.n_tile + c * 32;
+          if (base >= 0) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (n0 + j < p.Cout && c * 32 + j < p.n_tile) {
+                float o = __uint_as_float(a[j]);
+                if (bias != nullptr) o += bias[n0 + j];
+                if (p.resid != nullptr) o += __bfloat162float(p.resid[base + n0 + j]);
+                p.Y[base + n0 + j] = __float2bfloat16(o);
+              }
           }
         }
       }
@@ -353,6 +421,27 @@ __global__ void __launch_bounds__(256) rmsnorm_silu_cl_kernel(const bf16* __rest
 
 using namespace cb200;
 
+// As in the GEMM: the persistent grid is bounded by the pairs that the GPU can hold at once. One CTA per SM whatever the ring depth
+// (every ring is over half of the shared memory), so the figure for the largest shared-memory size holds for all.
+template <int RUN>
+static int launch_conv(cudaLaunchConfig_t& cfg, long tiles, int sms, const CUtensorMap& tx, const CUtensorMap& tc,
+                       const CUtensorMap& tw, const ConvParams& p, int* err) {
+  const auto kern = conv_cl_kernel<RUN>;
+  static int max_pairs = 0;
+  if (max_pairs == 0) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cv::kSmemMax);
+    if (e != cudaSuccess) return 100 + (int)e;
+    int n = 0;
+    cudaLaunchConfig_t c = cfg;
+    c.dynamicSmemBytes = cv::kSmemMax;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &c) != cudaSuccess || n < 1) return 600;
+    max_pairs = n;
+  }
+  cfg.gridDim = dim3(2 * (unsigned)std::min<long>(tiles, std::min(max_pairs, sms / 2)));
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tx, tc, tw, p, err);
+  return e == cudaSuccess ? 0 : 500 + (int)e;
+}
+
 // x [T_in, H_in, W_in, Cin] bf16; cache [cache_frames <= pad, H_in, W_in, Cin] or null; w [n_rows, ntaps * kblocks * 64] bf16 with
 // n_rows = tiles_n * n_tile; taps: ntaps x (dt, dh, dw), dt counted from the first of the `pad` frames in front of x.
 // out_map: {ot_mul, ot_add, oh_mul, oh_add, ow_mul, ow_add, out_H, out_W, out_C, oc_add}.
@@ -385,11 +474,15 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
   if (pad > 0 && max_dt < pad) return -52;      // the newest tap has to read X itself: otherwise a frame could be all padding
   // Columns of taps: for `run` = 3, 2 the whole list has to fall into (dt, dw) columns of exactly `run` adjacent rows, else 1.
   // (with a spatial stride neighbouring taps do not share rows of a strided box)
-  for (int run = hw_stride == 1 ? kMaxRun : 1; run >= 1; --run) {
+  int order[kMaxTaps], run = 1;
+  for (int i = 0; i < ntaps; ++i) order[i] = i;
+  std::stable_sort(order, order + ntaps, [&](int a, int b) { return taps[3 * a] < taps[3 * b]; });
+  for (run = hw_stride == 1 ? kMaxRun : 1; run >= 1; --run) {
     bool used[kMaxTaps] = {};
     int ng = 0;
     bool fits = ntaps % run == 0;
-    for (int i = 0; i < ntaps && fits; ++i) {
+    for (int q = 0; q < ntaps && fits; ++q) {
+      const int i = order[q];
       if (used[i]) continue;
       const int dt = taps[3 * i], dw = taps[3 * i + 2];
       int dh0 = taps[3 * i + 1];
@@ -397,8 +490,8 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
         for (int k = 0; k < ntaps; ++k)
           if (!used[k] && taps[3 * k] == dt && taps[3 * k + 2] == dw) dh0 = std::min(dh0, taps[3 * k + 1]);
       for (int j = 0; j < run && fits; ++j) {
-        int found = -1;
-        for (int k = run > 1 ? 0 : i; k < ntaps && found < 0; ++k)
+        int found = run > 1 ? -1 : i;
+        for (int k = 0; k < ntaps && found < 0; ++k)
           if (!used[k] && taps[3 * k] == dt && taps[3 * k + 2] == dw && taps[3 * k + 1] == dh0 + j) found = k;
         fits = found >= 0;
         if (fits) {
@@ -412,14 +505,13 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
       ++ng;
     }
     if (fits) {
-      p.run = run;
       p.ngroups = ng;
       break;
     }
   }
-  p.a_bytes = (TH + p.run - 1) * TW * BK * 2;
-  const int stage_bytes = p.a_bytes + p.run * n_tile * BK;
-  p.stages = std::min(kMaxStages, (kSmemMax - kSmemFixed) / stage_bytes);
+  const int stage_bytes = (TH + run - 1) * TW * BK * 2 + run * n_tile * BK;
+  const int fixed = kSmemFixed + (Cout <= kBiasMax ? (Cout * 4 + 15) / 16 * 16 : 0);
+  p.stages = std::min(kMaxStages, (kSmemMax - fixed) / stage_bytes);
   p.ot_mul = out_map[0];
   p.ot_add = out_map[1];
   p.oh_mul = out_map[2];
@@ -435,7 +527,7 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
   p.bias = bias;
   CUtensorMap tx, tc, tw;
   const uint64_t strides[3] = {(uint64_t)Cin * 2, (uint64_t)W_in * Cin * 2, (uint64_t)H_in * W_in * Cin * 2};
-  const uint32_t hw = (uint32_t)hw_stride, box[4] = {BK, TW * hw, (uint32_t)(TH + p.run - 1) * hw, 1}, step[4] = {1, hw, hw, 1};
+  const uint32_t hw = (uint32_t)hw_stride, box[4] = {BK, TW * hw, (uint32_t)(TH + run - 1) * hw, 1}, step[4] = {1, hw, hw, 1};
   {
     const uint64_t dims[4] = {(uint64_t)Cin, (uint64_t)W_in, (uint64_t)H_in, (uint64_t)T_in};
     const int rc = make_tmap_bf16(&tx, x, 4, dims, strides, box, 1, step);
@@ -452,19 +544,13 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
     const int rc = make_tmap_2d_bf16(&tw, w, kdim, (uint64_t)n_rows, kdim * 2, BK, (uint32_t)(n_tile / 2));
     if (rc) return rc;
   }
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(conv_cl_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
-    if (e != cudaSuccess) return 100 + (int)e;
-    attr = true;
-  }
   const long vox = (long)T_out * ((H_out + TH - 1) / TH) * ((W_out + TW - 1) / TW);
   const long tiles = (vox + 1) / 2 * p.tiles_n;
   if (tiles <= 0 || 2 * tiles > 0x7fffffffL) return -53;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * (sms / 2));
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = (size_t)p.stages * stage_bytes + kSmemFixed;
+  cfg.dynamicSmemBytes = (size_t)p.stages * stage_bytes + fixed;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -473,19 +559,9 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  // as in the GEMM: the persistent grid is bounded by the pairs that the GPU can hold at once. One CTA per SM whatever the ring
-  // depth (TMEM is allocated whole), so the figure for the largest shared-memory size holds for all
-  static int max_pairs = 0;
-  if (max_pairs == 0) {
-    int n = 0;
-    cudaLaunchConfig_t c = cfg;
-    c.dynamicSmemBytes = kSmemMax;
-    if (cudaOccupancyMaxActiveClusters(&n, conv_cl_kernel, &c) != cudaSuccess || n < 1) return 600;
-    max_pairs = n;
-  }
-  cfg.gridDim = dim3(2 * (unsigned)std::min<long>(tiles, std::min(max_pairs, sms / 2)));
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, conv_cl_kernel, tx, tc, tw, p, err);
-  return e == cudaSuccess ? 0 : 500 + (int)e;
+  return run == 3 ? launch_conv<3>(cfg, tiles, sms, tx, tc, tw, p, err)
+       : run == 2 ? launch_conv<2>(cfg, tiles, sms, tx, tc, tw, p, err)
+                  : launch_conv<1>(cfg, tiles, sms, tx, tc, tw, p, err);
 }
 
 extern "C" int cb200_rmsnorm_silu_cl(const void* x, const float* gamma, void* y, long n_vox, int C, int silu, cudaStream_t st) {
