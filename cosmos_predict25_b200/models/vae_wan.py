@@ -318,6 +318,7 @@ class WanVAE_(nn.Module):
             if clear_encoder_cache or cl.state is None:
                 cl.reset()
             run = cl.step
+            tw *= cl.windows_per_step(x.shape[-2], x.shape[-1], tw)
         else:
             run = lambda chunk: self.encoder(chunk, st)
         outs = [run(x[:, :, :1])]
@@ -355,7 +356,7 @@ class WanVAE_(nn.Module):
             # channels-last decoder on this package's convolution kernel; it keeps its own stream state
             if clear_decoder_cache or cl.state is None:
                 cl.reset()
-            outs = [cl.step(x[:, :, i: i + 1]) for i in range(z.shape[2])]
+            outs = [cl.step(x[:, :, lo:hi]) for lo, hi in cl.steps(*z.shape[2:])]
             if clear_decoder_cache:
                 cl.state = None
                 self._dec_state = None

@@ -13,8 +13,8 @@ step (cosmos_predict2/_src/predict2/tokenizers/wan2pt1.py:40-58, 84-137, 184-215
   * the temporal up-sampler's channel-to-frame interleave is an output mapping too (two launches, one per output-channel half);
   * RMS-norm + SiLU in front of a convolution is one element-wise kernel.
 
-The single-head frame attention of the middle block keeps torch's attention (head dimension 384) with its 1 x 1 projections on
-this package's GEMM. Weights are repacked once (``[C_out, taps, C_in padded to 64]`` bf16, fp32 bias) when the object is built.
+The single-head frame attention of the middle block runs on ``fa_wide`` (head dimension 384) with its 1 x 1 projections on this
+package's GEMM. Weights are repacked once (``[C_out, taps, C_in padded to 64]`` bf16, fp32 bias) when the object is built.
 """
 
 from __future__ import annotations
@@ -29,6 +29,7 @@ from ..ops import native
 from . import vae_parallel
 
 CACHE_T = 2
+STEP_BYTES = 3 << 29       # full-resolution activation of one streaming step (a step holds a handful of them; the stream one per layer)
 
 
 def _n_tile(cout: int) -> int:
@@ -198,11 +199,15 @@ class _AttnCL:
         y = native.load().rmsnorm_silu_cl(x, self.gamma, False)
         native.count_launch()
         qkv = F_ops.linear(y.view(T * H * W, C), self.w_qkv, self.b_qkv).view(T, H * W, 3, C)
-        q, k, v = (qkv[:, :, i].unsqueeze(1) for i in range(3))          # [T, 1, HW, C]
+        q, k, v = (qkv[:, :, i] for i in range(3))                        # [T, HW, C], a single head of dimension C
         if vae_parallel.active() is not None:                             # local rows attend to the whole frame
-            k, v = vae_parallel.gather_tokens(k.contiguous(), 2), vae_parallel.gather_tokens(v.contiguous(), 2)
-        o = F.scaled_dot_product_attention(q, k, v)                       # single head of dimension C
-        o = F_ops.linear(o.squeeze(1).reshape(T * H * W, C), self.w_proj, self.b_proj)
+            k, v = vae_parallel.gather_tokens(k.contiguous(), 1), vae_parallel.gather_tokens(v.contiguous(), 1)
+        if x.is_cuda and C == 384:
+            o = native.load().fa_wide(q, k, v, C ** -0.5)
+            native.count_launch()
+        else:                                                             # the kernel is built for the width of the released VAE
+            o = F.scaled_dot_product_attention(q.unsqueeze(1), k.unsqueeze(1), v.unsqueeze(1)).squeeze(1)
+        o = F_ops.linear(o.reshape(T * H * W, C), self.w_proj, self.b_proj)
         return o.view(T, H, W, C) + x
 
 
@@ -273,6 +278,15 @@ class DecoderCL:
 
     def reset(self):
         self.state = _Stream()
+
+    def steps(self, frames: int, h: int, w: int) -> List[Tuple[int, int]]:
+        """Ranges of latent frames to decode in one step each. A stream starts with a step of one frame (it skips the temporal
+        up-sampling); after that as many frames as keep a full-resolution activation within ``STEP_BYTES``, because one latent frame
+        is too few tiles for the low-resolution layers (384 channels at 88 x 160: 1.5 waves, 980 TFLOP/s; two frames 1,320)."""
+        per_frame = 4 * 64 * h * w * self.head.cin * 2
+        n = max(1, STEP_BYTES // per_frame)
+        cuts = [0] + list(range(1 if self.state is None or not self.state.store else n, frames, n)) + [frames]
+        return list(zip(cuts[:-1], cuts[1:]))
 
     @torch.no_grad()
     def step(self, x: torch.Tensor) -> torch.Tensor:
@@ -358,6 +372,13 @@ class EncoderCL:
 
     def reset(self):
         self.state = _Stream()
+
+    def windows_per_step(self, H: int, W: int, window: int) -> int:
+        """How many temporal windows one step takes: as many as keep a full-resolution activation within ``STEP_BYTES``. The result does
+        not depend on it when a window passes both temporal down-samplers without a remainder."""
+        if window % 4:
+            return 1
+        return max(1, STEP_BYTES // (window * H * W * self.conv1.cout * 2))
 
     @torch.no_grad()
     def step(self, x: torch.Tensor) -> torch.Tensor:

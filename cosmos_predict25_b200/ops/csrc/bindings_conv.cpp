@@ -82,10 +82,29 @@ Tensor rmsnorm_silu_cl(const Tensor& x, const Tensor& gamma, bool silu) {
   TORCH_CHECK(rc == 0, "rmsnorm_silu_cl launch failed with code ", rc);
   return y;
 }
+
+// softmax(q k^T * scale) v for one head of 384 channels: q [B, Sq, 384], k, v [B, Skv, 384] bf16, rows of any 16-byte aligned stride
+Tensor fa_wide(const Tensor& q, const Tensor& k, const Tensor& v, double scale) {
+  for (const Tensor* t : {&q, &k, &v}) {
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kBFloat16 && t->dim() == 3 && t->size(2) == 384 && t->stride(2) == 1 &&
+                    t->device() == q.device() && t->size(0) == q.size(0), "fa_wide: q, k, v must be CUDA bf16 [B, S, 384] with dense channels");
+    TORCH_CHECK(t->stride(1) % 8 == 0 && t->stride(0) % 8 == 0 && t->stride(1) > 0 && t->stride(0) > 0 &&
+                    reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "fa_wide: rows must start on 16-byte boundaries");
+  }
+  TORCH_CHECK(k.size(1) == v.size(1) && q.numel() > 0 && k.numel() > 0, "fa_wide: empty input or k / v of different length");
+  c10::cuda::CUDAGuard g(q.device());
+  Tensor o = at::empty({q.size(0), q.size(1), 384}, q.options());
+  const int rc = cb200_fa_wide(q.data_ptr(), q.stride(1), q.stride(0), k.data_ptr(), k.stride(1), k.stride(0), v.data_ptr(), v.stride(1),
+                               v.stride(0), o.data_ptr(), (int)q.size(0), (int)q.size(1), (int)k.size(1), (float)scale,
+                               cb200_error_word(q.get_device()), at::cuda::getCurrentCUDAStream().stream());
+  TORCH_CHECK(rc == 0, "fa_wide launch failed with code ", rc);
+  return o;
+}
 }  // namespace
 
 void register_conv_ops(torch::Library& m) {
   m.def("conv_cl(Tensor x, Tensor w, int n_tile, int Cout, int[] taps, int T_out, int H_out, int W_out, int[] out_map, Tensor(a!) y, "
         "Tensor? resid, Tensor? bias, Tensor? cache=None, int pad=0, int t_stride=1, int hw_stride=1) -> ()", &conv_cl);
+  m.def("fa_wide(Tensor q, Tensor k, Tensor v, float scale) -> Tensor", &fa_wide);
   m.def("rmsnorm_silu_cl(Tensor x, Tensor gamma, bool silu) -> Tensor", &rmsnorm_silu_cl);
 }

@@ -106,6 +106,19 @@ def test_strided_convolutions_match_torch_resample(H, W, C):
         _close(got, want, 3e-2, 2e-2, f"down-sampling, chunk of {T}")
 
 
+# queries and keys: below one tile, whole tiles, one row over, an odd and an even number of key tiles; large scores move the reference maximum
+@pytest.mark.parametrize("B,Sq,Skv,gain", [(1, 5, 7, 1.0), (2, 128, 64, 1.0), (1, 129, 65, 4.0), (3, 300, 1000, 8.0), (1, 1024, 1024, 1.0)])
+def test_wide_attention_matches_fp32(B, Sq, Skv, gain):
+    torch.manual_seed(8)
+    qkv = torch.randn(B, max(Sq, Skv), 3, 384, device=DEV).bfloat16()
+    q, k, v = qkv[:, :Sq, 0] * gain, qkv[:, :Skv, 1] * torch.linspace(0.2, 2, Skv, device=DEV)[:, None].bfloat16(), qkv[:, :Skv, 2]
+    got = native.load().fa_wide(q, k, v, 384 ** -0.5)
+    _no_kernel_error()
+    want = F.scaled_dot_product_attention(*(t.float().unsqueeze(1) for t in (q, k, v))).squeeze(1)
+    # probabilities and the result are rounded to bf16: 2^-9 of a weighted mean of unit-variance values each, plus the order of the sums
+    _close(got, want, 1e-2, 1e-2, "attention of width 384")
+
+
 @pytest.mark.parametrize("C", [8, 32, 48, 56, 96, 160, 192, 384, 392, 1024])
 def test_rmsnorm_silu_widths(C):
     torch.manual_seed(7)
