@@ -27,6 +27,22 @@ inline void check_f32(const Tensor& t, const char* name) {
   TORCH_CHECK(t.is_contiguous(), name, " must be contiguous");
 }
 
+// Rows of a per-frame modulation vector ([frames, D] fp32, e.g. a third of the columns of the modulation MLPs' output) as the
+// kernels read them: 16-byte aligned rows of any stride; anything else is copied.
+inline Tensor mod_rows(const Tensor& t, const char* name) {
+  TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kFloat && t.dim() == 2, name, " must be a 2-D float32 CUDA tensor");
+  const bool ok = t.stride(1) == 1 && t.stride(0) % 4 == 0 && t.stride(0) >= 0 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+  return ok ? t : t.clone(at::MemoryFormat::Contiguous);
+}
+// A norm weight as the kernels read it: bf16 or fp32, 16-byte aligned.
+inline Tensor norm_weight(const Tensor& w) {
+  if ((w.scalar_type() == at::kFloat || w.scalar_type() == at::kBFloat16) && w.is_contiguous() &&
+      reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 == 0)
+    return w;
+  return w.to(at::kFloat).clone(at::MemoryFormat::Contiguous);
+}
+inline int is_bf16(const Tensor& t) { return t.scalar_type() == at::kBFloat16 ? 1 : 0; }
+
 constexpr int kRowsPerCta = 32;
 constexpr int kRowsPerWarp = CB200_RMSNORM_BWD_ROWS_PER_WARP;
 
@@ -48,17 +64,16 @@ inline int* error_word(int device) { return cb200_error_word(device); }
 std::tuple<Tensor, Tensor, Tensor> ln_modulate_fwd(const Tensor& x, const Tensor& shift, const Tensor& scale, int64_t L,
                                                    double eps) {
   check_bf16(x, "x");
-  check_f32(shift, "shift");
-  check_f32(scale, "scale");
   c10::cuda::CUDAGuard g(x.device());
+  const Tensor sh = mod_rows(shift, "shift"), sc = mod_rows(scale, "scale");
   const int64_t rows = x.size(0), D = x.size(1);
   TORCH_CHECK(D % 8 == 0 && D <= 8192, "channel dim must be a multiple of 8 and <= 8192");
-  TORCH_CHECK(rows % L == 0 && shift.size(0) == rows / L && shift.size(1) == D, "shift/scale must be [rows/L, D]");
+  TORCH_CHECK(rows % L == 0 && shift.size(0) == rows / L && shift.size(1) == D && scale.sizes() == shift.sizes(), "shift/scale must be [rows/L, D]");
   Tensor y = at::empty_like(x);
   Tensor mean = at::empty({rows}, x.options().dtype(at::kFloat));
   Tensor rstd = at::empty({rows}, x.options().dtype(at::kFloat));
-  cb200_ln_modulate_fwd(x.data_ptr(), shift.data_ptr<float>(), scale.data_ptr<float>(), y.data_ptr(), mean.data_ptr<float>(),
-                        rstd.data_ptr<float>(), rows, (int)D, (int)L, (float)eps, stream());
+  cb200_ln_modulate_fwd(x.data_ptr(), sh.data_ptr<float>(), sc.data_ptr<float>(), y.data_ptr(), mean.data_ptr<float>(),
+                        rstd.data_ptr<float>(), rows, (int)D, (int)L, sh.stride(0), sc.stride(0), (float)eps, stream());
   return {y, mean, rstd};
 }
 
@@ -66,45 +81,45 @@ std::tuple<Tensor, Tensor, Tensor> ln_modulate_bwd(const Tensor& dy, const Tenso
                                                    const Tensor& scale, int64_t L) {
   check_bf16(dy, "dy");
   check_bf16(x, "x");
-  check_f32(scale, "scale");
   c10::cuda::CUDAGuard g(x.device());
+  const Tensor sc = mod_rows(scale, "scale");
   const int64_t rows = x.size(0), D = x.size(1), frames = rows / L;
   Tensor dx = at::empty_like(x);
   Tensor dshift = at::empty({frames, D}, scale.options());
   Tensor dscale = at::empty({frames, D}, scale.options());
   const int G = cb200_ln_groups_per_frame((int)L, kRowsPerCta);
   Tensor partials = at::empty({frames * G, 2, D}, scale.options());
-  cb200_ln_modulate_bwd(dy.data_ptr(), x.data_ptr(), mean.data_ptr<float>(), rstd.data_ptr<float>(), scale.data_ptr<float>(),
+  cb200_ln_modulate_bwd(dy.data_ptr(), x.data_ptr(), mean.data_ptr<float>(), rstd.data_ptr<float>(), sc.data_ptr<float>(),
                         dx.data_ptr(), dshift.data_ptr<float>(), dscale.data_ptr<float>(), partials.data_ptr<float>(), frames,
-                        (int)D, (int)L, kRowsPerCta, stream());
+                        (int)D, (int)L, kRowsPerCta, sc.stride(0), stream());
   return {dx, dshift, dscale};
 }
 
 Tensor gate_residual_fwd(const Tensor& x, const Tensor& gate, const Tensor& y, int64_t L) {
   check_bf16(x, "x");
   check_bf16(y, "y");
-  check_f32(gate, "gate");
   c10::cuda::CUDAGuard g(x.device());
+  const Tensor gt = mod_rows(gate, "gate");
   const int64_t rows = x.size(0), D = x.size(1);
   TORCH_CHECK(D % 8 == 0 && gate.size(0) == rows / L && gate.size(1) == D, "gate must be [rows/L, D]");
   Tensor out = at::empty_like(x);
-  cb200_gate_residual_fwd(x.data_ptr(), gate.data_ptr<float>(), y.data_ptr(), out.data_ptr(), rows, (int)D, (int)L, stream());
+  cb200_gate_residual_fwd(x.data_ptr(), gt.data_ptr<float>(), y.data_ptr(), out.data_ptr(), rows, (int)D, (int)L, gt.stride(0), stream());
   return out;
 }
 
 std::tuple<Tensor, Tensor> gate_residual_bwd(const Tensor& dout, const Tensor& gate, const Tensor& y, int64_t L) {
   check_bf16(dout, "dout");
   check_bf16(y, "y");
-  check_f32(gate, "gate");
   c10::cuda::CUDAGuard g(y.device());
+  const Tensor gt = mod_rows(gate, "gate");
   const int64_t rows = y.size(0), D = y.size(1), frames = rows / L;
   TORCH_CHECK(D <= 8192, "channel dim must be <= 8192");
   Tensor dy = at::empty_like(y);
   Tensor dgate = at::empty({frames, D}, gate.options());
   const int G = cb200_ln_groups_per_frame((int)L, kRowsPerCta);
   Tensor partials = at::empty({frames * G, D}, gate.options());
-  cb200_gate_residual_bwd(dout.data_ptr(), gate.data_ptr<float>(), y.data_ptr(), dy.data_ptr(), dgate.data_ptr<float>(),
-                          partials.data_ptr<float>(), frames, (int)D, (int)L, kRowsPerCta, stream());
+  cb200_gate_residual_bwd(dout.data_ptr(), gt.data_ptr<float>(), y.data_ptr(), dy.data_ptr(), dgate.data_ptr<float>(),
+                          partials.data_ptr<float>(), frames, (int)D, (int)L, kRowsPerCta, gt.stride(0), stream());
   return {dy, dgate};
 }
 
@@ -115,7 +130,8 @@ std::tuple<Tensor, Tensor> rmsnorm_rope_fwd(const Tensor& x, const Tensor& w, co
   c10::cuda::CUDAGuard g(x.device());
   const int64_t B = x.size(0), S = x.size(1), H = x.size(2), HD = x.size(3);
   TORCH_CHECK(HD == 128 || HD == 64, "head_dim must be 64 or 128");
-  Tensor wf = w.to(at::kFloat).contiguous();
+  TORCH_CHECK(w.numel() == HD && w.device() == x.device(), "w must hold head_dim values on the device of x");
+  const Tensor wf = norm_weight(w);
   const float* cp = nullptr;
   const float* sp = nullptr;
   if (cosv.has_value()) {
@@ -127,7 +143,7 @@ std::tuple<Tensor, Tensor> rmsnorm_rope_fwd(const Tensor& x, const Tensor& w, co
   }
   Tensor y = at::empty_like(x);
   Tensor rstd = at::empty({B, S, H}, x.options().dtype(at::kFloat));
-  cb200_rmsnorm_rope_fwd(x.data_ptr(), wf.data_ptr<float>(), cp, sp, y.data_ptr(), rstd.data_ptr<float>(), B * S * H, (int)S,
+  cb200_rmsnorm_rope_fwd(x.data_ptr(), wf.data_ptr(), is_bf16(wf), cp, sp, y.data_ptr(), rstd.data_ptr<float>(), B * S * H, (int)S,
                          (int)H, (int)HD, (float)eps, stream());
   return {y, rstd};
 }
@@ -150,14 +166,14 @@ std::tuple<Tensor, Tensor> rmsnorm_rope_bwd(const Tensor& dy, const Tensor& x, c
     TORCH_CHECK(cosv->dim() == 2 && cosv->size(0) == S && cosv->size(1) == HD / 2 && sinv->sizes() == cosv->sizes() &&
                     cosv->device() == x.device() && sinv->device() == x.device(), "cos/sin must be [S, D/2] on the device of x");
   }
-  Tensor wf = w.to(at::kFloat).contiguous();
+  const Tensor wf = norm_weight(w);
   const float* cp = cosv.has_value() ? cosv->data_ptr<float>() : nullptr;
   const float* sp = sinv.has_value() ? sinv->data_ptr<float>() : nullptr;
   Tensor dx = at::empty_like(x);
   Tensor dw = at::empty({HD}, x.options().dtype(at::kFloat));
   const int64_t blocks = cb200_rmsnorm_bwd_blocks(B * S * H, kRowsPerWarp);
   Tensor partials = at::empty({blocks, HD}, dw.options());
-  cb200_rmsnorm_rope_bwd(dy.data_ptr(), x.data_ptr(), wf.data_ptr<float>(), rstd.data_ptr<float>(), cp, sp, dx.data_ptr(),
+  cb200_rmsnorm_rope_bwd(dy.data_ptr(), x.data_ptr(), wf.data_ptr(), is_bf16(wf), rstd.data_ptr<float>(), cp, sp, dx.data_ptr(),
                          dw.data_ptr<float>(), partials.data_ptr<float>(), B * S * H, (int)S, (int)H, (int)HD, kRowsPerWarp,
                          stream());
   return {dx, dw};
@@ -325,17 +341,20 @@ Tensor gemm_impl(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& 
   }
   const void* resid_p = nullptr;
   const float* gate_p = nullptr;
+  Tensor gate_c;
+  long ld_gate = 0;
   if (resid != nullptr) {
     check_bf16(*resid, "resid");
-    check_f32(*gate, "gate");
+    gate_c = mod_rows(*gate, "gate");
+    ld_gate = gate_c.stride(0);
     TORCH_CHECK(resid->numel() == (int64_t)d.M * d.N && gate->size(-1) == d.N && gate->numel() == (d.M / L) * (int64_t)d.N,
                 "gated-residual epilogue shapes");
     resid_p = resid->data_ptr();
-    gate_p = gate->data_ptr<float>();
+    gate_p = gate_c.data_ptr<float>();
   }
   const int dev = a.get_device();
   const int rc = cb200_gemm_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), d.M, d.N, d.K, trans_a ? 1 : 0, trans_b ? 1 : 0, bias_p,
-                                 (int)act, pre_p, resid_p, gate_p, (int)L, error_word(dev), sm_count(dev), stream());
+                                 (int)act, pre_p, resid_p, gate_p, ld_gate, (int)L, error_word(dev), sm_count(dev), stream());
   TORCH_CHECK(rc == 0, "tcgen05 GEMM launch failed with code ", rc);
   return c;
 }
@@ -380,11 +399,12 @@ std::tuple<Tensor, Tensor> gemm_scatter_heads_peer(const Tensor& x, const Tensor
               "heads of 128 channels, divisible by the peer count");
   TORCH_CHECK(S > 0 && d.M % S == 0, "rows must be B * S");
   Tensor wf;
-  const float *wp = nullptr, *cp = nullptr, *sp = nullptr;
+  const void* wp = nullptr;
+  const float *cp = nullptr, *sp = nullptr;
   if (norm_w.has_value()) {
-    wf = norm_w->to(at::kFloat).contiguous();
-    TORCH_CHECK(wf.numel() == 128, "norm weight must be [128]");
-    wp = wf.data_ptr<float>();
+    wf = norm_weight(*norm_w);
+    TORCH_CHECK(wf.numel() == 128 && wf.device() == x.device(), "norm weight must be [128] on the device of x");
+    wp = wf.data_ptr();
     if (cosv.has_value()) {
       check_f32(*cosv, "cos");
       check_f32(*sinv, "sin");
@@ -401,7 +421,7 @@ std::tuple<Tensor, Tensor> gemm_scatter_heads_peer(const Tensor& x, const Tensor
   std::vector<int64_t> p(out_ptrs.begin(), out_ptrs.end());
   const int dev = x.get_device();
   const int rc = cb200_gemm_bf16_scatter_heads(x.data_ptr(), w.data_ptr(), d.M, d.N, d.K, p.data(), (int)p.size(), (int)rank, (int)S,
-                                               wp, cp, sp, (float)eps, keep_raw ? raw.data_ptr() : nullptr,
+                                               wp, wp != nullptr ? is_bf16(wf) : 0, cp, sp, (float)eps, keep_raw ? raw.data_ptr() : nullptr,
                                                keep_raw ? rstd.data_ptr<float>() : nullptr, error_word(dev), sm_count(dev), stream());
   TORCH_CHECK(rc == 0, "tcgen05 GEMM (head-scatter epilogue) launch failed with code ", rc);
   return {raw, rstd};
@@ -559,6 +579,10 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("ln_modulate_jvp(Tensor x, Tensor tx, Tensor shift, Tensor scale, Tensor? tshift, Tensor? tscale, int L, float eps) -> "
         "(Tensor, Tensor)", &ln_modulate_jvp);
   m.def("rmsnorm_rope_jvp(Tensor x, Tensor tx, Tensor w, Tensor? cos, Tensor? sin, float eps) -> (Tensor, Tensor)", &rmsnorm_rope_jvp);
+  m.def("skinny_wide(int a_k, int b_n, int b_k, bool b_bf16, bool out_bf16, bool silu_b, int N, int K) -> bool",
+        [](int64_t a_k, int64_t b_n, int64_t b_k, bool b_bf16, bool out_bf16, bool silu_b, int64_t N, int64_t K) {
+          return cb200_skinny_wide(a_k, b_n, b_k, b_bf16, out_bf16, silu_b, (int)N, (int)K) != 0;
+        });
   m.def("skinny_bgemm(Tensor a, int a_z, int a_r, int a_k, Tensor? b_ptrs, Tensor? b, int b_z, int b_n, int b_k, bool b_bf16, "
         "Tensor? add, int add_cols, int Z, int R, int N, int K, bool silu_a, bool silu_b, bool out_bf16, int ksplit) -> Tensor", &skinny_bgemm);
   m.def("gemm_pair_mode(int mode) -> int", &gemm_pair_mode);

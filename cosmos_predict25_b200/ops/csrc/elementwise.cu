@@ -61,7 +61,8 @@ __device__ __forceinline__ void store_f8(float* p, const float (&f)[8]) {
 template <int MV>
 __global__ void __launch_bounds__(kThreads) ln_modulate_fwd_kernel(
     const bf16* __restrict__ x, const float* __restrict__ shift, const float* __restrict__ scale,
-    bf16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int D, int L, float eps) {
+    bf16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int D, int L, long ld_shift, long ld_scale,
+    float eps) {
   __shared__ float red[64];
   const long row = blockIdx.x;
   const long frame = row / L;
@@ -97,8 +98,8 @@ __global__ void __launch_bounds__(kThreads) ln_modulate_fwd_kernel(
     rstd_out[row] = rstd;
   }
   bf16x8* yr = reinterpret_cast<bf16x8*>(y + row * D);
-  const float* sh = shift + frame * D;
-  const float* sc = scale + frame * D;
+  const float* sh = shift + frame * ld_shift;
+  const float* sc = scale + frame * ld_scale;
 #pragma unroll
   for (int i = 0; i < MV; ++i) {
     const int c = threadIdx.x + i * kThreads;
@@ -113,102 +114,90 @@ __global__ void __launch_bounds__(kThreads) ln_modulate_fwd_kernel(
   }
 }
 
-// Same operator for D <= 2048 with four rows per CTA: the loads of all four rows are in flight together and one pair of block
-// reductions serves the four rows, so the memory pipe does not idle behind a reduction per 4 KB row.
-constexpr int kLnRows = 4;
-__device__ __forceinline__ void block_sum_rows(float (&v)[kLnRows], float* red /* [kLnRows * 32] */) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int r = 0; r < kLnRows; ++r) v[r] = warp_sum(v[r]);
-  __syncthreads();
-  if (lane == 0) {
-#pragma unroll
-    for (int r = 0; r < kLnRows; ++r) red[r * 32 + warp] = v[r];
-  }
-  __syncthreads();
-  const int nwarps = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int r = 0; r < kLnRows; ++r) v[r] = warp_sum(lane < nwarps ? red[r * 32 + lane] : 0.f);
-}
-
-// A CTA takes `rows_per_cta` consecutive rows of ONE frame, four at a time: every thread keeps the shift / (1 + scale) values of
-// its 8 columns in registers for all of them (read per row, the two fp32 modulation vectors are 4x the bytes of the bf16 row and
-// made the kernel L2-bound).
-__global__ void __launch_bounds__(kThreads) ln_modulate_fwd_rows_kernel(
+// Same operator for D <= 256 NV: a warp owns R rows of one frame, all of whose 16-byte pieces are in flight together (kept packed),
+// and reduces them with shuffles alone. Bound by memory; with a CTA per four rows the two block-wide reductions (four barriers) kept
+// the memory pipe idle. The modulation vectors are four times a row's bytes and come from L1, whose bandwidth is the next limit: a
+// pair of rows shares them. Inside a denoising step: 46,800 rows of 2048 174 us before, 125 us now (155 with a row per warp); 512
+// rows 22 us before, 6.9 us with a row per warp (8.2 with pairs): a row per warp while the pairs would not fill the GPU.
+// shift / scale rows are `ld_*` apart: slices of the modulation MLPs' output serve as they lie.
+constexpr int kLnWarps = 4;
+template <int NV, int R>
+__global__ void __launch_bounds__(kLnWarps * 32) ln_modulate_fwd_warp_kernel(
     const bf16* __restrict__ x, const float* __restrict__ shift, const float* __restrict__ scale,
-    bf16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int D, int L, int rows_per_cta,
-    int groups_per_frame, float eps) {
-  __shared__ float red[kLnRows * 32];
-  const long frame = blockIdx.x / groups_per_frame;
-  const int g = blockIdx.x % groups_per_frame;
-  const int r_lo = g * rows_per_cta, r_hi = min(r_lo + rows_per_cta, L);
+    bf16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, long groups, int D, int L, int groups_per_frame,
+    long ld_shift, long ld_scale, float eps) {
+  const int lane = threadIdx.x & 31;
+  const long group = (long)blockIdx.x * kLnWarps + (threadIdx.x >> 5);
+  if (group >= groups) return;
+  const long frame = group / groups_per_frame;
+  const int r_in = (int)(group - frame * groups_per_frame) * R, n_here = min(R, L - r_in);
+  const long row0 = frame * L + r_in;
   const int nvec = D >> 3;
-  const int c = threadIdx.x;
-  const bool on = c < nvec;
-  float a[8], b[8];
-  if (on) {
-    load_f8(shift + frame * D + c * 8, a);
-    load_f8(scale + frame * D + c * 8, b);
+  bf16x8 v[R][NV];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) b[j] += 1.f;
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      if (r < n_here && lane + i * 32 < nvec) v[r][i] = reinterpret_cast<const bf16x8*>(x + (row0 + r) * D)[lane + i * 32];
+      else v[r][i] = bf16x8{};
+    }
+  float mean[R], rstd[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    float2 s2 = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s2 = add2(s2, __bfloat1622float2(v[r][i].v[j]));
+    mean[r] = s2.x + s2.y;
   }
-  for (int rb = r_lo; rb < r_hi; rb += kLnRows) {
-    const long row0 = frame * L + rb;
-    const int n_here = min(kLnRows, r_hi - rb);
-    float v[kLnRows][8];
-    float s[kLnRows];
 #pragma unroll
-    for (int r = 0; r < kLnRows; ++r) {
-      s[r] = 0.f;
-      if (on && r < n_here) {
-        unpack8(reinterpret_cast<const bf16x8*>(x + (row0 + r) * D)[c], v[r]);
-        const float2 t = add2(add2(CB200_P2(v[r], 0), CB200_P2(v[r], 1)), add2(CB200_P2(v[r], 2), CB200_P2(v[r], 3)));
-        s[r] = t.x + t.y;
-      } else {
+  for (int r = 0; r < R; ++r) mean[r] = warp_sum(mean[r]) / D;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[r][j] = 0.f;
-      }
-    }
-    block_sum_rows(s, red);
-    float mean[kLnRows], q[kLnRows];
+  for (int r = 0; r < R; ++r) {
+    const float2 nm = make_float2(-mean[r], -mean[r]);
+    float2 q2 = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int r = 0; r < kLnRows; ++r) {
-      mean[r] = s[r] / D;
-      q[r] = 0.f;
-      if (on) {
-        // v becomes the centred value; two elements per instruction
-        const float2 nm = make_float2(-mean[r], -mean[r]);
-        float2 acc = make_float2(0.f, 0.f);
+    for (int i = 0; i < NV; ++i)
+      if (lane + i * 32 < nvec) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float2 d = add2(CB200_P2(v[r], j), nm);
-          acc = fma2(d, d, acc);
-          v[r][2 * j] = d.x;
-          v[r][2 * j + 1] = d.y;
+          const float2 d = add2(__bfloat1622float2(v[r][i].v[j]), nm);
+          q2 = fma2(d, d, q2);
         }
-        q[r] = acc.x + acc.y;
       }
+    rstd[r] = q2.x + q2.y;
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    rstd[r] = rsqrtf(warp_sum(rstd[r]) / D + eps);
+    if (lane == 0 && r < n_here) {
+      mean_out[row0 + r] = mean[r];
+      rstd_out[row0 + r] = rstd[r];
     }
-    block_sum_rows(q, red);
+  }
+  const float* sh = shift + frame * ld_shift;
+  const float* sc = scale + frame * ld_scale;
+  const float2 one2 = make_float2(1.f, 1.f);
 #pragma unroll
-    for (int r = 0; r < kLnRows; ++r) {
-      if (r >= n_here) break;
-      const long row = row0 + r;
-      const float rstd = rsqrtf(q[r] / D + eps);
-      if (threadIdx.x == 0) {
-        mean_out[row] = mean[r];
-        rstd_out[row] = rstd;
-      }
-      if (on) {
-        float o[8];
-        const float2 rs2 = make_float2(rstd, rstd);
+  for (int i = 0; i < NV; ++i) {
+    const int c = lane + i * 32;
+    if (c < nvec) {
+      float a[8], b[8];
+      load_f8(sh + c * 8, a);
+      load_f8(sc + c * 8, b);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 t = fma2(mul2(CB200_P2(v[r], j), rs2), CB200_P2(b, j), CB200_P2(a, j));
-          o[2 * j] = t.x;
-          o[2 * j + 1] = t.y;
+      for (int r = 0; r < R; ++r) {
+        if (r < n_here) {
+          const float2 nm = make_float2(-mean[r], -mean[r]), rs2 = make_float2(rstd[r], rstd[r]);
+          bf16x8 o;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 t = fma2(mul2(add2(__bfloat1622float2(v[r][i].v[j]), nm), rs2), add2(CB200_P2(b, j), one2), CB200_P2(a, j));
+            o.v[j] = __floats2bfloat162_rn(t.x, t.y);
+          }
+          reinterpret_cast<bf16x8*>(y + (row0 + r) * D)[c] = o;
         }
-        reinterpret_cast<bf16x8*>(y + row * D)[c] = pack8(o);
       }
     }
   }
@@ -220,7 +209,7 @@ template <int MV>
 __global__ void __launch_bounds__(kThreads) ln_modulate_bwd_kernel(
     const bf16* __restrict__ dy, const bf16* __restrict__ x, const float* __restrict__ mean_in,
     const float* __restrict__ rstd_in, const float* __restrict__ scale, bf16* __restrict__ dx,
-    float* __restrict__ partials, int D, int L, int rows_per_cta, int groups_per_frame) {
+    float* __restrict__ partials, int D, int L, int rows_per_cta, int groups_per_frame, long ld_scale) {
   __shared__ float red[64];
   const long frame = blockIdx.x / groups_per_frame;
   const int g = blockIdx.x % groups_per_frame;
@@ -234,7 +223,7 @@ __global__ void __launch_bounds__(kThreads) ln_modulate_bwd_kernel(
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc_sh[i][j] = acc_sc[i][j] = 0.f;
     if (c < nvec) {
-      load_f8(scale + frame * D + c * 8, onep[i]);
+      load_f8(scale + frame * ld_scale + c * 8, onep[i]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) onep[i][j] += 1.f;
     }
@@ -365,7 +354,7 @@ __global__ void __launch_bounds__(1024) reduce_rows_kernel(const float* __restri
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads) gate_residual_fwd_kernel(
     const bf16* __restrict__ x, const float* __restrict__ gate, const bf16* __restrict__ y, bf16* __restrict__ out,
-    long nvec_total, int D, int L) {
+    long nvec_total, int D, int L, long ld_gate) {
   const int nvec = D >> 3;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec_total; i += (long)gridDim.x * blockDim.x) {
     const long row = i / nvec;
@@ -374,7 +363,7 @@ __global__ void __launch_bounds__(kThreads) gate_residual_fwd_kernel(
     float a[8], b[8], g[8], o[8];
     unpack8(reinterpret_cast<const bf16x8*>(x)[i], a);
     unpack8(reinterpret_cast<const bf16x8*>(y)[i], b);
-    load_f8(gate + frame * D + c * 8, g);
+    load_f8(gate + frame * ld_gate + c * 8, g);
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = a[j] + g[j] * b[j];
     reinterpret_cast<bf16x8*>(out)[i] = pack8(o);
@@ -384,7 +373,7 @@ __global__ void __launch_bounds__(kThreads) gate_residual_fwd_kernel(
 template <int MV>
 __global__ void __launch_bounds__(kThreads) gate_residual_bwd_kernel(
     const bf16* __restrict__ dout, const float* __restrict__ gate, const bf16* __restrict__ y, bf16* __restrict__ dy,
-    float* __restrict__ partials, int D, int L, int rows_per_cta, int groups_per_frame) {
+    float* __restrict__ partials, int D, int L, int rows_per_cta, int groups_per_frame, long ld_gate) {
   const long frame = blockIdx.x / groups_per_frame;
   const int g = blockIdx.x % groups_per_frame;
   const int r0 = g * rows_per_cta, r1 = min(r0 + rows_per_cta, L);
@@ -395,7 +384,7 @@ __global__ void __launch_bounds__(kThreads) gate_residual_bwd_kernel(
     const int c = threadIdx.x + i * kThreads;
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-    if (c < nvec) load_f8(gate + frame * D + c * 8, gt[i]);
+    if (c < nvec) load_f8(gate + frame * ld_gate + c * 8, gt[i]);
   }
   for (int r = r0; r < r1; ++r) {
     const long row = frame * L + r;
@@ -429,40 +418,50 @@ __global__ void __launch_bounds__(kThreads) gate_residual_bwd_kernel(
 // ------------------------------------------------------------------------------------------------
 // per-head RMSNorm + RoPE: one warp per (token, head), head_dim in {64, 128}; lane holds HD/32 values
 // ------------------------------------------------------------------------------------------------
-// Sixteen lanes per (token, head) row, HD / 16 elements (one 16- or 8-byte access) per lane, two rows per warp pass: half the
-// instructions per byte of a 32-lane layout (these kernels are bound by instruction issue, not by memory). The rotation partner
-// of element i (i +- HD/2) sits in lane ^ 8 at the same register index; reductions stay inside the 16-lane half.
+// Sixteen lanes per (token, head) row, two rows per warp pass. A lane holds P = HD / 32 elements of each half of the row, at the same
+// offset, so that the rotation partner of every element is in the lane itself and one cosine / sine vector serves both; reductions
+// stay inside the 16-lane half. Token and head of a row are counted along instead of divided out (64-bit divisions per row, a
+// shuffle per element and twice the table loads bound the earlier layout by instruction issue: 46,800 tokens x 16 heads 147 us,
+// now 90 us; the bytes take 59 us).
 constexpr int kRmsPasses = 4;        // forward: passes (of two rows) whose loads a warp keeps in flight together
 
-template <int E>
-__device__ __forceinline__ void load_row_bf16(const bf16* p, float (&v)[E]) {
-  if constexpr (E == 8) {
-    unpack8(*reinterpret_cast<const bf16x8*>(p), v);
-  } else {
+template <int P>
+__device__ __forceinline__ void load_part(const bf16* p, float2 (&v)[P / 2]) {
+  if constexpr (P == 4) {
     const uint2 raw = *reinterpret_cast<const uint2*>(p);
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-  }
-}
-template <int E>
-__device__ __forceinline__ void store_row_bf16(bf16* p, const float (&o)[E]) {
-  if constexpr (E == 8) {
-    *reinterpret_cast<bf16x8*>(p) = pack8(o);
+    v[0] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+    v[1] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
   } else {
-    uint2 raw;
-    *reinterpret_cast<__nv_bfloat162*>(&raw.x) = __floats2bfloat162_rn(o[0], o[1]);
-    *reinterpret_cast<__nv_bfloat162*>(&raw.y) = __floats2bfloat162_rn(o[2], o[3]);
-    *reinterpret_cast<uint2*>(p) = raw;
+    v[0] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
   }
 }
-template <int E>
-__device__ __forceinline__ void load_f32_vec(const float* p, float (&v)[E]) {
-#pragma unroll
-  for (int j = 0; j < E; j += 4) {
-    const float4 a = *reinterpret_cast<const float4*>(p + j);
-    v[j] = a.x; v[j + 1] = a.y; v[j + 2] = a.z; v[j + 3] = a.w;
+template <int P>
+__device__ __forceinline__ void store_part(bf16* p, const float2 (&v)[P / 2]) {
+  if constexpr (P == 4) {
+    uint2 raw;
+    *reinterpret_cast<__nv_bfloat162*>(&raw.x) = __floats2bfloat162_rn(v[0].x, v[0].y);
+    *reinterpret_cast<__nv_bfloat162*>(&raw.y) = __floats2bfloat162_rn(v[1].x, v[1].y);
+    *reinterpret_cast<uint2*>(p) = raw;
+  } else {
+    *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(v[0].x, v[0].y);
   }
+}
+template <int P>
+__device__ __forceinline__ void load_f32_part(const float* p, float2 (&v)[P / 2]) {
+  if constexpr (P == 4) {
+    const float4 a = *reinterpret_cast<const float4*>(p);
+    v[0] = make_float2(a.x, a.y);
+    v[1] = make_float2(a.z, a.w);
+  } else {
+    v[0] = *reinterpret_cast<const float2*>(p);
+  }
+}
+// norm weights starting at element `at`, stored as fp32 or bf16 (parameters are bf16: converting them on the host side cost a
+// launch per call)
+template <int P>
+__device__ __forceinline__ void load_weight_part(const void* w, int w_bf16, int at, float2 (&v)[P / 2]) {
+  if (w_bf16) load_part<P>(reinterpret_cast<const bf16*>(w) + at, v);
+  else load_f32_part<P>(reinterpret_cast<const float*>(w) + at, v);
 }
 __device__ __forceinline__ float half_warp_sum(float v) {   // over the 16 lanes of this half
   v += __shfl_xor_sync(0xffffffffu, v, 8);
@@ -471,85 +470,118 @@ __device__ __forceinline__ float half_warp_sum(float v) {   // over the 16 lanes
   v += __shfl_xor_sync(0xffffffffu, v, 1);
   return v;
 }
+// position in the sequence of consecutive (token, head) rows
+struct RowCursor {
+  int s, h;
+  __device__ RowCursor(long row, int S, int H) {
+    const long token = row / H;
+    h = (int)(row - token * H);
+    s = (int)(token % S);
+  }
+  __device__ void advance(int rows, int S, int H) {
+    h += rows;
+    while (h >= H) {
+      h -= H;
+      if (++s == S) s = 0;
+    }
+  }
+};
 
 template <int HD>
 __global__ void __launch_bounds__(256) rmsnorm_rope_fwd_kernel(
-    const bf16* __restrict__ x, const float* __restrict__ w, const float* __restrict__ cosv,
+    const bf16* __restrict__ x, const void* __restrict__ w, int w_bf16, const float* __restrict__ cosv,
     const float* __restrict__ sinv, bf16* __restrict__ y, float* __restrict__ rstd_out, long n_rows, int S, int H,
     float eps) {
-  constexpr int E = HD / 16;  // elements per lane (8 or 4)
+  constexpr int P = HD / 32, Q = P / 2;
   constexpr int U = kRmsPasses;
   const int lane = threadIdx.x & 31, sub = lane & 15, half = lane >> 4;
   const long row0 = ((long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (2 * U) + half;   // this lane's rows: row0 + 2u
-  float wv[E];
-  load_f32_vec<E>(w + sub * E, wv);
-  float v[U][E];
+  float2 lo[U][Q], hi[U][Q];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     if (row0 + 2 * u < n_rows) {
-      load_row_bf16<E>(x + (row0 + 2 * u) * HD + sub * E, v[u]);
+      const bf16* xr = x + (row0 + 2 * u) * HD + sub * P;
+      load_part<P>(xr, lo[u]);
+      load_part<P>(xr + HD / 2, hi[u]);
     } else {
 #pragma unroll
-      for (int j = 0; j < E; ++j) v[u][j] = 0.f;
+      for (int j = 0; j < Q; ++j) lo[u][j] = hi[u][j] = make_float2(0.f, 0.f);
     }
   }
+  float2 wl[Q], wh[Q];
+  load_weight_part<P>(w, w_bf16, sub * P, wl);
+  load_weight_part<P>(w, w_bf16, HD / 2 + sub * P, wh);
+  RowCursor at(row0 < n_rows ? row0 : 0, S, H);
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const long row = row0 + 2 * u;
     const bool valid = row < n_rows;          // both halves run every shuffle; only the accesses are predicated
-    const long s = valid ? (row / H) % S : 0;
-    float ss = 0.f;
+    float2 ss2 = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int j = 0; j < E; ++j) ss += v[u][j] * v[u][j];
-    ss = half_warp_sum(ss);
+    for (int j = 0; j < Q; ++j) ss2 = fma2(hi[u][j], hi[u][j], fma2(lo[u][j], lo[u][j], ss2));
+    const float ss = half_warp_sum(ss2.x + ss2.y);
     const float rstd = rsqrtf(ss / HD + eps);
     if (sub == 0 && valid) rstd_out[row] = rstd;
-    float o[E];
+    const float2 rs2 = make_float2(rstd, rstd);
 #pragma unroll
-    for (int j = 0; j < E; ++j) o[j] = v[u][j] * rstd * wv[j];
-    if (cosv != nullptr) {
-      float c[E], sn[E];
-      load_f32_vec<E>(cosv + s * (HD / 2) + (sub & 7) * E, c);
-      load_f32_vec<E>(sinv + s * (HD / 2) + (sub & 7) * E, sn);
+    for (int j = 0; j < Q; ++j) {
+      lo[u][j] = mul2(mul2(lo[u][j], rs2), wl[j]);
+      hi[u][j] = mul2(mul2(hi[u][j], rs2), wh[j]);
+    }
+    if (cosv != nullptr && valid) {
+      float2 c[Q], sn[Q];
+      load_f32_part<P>(cosv + (long)at.s * (HD / 2) + sub * P, c);
+      load_f32_part<P>(sinv + (long)at.s * (HD / 2) + sub * P, sn);
 #pragma unroll
-      for (int j = 0; j < E; ++j) {
-        const float other = __shfl_xor_sync(0xffffffffu, o[j], 8);
-        o[j] = (sub < 8) ? (o[j] * c[j] - other * sn[j]) : (o[j] * c[j] + other * sn[j]);
+      for (int j = 0; j < Q; ++j) {
+        const float2 a = lo[u][j], b = hi[u][j], ns = make_float2(-sn[j].x, -sn[j].y);
+        lo[u][j] = fma2(b, ns, mul2(a, c[j]));
+        hi[u][j] = fma2(a, sn[j], mul2(b, c[j]));
       }
     }
-    if (valid) store_row_bf16<E>(y + row * HD + sub * E, o);
+    if (valid) {
+      bf16* yr = y + row * HD + sub * P;
+      store_part<P>(yr, lo[u]);
+      store_part<P>(yr + HD / 2, hi[u]);
+    }
+    at.advance(2, S, H);
   }
 }
 
 // backward: `rows_per_warp` consecutive rows per warp (two per pass) to amortise the weight-gradient partial.
 template <int HD>
 __global__ void __launch_bounds__(256) rmsnorm_rope_bwd_kernel(
-    const bf16* __restrict__ dy, const bf16* __restrict__ x, const float* __restrict__ w,
+    const bf16* __restrict__ dy, const bf16* __restrict__ x, const void* __restrict__ w, int w_bf16,
     const float* __restrict__ rstd_in, const float* __restrict__ cosv, const float* __restrict__ sinv,
     bf16* __restrict__ dx, float* __restrict__ dw_partials, long n_rows, int S, int H, int rows_per_warp) {
-  constexpr int E = HD / 16;
+  constexpr int P = HD / 32, Q = P / 2;
   __shared__ float sm[8][HD];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 15, half = lane >> 4;
   const long warp_global = (long)blockIdx.x * 8 + warp;
   const long r0 = warp_global * rows_per_warp;
   const long r_end = min(r0 + (long)rows_per_warp, n_rows);
-  float wv[E], dwacc[E];
-  load_f32_vec<E>(w + sub * E, wv);
+  float2 wl[Q], wh[Q], dwl[Q], dwh[Q];
+  load_weight_part<P>(w, w_bf16, sub * P, wl);
+  load_weight_part<P>(w, w_bf16, HD / 2 + sub * P, wh);
 #pragma unroll
-  for (int j = 0; j < E; ++j) dwacc[j] = 0.f;
-  constexpr int U = 2;      // passes (of two rows) whose loads are in flight together
+  for (int j = 0; j < Q; ++j) dwl[j] = dwh[j] = make_float2(0.f, 0.f);
+  constexpr int U = 4;      // passes (of two rows) whose loads are in flight together
+  RowCursor at(min(r0 + half, n_rows - 1), S, H);
   for (long rb = r0; rb < r_end; rb += 2 * U) {
-    float dU[U][E], xU[U][E], rsU[U];
+    float2 dl[U][Q], dh[U][Q], xl[U][Q], xh[U][Q];
+    float rsU[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long row = rb + 2 * u + half;
       if (row < r_end) {
-        load_row_bf16<E>(dy + row * HD + sub * E, dU[u]);
-        load_row_bf16<E>(x + row * HD + sub * E, xU[u]);
+        load_part<P>(dy + row * HD + sub * P, dl[u]);
+        load_part<P>(dy + row * HD + HD / 2 + sub * P, dh[u]);
+        load_part<P>(x + row * HD + sub * P, xl[u]);
+        load_part<P>(x + row * HD + HD / 2 + sub * P, xh[u]);
         rsU[u] = rstd_in[row];
       } else {
 #pragma unroll
-        for (int j = 0; j < E; ++j) dU[u][j] = xU[u][j] = 0.f;
+        for (int j = 0; j < Q; ++j) dl[u][j] = dh[u][j] = xl[u][j] = xh[u][j] = make_float2(0.f, 0.f);
         rsU[u] = 0.f;
       }
     }
@@ -557,43 +589,59 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_bwd_kernel(
     for (int u = 0; u < U; ++u) {
       const long row = rb + 2 * u + half;
       const bool valid = row < r_end;
-      const long s = valid ? (row / H) % S : 0;
-      float d[E];
+      if (cosv != nullptr && valid) {
+        float2 c[Q], sn[Q];
+        load_f32_part<P>(cosv + (long)at.s * (HD / 2) + sub * P, c);
+        load_f32_part<P>(sinv + (long)at.s * (HD / 2) + sub * P, sn);
 #pragma unroll
-      for (int j = 0; j < E; ++j) d[j] = dU[u][j];
-      if (cosv != nullptr) {
-        float c[E], sn[E];
-        load_f32_vec<E>(cosv + s * (HD / 2) + (sub & 7) * E, c);
-        load_f32_vec<E>(sinv + s * (HD / 2) + (sub & 7) * E, sn);
-#pragma unroll
-        for (int j = 0; j < E; ++j) {
-          const float other = __shfl_xor_sync(0xffffffffu, d[j], 8);
-          d[j] = (sub < 8) ? (d[j] * c[j] + other * sn[j]) : (d[j] * c[j] - other * sn[j]);
+        for (int j = 0; j < Q; ++j) {
+          const float2 a = dl[u][j], b = dh[u][j], ns = make_float2(-sn[j].x, -sn[j].y);
+          dl[u][j] = fma2(b, sn[j], mul2(a, c[j]));
+          dh[u][j] = fma2(a, ns, mul2(b, c[j]));
         }
       }
       const float rstd = rsU[u];
-      float dot = 0.f;
-      float gv[E];
+      const float2 rs2 = make_float2(rstd, rstd);
+      float2 dot2 = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int j = 0; j < E; ++j) {
-        dwacc[j] += d[j] * xU[u][j] * rstd;
-        gv[j] = d[j] * wv[j];
-        dot += gv[j] * xU[u][j];
+      for (int j = 0; j < Q; ++j) {
+        dwl[j] = fma2(mul2(dl[u][j], xl[u][j]), rs2, dwl[j]);
+        dwh[j] = fma2(mul2(dh[u][j], xh[u][j]), rs2, dwh[j]);
+        dl[u][j] = mul2(dl[u][j], wl[j]);
+        dh[u][j] = mul2(dh[u][j], wh[j]);
+        dot2 = fma2(dh[u][j], xh[u][j], fma2(dl[u][j], xl[u][j], dot2));
       }
-      dot = half_warp_sum(dot);
+      const float dot = half_warp_sum(dot2.x + dot2.y);
       const float k = dot * rstd * rstd * rstd / HD;
-      float o[E];
+      const float2 nk = make_float2(-k, -k);
 #pragma unroll
-      for (int j = 0; j < E; ++j) o[j] = rstd * gv[j] - xU[u][j] * k;
-      if (valid) store_row_bf16<E>(dx + row * HD + sub * E, o);
+      for (int j = 0; j < Q; ++j) {
+        dl[u][j] = fma2(xl[u][j], nk, mul2(dl[u][j], rs2));
+        dh[u][j] = fma2(xh[u][j], nk, mul2(dh[u][j], rs2));
+      }
+      if (valid) {
+        store_part<P>(dx + row * HD + sub * P, dl[u]);
+        store_part<P>(dx + row * HD + HD / 2 + sub * P, dh[u]);
+      }
+      at.advance(2, S, H);
     }
   }
   // the two halves of the warp hold partial sums of the same columns
 #pragma unroll
-  for (int j = 0; j < E; ++j) dwacc[j] += __shfl_xor_sync(0xffffffffu, dwacc[j], 16);
+  for (int j = 0; j < Q; ++j) {
+    dwl[j].x += __shfl_xor_sync(0xffffffffu, dwl[j].x, 16);
+    dwl[j].y += __shfl_xor_sync(0xffffffffu, dwl[j].y, 16);
+    dwh[j].x += __shfl_xor_sync(0xffffffffu, dwh[j].x, 16);
+    dwh[j].y += __shfl_xor_sync(0xffffffffu, dwh[j].y, 16);
+  }
   if (half == 0) {
 #pragma unroll
-    for (int j = 0; j < E; ++j) sm[warp][sub * E + j] = dwacc[j];
+    for (int j = 0; j < Q; ++j) {
+      sm[warp][sub * P + 2 * j] = dwl[j].x;
+      sm[warp][sub * P + 2 * j + 1] = dwl[j].y;
+      sm[warp][HD / 2 + sub * P + 2 * j] = dwh[j].x;
+      sm[warp][HD / 2 + sub * P + 2 * j + 1] = dwh[j].y;
+    }
   }
   __syncthreads();
   if (threadIdx.x < HD) {
@@ -723,22 +771,22 @@ extern "C" {
 int cb200_ln_groups_per_frame(int L, int rows_per_cta) { return (L + rows_per_cta - 1) / rows_per_cta; }
 
 void cb200_ln_modulate_fwd(const void* x, const float* shift, const float* scale, void* y, float* mean, float* rstd,
-                           long rows, int D, int L, float eps, cudaStream_t st) {
-#define LAUNCH(MV) ln_modulate_fwd_kernel<MV><<<(unsigned)rows, kThreads, 0, st>>>((const bf16*)x, shift, scale, (bf16*)y, mean, rstd, D, L, eps)
-  if (D <= 2048) {
-    constexpr int kRowsPerCta = 32;
-    const int G = (L + kRowsPerCta - 1) / kRowsPerCta;
-    ln_modulate_fwd_rows_kernel<<<(unsigned)((rows / L) * G), kThreads, 0, st>>>((const bf16*)x, shift, scale, (bf16*)y, mean, rstd, D, L,
-                                                                               kRowsPerCta, G, eps);
-  } else if (D <= 4096) LAUNCH(2); else LAUNCH(4);
+                           long rows, int D, int L, long ld_shift, long ld_scale, float eps, cudaStream_t st) {
+#define LAUNCH(MV) ln_modulate_fwd_kernel<MV><<<(unsigned)rows, kThreads, 0, st>>>((const bf16*)x, shift, scale, (bf16*)y, mean, rstd, D, L, ld_shift, ld_scale, eps)
+#define LAUNCH_WARP(NV, R) ln_modulate_fwd_warp_kernel<NV, R><<<(unsigned)((rows / L * ((L + R - 1) / R) + kLnWarps - 1) / kLnWarps), kLnWarps * 32, 0, st>>>((const bf16*)x, shift, scale, (bf16*)y, mean, rstd, rows / L * ((L + R - 1) / R), D, L, (L + R - 1) / R, ld_shift, ld_scale, eps)
+  const bool pairs = rows >= 2 * 148 * 3 * kLnWarps && L > 1;      // three CTAs of pairs on every SM
+  if (D <= 1024) { if (pairs) LAUNCH_WARP(4, 2); else LAUNCH_WARP(4, 1); }
+  else if (D <= 2048) { if (pairs) LAUNCH_WARP(8, 2); else LAUNCH_WARP(8, 1); }
+  else if (D <= 4096) LAUNCH(2); else LAUNCH(4);
+#undef LAUNCH_WARP
 #undef LAUNCH
 }
 
 void cb200_ln_modulate_bwd(const void* dy, const void* x, const float* mean, const float* rstd, const float* scale,
                            void* dx, float* dshift, float* dscale, float* partials, long frames, int D, int L,
-                           int rows_per_cta, cudaStream_t st) {
+                           int rows_per_cta, long ld_scale, cudaStream_t st) {
   const int G = cb200_ln_groups_per_frame(L, rows_per_cta);
-#define LAUNCH(MV) ln_modulate_bwd_kernel<MV><<<(unsigned)(frames * G), kThreads, 0, st>>>((const bf16*)dy, (const bf16*)x, mean, rstd, scale, (bf16*)dx, partials, D, L, rows_per_cta, G)
+#define LAUNCH(MV) ln_modulate_bwd_kernel<MV><<<(unsigned)(frames * G), kThreads, 0, st>>>((const bf16*)dy, (const bf16*)x, mean, rstd, scale, (bf16*)dx, partials, D, L, rows_per_cta, G, ld_scale)
   if (D <= 2048) LAUNCH(1); else if (D <= 4096) LAUNCH(2); else LAUNCH(4);
 #undef LAUNCH
   dim3 grid((D + 255) / 256, (unsigned)frames);
@@ -746,29 +794,29 @@ void cb200_ln_modulate_bwd(const void* dy, const void* x, const float* mean, con
 }
 
 void cb200_gate_residual_fwd(const void* x, const float* gate, const void* y, void* out, long rows, int D, int L,
-                             cudaStream_t st) {
+                             long ld_gate, cudaStream_t st) {
   const long nvec = rows * (D >> 3);
   gate_residual_fwd_kernel<<<grid_for(nvec, kThreads, 148 * 16), kThreads, 0, st>>>((const bf16*)x, gate, (const bf16*)y,
-                                                                                    (bf16*)out, nvec, D, L);
+                                                                                    (bf16*)out, nvec, D, L, ld_gate);
 }
 
 void cb200_gate_residual_bwd(const void* dout, const float* gate, const void* y, void* dy, float* dgate, float* partials,
-                             long frames, int D, int L, int rows_per_cta, cudaStream_t st) {
+                             long frames, int D, int L, int rows_per_cta, long ld_gate, cudaStream_t st) {
   const int G = cb200_ln_groups_per_frame(L, rows_per_cta);
-#define LAUNCH(MV) gate_residual_bwd_kernel<MV><<<(unsigned)(frames * G), kThreads, 0, st>>>((const bf16*)dout, gate, (const bf16*)y, (bf16*)dy, partials, D, L, rows_per_cta, G)
+#define LAUNCH(MV) gate_residual_bwd_kernel<MV><<<(unsigned)(frames * G), kThreads, 0, st>>>((const bf16*)dout, gate, (const bf16*)y, (bf16*)dy, partials, D, L, rows_per_cta, G, ld_gate)
   if (D <= 2048) LAUNCH(1); else if (D <= 4096) LAUNCH(2); else LAUNCH(4);
 #undef LAUNCH
   dim3 grid((D + 255) / 256, (unsigned)frames);
   reduce_partials_kernel<<<grid, 256, 0, st>>>(partials, dgate, nullptr, D, G, 1);
 }
 
-void cb200_rmsnorm_rope_fwd(const void* x, const float* w, const float* cosv, const float* sinv, void* y, float* rstd,
+void cb200_rmsnorm_rope_fwd(const void* x, const void* w, int w_bf16, const float* cosv, const float* sinv, void* y, float* rstd,
                             long n_rows, int S, int H, int HD, float eps, cudaStream_t st) {
   const unsigned blocks = (unsigned)((n_rows + 16 * kRmsPasses - 1) / (16 * kRmsPasses));   // 8 warps x 2 rows x passes per CTA
   if (HD == 128)
-    rmsnorm_rope_fwd_kernel<128><<<blocks, 256, 0, st>>>((const bf16*)x, w, cosv, sinv, (bf16*)y, rstd, n_rows, S, H, eps);
+    rmsnorm_rope_fwd_kernel<128><<<blocks, 256, 0, st>>>((const bf16*)x, w, w_bf16, cosv, sinv, (bf16*)y, rstd, n_rows, S, H, eps);
   else
-    rmsnorm_rope_fwd_kernel<64><<<blocks, 256, 0, st>>>((const bf16*)x, w, cosv, sinv, (bf16*)y, rstd, n_rows, S, H, eps);
+    rmsnorm_rope_fwd_kernel<64><<<blocks, 256, 0, st>>>((const bf16*)x, w, w_bf16, cosv, sinv, (bf16*)y, rstd, n_rows, S, H, eps);
 }
 
 long cb200_rmsnorm_bwd_blocks(long n_rows, int rows_per_warp) {
@@ -776,15 +824,15 @@ long cb200_rmsnorm_bwd_blocks(long n_rows, int rows_per_warp) {
   return (warps + 7) / 8;
 }
 
-void cb200_rmsnorm_rope_bwd(const void* dy, const void* x, const float* w, const float* rstd, const float* cosv,
+void cb200_rmsnorm_rope_bwd(const void* dy, const void* x, const void* w, int w_bf16, const float* rstd, const float* cosv,
                             const float* sinv, void* dx, float* dw, float* partials, long n_rows, int S, int H, int HD,
                             int rows_per_warp, cudaStream_t st) {
   const long blocks = cb200_rmsnorm_bwd_blocks(n_rows, rows_per_warp);
   if (HD == 128)
-    rmsnorm_rope_bwd_kernel<128><<<(unsigned)blocks, 256, 0, st>>>((const bf16*)dy, (const bf16*)x, w, rstd, cosv, sinv,
+    rmsnorm_rope_bwd_kernel<128><<<(unsigned)blocks, 256, 0, st>>>((const bf16*)dy, (const bf16*)x, w, w_bf16, rstd, cosv, sinv,
                                                                    (bf16*)dx, partials, n_rows, S, H, rows_per_warp);
   else
-    rmsnorm_rope_bwd_kernel<64><<<(unsigned)blocks, 256, 0, st>>>((const bf16*)dy, (const bf16*)x, w, rstd, cosv, sinv,
+    rmsnorm_rope_bwd_kernel<64><<<(unsigned)blocks, 256, 0, st>>>((const bf16*)dy, (const bf16*)x, w, w_bf16, rstd, cosv, sinv,
                                                                   (bf16*)dx, partials, n_rows, S, H, rows_per_warp);
   reduce_rows_kernel<<<(HD + 31) / 32, 1024, 0, st>>>(partials, dw, HD, (int)blocks);
 }

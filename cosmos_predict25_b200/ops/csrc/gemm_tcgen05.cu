@@ -53,7 +53,8 @@ constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + 1024 /*alignment s
 // RoPE) and stored straight into the staging buffer of the rank that owns the head, at its place in the gathered sequence.
 struct HeadScatter {
   int64_t ptrs[8];    // staging buffers of the P ranks, each [B, P * S, Hl, 128] bf16
-  const float* w;     // [128] RMSNorm weight or nullptr
+  const void* w;      // [128] RMSNorm weight (fp32, or bf16 with w_bf16) or nullptr
+  int w_bf16;
   const float* cosv;  // [S, 64] or nullptr
   const float* sinv;
   int S, Hl, P, rank;
@@ -62,6 +63,10 @@ struct HeadScatter {
   float* rstd_out;    // optional [M, N / 128]: reciprocal RMS of every (token, head), with ``raw``
 };
 
+__device__ __forceinline__ float norm_weight(const HeadScatter& hs, int i) {
+  return hs.w_bf16 ? __bfloat162float(reinterpret_cast<const bf16*>(hs.w)[i]) : reinterpret_cast<const float*>(hs.w)[i];
+}
+
 struct GemmEpilogue {
   HeadScatter hs;     // hs.P == 0: disabled
   bf16* C;
@@ -69,7 +74,8 @@ struct GemmEpilogue {
                       // (full 256-column tiles only)
   const bf16* bias;   // optional [N]
   const bf16* resid;  // optional [M, N] (gated residual)
-  const float* gate;  // optional [M / L, N]
+  const float* gate;  // optional [M / L] rows of N, ld_gate elements apart
+  long ld_gate;
   int act;            // 0 none, 1 gelu(erf)
   int L;              // rows per gate vector
 };
@@ -409,8 +415,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
               if (ep.hs.w != nullptr) {
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
-                  a[j] *= rstd * ep.hs.w[c * 32 + j];
-                  bb[j] *= rstd * ep.hs.w[64 + c * 32 + j];
+                  a[j] *= rstd * norm_weight(ep.hs, c * 32 + j);
+                  bb[j] *= rstd * norm_weight(ep.hs, 64 + c * 32 + j);
                 }
                 if (ep.hs.cosv != nullptr) {
                   // this row's 32 cosines and sines come in through the staging block with coalesced loads (8 lanes per
@@ -456,7 +462,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         if (++acc == 2) { acc = 0; acc_ph ^= 1; }
         continue;
       }
-      const float* gate_row = (ep.gate != nullptr && row < M) ? ep.gate + (size_t)(row / ep.L) * N : nullptr;
+      const float* gate_row = (ep.gate != nullptr && row < M) ? ep.gate + (size_t)(row / ep.L) * ep.ld_gate : nullptr;
       if (vec_ok && n0 + BN <= N) {
         // ---- full-width tile: every global access of the epilogue goes through the warp's 4 KB staging block, so that a
         // warp instruction moves four contiguous 128-byte row segments instead of 32 scattered 16-byte pieces (the scattered
@@ -753,14 +759,15 @@ extern "C" int cb200_gemm_pair_mode(int mode) {
 }
 
 extern "C" int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int b_mn,
-                               const void* bias, int act, void* pre, const void* resid, const float* gate, int L, int* err,
-                               int sms, cudaStream_t st) {
+                               const void* bias, int act, void* pre, const void* resid, const float* gate, long ld_gate, int L,
+                               int* err, int sms, cudaStream_t st) {
   GemmEpilogue ep{};
   ep.C = (bf16*)C;
   ep.pre = (bf16*)pre;
   ep.bias = (const bf16*)bias;
   ep.resid = (const bf16*)resid;
   ep.gate = gate;
+  ep.ld_gate = ld_gate;
   ep.act = act;
   ep.L = L > 0 ? L : 1;
   if (cb200_gemm_pair_mode(-1) == 1 && M >= 2 * BM && N % 8 == 0) {
@@ -779,7 +786,7 @@ extern "C" int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int
 // `norm_w` (optional), rotated by cos/sin [S, 64] (optional, needs norm_w) and stored into staging buffer ptrs[head / Hl] at
 // [b, rank * S + s, head % Hl, :].  The buffers may live on peer GPUs (plain stores over NVLink).
 extern "C" int cb200_gemm_bf16_scatter_heads(const void* A, const void* W, int M, int N, int K, const int64_t* ptrs, int P,
-                                             int rank, int S, const float* norm_w, const float* cosv, const float* sinv,
+                                             int rank, int S, const void* norm_w, int norm_bf16, const float* cosv, const float* sinv,
                                              float eps, void* raw, float* rstd_out, int* err, int sms, cudaStream_t st) {
   if (P < 1 || P > 8 || N % 128 != 0 || (N / 128) % P != 0 || S <= 0 || M % S != 0) return -21;
   if (cosv != nullptr && norm_w == nullptr) return -22;
@@ -787,6 +794,7 @@ extern "C" int cb200_gemm_bf16_scatter_heads(const void* A, const void* W, int M
   GemmEpilogue ep{};
   for (int i = 0; i < P; ++i) ep.hs.ptrs[i] = ptrs[i];
   ep.hs.w = norm_w;
+  ep.hs.w_bf16 = norm_bf16;
   ep.hs.cosv = cosv;
   ep.hs.sinv = sinv;
   ep.hs.S = S;

@@ -11,18 +11,18 @@ extern "C" {
 // elementwise.cu
 int cb200_ln_groups_per_frame(int L, int rows_per_cta);
 void cb200_ln_modulate_fwd(const void* x, const float* shift, const float* scale, void* y, float* mean, float* rstd,
-                           long rows, int D, int L, float eps, cudaStream_t st);
+                           long rows, int D, int L, long ld_shift, long ld_scale, float eps, cudaStream_t st);
 void cb200_ln_modulate_bwd(const void* dy, const void* x, const float* mean, const float* rstd, const float* scale,
                            void* dx, float* dshift, float* dscale, float* partials, long frames, int D, int L,
-                           int rows_per_cta, cudaStream_t st);
+                           int rows_per_cta, long ld_scale, cudaStream_t st);
 void cb200_gate_residual_fwd(const void* x, const float* gate, const void* y, void* out, long rows, int D, int L,
-                             cudaStream_t st);
+                             long ld_gate, cudaStream_t st);
 void cb200_gate_residual_bwd(const void* dout, const float* gate, const void* y, void* dy, float* dgate, float* partials,
-                             long frames, int D, int L, int rows_per_cta, cudaStream_t st);
-void cb200_rmsnorm_rope_fwd(const void* x, const float* w, const float* cosv, const float* sinv, void* y, float* rstd,
+                             long frames, int D, int L, int rows_per_cta, long ld_gate, cudaStream_t st);
+void cb200_rmsnorm_rope_fwd(const void* x, const void* w, int w_bf16, const float* cosv, const float* sinv, void* y, float* rstd,
                             long n_rows, int S, int H, int HD, float eps, cudaStream_t st);
 long cb200_rmsnorm_bwd_blocks(long n_rows, int rows_per_warp);
-void cb200_rmsnorm_rope_bwd(const void* dy, const void* x, const float* w, const float* rstd, const float* cosv,
+void cb200_rmsnorm_rope_bwd(const void* dy, const void* x, const void* w, int w_bf16, const float* rstd, const float* cosv,
                             const float* sinv, void* dx, float* dw, float* partials, long n_rows, int S, int H, int HD,
                             int rows_per_warp, cudaStream_t st);
 void cb200_gelu_fwd(const void* x, void* y, long n, cudaStream_t st);
@@ -51,14 +51,16 @@ int cb200_skinny_bgemm(const float* a, long a_z, long a_r, long a_k, const long 
                        long b_k, int b_is_bf16, void* c, long c_z, int ldc, int c_is_bf16, const float* add, int ld_add, int add_cols,
                        int Z, int R, int N, int K, int silu_a, int silu_b, int ksplit, cudaStream_t st);
 
+int cb200_skinny_wide(long a_k, long b_n, long b_k, int b_is_bf16, int c_is_bf16, int silu_b, int N, int K);   // 1: 256-column tiles
+
 // gemm_tcgen05.cu
 int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int b_mn, const void* bias,
-                    int act, void* pre, const void* resid, const float* gate, int L, int* err, int sms, cudaStream_t st);
+                    int act, void* pre, const void* resid, const float* gate, long ld_gate, int L, int* err, int sms, cudaStream_t st);
 int cb200_gemm_pair_mode(int mode);   // 0 / 1 sets, -1 reads; returns the previous mode (1 = CTA-pair tiles where the shape allows)
 int cb200_gemm_bf16_gather(const void* A, void* ws, void* C, int M, int rows, int ld, int b_mn, const int64_t* shard_ptrs, int P,
                            int chunk_rows, int* counters, const void* bias, int act, void* pre, int* err, int sms, cudaStream_t st);
 int cb200_gemm_bf16_scatter_heads(const void* A, const void* W, int M, int N, int K, const int64_t* ptrs, int P, int rank, int S,
-                                  const float* norm_w, const float* cosv, const float* sinv, float eps, void* raw, float* rstd_out, int* err, int sms,
+                                  const void* norm_w, int norm_bf16, const float* cosv, const float* sinv, float eps, void* raw, float* rstd_out, int* err, int sms,
                                   cudaStream_t st);
 }
 

@@ -83,7 +83,7 @@ extern "C" int cb200_rmsnorm_rope_bwd_noalloc(const void* dy, const void* x, con
     return CB200_NOALLOC_ERR_CUDA;
   }
   // every partial slot [0, ctas) x [0, HD) is written by the first kernel before the second one sums it
-  cb200_rmsnorm_rope_bwd(dy, x, w, rstd, cosv, sinv, dx, dw, scratch, n_rows, S, H, HD, kRowsPerWarp, stream);
+  cb200_rmsnorm_rope_bwd(dy, x, w, 0, rstd, cosv, sinv, dx, dw, scratch, n_rows, S, H, HD, kRowsPerWarp, stream);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error(errbuf, errbuf_len, "rmsnorm_rope_bwd_noalloc: kernel launch failed with CUDA error %ld", (long)e);

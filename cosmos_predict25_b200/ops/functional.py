@@ -161,15 +161,19 @@ def _linear_fm(x, w, bias, act):
 # --------------------------------------------------------------------------------------
 # AdaLN: LayerNorm + modulate
 # --------------------------------------------------------------------------------------
+def _mod_rows(t: torch.Tensor, frames: int, D: int) -> torch.Tensor:
+    """[B, T, D] modulation vectors as fp32 rows; a slice of the modulation MLPs' output stays where it lies (strided rows)."""
+    return t.float().reshape(frames, D)
+
+
 class _LnModulate(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, shift, scale, eps):
         ops = native.load()
         B, T, L, D = x.shape
         xc = x.contiguous()
-        shift_c = shift.float().contiguous()
-        scale_c = scale.float().contiguous()
-        y, mean, rstd = ops.ln_modulate_fwd(xc.view(B * T * L, D), shift_c.view(B * T, D), scale_c.view(B * T, D), L, eps)
+        scale_c = _mod_rows(scale, B * T, D)
+        y, mean, rstd = ops.ln_modulate_fwd(xc.view(B * T * L, D), _mod_rows(shift, B * T, D), scale_c, L, eps)
         native.count_launch()
         ctx.save_for_backward(xc, scale_c, mean, rstd)
         ctx.dims = (B, T, L, D)
@@ -182,7 +186,7 @@ class _LnModulate(torch.autograd.Function):
         x, scale, mean, rstd = ctx.saved_tensors
         B, T, L, D = ctx.dims
         dx, dshift, dscale = ops.ln_modulate_bwd(
-            dy.contiguous().view(B * T * L, D), x.view(B * T * L, D), mean, rstd, scale.view(B * T, D), L
+            dy.contiguous().view(B * T * L, D), x.view(B * T * L, D), mean, rstd, scale, L
         )
         native.count_launch(2)
         return (dx.view(B, T, L, D), dshift.view(B, T, D).to(ctx.in_dtypes[0]),
@@ -206,9 +210,9 @@ class _GateResidual(torch.autograd.Function):
     def forward(ctx, x, gate, y):
         ops = native.load()
         B, T, L, D = x.shape
-        gate_c = gate.float().contiguous()
+        gate_c = _mod_rows(gate, B * T, D)
         yc = y.contiguous()
-        out = ops.gate_residual_fwd(x.contiguous().view(-1, D), gate_c.view(B * T, D), yc.view(-1, D), L)
+        out = ops.gate_residual_fwd(x.contiguous().view(-1, D), gate_c, yc.view(-1, D), L)
         native.count_launch()
         ctx.save_for_backward(gate_c, yc)
         ctx.dims = (B, T, L, D)
@@ -221,7 +225,7 @@ class _GateResidual(torch.autograd.Function):
         gate, y = ctx.saved_tensors
         B, T, L, D = ctx.dims
         dout = dout.contiguous()
-        dy, dgate = ops.gate_residual_bwd(dout.view(-1, D), gate.view(B * T, D), y.view(-1, D), L)
+        dy, dgate = ops.gate_residual_bwd(dout.view(-1, D), gate, y.view(-1, D), L)
         native.count_launch(2)
         return dout, dgate.view(B, T, D).to(ctx.gate_dtype), dy.view(B, T, L, D)
 
@@ -546,7 +550,7 @@ class _LinearGateResidual(torch.autograd.Function):
         B, T, L, D = resid.shape
         h2d = h.reshape(-1, h.shape[-1])
         h2d = h2d if h2d.is_contiguous() else h2d.contiguous()
-        gate_c = gate.float().contiguous().view(B * T, D)
+        gate_c = _mod_rows(gate, B * T, D)
         out, y = native.load().gemm_bf16_gate_residual_pre(h2d, w, resid.contiguous().view(-1, D), gate_c, L)
         native.count_launch()
         ctx.save_for_backward(h2d, w, gate_c, y)
@@ -579,7 +583,7 @@ def linear_gate_residual(h: torch.Tensor, w: torch.Tensor, resid: torch.Tensor, 
     if resid.is_cuda and not needs_grad and _native_gemm_ok(h2d, w) and h2d.shape[0] % 8 == 0 \
             and getattr(w, "_cb200_gather", None) is None:
         out = native.load().gemm_bf16_gate_residual(h2d.contiguous(), w, resid.contiguous().view(-1, D),
-                                                    gate.float().contiguous().view(B * T, D), L)
+                                                    _mod_rows(gate, B * T, D), L)
         native.count_launch()
         return out.view(B, T, L, D)
     if (resid.is_cuda and needs_grad and _native_gemm_ok(h2d, w) and h2d.shape[0] % 8 == 0 and w.shape[0] % 256 == 0
@@ -618,16 +622,20 @@ def _skinny_ok(a: torch.Tensor, weights: Sequence[torch.Tensor], ignore_forward_
                                                                    for w in weights) and hasattr(native.load(), "skinny_bgemm"))
 
 
-def _skinny_split(Z: int, R: int, N: int, K: int) -> int:
-    """Ranges of the reduction per problem: enough CTAs to fill the GPU when the output is a few tiles and K is long."""
+def _skinny_split(Z: int, R: int, N: int, K: int, wide: bool) -> int:
+    """Ranges of the reduction per problem: enough CTAs to fill the GPU when the output is a few tiles and K is long. ``wide``: the
+    256-column kernel, four CTAs per SM, ranges of at least two of its 64-deep stages."""
+    if wide:
+        tiles = Z * ((R + 47) // 48) * ((N + 255) // 256)
+        return max(1, min(K // 128, 592 // max(tiles, 1), 65535 // Z))
     tiles = Z * ((R + 63) // 64) * ((N + 63) // 64)
     return max(1, min((K + 255) // 256, 296 // max(tiles, 1), 65535 // Z))
 
 
 def _skinny_call(ops, Z, R, N, K, *args):
     """args = the operator's arguments up to ``out_bf16``; splits long reductions and adds the partial sums."""
-    out_bf16 = args[-1]
-    S = 1 if out_bf16 else _skinny_split(Z, R, N, K)
+    _, _, _, a_k, _, _, _, b_n, b_k, bf16, _, _, _, _, _, _, _, silu_b, out_bf16 = args
+    S = 1 if out_bf16 else _skinny_split(Z, R, N, K, ops.skinny_wide(a_k, b_n, b_k, bf16, out_bf16, silu_b, N, K))
     out = ops.skinny_bgemm(*args, S)
     native.count_launch()
     return out if S == 1 else out.view(Z, S, R, N).sum(1)

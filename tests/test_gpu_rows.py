@@ -1,0 +1,94 @@
+"""Edges of the row-wise kernels: modulation vectors that are slices of a wider buffer, channel counts around the widths a warp
+holds, head counts that do not divide a warp's rows, row counts around the tiles of the few-row GEMM."""
+
+import math
+
+import pytest
+import torch
+
+from cosmos_predict25_b200.ops import functional as F_ops
+from cosmos_predict25_b200.ops import native, ref
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _max_rel(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm()).item()
+
+
+@pytest.mark.parametrize("D,L,T", [(8, 3, 2), (1024, 5, 3), (1032, 4, 1), (2048, 1, 7), (2056, 3, 2), (1024, 1777, 3),
+                                   (1800, 3553, 1)])
+@pytest.mark.parametrize("offset", [0, 2])
+def test_modulation_slices_are_read_in_place(D, L, T, offset):
+    """shift / scale / gate as thirds of one buffer; ``offset`` moves them off the 16-byte boundary (they are copied then)."""
+    torch.manual_seed(0)
+    x = torch.randn(1, T, L, D, device=DEV).bfloat16()
+    y = torch.randn(1, T, L, D, device=DEV).bfloat16()
+    buf = torch.randn(1, T, 3 * D + 4, device=DEV)
+    sh, sc, g = (buf[..., offset + i * D: offset + (i + 1) * D] for i in range(3))
+    mean_sq = 2.0 ** -9      # one bf16 rounding of the result (2^-9 relative), measured in the 2-norm
+    assert _max_rel(F_ops.ln_modulate(x, sh, sc), ref.ln_modulate(x.double(), sh.double(), sc.double())) < 1.5 * mean_sq
+    assert _max_rel(F_ops.gate_residual(x, g, y), x.double() + g.double().unsqueeze(2) * y.double()) < 1.5 * mean_sq
+    dout = torch.randn_like(y)
+    dy, dg = native.load().gate_residual_bwd(dout.view(-1, D), g.reshape(T, D), y.view(-1, D), L)
+    assert _max_rel(dy.view_as(y), dout.double() * g.double().unsqueeze(2)) < 1.5 * mean_sq
+    assert _max_rel(dg.view(1, T, D), (dout.double() * y.double()).sum(2)) < 1e-5
+
+
+def test_gated_gemm_epilogue_reads_strided_gates():
+    torch.manual_seed(1)
+    B, T, L, D, K = 1, 3, 88, 256, 128
+    h = torch.randn(B, T * L, K, device=DEV).bfloat16()
+    w = (torch.randn(D, K, device=DEV) / math.sqrt(K)).bfloat16()
+    x = torch.randn(B, T, L, D, device=DEV).bfloat16()
+    gate = torch.randn(B, T, 3 * D, device=DEV)[..., D:2 * D]
+    with torch.no_grad():
+        got = F_ops.linear_gate_residual(h, w, x, gate)
+    want = x.double() + gate.double().unsqueeze(2) * (h.double() @ w.double().t()).view(B, T, L, D)
+    assert _max_rel(got, want) < 1.5 * 2.0 ** -9
+
+
+@pytest.mark.parametrize("HD,H,S,B", [(128, 5, 7, 2), (128, 16, 33, 1), (64, 3, 130, 2), (128, 40, 3, 1), (64, 1, 1, 1)])
+@pytest.mark.parametrize("wdtype", [torch.bfloat16, torch.float32])
+def test_rmsnorm_rope_head_counts(HD, H, S, B, wdtype):
+    torch.manual_seed(2)
+    x = torch.randn(B, S, H, HD, device=DEV).bfloat16().requires_grad_(True)
+    w = (1 + 0.2 * torch.randn(HD, device=DEV)).to(wdtype).requires_grad_(True)
+    half = torch.randn(S, HD // 2, device=DEV)
+    rope = F_ops.RopeTable(torch.cat([half, half], 1))
+    dy = torch.randn(B, S, H, HD, device=DEV).bfloat16()
+    for table in (rope, None):
+        x.grad = w.grad = None
+        y = F_ops.rmsnorm_rope(x, w, table, 1e-6)
+        y.backward(dy)
+        xr, wr = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+        n = xr * torch.rsqrt(xr.pow(2).mean(-1, keepdim=True) + 1e-6) * wr
+        if table is not None:
+            c, s = half.double().cos()[None, :, None], half.double().sin()[None, :, None]
+            a, b = n[..., :HD // 2], n[..., HD // 2:]
+            n = torch.cat([a * c - b * s, b * c + a * s], -1)
+        n.backward(dy.double())
+        assert _max_rel(y, n) < 1.5 * 2.0 ** -9
+        assert _max_rel(x.grad, xr.grad) < 1.5 * 2.0 ** -9
+        assert _max_rel(w.grad, wr.grad) < (2.0 ** -8 if wdtype == torch.bfloat16 else 1e-5)
+
+
+# rows around the tiles of 4, 16, 32 and 48; columns off the 256-column tile; a reduction that is no multiple of the 64-deep stage
+@pytest.mark.parametrize("R", [1, 4, 5, 16, 17, 32, 33, 48, 49, 100])
+@pytest.mark.parametrize("K,N,Z", [(72, 264, 2), (2048, 256, 3), (256, 520, 1), (8, 8, 2)])
+def test_few_row_gemm_tiles(R, K, N, Z):
+    torch.manual_seed(3)
+    store = torch.randn(Z * N * K + 1, device=DEV).bfloat16() / math.sqrt(K)
+    for off in (0, 1):                          # off a 16-byte boundary: the weight is staged element by element
+        ws = [store[off + z * N * K: off + (z + 1) * N * K].view(N, K) for z in range(Z)]
+        a = torch.randn(Z, R, K, device=DEV)
+        add = torch.randn(R, N // 2, device=DEV)
+        got = F_ops.skinny_linears(a, ws, silu=True, add=add)
+        want = torch.nn.functional.silu(a.double()) @ torch.stack(ws).double().transpose(1, 2)
+        want[..., :N // 2] += add.double()
+        assert _max_rel(got, want) < 1e-6       # fp32 products and sums: 2^-24 per term of a random walk, SiLU by the fast exponential
+        dout = torch.randn(Z, R, N, device=DEV)
+        da = F_ops._skinny_call(native.load(), Z, R, K, N, dout, R * N, N, 1, F_ops._ptr_table(ws), None, 0, 1, K, True, None, 0, Z, R, K, N,
+                                False, False, False)
+        assert _max_rel(da, dout.double() @ torch.stack(ws).double()) < 1e-6
