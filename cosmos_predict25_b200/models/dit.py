@@ -24,6 +24,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops import functional as ops
+from ..ops import native
 from ..parallel import ulysses
 
 
@@ -516,6 +517,59 @@ class Block(nn.Module):
         return x
 
 
+_HOOKS = ("_forward_hooks", "_forward_pre_hooks")
+
+
+def _unhooked(*modules: nn.Module) -> bool:
+    return not any(getattr(m, h) for m in modules for h in _HOOKS) and not any("forward" in m.__dict__ for m in modules)
+
+
+def _plain_linear(m: nn.Module) -> bool:
+    return (type(m) is FusedLinear and m.bias is None and m.weight.dtype == torch.bfloat16 and m.weight.is_contiguous()
+            and getattr(m.weight, "_cb200_gather", None) is None)
+
+
+def _native_call_ok(x: torch.Tensor) -> bool:
+    """Whether a sequence of kernels may be issued as one native operator: no autograd, no forward-mode tangents, no dispatch mode or
+    global module hook that would want to see the single operators, and the kernels not replaced by library calls."""
+    glob = torch.nn.modules.module
+    return (x.is_cuda and x.dtype == torch.bfloat16 and not torch.is_grad_enabled() and not native.forward_mode() and native.available()
+            and ops.settings.gemm == "native" and ops.settings.attention == "native" and torch._C._len_torch_dispatch_stack() == 0
+            and torch._C._len_torch_function_stack() == 0 and not torch.compiler.is_compiling()
+            and not glob._global_forward_hooks and not glob._global_forward_pre_hooks)
+
+
+def native_block_weights(blocks, x: torch.Tensor, cross_kv) -> Optional[Tuple[List[torch.Tensor], List[torch.Tensor], float]]:
+    """The weights, keys / values and norm epsilon that the native block loop takes (``dit_blocks``), or None when a block is anything
+    but plain: adapters, biases, sparse or distributed attention, an image context, hooks, other types or head sizes."""
+    B, T, L, D = x.shape
+    if not _native_call_ok(x) or len(cross_kv) != len(blocks) or D % 128 or D > 8192 or B * T * L % 8:
+        return None
+    weights, kvs, eps = [], [], None
+    for blk, (k, v) in zip(blocks, cross_kv):
+        if type(blk) is not Block or type(blk.self_attn) is not Attention or type(blk.cross_attn) is not Attention or type(blk.mlp) is not GPT2FeedForward:
+            return None
+        sa, ca, mlp = blk.self_attn, blk.cross_attn, blk.mlp
+        linears = (sa.q_proj, sa.k_proj, sa.v_proj, sa.output_proj, ca.q_proj, ca.output_proj, mlp.layer1, mlp.layer2)
+        norms = (sa.q_norm, sa.k_norm, ca.q_norm)
+        if (sa.head_dim != 128 or ca.head_dim != 128 or sa.n_heads * 128 != D or ca.n_heads * 128 != D or sa.sparse_op is not None
+                or sa.cp_group is not None or not all(map(_plain_linear, linears)) or mlp.layer1.act != "gelu" or mlp.layer1.out_features % 64
+                or any(l.act != "none" for l in linears[:6]) or mlp.layer2.act != "none" or any(type(n) is not RMSNorm for n in norms)
+                or not _unhooked(blk, sa, ca, mlp, *linears, *norms)):
+            return None
+        for n in norms:
+            eps = n.eps if eps is None else eps
+            if n.eps != eps:
+                return None
+        for t in (k, v):
+            if t.dtype != torch.bfloat16 or not t.is_contiguous() or t.dim() != 4 or t.shape[0] != B or t.shape[2:] != (D // 128, 128):
+                return None
+        weights += [l.weight for l in linears[:4]] + [sa.q_norm.weight, sa.k_norm.weight] + [ca.q_proj.weight, ca.output_proj.weight,
+                                                                                            ca.q_norm.weight, mlp.layer1.weight, mlp.layer2.weight]
+        kvs += [k, v]
+    return weights, kvs, eps
+
+
 class FinalLayer(nn.Module):
     def __init__(self, cfg: DiTConfig):
         super().__init__()
@@ -640,7 +694,29 @@ class CosmosDiT(nn.Module):
 
     def build_context_cache(self, crossattn_emb: torch.Tensor) -> ContextCache:
         ctx = self.project_context(crossattn_emb)
-        return ContextCache(ctx, [b.cross_attn.project_kv(ctx) for b in self.blocks])
+        kv = self._context_kv_native(ctx)
+        return ContextCache(ctx, kv if kv is not None else [b.cross_attn.project_kv(ctx) for b in self.blocks])
+
+    def _context_kv_native(self, ctx: torch.Tensor) -> Optional[List[Tuple[torch.Tensor, torch.Tensor]]]:
+        """Every block's keys and values by one native operator, or None when a projection is not plain."""
+        if ctx.dim() != 3 or not _native_call_ok(ctx) or not ctx.is_contiguous() or ctx.shape[0] * ctx.shape[1] % 8 or ctx.shape[2] % 64:
+            return None
+        weights, eps = [], None
+        for b in self.blocks:
+            ca = b.cross_attn
+            if (type(ca) is not Attention or ca.head_dim != 128 or not _plain_linear(ca.k_proj) or not _plain_linear(ca.v_proj)
+                    or ca.k_proj.act != "none" or ca.v_proj.act != "none" or ca.v_proj.out_features != ca.k_proj.out_features
+                    or ca.k_proj.in_features != ctx.shape[2] or type(ca.k_norm) is not RMSNorm or not _unhooked(ca.k_proj, ca.v_proj, ca.k_norm)):
+                return None
+            eps = ca.k_norm.eps if eps is None else eps
+            if ca.k_norm.eps != eps:
+                return None
+            weights += [ca.k_proj.weight, ca.v_proj.weight, ca.k_norm.weight]
+        if not weights:
+            return None
+        kv = native.load().dit_context_kv(ctx, weights, eps)
+        native.count_launch(3 * len(self.blocks))
+        return list(zip(kv[0::2], kv[1::2]))
 
     def _embed(self, x_B_C_T_H_W, condition_mask, padding_mask):
         B, C, T, H, W = x_B_C_T_H_W.shape
@@ -717,7 +793,14 @@ class CosmosDiT(nn.Module):
                 and all(_plain_adaln(m) for b in self.blocks for m in b.adaln_mlps())):
             # the modulation vectors depend only on the timestep embedding: all 3 x L MLPs in two launches, once per forward
             all_mods = run_adaln_many([m for b in self.blocks for m in b.adaln_mlps()], emb, lora, cfg.use_wan_fp32_strategy)
-        for i, block in enumerate(self.blocks):
+        plain = native_block_weights(self.blocks, x, cross_kv) \
+            if all_mods is not None and all_mods.dtype == torch.float32 and cross_kv and extra is None else None
+        if plain is not None:
+            weights, kvs, eps = plain
+            cos, sin = rope.cos_sin() if rope is not None else (None, None)
+            x = native.load().dit_blocks(x.contiguous(), all_mods, cos, sin, weights, kvs, 1e-6, eps)
+            native.count_launch(16 * len(self.blocks))
+        for i, block in enumerate(self.blocks if plain is None else ()):
             kv = cross_kv[i] if cross_kv else None
             mods = None if all_mods is None else all_mods[3 * i: 3 * i + 3]
             x = run_block(block, cfg.checkpoint_mode if self.training else "none", x, emb, context, rope, lora, extra, kv, mods)

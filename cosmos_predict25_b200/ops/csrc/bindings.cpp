@@ -549,6 +549,7 @@ int64_t kernel_error(int64_t device, bool clear) {
 void register_attention_ops(torch::Library& m);
 void register_peer_ops(torch::Library& m);
 void register_conv_ops(torch::Library& m);
+void register_dit_ops(torch::Library& m);
 
 TORCH_LIBRARY(cosmos_b200, m) {
   m.def("ln_modulate_fwd(Tensor x, Tensor shift, Tensor scale, int L, float eps) -> (Tensor, Tensor, Tensor)", &ln_modulate_fwd);
@@ -590,6 +591,7 @@ TORCH_LIBRARY(cosmos_b200, m) {
   register_attention_ops(m);
   register_peer_ops(m);
   register_conv_ops(m);
+  register_dit_ops(m);
 }
 
 TORCH_LIBRARY_IMPL(cosmos_b200, CUDA, m) {
