@@ -107,19 +107,29 @@ __device__ __forceinline__ void red_release_gpu_add(int* p, int v) {
 // [128 r, 128 r + 128) of the A tile and of the B tile into its own shared memory (half the B bytes per CTA and per MMA), the even
 // CTA issues M = 256 MMAs that read both shared memories, each CTA's TMEM receives its 128 rows and its epilogue warps drain them.
 // Six 32 KB stages instead of four 48 KB ones.
-template <int A_MN, int B_MN, bool GATHER, bool CTA2 = false>
+//
+// SPLIT > 1: a cluster of SPLIT pairs works on ONE tile, each pair on its share of the contraction dimension, for outputs of so few
+// tiles that most of the GPU would idle while a handful of SMs pull the operands (a 512 x 2048 output is 16 tiles: 32 SMs fetch 1 MB
+// each at K = 2048). The fp32 partial tiles are exchanged through distributed shared memory - pair s receives the SPLIT - 1 other
+// partials of its 256 / SPLIT columns in the shared memory that the operand ring no longer needs - added in a fixed order (the
+// result is deterministic) and put back into TMEM, from where the ordinary epilogue finishes those columns.
+template <int A_MN, int B_MN, bool GATHER, bool CTA2 = false, int SPLIT = 1>
 __global__ void __launch_bounds__(kGemmThreads + (GATHER ? kGatherWarps * 32 : 0), 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, int M, int N, int K,
                  GemmEpilogue ep, GatherB gb, int* __restrict__ err) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   static_assert(!(CTA2 && GATHER), "the gather mode runs on single-CTA tiles");
+  static_assert(SPLIT == 1 || (CTA2 && (SPLIT == 2 || SPLIT == 4)), "split tiles: clusters of two or four pairs");
   constexpr int STG = CTA2 ? 6 : kStages;                                   // pipeline stages
   constexpr int STG_BYTES = CTA2 ? (kABytes + kBBytes / 2) : kStageBytes;   // bytes per stage in this CTA
   constexpr int TM = CTA2 ? 2 * BM : BM;                                    // output rows per tile (per pair with CTA2)
   static_assert(STG * STG_BYTES == kStages * kStageBytes, "both layouts fill the same shared-memory window");
-  const uint32_t pair_rank = CTA2 ? cluster_ctarank() : 0u;
-  const int first_tile = CTA2 ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, tile_step = CTA2 ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+  const uint32_t cta_rank = CTA2 ? cluster_ctarank() : 0u, pair_rank = cta_rank & 1u, lead_rank = cta_rank & ~1u;
+  const int split = (int)(cta_rank >> 1);                    // this pair's share of the tile's contraction (SPLIT > 1)
+  const uint16_t pair_mask = (uint16_t)(3u << lead_rank);
+  constexpr int kCtasPerTile = CTA2 ? 2 * SPLIT : 1;
+  const int first_tile = (int)blockIdx.x / kCtasPerTile, tile_step = (int)gridDim.x / kCtasPerTile;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STG * STG_BYTES);
   uint64_t* full = bars;                    // [STG]
   uint64_t* empty = bars + STG;             // [STG]
@@ -132,7 +142,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int tiles_m = (M + TM - 1) / TM, tiles_n = (N + BN - 1) / BN;
   const int n_tiles = tiles_m * tiles_n;
-  const int k_blocks = (K + BK - 1) / BK;
+  const int k_all = (K + BK - 1) / BK;
+  const int kb_first = SPLIT > 1 ? k_all * split / SPLIT : 0, k_blocks = SPLIT > 1 ? k_all * (split + 1) / SPLIT - kb_first : k_all;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STG; ++s) {
@@ -196,11 +207,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           if (!mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
           uint8_t* sa = smem + s * STG_BYTES;
           uint8_t* sb = sa + kABytes;
-          const int k0 = kb * BK;
+          const int k0 = (kb_first + kb) * BK;
           if (CTA2) {
             // all bytes of the pair's stage are counted on the leader's barrier: the leader announces them, both CTAs load
             if (pair_rank == 0) mbar_arrive_expect_tx(&full[s], 2 * STG_BYTES);
-            const uint32_t bar = mapa_shared(smem_u32(&full[s]), 0);
+            const uint32_t bar = mapa_shared(smem_u32(&full[s]), lead_rank);
             if (A_MN == 0) {
               tma_load_2d_pair(sa, &tma_a, bar, k0, m0);
             } else {
@@ -232,6 +243,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         }
       }
       if (!ok) { atomicCAS(err, 0, 1); *abort_flag = 1; }
+    }
+    if (SPLIT > 1) {                 // the two exchange barriers of the epilogue warps below take every warp of the cluster
+      __syncwarp();
+      cluster_sync_all();
+      cluster_sync_all();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
@@ -265,16 +281,21 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             else umma_ss_w(d_tmem, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u, leader);
           }
           // slot reusable once these MMAs have read it (with CTA2: in both CTAs)
-          if (CTA2) umma_commit_pair_w(&empty[s], leader);
+          if (CTA2) umma_commit_pair_w(&empty[s], leader, pair_mask);
           else umma_commit_w(&empty[s], leader);
           if (++s == STG) { s = 0; ph ^= 1; }
         }
         if (!ok) break;
-        if (CTA2) umma_commit_pair_w(&acc_full[acc], leader);
+        if (CTA2) umma_commit_pair_w(&acc_full[acc], leader, pair_mask);
         else umma_commit_w(&acc_full[acc], leader);
         if (++acc == 2) { acc = 0; acc_ph ^= 1; }
       }
       if (!ok && lane == 0) { atomicCAS(err, 0, 2); *abort_flag = 1; }
+    }
+    if (SPLIT > 1) {
+      __syncwarp();
+      cluster_sync_all();
+      cluster_sync_all();
     }
   } else if (GATHER && warp >= 10) {
     // ------------------------------------------------------------------ gather warps
@@ -329,14 +350,70 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     uint32_t acc_ph = 0;
     bool ok = true;
     const bool vec_ok = (N % 8) == 0;
-    const uint32_t acc_empty_leader[2] = {CTA2 ? mapa_shared(smem_u32(&acc_empty[0]), 0) : 0u,
-                                          CTA2 ? mapa_shared(smem_u32(&acc_empty[1]), 0) : 0u};
+    const uint32_t acc_empty_leader[2] = {CTA2 ? mapa_shared(smem_u32(&acc_empty[0]), lead_rank) : 0u,
+                                          CTA2 ? mapa_shared(smem_u32(&acc_empty[1]), lead_rank) : 0u};
     for (int t = first_tile; t < n_tiles && ok; t += tile_step) {
       const int m0 = (t / tiles_n) * TM + (CTA2 ? (int)pair_rank * BM : 0), n0 = (t % tiles_n) * BN;
-      if (!mbar_wait(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
+      ok = mbar_wait(&acc_full[acc], acc_ph, abort_flag);
+      if (SPLIT == 1 && !ok) break;
       tc_fence_after();
       const int row = m0 + quarter * 32 + lane;
       const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
+      if (SPLIT > 1) {
+        // One tile per cluster: this code runs once. Block (src, float4 column g of the slice) of the receiving CTA holds 128 rows x
+        // 16 bytes, so that the lanes of a warp write and read 512 contiguous bytes.
+        constexpr int kSlice = BN / SPLIT;
+        const int r_tile = quarter * 32 + lane;
+        __syncwarp();
+        cluster_sync_all();            // every pair's MMAs are complete: the operand rings are free
+        if (ok) {
+#pragma unroll 1
+          for (int c = part * 4; c < part * 4 + 4; ++c) {
+            const int dst = c * 32 / kSlice;
+            if (dst == split) continue;
+            uint32_t r[32];
+            tmem_ld32(t_row + c * 32, r);
+            tmem_ld_wait();
+            const uint32_t base = mapa_shared(smem_u32(smem), (uint32_t)(2 * dst) + pair_rank) +
+                                  (uint32_t)((split * (kSlice / 4) + (c * 32 - dst * kSlice) / 4) * (BM * 16) + r_tile * 16);
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              st_cluster_v4(base + q * (BM * 16), __uint_as_float(r[q * 4]), __uint_as_float(r[q * 4 + 1]), __uint_as_float(r[q * 4 + 2]),
+                            __uint_as_float(r[q * 4 + 3]));
+          }
+        }
+        __syncwarp();
+        cluster_sync_all();            // every partial has arrived
+        if (!ok) break;
+        if (part != split * kSlice / 128) break;      // the slice's columns belong to the warps of one half
+#pragma unroll 1
+        for (int c = split * kSlice / 32; c < (split + 1) * kSlice / 32; ++c) {
+          uint32_t own[32];
+          tmem_ld32(t_row + c * 32, own);
+          tmem_ld_wait();
+          float sum[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) sum[j] = 0.f;
+#pragma unroll
+          for (int src = 0; src < SPLIT; ++src) {
+            if (src == split) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) sum[j] += __uint_as_float(own[j]);
+            } else {
+              const uint8_t* in = smem + (src * (kSlice / 4) + (c * 32 - split * kSlice) / 4) * (BM * 16) + r_tile * 16;
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                const float4 f = *reinterpret_cast<const float4*>(in + q * (BM * 16));
+                sum[q * 4] += f.x; sum[q * 4 + 1] += f.y; sum[q * 4 + 2] += f.z; sum[q * 4 + 3] += f.w;
+              }
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 32; ++j) own[j] = __float_as_uint(sum[j]);
+          tmem_st32(t_row + c * 32, own);
+        }
+        tmem_st_wait();
+      }
       if (ep.hs.P > 0) {
         // ---- fused head scatter: this thread owns one token row; a 256-wide tile holds two complete heads
         // tcgen05.ld is warp-collective: every lane runs every load, rows past M only skip their stores
@@ -492,6 +569,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 #pragma unroll 1
         for (int pass = 0; pass < 2; ++pass) {
           const int coff = part * 128 + pass * 64;              // column offset inside the tile
+          if (SPLIT == 4 && coff != split * 64) continue;       // this pair finishes 64 columns (with SPLIT 2: the 128 of this warp)
           const int colbase = n0 + coff;
           if (ep.pre != nullptr && (ep.act == 1 || ep.gate != nullptr)) {
             // second output first (TMEM is read again below): the pre-activation of a GELU, or the plain product of a
@@ -744,6 +822,69 @@ static int launch_gemm_pair(const void* A, const void* B, int M, int N, int K, c
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
 
+// Split tiles (template flag SPLIT): a cluster of SPLIT pairs per 256 x 256 tile, as many clusters as tiles.
+template <int A_MN, int B_MN, int SPLIT>
+static int launch_gemm_split(const void* A, const void* B, int M, int N, int K, const GemmEpilogue& ep, int* err, cudaStream_t st,
+                             int* clusters) {
+  auto kern = gemm_bf16_kernel<A_MN, B_MN, false, true, SPLIT>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kGemmThreads);
+  cfg.dynamicSmemBytes = kSmemBytes;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2 * SPLIT;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  static int max_clusters = 0;       // clusters that the GPU holds at once
+  if (max_clusters == 0) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+    if (e != cudaSuccess) return 100 + (int)e;
+    int n = 0;
+    cfg.gridDim = dim3(2 * SPLIT);
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) return 600;
+    max_clusters = n;
+  }
+  if (clusters != nullptr) {         // only asked for the capacity
+    *clusters = max_clusters;
+    return 0;
+  }
+  CUtensorMap ta, tb;
+  int rc;
+  if (A_MN == 0) rc = make_tmap_2d_bf16(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, BM);
+  else rc = make_tmap_2d_bf16(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)M * 2, 64, BK);
+  if (rc) return rc;
+  if (B_MN == 0) rc = make_tmap_2d_bf16(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, BK, BN / 2);
+  else rc = make_tmap_2d_bf16(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)N * 2, 64, BK);
+  if (rc) return rc;
+  cfg.gridDim = dim3(2 * SPLIT * ((M + 2 * BM - 1) / (2 * BM)) * (N / BN));
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, M, N, K, ep, GatherB{}, err);
+  return e == cudaSuccess ? 0 : 500 + (int)e;
+}
+
+// One tile per pair, or clusters of 2 or 4 pairs per tile: whichever takes fewer k-blocks in a row, waves counted, with kExchange
+// k-blocks' time for the exchange of partial tiles. Six k-blocks: measured 9.1 us
+// against 7.0 us of fixed time, 0.3 us a k-block. 512 x 2048 from K = 2048: 18.7 -> 13.9 us, from K = 8192: 46.9 -> 28; 1024 x 1024 from
+// K = 100,352 (the text projection): 460 -> 241 us.
+template <int A_MN, int B_MN>
+static int launch_gemm_any(const void* A, const void* B, int M, int N, int K, const GemmEpilogue& ep, int* err, int sms, cudaStream_t st) {
+  const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN), kb = (K + BK - 1) / BK;
+  const int pairs = sms / 2;
+  if (N % BN == 0 && ep.hs.P == 0 && 2 * tiles <= pairs && kb >= 8) {
+    constexpr long kExchange = 6;
+    int c2 = 0, c4 = 0;
+    int rc = launch_gemm_split<A_MN, B_MN, 2>(A, B, M, N, K, ep, err, st, &c2);
+    if (rc) return rc;
+    if ((rc = launch_gemm_split<A_MN, B_MN, 4>(A, B, M, N, K, ep, err, st, &c4))) return rc;
+    const long t1 = kb, t2 = ((tiles + c2 - 1) / c2) * ((kb + 1) / 2 + kExchange), t4 = ((tiles + c4 - 1) / c4) * ((kb + 3) / 4 + kExchange);
+    if (t4 < t1 && t4 <= t2) return launch_gemm_split<A_MN, B_MN, 4>(A, B, M, N, K, ep, err, st, nullptr);
+    if (t2 < t1) return launch_gemm_split<A_MN, B_MN, 2>(A, B, M, N, K, ep, err, st, nullptr);
+  }
+  return launch_gemm_pair<A_MN, B_MN>(A, B, M, N, K, ep, err, sms, st);
+}
+
 // 0: single-CTA tiles; 1 (default): CTA pairs where the shape allows (measured 8-45 % faster on the 2B shapes: half the B-operand
 // bytes per CTA). COSMOS_B200_GEMM_PAIR=0 selects single-CTA tiles; cb200_gemm_pair_mode switches at run time (the kernel
 // benchmark compares the two).
@@ -771,10 +912,10 @@ extern "C" int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int
   ep.act = act;
   ep.L = L > 0 ? L : 1;
   if (cb200_gemm_pair_mode(-1) == 1 && M >= 2 * BM && N % 8 == 0) {
-    if (a_mn == 0 && b_mn == 0) return launch_gemm_pair<0, 0>(A, B, M, N, K, ep, err, sms, st);
-    if (a_mn == 0 && b_mn == 1) return launch_gemm_pair<0, 1>(A, B, M, N, K, ep, err, sms, st);
-    if (a_mn == 1 && b_mn == 0) return launch_gemm_pair<1, 0>(A, B, M, N, K, ep, err, sms, st);
-    return launch_gemm_pair<1, 1>(A, B, M, N, K, ep, err, sms, st);
+    if (a_mn == 0 && b_mn == 0) return launch_gemm_any<0, 0>(A, B, M, N, K, ep, err, sms, st);
+    if (a_mn == 0 && b_mn == 1) return launch_gemm_any<0, 1>(A, B, M, N, K, ep, err, sms, st);
+    if (a_mn == 1 && b_mn == 0) return launch_gemm_any<1, 0>(A, B, M, N, K, ep, err, sms, st);
+    return launch_gemm_any<1, 1>(A, B, M, N, K, ep, err, sms, st);
   }
   if (a_mn == 0 && b_mn == 0) return launch_gemm<0, 0>(A, B, M, N, K, ep, err, sms, st);
   if (a_mn == 0 && b_mn == 1) return launch_gemm<0, 1>(A, B, M, N, K, ep, err, sms, st);

@@ -323,6 +323,10 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t local_smem_addr, uint32
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(rank));
   return r;
 }
+// 16 bytes into the shared memory of another CTA of the cluster
+__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, float a, float b, float c, float d) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -363,17 +367,16 @@ __device__ __forceinline__ void umma_ss_pair_w(uint32_t tmem_d, uint64_t desc_a,
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
-// arrive on the mbarrier at this shared-memory offset in BOTH CTAs of the pair when the MMAs issued so far have completed
-__device__ __forceinline__ void umma_commit_pair_w(uint64_t* bar, uint32_t leader) {
+// arrive on the mbarrier at this shared-memory offset in BOTH CTAs of the pair when the MMAs issued so far have completed;
+// `ranks`: one bit per cluster rank of the pair (ranks 0 and 1 in a cluster of one pair)
+__device__ __forceinline__ void umma_commit_pair_w(uint64_t* bar, uint32_t leader, uint16_t ranks = 3) {
   asm volatile(
       "{\n\t"
       ".reg .pred q;\n\t"
-      ".reg .b16 m;\n\t"
       "setp.ne.b32 q, %1, 0;\n\t"
-      "mov.b16 m, 3;\n\t"
-      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %2;\n\t"
       "}\n"
-      ::"r"(smem_u32(bar)), "r"(leader)
+      ::"r"(smem_u32(bar)), "r"(leader), "h"(ranks)
       : "memory");
 }
 

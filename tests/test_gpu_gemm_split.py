@@ -1,0 +1,59 @@
+"""GEMMs whose output is a few tiles: clusters of two or four CTA pairs share a tile's contraction and exchange partial tiles through
+distributed shared memory. Ragged rows, contractions that do not divide by the split, every operand order and epilogue."""
+
+import math
+
+import pytest
+import torch
+
+from cosmos_predict25_b200.ops import native
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+ROUND = 1.5 * 2.0 ** -9        # one bf16 rounding of the result in the 2-norm
+
+
+def _rel(a, b):
+    return ((a.double() - b).norm() / b.norm()).item()
+
+
+def _check():
+    torch.cuda.synchronize()
+    assert native.load().kernel_error(0, True) == 0
+
+
+# tiles x k-blocks: below the split's limit, both splits, uneven shares (9, 13, 33 blocks), more tiles than half the pairs (no split)
+@pytest.mark.parametrize("M,N,K", [(256, 256, 448), (256, 256, 576), (264, 512, 832), (520, 2048, 2048), (512, 2048, 8192), (1000, 1024, 2112),
+                                   (2056, 1024, 1536), (2304, 1024, 2048), (7040, 2048, 1024)])
+@pytest.mark.parametrize("trans_a,trans_b", [(False, False), (False, True), (True, False), (True, True)])
+def test_operand_orders(M, N, K, trans_a, trans_b):
+    torch.manual_seed(0)
+    a = torch.randn(M, K, device=DEV).bfloat16()
+    b = (torch.randn(N, K, device=DEV) / math.sqrt(K)).bfloat16()
+    want = a.double() @ b.double().t()
+    args = (a.t().contiguous() if trans_a else a, b.t().contiguous() if trans_b else b, None, 0, trans_a, trans_b)
+    got = native.load().gemm_bf16(*args)
+    again = native.load().gemm_bf16(*args)
+    _check()
+    assert _rel(got, want) < ROUND and torch.equal(got, again)
+
+
+@pytest.mark.parametrize("M,N,K", [(264, 512, 832), (512, 1024, 4096), (2048, 512, 640)])
+def test_epilogues(M, N, K):
+    torch.manual_seed(1)
+    ops = native.load()
+    a = torch.randn(M, K, device=DEV).bfloat16()
+    b = (torch.randn(N, K, device=DEV) / math.sqrt(K)).bfloat16()
+    bias = torch.randn(N, device=DEV).bfloat16()
+    L = 8
+    gate = torch.randn(M // L, 3 * N, device=DEV)[:, N:2 * N]
+    resid = torch.randn(M, N, device=DEV).bfloat16()
+    prod = a.double() @ b.double().t()
+    pre_want = prod + bias.double()
+    y, pre = ops.gemm_bf16_gelu_pre(a, b, bias)
+    out, p = ops.gemm_bf16_gate_residual_pre(a, b, resid, gate, L)
+    only = ops.gemm_bf16_gate_residual(a, b, resid, gate, L)
+    _check()
+    assert _rel(pre, pre_want) < ROUND and _rel(y, torch.nn.functional.gelu(pre_want)) < ROUND
+    sum_want = resid.double() + gate.double().repeat_interleave(L, 0) * prod
+    assert _rel(p, prod) < ROUND and _rel(out, sum_want) < ROUND and torch.equal(out, only)
