@@ -54,4 +54,27 @@ __device__ __forceinline__ float scrub(float x) {
   return (fabsf(x) <= 3.402823466e+38f) ? x : 0.f;
 }
 
+// Programmatic dependent launch: a kernel launched with `launch_pdl` may start before the kernel in front of it on the stream has
+// ended - its set-up (barriers, TMEM, descriptors) and its launch then overlap that kernel's tail. Every thread block of such a kernel
+// calls pdl_wait() before its first access to global memory; the call returns when the kernel in front is complete and its writes
+// are visible. pdl_trigger() lets the next kernel start; it comes after the block's own TMEM allocation, so that a waiting kernel
+// never holds what a block of this one still needs (the next kernel starts only when every block has triggered or ended).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+static inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 }  // namespace cb200

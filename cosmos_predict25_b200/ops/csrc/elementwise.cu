@@ -126,6 +126,8 @@ __global__ void __launch_bounds__(kLnWarps * 32) ln_modulate_fwd_warp_kernel(
     const bf16* __restrict__ x, const float* __restrict__ shift, const float* __restrict__ scale,
     bf16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, long groups, int D, int L, int groups_per_frame,
     long ld_shift, long ld_scale, float eps) {
+  pdl_trigger();                     // launched with programmatic serialisation (see common.cuh)
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long group = (long)blockIdx.x * kLnWarps + (threadIdx.x >> 5);
   if (group >= groups) return;
@@ -494,6 +496,8 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_fwd_kernel(
     float eps) {
   constexpr int P = HD / 32, Q = P / 2;
   constexpr int U = kRmsPasses;
+  pdl_trigger();                     // launched with programmatic serialisation (see common.cuh)
+  pdl_wait();
   const int lane = threadIdx.x & 31, sub = lane & 15, half = lane >> 4;
   const long row0 = ((long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (2 * U) + half;   // this lane's rows: row0 + 2u
   float2 lo[U][Q], hi[U][Q];
@@ -773,7 +777,7 @@ int cb200_ln_groups_per_frame(int L, int rows_per_cta) { return (L + rows_per_ct
 void cb200_ln_modulate_fwd(const void* x, const float* shift, const float* scale, void* y, float* mean, float* rstd,
                            long rows, int D, int L, long ld_shift, long ld_scale, float eps, cudaStream_t st) {
 #define LAUNCH(MV) ln_modulate_fwd_kernel<MV><<<(unsigned)rows, kThreads, 0, st>>>((const bf16*)x, shift, scale, (bf16*)y, mean, rstd, D, L, ld_shift, ld_scale, eps)
-#define LAUNCH_WARP(NV, R) ln_modulate_fwd_warp_kernel<NV, R><<<(unsigned)((rows / L * ((L + R - 1) / R) + kLnWarps - 1) / kLnWarps), kLnWarps * 32, 0, st>>>((const bf16*)x, shift, scale, (bf16*)y, mean, rstd, rows / L * ((L + R - 1) / R), D, L, (L + R - 1) / R, ld_shift, ld_scale, eps)
+#define LAUNCH_WARP(NV, R) launch_pdl(ln_modulate_fwd_warp_kernel<NV, R>, dim3((unsigned)((rows / L * ((L + R - 1) / R) + kLnWarps - 1) / kLnWarps)), dim3(kLnWarps * 32), 0, st, (const bf16*)x, shift, scale, (bf16*)y, mean, rstd, rows / L * ((L + R - 1) / R), D, L, (L + R - 1) / R, ld_shift, ld_scale, eps)
   const bool pairs = rows >= 2 * 148 * 3 * kLnWarps && L > 1;      // three CTAs of pairs on every SM
   if (D <= 1024) { if (pairs) LAUNCH_WARP(4, 2); else LAUNCH_WARP(4, 1); }
   else if (D <= 2048) { if (pairs) LAUNCH_WARP(8, 2); else LAUNCH_WARP(8, 1); }
@@ -814,9 +818,9 @@ void cb200_rmsnorm_rope_fwd(const void* x, const void* w, int w_bf16, const floa
                             long n_rows, int S, int H, int HD, float eps, cudaStream_t st) {
   const unsigned blocks = (unsigned)((n_rows + 16 * kRmsPasses - 1) / (16 * kRmsPasses));   // 8 warps x 2 rows x passes per CTA
   if (HD == 128)
-    rmsnorm_rope_fwd_kernel<128><<<blocks, 256, 0, st>>>((const bf16*)x, w, w_bf16, cosv, sinv, (bf16*)y, rstd, n_rows, S, H, eps);
+    launch_pdl(rmsnorm_rope_fwd_kernel<128>, dim3(blocks), dim3(256), 0, st, (const bf16*)x, w, w_bf16, cosv, sinv, (bf16*)y, rstd, n_rows, S, H, eps);
   else
-    rmsnorm_rope_fwd_kernel<64><<<blocks, 256, 0, st>>>((const bf16*)x, w, w_bf16, cosv, sinv, (bf16*)y, rstd, n_rows, S, H, eps);
+    launch_pdl(rmsnorm_rope_fwd_kernel<64>, dim3(blocks), dim3(256), 0, st, (const bf16*)x, w, w_bf16, cosv, sinv, (bf16*)y, rstd, n_rows, S, H, eps);
 }
 
 long cb200_rmsnorm_bwd_blocks(long n_rows, int rows_per_warp) {

@@ -157,9 +157,13 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
   // A CTA that starts after another one has reported an error leaves at once (the whole grid then drains in microseconds
   // instead of running every CTA into its own wait limit). One thread reads the word so that the decision is CTA-uniform.
+  // It is read ahead of the wait for the kernel in front: only errors of kernels before that one are sure to be seen.
   if (threadIdx.x == 0) *abort_flag = *reinterpret_cast<volatile int*>(err);
   __syncthreads();
-  if (*abort_flag != 0) return;
+  if (*abort_flag != 0) {
+    pdl_wait();
+    return;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -183,6 +187,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();                     // launched with programmatic serialisation (see common.cuh)
+  pdl_wait();
 
   // With REGS every role branch starts by re-dividing the registers of its warpgroup (the instruction has to sit inside the
   // branch: the compiler takes the smallest limit that reaches a join point as the limit of everything after it).
@@ -509,8 +515,7 @@ static int launch_fa_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
     attr = true;
   }
   dim3 grid((Sq + QT * BQ - 1) / (QT * BQ), H, B);
-  kern<<<grid, Sh::kThreads, Sh::kSmem, st>>>(tq, tk, tv, (bf16*)o, lse, Sq, Skv, H, scale * 1.4426950408889634f, sc, na, err);
-  return (int)cudaGetLastError();
+  return (int)launch_pdl(kern, grid, dim3(Sh::kThreads), Sh::kSmem, st, tq, tk, tv, (bf16*)o, lse, Sq, Skv, H, scale * 1.4426950408889634f, sc, na, err);
 }
 
 // the variant the operators use: exponentials split between the special-function unit and the FMA pipe, half-row hand-off

@@ -171,6 +171,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   if (CTA2) cluster_sync_all();      // the other CTA's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (CTA2) {                        // launched with programmatic serialisation (see common.cuh)
+    pdl_trigger();
+    pdl_wait();
+  }
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -801,13 +805,15 @@ static int launch_gemm_pair(const void* A, const void* B, int M, int N, int K, c
   cfg.blockDim = dim3(kGemmThreads);
   cfg.dynamicSmemBytes = kSmemBytes;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   // A persistent grid must be resident as a whole: the pairs that the GPU can hold at once (a pair lives inside one GPC, so a
   // GPC with an odd number of free SMs leaves one out) bound the grid, otherwise late pairs would run after the others.
   static int max_pairs = 0;
@@ -831,13 +837,15 @@ static int launch_gemm_split(const void* A, const void* B, int M, int N, int K, 
   cfg.blockDim = dim3(kGemmThreads);
   cfg.dynamicSmemBytes = kSmemBytes;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2 * SPLIT;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   static int max_clusters = 0;       // clusters that the GPU holds at once
   if (max_clusters == 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
