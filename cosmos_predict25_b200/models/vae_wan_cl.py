@@ -11,7 +11,8 @@ step (cosmos_predict2/_src/predict2/tokenizers/wan2pt1.py:40-58, 84-137, 184-215
     pre-summed weights: output pixel (2y + a, 2x + b) only ever sees a 2 x 2 neighbourhood of the input, so 4 taps replace 9 and
     the up-sampled frame is never materialised; the phases interleave through the kernel's output mapping;
   * the temporal up-sampler's channel-to-frame interleave is an output mapping too (two launches, one per output-channel half);
-  * RMS-norm + SiLU in front of a convolution is one element-wise kernel.
+  * RMS-norm + SiLU in front of a convolution is part of the epilogue of the convolution before it while one tile holds all channels
+    (96 and 192), else one element-wise kernel.
 
 The single-head frame attention of the middle block runs on ``fa_wide`` (head dimension 384) with its 1 x 1 projections on this
 package's GEMM. Weights are repacked once (``[C_out, taps, C_in padded to 64]`` bf16, fp32 bias) when the object is built.
@@ -75,36 +76,57 @@ class ConvCL:
             return vae_parallel.exchange_rows(x, 1, 1), self.taps_halo
         return x, self.taps
 
-    def _launch(self, x, taps, t_out, h_out, w_out, out, out_map, resid, cache=None, pad=0):
-        if out is None:
+    def _launch(self, x, taps, t_out, h_out, w_out, out, out_map, resid, cache=None, pad=0, norm=None, normed=None, raw=True):
+        if out is None and raw:
             out = torch.empty(t_out, h_out, w_out, self.cout, dtype=torch.bfloat16, device=x.device)
+        if norm is not None and normed is None:
+            normed = torch.empty(t_out, h_out, w_out, self.cout, dtype=torch.bfloat16, device=x.device)
+        dst = out if raw else normed
         if out_map is None:
-            out_map = [1, 0, 1, 0, 1, 0, out.shape[1], out.shape[2], out.shape[3], 0]
-        native.load().conv_cl(x, self.w, self.n_tile, self.cout, taps, t_out, h_out, w_out, out_map, out, resid, self.bias, cache, pad,
-                              self.t_stride, self.hw_stride)
+            out_map = [1, 0, 1, 0, 1, 0, dst.shape[1], dst.shape[2], dst.shape[3], 0]
+        native.load().conv_cl(x, self.w, self.n_tile, self.cout, taps, t_out, h_out, w_out, out_map, dst, resid, self.bias, cache, pad,
+                              self.t_stride, self.hw_stride, normed, None if norm is None else norm[0], norm is None or norm[1], raw)
         native.count_launch()
-        return out
+        return out if norm is None else (out, normed)
 
-    def strided(self, x: torch.Tensor) -> torch.Tensor:
-        """The spatially strided convolution of every frame of ``x``; pixels past the bottom / right edge are zeros."""
+    def _finish(self, y: torch.Tensor, norm, raw: bool):
+        """What a launch with ``norm`` returns, from its raw output: the norm as a kernel of its own."""
+        if norm is None:
+            return y
+        n = native.load().rmsnorm_silu_cl(y, norm[0], norm[1])
+        native.count_launch()
+        return (y if raw else None), n
+
+    def fuses_norm(self, x: torch.Tensor) -> bool:
+        """The epilogue normalises when one N tile holds all channels (up to 256)."""
+        return x.is_cuda and self.cout <= self.n_tile and self.cout % 8 == 0
+
+    def strided(self, x: torch.Tensor, norm=None) -> torch.Tensor:
+        """The spatially strided convolution of every frame of ``x``; pixels past the bottom / right edge are zeros. ``norm`` as in
+        ``causal``."""
         T, H, W, _ = x.shape
         if not x.is_cuda:                                      # plain definition: stride 1, every second pixel
-            return self(x, T)[:, ::self.hw_stride, ::self.hw_stride].contiguous()
-        return self._launch(x, self.taps, T, H // self.hw_stride, W // self.hw_stride, None, None, None)
+            return self._finish(self(x, T)[:, ::self.hw_stride, ::self.hw_stride].contiguous(), norm, True)
+        fused = norm if self.fuses_norm(x) else None
+        y = self._launch(x, self.taps, T, H // self.hw_stride, W // self.hw_stride, None, None, None, norm=fused)
+        return y if fused is not None else self._finish(y, norm, True)
 
-    def causal(self, x: torch.Tensor, state: "_Stream", pad_frames: int = CACHE_T, resid: Optional[torch.Tensor] = None) -> torch.Tensor:
+    def causal(self, x: torch.Tensor, state: "_Stream", pad_frames: int = CACHE_T, resid: Optional[torch.Tensor] = None, norm=None,
+               raw: bool = True):
         """The causal convolution of the chunk ``x`` with the ``pad_frames`` input frames before it, which the stream carries (zeros
-        before the first chunk); leaves this chunk's last frames in the stream."""
+        before the first chunk); leaves this chunk's last frames in the stream. ``norm`` = (gamma, silu) of the RMS-norm that follows:
+        the result is then (output, normalised output), the first None with ``raw`` False."""
         T, H, W, _ = x.shape
         t_out = T // self.t_stride
         if not x.is_cuda:
             full = _with_cache(self, x, state, pad_frames)
-            return self(full, T, resid=resid)[:t_out * self.t_stride:self.t_stride].contiguous()
+            return self._finish(self(full, T, resid=resid)[:t_out * self.t_stride:self.t_stride].contiguous(), norm, raw)
         x, taps = self._halo(x)
         prev = state.store.get(id(self))
-        out = self._launch(x, taps, t_out, H, W, None, None, resid, prev, pad_frames)
+        fused = norm if self.fuses_norm(x) else None
+        y = self._launch(x, taps, t_out, H, W, None, None, resid, prev, pad_frames, fused, None, raw or fused is None)
         state.store[id(self)] = _last_frames(prev, x, pad_frames)
-        return out
+        return y if fused is not None else self._finish(y, norm, raw)
 
 
 def _last_frames(prev: Optional[torch.Tensor], x: torch.Tensor, n: int) -> torch.Tensor:
@@ -146,6 +168,39 @@ def _upsample_conv2d_phases(conv2d, device) -> List[Tuple[ConvCL, int, int]]:
     return phases
 
 
+class _Layer:
+    """``run(x, state, xn, norm)``: ``xn`` is the layer's normalised input when the layer in front has produced it; ``norm`` = (gamma, silu)
+    of the RMS-norm with which the layer behind begins. Returns the output and, when a convolution's epilogue has made it, the
+    normalised output."""
+
+    def run(self, x, state, xn=None, norm=None):
+        raise NotImplementedError
+
+    def __call__(self, x, state):
+        return self.run(x, state)[0]
+
+
+def _wants(layer):
+    """(gamma, silu) of the RMS-norm with which a layer begins, or None."""
+    if isinstance(layer, _ResBlockCL):
+        return layer.g1, True
+    if isinstance(layer, _AttnCL):
+        return layer.gamma, False
+    return None
+
+
+def _run_layers(layers, y, yn, state, last):
+    """The layers in order, each told which norm the layer behind it begins with (``last``: behind the last one), so that a convolution
+    can produce the normalised tensor beside or instead of the raw one. Returns the last layer's normalised output."""
+    for i, layer in enumerate(layers):
+        norm = _wants(layers[i + 1]) if i + 1 < len(layers) else last
+        y, yn = layer.run(y, state, yn, norm)
+    if yn is None:
+        yn = native.load().rmsnorm_silu_cl(y, *last)
+        native.count_launch()
+    return yn
+
+
 class _Stream:
     """Last two input frames of every causal convolution (keyed by the ConvCL object)."""
 
@@ -164,7 +219,7 @@ def _with_cache(conv: ConvCL, x: torch.Tensor, state: _Stream, pad_frames: int =
     return full
 
 
-class _ResBlockCL:
+class _ResBlockCL(_Layer):
     def __init__(self, block, device):
         res = block.residual
         self.g1 = res[0].gamma.detach().float().reshape(-1).to(device).contiguous()
@@ -173,18 +228,17 @@ class _ResBlockCL:
         self.c2 = _conv3d(res[6], device)
         self.short = _conv3d(block.shortcut, device) if not isinstance(block.shortcut, torch.nn.Identity) else None
 
-    def __call__(self, x, state):
-        ops = native.load()
-        T = x.shape[0]
-        h = self.short(x, T) if self.short is not None else x
-        y = ops.rmsnorm_silu_cl(x, self.g1, True)
-        y = self.c1.causal(y, state)
-        y = ops.rmsnorm_silu_cl(y, self.g2, True)
-        native.count_launch(2)
-        return self.c2.causal(y, state, resid=h)
+    def run(self, x, state, xn=None, norm=None):
+        h = self.short(x, x.shape[0]) if self.short is not None else x
+        if xn is None:
+            xn = native.load().rmsnorm_silu_cl(x, self.g1, True)
+            native.count_launch()
+        _, y = self.c1.causal(xn, state, norm=(self.g2, True), raw=False)
+        out = self.c2.causal(y, state, resid=h, norm=norm)
+        return out if norm is not None else (out, None)
 
 
-class _AttnCL:
+class _AttnCL(_Layer):
     def __init__(self, block, device):
         C = block.dim
         self.C = C
@@ -194,10 +248,12 @@ class _AttnCL:
         self.w_proj = block.proj.weight.detach().reshape(C, C).to(device=device, dtype=torch.bfloat16).contiguous()
         self.b_proj = block.proj.bias.detach().to(device=device, dtype=torch.bfloat16).contiguous()
 
-    def __call__(self, x, state):
+    def run(self, x, state, xn=None, norm=None):
         T, H, W, C = x.shape
-        y = native.load().rmsnorm_silu_cl(x, self.gamma, False)
-        native.count_launch()
+        y = xn
+        if y is None:
+            y = native.load().rmsnorm_silu_cl(x, self.gamma, False)
+            native.count_launch()
         qkv = F_ops.linear(y.view(T * H * W, C), self.w_qkv, self.b_qkv).view(T, H * W, 3, C)
         q, k, v = (qkv[:, :, i] for i in range(3))                        # [T, HW, C], a single head of dimension C
         if vae_parallel.active() is not None:                             # local rows attend to the whole frame
@@ -208,10 +264,10 @@ class _AttnCL:
         else:                                                             # the kernel is built for the width of the released VAE
             o = F.scaled_dot_product_attention(q.unsqueeze(1), k.unsqueeze(1), v.unsqueeze(1)).squeeze(1)
         o = F_ops.linear(o.reshape(T * H * W, C), self.w_proj, self.b_proj)
-        return o.view(T, H, W, C) + x
+        return o.view(T, H, W, C) + x, None
 
 
-class _UpsampleCL:
+class _UpsampleCL(_Layer):
     def __init__(self, mod, device):
         self.mode = mod.mode
         self.dim = mod.dim
@@ -227,7 +283,7 @@ class _UpsampleCL:
                 self.time.append(ConvCL(wt, b[s * C:(s + 1) * C] if b is not None else None, _causal3_taps(3, 1, 1), device))
         self._key = object()
 
-    def __call__(self, x, state):
+    def run(self, x, state, xn=None, norm=None):
         T, H, W, C = x.shape
         if self.time is not None:
             prev = state.store.get(id(self._key))
@@ -243,9 +299,16 @@ class _UpsampleCL:
                 T = 2 * T
         cout = self.phases[0][0].cout
         out = torch.empty(T, 2 * H, 2 * W, cout, dtype=x.dtype, device=x.device)
+        fused = norm is not None and self.phases[0][0].fuses_norm(x)
+        normed = torch.empty_like(out) if fused else None
         for conv, a, b in self.phases:
-            conv(x, T, out=out, out_map=[1, 0, 2, a, 2, b, 2 * H, 2 * W, cout, 0], h_out=H, w_out=W)
-        return out
+            out_map = [1, 0, 2, a, 2, b, 2 * H, 2 * W, cout, 0]
+            if fused:
+                xh, taps = conv._halo(x)
+                conv._launch(xh, taps, T, H, W, out, out_map, None, norm=norm, normed=normed)
+            else:
+                conv(x, T, out=out, out_map=out_map, h_out=H, w_out=W)
+        return out, normed
 
 
 class DecoderCL:
@@ -298,12 +361,9 @@ class DecoderCL:
         T, h, w = x.shape[2:]
         xin = torch.zeros(T, h, w, self.z_pad, dtype=torch.bfloat16, device=self.device)
         xin[..., : self.z_dim] = x[0].permute(1, 2, 3, 0)
-        y = self.conv1.causal(xin, st)
-        for layer in self.layers:
-            y = layer(y, st)
-        y = native.load().rmsnorm_silu_cl(y, self.head_gamma, True)
-        native.count_launch()
-        y = self.head.causal(y, st)
+        first = _wants(self.layers[0])
+        y, yn = self.conv1.causal(xin, st, norm=first) if first is not None else (self.conv1.causal(xin, st), None)
+        y = self.head.causal(_run_layers(self.layers, y, yn, st, (self.head_gamma, True)), st)
         return y.permute(3, 0, 1, 2).unsqueeze(0)
 
 
@@ -314,7 +374,7 @@ def supported(decoder, z: torch.Tensor) -> bool:
 
 
 # ------------------------------------------------------------------------------------------------------------------ encoder
-class _DownsampleCL:
+class _DownsampleCL(_Layer):
     """``ZeroPad2d((0, 1, 0, 1)) + Conv2d(3 x 3, stride 2)`` and, for the 3-D mode, the causal ``(3, 1, 1)`` convolution with
     temporal stride 2 (wan2pt1.py:84-137): strided launches of the convolution kernel. Pixels past the bottom / right edge read its
     out-of-range fill, which is the zero padding; the time convolution's input is [last frame of the previous chunk | chunk]."""
@@ -330,14 +390,15 @@ class _DownsampleCL:
             wt = mod.time_conv.weight.detach().float()[:, :, :, 0, 0].permute(0, 2, 1)          # [C, 3, C]
             self.time = ConvCL(wt, mod.time_conv.bias, _causal3_taps(3, 1, 1), device, t_stride=2)
 
-    def __call__(self, x, state):
-        y = self.space.strided(x)
-        if self.time is None:
-            return y
-        if id(self.time) not in state.store:                             # first chunk: no temporal down-sampling
-            state.store[id(self.time)] = y[-1:]
-            return y
-        return self.time.causal(y, state, pad_frames=1)
+    def run(self, x, state, xn=None, norm=None):
+        first = self.time is not None and id(self.time) not in state.store
+        if self.time is None or first:                                   # first chunk: no temporal down-sampling
+            y = self.space.strided(x, norm)
+            if first:
+                state.store[id(self.time)] = (y if norm is None else y[0])[-1:]
+            return (y, None) if norm is None else y
+        y = self.time.causal(self.space.strided(x), state, pad_frames=1, norm=norm)
+        return (y, None) if norm is None else y
 
 
 class EncoderCL:
@@ -390,12 +451,9 @@ class EncoderCL:
         T, H, W = x.shape[2:]
         xin = torch.zeros(T, H, W, self.in_pad, dtype=torch.bfloat16, device=self.device)
         xin[..., : self.cin] = x[0].permute(1, 2, 3, 0)
-        y = self.conv1.causal(xin, st)
-        for layer in self.layers:
-            y = layer(y, st)
-        y = native.load().rmsnorm_silu_cl(y, self.head_gamma, True)
-        native.count_launch()
-        y = self.head.causal(y, st)
+        first = _wants(self.layers[0])
+        y, yn = self.conv1.causal(xin, st, norm=first) if first is not None else (self.conv1.causal(xin, st), None)
+        y = self.head.causal(_run_layers(self.layers, y, yn, st, (self.head_gamma, True)), st)
         return y.permute(3, 0, 1, 2).unsqueeze(0)
 
 

@@ -26,7 +26,8 @@ int sm_count(int device) {
 // x: the frames of `cache` are the last of these, frames before them are zeros; out_map: 10 ints (see ConvParams); y is written in place.
 void conv_cl(const Tensor& x, const Tensor& w, int64_t n_tile, int64_t Cout, c10::ArrayRef<int64_t> taps, int64_t T_out, int64_t H_out,
              int64_t W_out, c10::ArrayRef<int64_t> out_map, Tensor y, const c10::optional<Tensor>& resid,
-             const c10::optional<Tensor>& bias, const c10::optional<Tensor>& cache, int64_t pad, int64_t t_stride, int64_t hw_stride) {
+             const c10::optional<Tensor>& bias, const c10::optional<Tensor>& cache, int64_t pad, int64_t t_stride, int64_t hw_stride,
+             const c10::optional<Tensor>& y_norm, const c10::optional<Tensor>& gamma, bool silu, bool write_raw) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.is_contiguous() && x.dim() == 4, "x must be contiguous CUDA bf16 [T, H, W, C]");
   TORCH_CHECK(w.is_cuda() && w.scalar_type() == at::kBFloat16 && w.is_contiguous() && w.dim() == 2 && w.device() == x.device(),
               "w must be contiguous CUDA bf16 [rows, K] on the device of x");
@@ -56,6 +57,12 @@ void conv_cl(const Tensor& x, const Tensor& w, int64_t n_tile, int64_t Cout, c10
   if (bias.has_value())
     TORCH_CHECK(bias->is_cuda() && bias->scalar_type() == at::kFloat && bias->is_contiguous() && bias->device() == x.device() &&
                     bias->numel() >= Cout, "bias must be contiguous CUDA fp32 [Cout]");
+  TORCH_CHECK(y_norm.has_value() == gamma.has_value() && (write_raw || y_norm.has_value()), "give gamma with y_norm; without it the raw output is written");
+  if (y_norm.has_value())
+    TORCH_CHECK(y_norm->is_cuda() && y_norm->scalar_type() == at::kBFloat16 && y_norm->is_contiguous() && y_norm->device() == x.device() &&
+                    y_norm->numel() >= last && Cout <= n_tile && Cout % 8 == 0 && out_C % 8 == 0 && oc_add % 8 == 0 && gamma->is_cuda() &&
+                    gamma->scalar_type() == at::kFloat && gamma->is_contiguous() && gamma->numel() == Cout && gamma->device() == x.device(),
+                "y_norm must cover the output map, gamma be fp32 [Cout], and all channels lie in one N tile");
   c10::cuda::CUDAGuard g(x.device());
   std::vector<int> tp(taps.begin(), taps.end()), om(out_map.begin(), out_map.end());
   const int dev = x.get_device();
@@ -63,7 +70,8 @@ void conv_cl(const Tensor& x, const Tensor& w, int64_t n_tile, int64_t Cout, c10
                                cache.has_value() ? cache->data_ptr() : nullptr, cache.has_value() ? (int)cache->size(0) : 0, (int)pad,
                                (int)t_stride, (int)hw_stride, w.data_ptr(), (int)w.size(0), (int)n_tile, (int)Cout, tp.data(), (int)ntaps, (int)T_out, (int)H_out, (int)W_out, om.data(), y.data_ptr(),
                                resid.has_value() ? resid->data_ptr() : nullptr, bias.has_value() ? bias->data_ptr<float>() : nullptr,
-                               cb200_error_word(dev), sm_count(dev), at::cuda::getCurrentCUDAStream().stream());
+                               y_norm.has_value() ? y_norm->data_ptr() : nullptr, gamma.has_value() ? gamma->data_ptr<float>() : nullptr,
+                               silu ? 1 : 0, write_raw ? 1 : 0, cb200_error_word(dev), sm_count(dev), at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(rc == 0, "conv_cl launch failed with code ", rc);
 }
 
@@ -104,7 +112,8 @@ Tensor fa_wide(const Tensor& q, const Tensor& k, const Tensor& v, double scale) 
 
 void register_conv_ops(torch::Library& m) {
   m.def("conv_cl(Tensor x, Tensor w, int n_tile, int Cout, int[] taps, int T_out, int H_out, int W_out, int[] out_map, Tensor(a!) y, "
-        "Tensor? resid, Tensor? bias, Tensor? cache=None, int pad=0, int t_stride=1, int hw_stride=1) -> ()", &conv_cl);
+        "Tensor? resid, Tensor? bias, Tensor? cache=None, int pad=0, int t_stride=1, int hw_stride=1, "
+        "Tensor(b!)? y_norm=None, Tensor? gamma=None, bool silu=True, bool write_raw=True) -> ()", &conv_cl);
   m.def("fa_wide(Tensor q, Tensor k, Tensor v, float scale) -> Tensor", &fa_wide);
   m.def("rmsnorm_silu_cl(Tensor x, Tensor gamma, bool silu) -> Tensor", &rmsnorm_silu_cl);
 }

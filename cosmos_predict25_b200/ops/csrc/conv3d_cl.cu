@@ -51,6 +51,7 @@ constexpr int kMaxStages = 8;
 constexpr int kStageOut = 32 * 64;            // staging block of an epilogue warp: 32 voxels x 32 channels
 constexpr int kBiasMax = 1024;                // channels whose bias is kept in shared memory
 constexpr int kSmemMax = 227 * 1024, kSmemFixed = 1024 /*alignment slack*/ + 256 /*barriers*/ + 8 * kStageOut;
+constexpr int kSumSq = 2 * 2 * BM * 4;       // partial sums of squares: accumulator, column half, row
 }  // namespace cv
 
 struct ConvParams {
@@ -69,6 +70,12 @@ struct ConvParams {
   bf16* Y;
   const bf16* resid;            // optional, same addressing as Y
   const float* bias;            // optional [Cout]
+  // optional: the RMS-norm (+ SiLU) that the next convolution's input goes through, of the finished value and in the same epilogue:
+  // Yn = [silu](v / max(||v||, 1e-12) * norm_scale * gamma) over the channels, same addressing as Y. Needs all channels in one N tile.
+  bf16* Yn;
+  const float* gamma;           // [Cout], 16-byte aligned
+  float norm_scale;             // sqrt(Cout)
+  int silu, write_raw;          // write_raw 0: only Yn is stored
 };
 
 template <int RUN>
@@ -89,7 +96,9 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint8_t* stage_out = smem + p.stages * stage_bytes + 256;
-  float* bias_s = reinterpret_cast<float*>(stage_out + 8 * kStageOut);   // [Cout] when Cout <= kBiasMax
+  float* ssq = reinterpret_cast<float*>(stage_out + 8 * kStageOut);      // with a fused norm: sums of squares, then gamma
+  float* gamma_s = ssq + kSumSq / 4;
+  float* bias_s = p.Yn != nullptr ? gamma_s + 256 : ssq;   // [Cout] when Cout <= kBiasMax
 
   // the shuffle makes the warp index (and every role branch below) provably warp-uniform for the compiler
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -113,6 +122,8 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   }
   if (p.bias != nullptr && p.Cout <= kBiasMax)
     for (int i = threadIdx.x; i < p.Cout; i += kThreads) bias_s[i] = p.bias[i];
+  if (p.Yn != nullptr)
+    for (int i = threadIdx.x; i < p.Cout; i += kThreads) gamma_s[i] = p.gamma[i] * p.norm_scale;
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, 512);
     tmem_relinquish_pair();
@@ -277,6 +288,26 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         if (p.resid != nullptr && c_lo < c_hi) fetch(c_lo);
         if (!mbar_wait(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
         tc_fence_after();
+        // this thread's 32 channels of chunk c, staged and stored as 64-byte runs
+        auto emit = [&](bf16* dst, int c, const uint32_t (&a)[32]) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            uint4 o;
+            __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              o2[j] = __floats2bfloat162_rn(__uint_as_float(a[q * 8 + 2 * j]), __uint_as_float(a[q * 8 + 2 * j + 1]));
+            *reinterpret_cast<uint4*>(slot(lane, q)) = o;
+          }
+          __syncwarp();
+          const int n = nt * p.n_tile + c * 32 + piece * 8;
+#pragma unroll
+          for (int it = 0; it < 4; ++it)
+            if (off[it] >= 0 && n < p.Cout && c * 32 + piece * 8 < p.n_tile)
+              *reinterpret_cast<uint4*>(dst + off[it] + n) = *reinterpret_cast<const uint4*>(slot(it * 8 + (lane >> 2), piece));
+          __syncwarp();
+        };
+        float ss = 0.f;
 #pragma unroll 1
         for (int c = c_lo; c < c_hi; ++c) {
           const int n0 = nt * p.n_tile + c * 32;
@@ -284,9 +315,20 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
           tmem_ld32(t_row + c * 32, a);                   // warp-collective; columns past the tile are loaded and not stored
           tmem_ld_wait();
           if (bias != nullptr) {
+            if (n0 + 32 <= p.Cout && bias == bias_s) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (n0 + j < p.Cout) a[j] = __float_as_uint(__uint_as_float(a[j]) + bias[n0 + j]);
+              for (int j = 0; j < 32; j += 4) {
+                const float4 f = *reinterpret_cast<const float4*>(bias_s + n0 + j);
+                a[j] = __float_as_uint(__uint_as_float(a[j]) + f.x);
+                a[j + 1] = __float_as_uint(__uint_as_float(a[j + 1]) + f.y);
+                a[j + 2] = __float_as_uint(__uint_as_float(a[j + 2]) + f.z);
+                a[j + 3] = __float_as_uint(__uint_as_float(a[j + 3]) + f.w);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (n0 + j < p.Cout) a[j] = __float_as_uint(__uint_as_float(a[j]) + bias[n0 + j]);
+            }
           }
           if (p.resid != nullptr) {
             // the sum is rounded once: the residual comes through the staging block to the thread that owns the voxel
@@ -306,22 +348,61 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
               }
             }
           }
+          if (p.Yn != nullptr) {
+            // the finished values go back to TMEM for the second pass
+            if (n0 + 32 <= p.Cout) {
+              float2 s2[4] = {make_float2(ss, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint4 o;
-            __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
+              for (int j = 0; j < 16; ++j) {
+                const float2 v = make_float2(__uint_as_float(a[2 * j]), __uint_as_float(a[2 * j + 1]));
+                s2[j & 3] = fma2(v, v, s2[j & 3]);
+              }
+              const float2 t = add2(add2(s2[0], s2[1]), add2(s2[2], s2[3]));
+              ss = t.x + t.y;
+            } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-              o2[j] = __floats2bfloat162_rn(__uint_as_float(a[q * 8 + 2 * j]), __uint_as_float(a[q * 8 + 2 * j + 1]));
-            *reinterpret_cast<uint4*>(slot(lane, q)) = o;
+              for (int j = 0; j < 32; ++j)
+                if (n0 + j < p.Cout) ss = fmaf(__uint_as_float(a[j]), __uint_as_float(a[j]), ss);
+            }
+            tmem_st32(t_row + c * 32, a);
           }
-          __syncwarp();
-          const int n = n0 + piece * 8;
+          if (p.write_raw) emit(p.Y, c, a);
+        }
+        if (p.Yn != nullptr) {
+          // the two warps of a lane quarter hold half of a voxel's channels each
+          float* mine_s = ssq + (acc * 2 + part) * BM + quarter * 32 + lane;
+          const float* other_s = ssq + (acc * 2 + (part ^ 1)) * BM + quarter * 32 + lane;
+          *mine_s = ss;
+          tmem_st_wait();
+          asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory");
+          const float total = part == 0 ? ss + *other_s : *other_s + ss;
+          const float inv = 1.f / fmaxf(sqrtf(total), 1e-12f);
+#pragma unroll 1
+          for (int c = c_lo; c < c_hi; ++c) {
+            uint32_t a[32];
+            tmem_ld32(t_row + c * 32, a);
+            tmem_ld_wait();
+            const float2 inv2 = make_float2(inv, inv);
 #pragma unroll
-          for (int it = 0; it < 4; ++it)
-            if (off[it] >= 0 && n < p.Cout && c * 32 + piece * 8 < p.n_tile)
-              *reinterpret_cast<uint4*>(p.Y + off[it] + n) = *reinterpret_cast<const uint4*>(slot(it * 8 + (lane >> 2), piece));
-          __syncwarp();
+            for (int j = 0; j < 32; j += 4) {
+              // gamma past the last channel is whatever follows it in shared memory: those columns are not stored
+              const float4 g = *reinterpret_cast<const float4*>(gamma_s + c * 32 + j);
+              const float2 z0 = mul2(mul2(make_float2(__uint_as_float(a[j]), __uint_as_float(a[j + 1])), inv2), make_float2(g.x, g.y));
+              const float2 z1 = mul2(mul2(make_float2(__uint_as_float(a[j + 2]), __uint_as_float(a[j + 3])), inv2), make_float2(g.z, g.w));
+              a[j] = __float_as_uint(z0.x);
+              a[j + 1] = __float_as_uint(z0.y);
+              a[j + 2] = __float_as_uint(z1.x);
+              a[j + 3] = __float_as_uint(z1.y);
+            }
+            if (p.silu) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                const float z = __uint_as_float(a[j]);
+                a[j] = __float_as_uint(__fdividef(z, 1.f + __expf(-z)));
+              }
+            }
+            emit(p.Yn, c, a);
+          }
         }
       } else {
         const long base = offset(quarter * 32 + lane);
@@ -447,7 +528,8 @@ static int launch_conv(cudaLaunchConfig_t& cfg, long tiles, int sms, const CUten
 // out_map: {ot_mul, ot_add, oh_mul, oh_add, ow_mul, ow_add, out_H, out_W, out_C, oc_add}.
 extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Cin, const void* cache, int cache_frames, int pad, int t_stride,
                              int hw_stride, const void* w, int n_rows, int n_tile, int Cout, const int* taps, int ntaps, int T_out, int H_out, int W_out, const int* out_map,
-                             void* y, const void* resid, const float* bias, int* err, int sms, cudaStream_t st) {
+                             void* y, const void* resid, const float* bias, void* y_norm, const float* gamma, int silu, int write_raw,
+                             int* err, int sms, cudaStream_t st) {
   using namespace cv;
   if (Cin % 16 != 0 || Cin < 16 || ntaps < 1 || ntaps > kMaxTaps || n_tile % 16 != 0 || n_tile < 16 || n_tile > 256 ||
       n_rows % n_tile != 0 || Cout > n_rows || Cout < 1 || pad < 0 || pad > 64 || cache_frames < 0 || cache_frames > pad || t_stride < 1 || t_stride > 8 || hw_stride < 1 || hw_stride > 2)
@@ -510,7 +592,7 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
     }
   }
   const int stage_bytes = (TH + run - 1) * TW * BK * 2 + run * n_tile * BK;
-  const int fixed = kSmemFixed + (Cout <= kBiasMax ? (Cout * 4 + 15) / 16 * 16 : 0);
+  const int fixed = kSmemFixed + (Cout <= kBiasMax ? (Cout * 4 + 15) / 16 * 16 : 0) + (y_norm != nullptr ? kSumSq + 256 * 4 : 0);
   p.stages = std::min(kMaxStages, (kSmemMax - fixed) / stage_bytes);
   p.ot_mul = out_map[0];
   p.ot_add = out_map[1];
@@ -525,6 +607,13 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
   p.Y = (bf16*)y;
   p.resid = (const bf16*)resid;
   p.bias = bias;
+  if (y_norm != nullptr && (p.tiles_n != 1 || gamma == nullptr || ((p.out_C | p.oc_add | Cout) & 7) != 0)) return -55;
+  if (y_norm == nullptr && !write_raw) return -55;
+  p.Yn = (bf16*)y_norm;
+  p.gamma = gamma;
+  p.norm_scale = sqrtf((float)Cout);
+  p.silu = silu;
+  p.write_raw = write_raw;
   CUtensorMap tx, tc, tw;
   const uint64_t strides[3] = {(uint64_t)Cin * 2, (uint64_t)W_in * Cin * 2, (uint64_t)H_in * W_in * Cin * 2};
   const uint32_t hw = (uint32_t)hw_stride, box[4] = {BK, TW * hw, (uint32_t)(TH + run - 1) * hw, 1}, step[4] = {1, hw, hw, 1};

@@ -116,7 +116,7 @@ extern "C" {
 // conv3d_cl.cu
 int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Cin, const void* cache, int cache_frames, int pad, int t_stride,
                   int hw_stride, const void* w, int n_rows, int n_tile, int Cout, const int* taps, int ntaps, int T_out, int H_out, int W_out, const int* out_map, void* y, const void* resid,
-                  const float* bias, int* err, int sms, cudaStream_t st);
+                  const float* bias, void* y_norm, const float* gamma, int silu, int write_raw, int* err, int sms, cudaStream_t st);
 // fa_wide.cu
 int cb200_fa_wide(const void* q, long q_row, long q_batch, const void* k, long k_row, long k_batch, const void* v, long v_row, long v_batch,
                   void* o, int B, int Sq, int Skv, float scale, int* err, cudaStream_t st);

@@ -106,6 +106,41 @@ def test_strided_convolutions_match_torch_resample(H, W, C):
         _close(got, want, 3e-2, 2e-2, f"down-sampling, chunk of {T}")
 
 
+# one and several 32-channel chunks per column half, uneven halves; N tiles that are no whole chunks; with and without residual and raw
+# output; the interleaved output of an up-sampling phase
+@pytest.mark.parametrize("Cout", [8, 48, 96, 192, 256])
+@pytest.mark.parametrize("silu,raw,resid", [(True, False, False), (False, True, True), (True, True, False)])
+def test_norm_in_the_epilogue(Cout, silu, raw, resid):
+    from cosmos_predict25_b200.models import vae_wan_cl
+    torch.manual_seed(9)
+    T, H, W, Cin = 2, 11, 20, 64
+    w = (torch.randn(Cout, Cin, 3, 3, 3, device=DEV) / (27 * Cin) ** 0.5).bfloat16().float()
+    b, g = torch.randn(Cout, device=DEV), 1 + 0.2 * torch.randn(Cout, device=DEV)
+    cl = vae_wan_cl.ConvCL(w.permute(0, 2, 3, 4, 1).reshape(Cout, -1, Cin), b, vae_wan_cl._causal3_taps(3, 3, 3), DEV)
+    x = torch.randn(1, Cin, T, H, W, device=DEV).bfloat16()
+    r = torch.randn(T, H, W, Cout, device=DEV).bfloat16() if resid else None
+    y, n = cl.causal(x[0].permute(1, 2, 3, 0).contiguous(), vae_wan_cl._Stream(), resid=r, norm=(g, silu), raw=raw)
+    _no_kernel_error()
+    want = F.conv3d(F.pad(x.float(), (1, 1, 1, 1, 2, 0)), w, b)[0].permute(1, 2, 3, 0) + (r.float() if resid else 0)
+    wn = F.normalize(want, dim=-1) * Cout ** 0.5 * g
+    assert cl.fuses_norm(x) and (y is not None) == raw
+    if raw:
+        _close(y, want, 4e-3, 1e-2, "conv")
+    _close(n, F.silu(wn) if silu else wn, 4e-3, 1e-2, "norm of the conv")
+
+
+def test_norm_behind_upsampling_phases():
+    from cosmos_predict25_b200.models import vae_wan, vae_wan_cl
+    torch.manual_seed(10)
+    mod = vae_wan.Resample(128, "upsample2d").to(DEV)
+    up, g = vae_wan_cl._UpsampleCL(mod, DEV), 1 + 0.2 * torch.randn(64, device=DEV)
+    x = torch.randn(2, 12, 20, 128, device=DEV).bfloat16()
+    y, n = up.run(x, vae_wan_cl._Stream(), None, (g, True))
+    _no_kernel_error()
+    assert torch.equal(y, up(x, vae_wan_cl._Stream()))
+    _close(n, F.silu(F.normalize(y.float(), dim=-1) * 8 * g), 1e-2, 2e-2, "norm")       # the epilogue normalises before y is rounded
+
+
 # queries and keys: below one tile, whole tiles, one row over, an odd and an even number of key tiles; large scores move the reference maximum
 @pytest.mark.parametrize("B,Sq,Skv,gain", [(1, 5, 7, 1.0), (2, 128, 64, 1.0), (1, 129, 65, 4.0), (3, 300, 1000, 8.0), (1, 1024, 1024, 1.0)])
 def test_wide_attention_matches_fp32(B, Sq, Skv, gain):
