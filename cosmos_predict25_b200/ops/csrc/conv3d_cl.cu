@@ -51,7 +51,7 @@ constexpr int kMaxStages = 8;
 constexpr int kStageOut = 32 * 64;            // staging block of an epilogue warp: 32 voxels x 32 channels
 constexpr int kBiasMax = 1024;                // channels whose bias is kept in shared memory
 constexpr int kSmemMax = 227 * 1024, kSmemFixed = 1024 /*alignment slack*/ + 256 /*barriers*/ + 8 * kStageOut;
-constexpr int kSumSq = 2 * 2 * BM * 4;       // partial sums of squares: accumulator, column half, row
+constexpr int kSumSq = 2 * 2 * BM * 4;       // partial sums of squares: buffer, column half, row
 }  // namespace cv
 
 struct ConvParams {
@@ -78,7 +78,10 @@ struct ConvParams {
   int silu, write_raw;          // write_raw 0: only Yn is stored
 };
 
-template <int RUN>
+// STACK = 2 (narrow layers, N tile <= 128): a CTA owns two voxel tiles, one below the other, with an accumulator each; their A box is
+// one of 16 + RUN - 1 rows and every B row in shared memory serves both: 486 instead of 684 KB per 128 voxels of a 3 x 3 x 3
+// convolution with 96 channels. 4 frames of 704 x 1280: 1637 -> 1366 us (1,315 TFLOP/s).
+template <int RUN, int STACK>
 __global__ void __launch_bounds__(cv::kThreads, 1)
 conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_w,
                const __grid_constant__ ConvParams p, int* __restrict__ err) {
@@ -86,7 +89,7 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int b_half = p.n_tile * (BK * 2 / 2);                  // bytes of one tap's B rows in this CTA (half of the N tile)
-  constexpr int a_bytes = (TH + RUN - 1) * TW * BK * 2;
+  constexpr int a_bytes = (TH * STACK + RUN - 1) * TW * BK * 2;
   const int stage_bytes = a_bytes + RUN * b_half;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + p.stages * stage_bytes);
   uint64_t* full = bars;                      // [stages], the even CTA's count the bytes of both
@@ -103,7 +106,7 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   // the shuffle makes the warp index (and every role branch below) provably warp-uniform for the compiler
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
-  const int tiles_w = (p.W_out + TW - 1) / TW, tiles_h = (p.H_out + TH - 1) / TH;
+  const int tiles_w = (p.W_out + TW - 1) / TW, tiles_h = (p.H_out + TH * STACK - 1) / (TH * STACK);
   const int vox_tiles = p.T_out * tiles_h * tiles_w;
   const int n_tiles = (vox_tiles + 1) / 2 * p.tiles_n;         // tiles of the pair: two voxel tiles x one N tile
   const int first_tile = (int)(blockIdx.x >> 1), tile_step = (int)(gridDim.x >> 1);
@@ -143,7 +146,7 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     v = min(v, vox_tiles - 1);
     w0 = (v % tiles_w) * TW;
     v /= tiles_w;
-    h0 = (v % tiles_h) * TH;
+    h0 = (v % tiles_h) * (TH * STACK);
     tf = v / tiles_h;
   };
   // groups whose frame is zero padding for both tiles of the pair are left out: the later tile's frame decides, and the groups
@@ -215,25 +218,25 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
           const int ksteps = (p.Cin - kb * BK) / 16;   // below 4 in the last block of, e.g., C_in = 96: 32 real channels
           // straight-line issue: one warp issues every MMA of the pair, and a narrow MMA (N = 96: 48 clocks) is over before a
           // loop with descriptor arithmetic gets to the next one (64 -> 16 channels, 27 taps: 6.8 us a tile as loops, 4.4 us)
+          auto issue = [&](int j, int k) {
+            const uint64_t db = db_s + (uint32_t)(j * (b_half >> 4) + k * 2);
+#pragma unroll
+            for (int u = 0; u < STACK; ++u)
+              umma_ss_pair_w(d_tmem + u * 128, da_s + (uint32_t)(((u * TH + j) * TW * 128 + k * 32) >> 4), db, idesc, (j | k) ? 1u : first, leader);
+          };
           if (ksteps >= 4) {
 #pragma unroll
             for (int j = 0; j < RUN; ++j)
 #pragma unroll
-              for (int k = 0; k < 4; ++k)
-                umma_ss_pair_w(d_tmem, da_s + (uint32_t)((j * TW * 128 + k * 32) >> 4),
-                               db_s + (uint32_t)(j * (b_half >> 4) + k * 2), idesc, (j | k) ? 1u : first, leader);
+              for (int k = 0; k < 4; ++k) issue(j, k);
           } else if (ksteps == 2) {
 #pragma unroll
             for (int j = 0; j < RUN; ++j)
 #pragma unroll
-              for (int k = 0; k < 2; ++k)
-                umma_ss_pair_w(d_tmem, da_s + (uint32_t)((j * TW * 128 + k * 32) >> 4),
-                               db_s + (uint32_t)(j * (b_half >> 4) + k * 2), idesc, (j | k) ? 1u : first, leader);
+              for (int k = 0; k < 2; ++k) issue(j, k);
           } else {
             for (int j = 0; j < RUN; ++j)
-              for (int k = 0; k < ksteps; ++k)
-                umma_ss_pair_w(d_tmem, da_s + (uint32_t)((j * TW * 128 + k * 32) >> 4),
-                               db_s + (uint32_t)(j * (b_half >> 4) + k * 2), idesc, (j | k) ? 1u : first, leader);
+              for (int k = 0; k < ksteps; ++k) issue(j, k);
           }
           first = 1u;
           umma_commit_pair_w(&empty[s], leader);  // slot reusable in both CTAs once these MMAs have read it
@@ -257,6 +260,7 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     int acc = 0;
     uint32_t acc_ph = 0;
     bool ok = true;
+    int ss_buf = 0;
     const bool vec_ok = ((p.out_C | p.oc_add | p.Cout) & 7) == 0;
     const float* bias = p.bias != nullptr && p.Cout <= kBiasMax ? bias_s : p.bias;
     const uint32_t acc_empty_leader[2] = {mapa_shared(smem_u32(&acc_empty[0]), 0), mapa_shared(smem_u32(&acc_empty[1]), 0)};
@@ -264,13 +268,16 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       int nt, w0, h0, tf;
       bool mine;
       decode(t, nt, w0, h0, tf, mine);
+      bool arrived = false;              // whether the accumulators of this tile have been waited for
+#pragma unroll 1
+      for (int u = 0; u < STACK; ++u, h0 += TH) {
       // element offset of a voxel of the tile (row r = 16 h + w), or -1 outside the frame
       auto offset = [&](int r) -> long {
         const int h = h0 + (r >> 4), w = w0 + (r & 15);
         if (!mine || h >= p.H_out || w >= p.W_out) return -1;
         return (((long)(tf * p.ot_mul + p.ot_add) * p.out_H + (h * p.oh_mul + p.oh_add)) * p.out_W + (w * p.ow_mul + p.ow_add)) * p.out_C + p.oc_add;
       };
-      const uint32_t t_row = tmem_base + acc * 256 + ((uint32_t)(quarter * 32) << 16);
+      const uint32_t t_row = tmem_base + acc * 256 + u * 128 + ((uint32_t)(quarter * 32) << 16);
       if (vec_ok) {
         const int piece = lane & 3;                       // 16-byte piece of the 64-byte run that this lane moves
         long off[4];                                      // voxels quarter * 32 + 8 it + lane / 4
@@ -286,7 +293,8 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
             if (off[it] >= 0 && n < p.Cout) res[it] = *reinterpret_cast<const uint4*>(p.resid + off[it] + n);
         };
         if (p.resid != nullptr && c_lo < c_hi) fetch(c_lo);
-        if (!mbar_wait(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
+        if (!arrived && !mbar_wait(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
+        arrived = true;
         tc_fence_after();
         // this thread's 32 channels of chunk c, staged and stored as 64-byte runs
         auto emit = [&](bf16* dst, int c, const uint32_t (&a)[32]) {
@@ -370,8 +378,9 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         }
         if (p.Yn != nullptr) {
           // the two warps of a lane quarter hold half of a voxel's channels each
-          float* mine_s = ssq + (acc * 2 + part) * BM + quarter * 32 + lane;
-          const float* other_s = ssq + (acc * 2 + (part ^ 1)) * BM + quarter * 32 + lane;
+          float* mine_s = ssq + (ss_buf * 2 + part) * BM + quarter * 32 + lane;
+          const float* other_s = ssq + (ss_buf * 2 + (part ^ 1)) * BM + quarter * 32 + lane;
+          ss_buf ^= 1;                   // two buffers: a warp is at most one tile ahead of its partner
           *mine_s = ss;
           tmem_st_wait();
           asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory");
@@ -406,7 +415,8 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         }
       } else {
         const long base = offset(quarter * 32 + lane);
-        if (!mbar_wait(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
+        if (!arrived && !mbar_wait(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
+        arrived = true;
         tc_fence_after();
 #pragma unroll 1
         for (int c = c_lo; c < c_hi; ++c) {
@@ -426,6 +436,8 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
           }
         }
       }
+      }
+      if (!ok) break;
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(acc_empty_leader[acc]);
@@ -504,10 +516,10 @@ using namespace cb200;
 
 // As in the GEMM: the persistent grid is bounded by the pairs that the GPU can hold at once. One CTA per SM whatever the ring depth
 // (every ring is over half of the shared memory), so the figure for the largest shared-memory size holds for all.
-template <int RUN>
+template <int RUN, int STACK>
 static int launch_conv(cudaLaunchConfig_t& cfg, long tiles, int sms, const CUtensorMap& tx, const CUtensorMap& tc,
                        const CUtensorMap& tw, const ConvParams& p, int* err) {
-  const auto kern = conv_cl_kernel<RUN>;
+  const auto kern = conv_cl_kernel<RUN, STACK>;
   static int max_pairs = 0;
   if (max_pairs == 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cv::kSmemMax);
@@ -591,7 +603,11 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
       break;
     }
   }
-  const int stage_bytes = (TH + run - 1) * TW * BK * 2 + run * n_tile * BK;
+  // two stacked tiles per CTA for narrow layers, unless the frame's last rows would leave more than a fifth of them empty
+  const int rows8 = (H_out + TH - 1) / TH, rows16 = (H_out + 2 * TH - 1) / (2 * TH);
+  const int stack = run == 3 && n_tile <= 128 && rows16 * 10 <= rows8 * 6 ? 2 : 1;
+  const int box_rows = TH * stack + run - 1;
+  const int stage_bytes = box_rows * TW * BK * 2 + run * n_tile * BK;
   const int fixed = kSmemFixed + (Cout <= kBiasMax ? (Cout * 4 + 15) / 16 * 16 : 0) + (y_norm != nullptr ? kSumSq + 256 * 4 : 0);
   p.stages = std::min(kMaxStages, (kSmemMax - fixed) / stage_bytes);
   p.ot_mul = out_map[0];
@@ -616,7 +632,7 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
   p.write_raw = write_raw;
   CUtensorMap tx, tc, tw;
   const uint64_t strides[3] = {(uint64_t)Cin * 2, (uint64_t)W_in * Cin * 2, (uint64_t)H_in * W_in * Cin * 2};
-  const uint32_t hw = (uint32_t)hw_stride, box[4] = {BK, TW * hw, (uint32_t)(TH + run - 1) * hw, 1}, step[4] = {1, hw, hw, 1};
+  const uint32_t hw = (uint32_t)hw_stride, box[4] = {BK, TW * hw, (uint32_t)box_rows * hw, 1}, step[4] = {1, hw, hw, 1};
   {
     const uint64_t dims[4] = {(uint64_t)Cin, (uint64_t)W_in, (uint64_t)H_in, (uint64_t)T_in};
     const int rc = make_tmap_bf16(&tx, x, 4, dims, strides, box, 1, step);
@@ -633,7 +649,7 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
     const int rc = make_tmap_2d_bf16(&tw, w, kdim, (uint64_t)n_rows, kdim * 2, BK, (uint32_t)(n_tile / 2));
     if (rc) return rc;
   }
-  const long vox = (long)T_out * ((H_out + TH - 1) / TH) * ((W_out + TW - 1) / TW);
+  const long vox = (long)T_out * (stack == 2 ? rows16 : rows8) * ((W_out + TW - 1) / TW);
   const long tiles = (vox + 1) / 2 * p.tiles_n;
   if (tiles <= 0 || 2 * tiles > 0x7fffffffL) return -53;
   cudaLaunchConfig_t cfg = {};
@@ -648,9 +664,10 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return run == 3 ? launch_conv<3>(cfg, tiles, sms, tx, tc, tw, p, err)
-       : run == 2 ? launch_conv<2>(cfg, tiles, sms, tx, tc, tw, p, err)
-                  : launch_conv<1>(cfg, tiles, sms, tx, tc, tw, p, err);
+  return stack == 2 ? launch_conv<3, 2>(cfg, tiles, sms, tx, tc, tw, p, err)
+       : run == 3   ? launch_conv<3, 1>(cfg, tiles, sms, tx, tc, tw, p, err)
+       : run == 2   ? launch_conv<2, 1>(cfg, tiles, sms, tx, tc, tw, p, err)
+                    : launch_conv<1, 1>(cfg, tiles, sms, tx, tc, tw, p, err);
 }
 
 extern "C" int cb200_rmsnorm_silu_cl(const void* x, const float* gamma, void* y, long n_vox, int C, int silu, cudaStream_t st) {
