@@ -123,10 +123,6 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     *abort_flag = 0;
     fence_barrier_init();
   }
-  if (p.bias != nullptr && p.Cout <= kBiasMax)
-    for (int i = threadIdx.x; i < p.Cout; i += kThreads) bias_s[i] = p.bias[i];
-  if (p.Yn != nullptr)
-    for (int i = threadIdx.x; i < p.Cout; i += kThreads) gamma_s[i] = p.gamma[i] * p.norm_scale;
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, 512);
     tmem_relinquish_pair();
@@ -136,6 +132,13 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   cluster_sync_all();                         // the other CTA's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();                              // launched with programmatic serialisation (see common.cuh)
+  pdl_wait();
+  if (p.bias != nullptr && p.Cout <= kBiasMax)
+    for (int i = threadIdx.x; i < p.Cout; i += kThreads) bias_s[i] = p.bias[i];
+  if (p.Yn != nullptr)
+    for (int i = threadIdx.x; i < p.Cout; i += kThreads) gamma_s[i] = p.gamma[i] * p.norm_scale;
+  __syncthreads();
 
   // pair tile -> N tile and this CTA's voxel tile (a trailing odd tile is computed by both CTAs and stored by the even one);
   // N tiles of one voxel pair are neighbours so that they run at the same time and share the activation boxes through L2
@@ -467,6 +470,8 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
 template <int G, int NV>
 __global__ void __launch_bounds__(256) rmsnorm_silu_cl_kernel(const bf16* __restrict__ x, const float* __restrict__ gamma,
                                                                 bf16* __restrict__ y, long n_vox, int C, float scale, int silu) {
+  pdl_trigger();                                       // launched with programmatic serialisation (see common.cuh)
+  pdl_wait();
   const int sub = threadIdx.x % G;
   const long v = (long)blockIdx.x * (256 / G) + threadIdx.x / G;
   const bool live = v < n_vox;                         // no early return: the reduction below is warp-wide
@@ -657,13 +662,15 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = (size_t)p.stages * stage_bytes + fixed;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   return stack == 2 ? launch_conv<3, 2>(cfg, tiles, sms, tx, tc, tw, p, err)
        : run == 3   ? launch_conv<3, 1>(cfg, tiles, sms, tx, tc, tw, p, err)
        : run == 2   ? launch_conv<2, 1>(cfg, tiles, sms, tx, tc, tw, p, err)
@@ -675,7 +682,7 @@ extern "C" int cb200_rmsnorm_silu_cl(const void* x, const float* gamma, void* y,
   const float scale = sqrtf((float)C);
   auto run = [&](auto kern, int lanes) {
     const int per_block = 256 / lanes;
-    kern<<<(unsigned)((n_vox + per_block - 1) / per_block), 256, 0, st>>>((const bf16*)x, gamma, (bf16*)y, n_vox, C, scale, silu);
+    launch_pdl(kern, dim3((unsigned)((n_vox + per_block - 1) / per_block)), dim3(256), 0, st, (const bf16*)x, gamma, (bf16*)y, n_vox, C, scale, silu);
   };
   // three pieces per lane while that fills the lanes (C = 96, 192, 384: no idle lane); the widest rows take four
   if (C <= 48) run(rmsnorm_silu_cl_kernel<2, 3>, 2);

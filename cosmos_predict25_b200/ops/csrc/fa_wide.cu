@@ -87,6 +87,8 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();                              // launched with programmatic serialisation (see common.cuh)
+  pdl_wait();
 
   if (warp == 4) {
     // -------------------------------------------------------------------- TMA producer
@@ -314,6 +316,6 @@ extern "C" int cb200_fa_wide(const void* q, long q_row, long q_batch, const void
     if (e != cudaSuccess) return 100 + (int)e;
     attr = true;
   }
-  fa_wide_kernel<<<dim3((Sq + BQ - 1) / BQ, B), kThreads, kSmem, st>>>(tq, tk, tv, (bf16*)o, Sq, Skv, scale * 1.4426950408889634f, err);
-  return (int)cudaGetLastError();
+  return (int)launch_pdl(fa_wide_kernel, dim3((Sq + BQ - 1) / BQ, B), dim3(kThreads), kSmem, st, tq, tk, tv, (bf16*)o, Sq, Skv,
+                         scale * 1.4426950408889634f, err);
 }

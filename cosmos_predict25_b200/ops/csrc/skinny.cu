@@ -147,6 +147,8 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes
 template <int RT, bool KFAST>
 __global__ void __launch_bounds__(kFsThreads) skinny_wide_kernel(SkinnyParams p) {
   using Sh = FsShape<RT, KFAST>;
+  pdl_trigger();                       // launched with programmatic serialisation (see common.cuh)
+  pdl_wait();
   extern __shared__ __align__(16) uint8_t fs_smem[];
   __nv_bfloat16* Ws = reinterpret_cast<__nv_bfloat16*>(fs_smem);
   float* As = reinterpret_cast<float*>(fs_smem + 2 * (size_t)Sh::kW * 2);
@@ -294,8 +296,7 @@ static int launch_skinny_wide(const SkinnyParams& p, int Z, cudaStream_t st) {
   }
   dim3 grid((p.N + kFsN - 1) / kFsN, (p.R + RT - 1) / RT, Z * p.ksplit);
   if (grid.y > 65535) return -1;
-  skinny_wide_kernel<RT, KFAST><<<grid, kFsThreads, Sh::kSmem, st>>>(p);
-  return 0;
+  return (int)launch_pdl(skinny_wide_kernel<RT, KFAST>, grid, dim3(kFsThreads), Sh::kSmem, st, p);
 }
 
 }  // namespace cb200
