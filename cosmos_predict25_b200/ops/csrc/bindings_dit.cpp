@@ -1,9 +1,10 @@
 // The sampling-time path of the DiT in native code: all transformer blocks of a denoising step (and the cross-attention keys / values
-// of all blocks for a prompt) as ONE operator each, which launches the package's kernels back to back. A block is 16 launches;
+// of all blocks for a prompt) as ONE operator each, which launches the package's kernels back to back. A block is 16 launches
+// (14 here: q, k and v are one GEMM over three weights);
 // issued one by one through Python and the dispatcher they cost about 25 us of host time each, more than most of them take on the GPU
 // for an image of 256 x 256 (512 tokens with guidance): 12.9 ms a step, 8.0 ms
-// with this loop (4.2 ms of it host time). The kernels and their order are those of
-// models/dit.py: Block.forward, so the results are the same bits.
+// with this loop (4.2 ms of it host time). The kernels are those of models/dit.py:
+// Block.forward and so are the sums, except where more tiles in a launch change how a contraction is split.
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
@@ -12,6 +13,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <initializer_list>
 #include <vector>
 
 #include "launchers.h"
@@ -55,6 +57,10 @@ struct Launcher {
             const float* gate = nullptr, int64_t ld_gate = 0, int64_t L = 1) const {
     const int rc = cb200_gemm_bf16(a, w, c, (int)M, (int)N, (int)K, 0, 0, nullptr, act, nullptr, resid, gate, ld_gate, (int)L, err, sms, st);
     TORCH_CHECK(rc == 0, "tcgen05 GEMM launch failed with code ", rc);
+  }
+  void gemms(const void* a, std::initializer_list<const void*> w, std::initializer_list<void*> c, int64_t M, int64_t N, int64_t K) const {
+    const int rc = cb200_gemm_bf16_group(a, w.begin(), c.begin(), (int)w.size(), (int)M, (int)N, (int)K, err, sms, st);
+    TORCH_CHECK(rc == 0, "tcgen05 GEMM (several weights) launch failed with code ", rc);
   }
   void attention(const void* q, const void* k, const void* v, void* o, float* lse, int64_t B, int64_t Sq, int64_t Skv, int64_t H) const {
     const int rc = cb200_fa_fwd(q, k, v, o, lse, (int)B, (int)Sq, (int)Skv, (int)H, (float)(1.0 / std::sqrt(128.0)), 0, err, st);
@@ -109,10 +115,8 @@ Tensor dit_blocks(const Tensor& x, const Tensor& mods, const c10::optional<Tenso
     std::swap(nxt, spare);
   };
   std::vector<Tensor> keep;
-  // projection to heads, normalised and rotated; the attention output's place holds the projection meanwhile
-  auto project = [&](const Tensor& wt, const Norm& w, const float* c, const float* s, void* dst) {
-    run.gemm(hp, weight(wt, x, D, D), o, M, D, D);
-    cb200_rmsnorm_rope_fwd(o, w.p, w.bf16, c, s, dst, rn, M * H, (int)S, (int)H, 128, (float)rms_eps, run.st);
+  auto rms = [&](const void* raw, const Norm& w, const float* c, const float* s, void* dst) {
+    cb200_rmsnorm_rope_fwd(raw, w.p, w.bf16, c, s, dst, rn, M * H, (int)S, (int)H, 128, (float)rms_eps, run.st);
   };
   for (int64_t i = 0; i < n; ++i) {
     const Tensor* w = &weights[i * kPerBlock];
@@ -128,13 +132,15 @@ Tensor dit_blocks(const Tensor& x, const Tensor& mods, const c10::optional<Tenso
       step();
     };
     ln(0);
-    run.gemm(hp, weight(w[2], x, D, D), v, M, D, D);
-    project(w[0], norm(w[4], x, keep), cp, sp, q);
-    project(w[1], norm(w[5], x, keep), cp, sp, k);
+    // the attention output's and the next residual stream's places hold the raw projections meanwhile
+    run.gemms(hp, {weight(w[0], x, D, D), weight(w[1], x, D, D), weight(w[2], x, D, D)}, {o, nxt, v}, M, D, D);
+    rms(o, norm(w[4], x, keep), cp, sp, q);
+    rms(nxt, norm(w[5], x, keep), cp, sp, k);
     run.attention(q, k, v, o, lp, B, S, S, H);
     add(0, o, weight(w[3], x, D, D), D);
     ln(1);
-    project(w[6], norm(w[8], x, keep), nullptr, nullptr, q);
+    run.gemm(hp, weight(w[6], x, D, D), o, M, D, D);
+    rms(o, norm(w[8], x, keep), nullptr, nullptr, q);
     run.attention(q, kv[2 * i].data_ptr(), kv[2 * i + 1].data_ptr(), o, lp, B, S, Skv, H);
     add(1, o, weight(w[7], x, D, D), D);
     ln(2);
@@ -165,8 +171,7 @@ std::vector<Tensor> dit_context_kv(const Tensor& context, at::TensorList weights
       rstd = at::empty({M * H}, context.options().dtype(at::kFloat));
       raw = at::empty({M * D}, context.options());
     }
-    run.gemm(context.data_ptr(), weight(weights[3 * i], context, D, C), raw.data_ptr(), M, D, C);
-    run.gemm(context.data_ptr(), weight(weights[3 * i + 1], context, D, C), v.data_ptr(), M, D, C);
+    run.gemms(context.data_ptr(), {weight(weights[3 * i], context, D, C), weight(weights[3 * i + 1], context, D, C)}, {raw.data_ptr(), v.data_ptr()}, M, D, C);
     const Norm w = norm(weights[3 * i + 2], context, keep);
     cb200_rmsnorm_rope_fwd(raw.data_ptr(), w.p, w.bf16, nullptr, nullptr, k.data_ptr(), rstd.data_ptr<float>(), M * H, (int)S, (int)H, 128,
                            (float)rms_eps, run.st);

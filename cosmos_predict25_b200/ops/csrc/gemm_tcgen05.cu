@@ -70,6 +70,10 @@ __device__ __forceinline__ float norm_weight(const HeadScatter& hs, int i) {
 struct GemmEpilogue {
   HeadScatter hs;     // hs.P == 0: disabled
   bf16* C;
+  // up to three products of one A with weights of the same shape [N, K] in one launch (q, k, v; the context's k, v): N tiles
+  // [g tiles, (g + 1) tiles) belong to weight g, whose tensor map is tma_b, tma_b1 or tma_b2 and whose product goes to C, C1 or C2
+  bf16 *C1, *C2;
+  int groups;         // 1 to 3; more than one only without bias, activation, residual and head scatter
   bf16* pre;          // optional second output: the pre-activation (act == 1) or the product before the gated residual
                       // (full 256-column tiles only)
   const bf16* bias;   // optional [N]
@@ -115,7 +119,8 @@ __device__ __forceinline__ void red_release_gpu_add(int* p, int v) {
 // result is deterministic) and put back into TMEM, from where the ordinary epilogue finishes those columns.
 template <int A_MN, int B_MN, bool GATHER, bool CTA2 = false, int SPLIT = 1>
 __global__ void __launch_bounds__(kGemmThreads + (GATHER ? kGatherWarps * 32 : 0), 1)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, int M, int N, int K,
+gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
+                 const __grid_constant__ CUtensorMap tma_b1, const __grid_constant__ CUtensorMap tma_b2, int M, int N, int K,
                  GemmEpilogue ep, GatherB gb, int* __restrict__ err) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -140,7 +145,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 
   // the shuffle makes the warp index (and every role branch below) provably warp-uniform for the compiler
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int tiles_m = (M + TM - 1) / TM, tiles_n = (N + BN - 1) / BN;
+  const int tiles_m = (M + TM - 1) / TM, tiles_g = (N + BN - 1) / BN;
+  const int tiles_n = CTA2 ? tiles_g * ep.groups : tiles_g;      // N tiles of all weights
   const int n_tiles = tiles_m * tiles_n;
   const int k_all = (K + BK - 1) / BK;
   const int kb_first = SPLIT > 1 ? k_all * split / SPLIT : 0, k_blocks = SPLIT > 1 ? k_all * (split + 1) / SPLIT - kb_first : k_all;
@@ -200,7 +206,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       };
       for (int t = first_tile; t < n_tiles && ok; t += tile_step) {
         // with CTA2 this CTA fetches its 128 rows of the pair's A tile and its 128 rows of the B tile
-        const int m0 = (t / tiles_n) * TM + (CTA2 ? (int)pair_rank * BM : 0), n0 = (t % tiles_n) * BN + (CTA2 ? (int)pair_rank * (BN / 2) : 0);
+        const int grp = CTA2 ? t % tiles_n / tiles_g : 0;
+        const CUtensorMap* tb = CTA2 && grp > 0 ? (grp == 1 ? &tma_b1 : &tma_b2) : &tma_b;
+        const int m0 = (t / tiles_n) * TM + (CTA2 ? (int)pair_rank * BM : 0);
+        const int n0 = (t % tiles_n - grp * tiles_g) * BN + (CTA2 ? (int)pair_rank * (BN / 2) : 0);
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (GATHER) {
             // rows of the weight this stage reads: an N tile of 256 rows (forward) or 64 rows of the contraction dimension (dgrad)
@@ -223,10 +232,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
               for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * 8192, &tma_a, bar, m0 + j * 64, k0);
             }
             if (B_MN == 0) {
-              tma_load_2d_pair(sb, &tma_b, bar, k0, n0);
+              tma_load_2d_pair(sb, tb, bar, k0, n0);
             } else {
 #pragma unroll
-              for (int j = 0; j < BN / 128; ++j) tma_load_2d_pair(sb + j * 8192, &tma_b, bar, n0 + j * 64, k0);
+              for (int j = 0; j < BN / 128; ++j) tma_load_2d_pair(sb + j * 8192, tb, bar, n0 + j * 64, k0);
             }
           } else {
             mbar_arrive_expect_tx(&full[s], kStageBytes);
@@ -357,7 +366,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     const uint32_t acc_empty_leader[2] = {CTA2 ? mapa_shared(smem_u32(&acc_empty[0]), lead_rank) : 0u,
                                           CTA2 ? mapa_shared(smem_u32(&acc_empty[1]), lead_rank) : 0u};
     for (int t = first_tile; t < n_tiles && ok; t += tile_step) {
-      const int m0 = (t / tiles_n) * TM + (CTA2 ? (int)pair_rank * BM : 0), n0 = (t % tiles_n) * BN;
+      const int grp = CTA2 ? t % tiles_n / tiles_g : 0;
+      bf16* const out = CTA2 && grp > 0 ? (grp == 1 ? ep.C1 : ep.C2) : ep.C;
+      const int m0 = (t / tiles_n) * TM + (CTA2 ? (int)pair_rank * BM : 0), n0 = (t % tiles_n - grp * tiles_g) * BN;
       ok = mbar_wait(&acc_full[acc], acc_ph, abort_flag);
       if (SPLIT == 1 && !ok) break;
       tc_fence_after();
@@ -642,7 +653,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             }
             stage_chunk(c, v);                                  // in place: a thread only ever touches its own row here
           }
-          write_out(ep.C, colbase);
+          write_out(out, colbase);
         }
         tc_fence_before();
         __syncwarp();
@@ -716,10 +727,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
               __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
               for (int j = 0; j < 4; ++j) o2[j] = __floats2bfloat162_rn(v[q * 8 + 2 * j], v[q * 8 + 2 * j + 1]);
-              *reinterpret_cast<uint4*>(ep.C + off + q * 8) = o;
+              *reinterpret_cast<uint4*>(out + off + q * 8) = o;
             }
           } else {
-            for (int j = 0; j < 32 && col0 + j < N; ++j) ep.C[off + j] = __float2bfloat16(v[j]);
+            for (int j = 0; j < 32 && col0 + j < N; ++j) out[off + j] = __float2bfloat16(v[j]);
           }
         }
       }
@@ -776,22 +787,25 @@ static int launch_gemm(const void* A, const void* B, int M, int N, int K, const 
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   // with a gather every SM takes part (its gather warps work even when it has no tile): the grid is the whole machine
   const int grid = GATHER ? sms : (tiles < sms ? tiles : sms);
-  kern<<<grid, kGemmThreads + (GATHER ? kGatherWarps * 32 : 0), kSmemBytes, st>>>(ta, tb, M, N, K, ep, gb, err);
+  kern<<<grid, kGemmThreads + (GATHER ? kGatherWarps * 32 : 0), kSmemBytes, st>>>(ta, tb, tb, tb, M, N, K, ep, gb, err);
   return (int)cudaGetLastError();
 }
 
 // Same contraction on CTA pairs (template flag CTA2): clusters of two CTAs, one 256 x 256 tile per pair.
 template <int A_MN, int B_MN>
-static int launch_gemm_pair(const void* A, const void* B, int M, int N, int K, const GemmEpilogue& ep, int* err, int sms,
+static int launch_gemm_pair(const void* A, const void* const* B, int M, int N, int K, const GemmEpilogue& ep, int* err, int sms,
                             cudaStream_t st) {
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tb[3];
   int rc;
   if (A_MN == 0) rc = make_tmap_2d_bf16(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, BM);
   else rc = make_tmap_2d_bf16(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)M * 2, 64, BK);
   if (rc) return rc;
-  if (B_MN == 0) rc = make_tmap_2d_bf16(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, BK, BN / 2);   // each CTA loads half the columns
-  else rc = make_tmap_2d_bf16(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)N * 2, 64, BK);
-  if (rc) return rc;
+  for (int g = 0; g < 3; ++g) {
+    const void* w = B[g < ep.groups ? g : 0];
+    if (B_MN == 0) rc = make_tmap_2d_bf16(&tb[g], w, (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, BK, BN / 2);   // each CTA loads half the columns
+    else rc = make_tmap_2d_bf16(&tb[g], w, (uint64_t)N, (uint64_t)K, (uint64_t)N * 2, 64, BK);
+    if (rc) return rc;
+  }
   static bool attr_set = false;
   auto kern = gemm_bf16_kernel<A_MN, B_MN, false, true>;
   if (!attr_set) {
@@ -799,7 +813,7 @@ static int launch_gemm_pair(const void* A, const void* B, int M, int N, int K, c
     if (e != cudaSuccess) return 100 + (int)e;
     attr_set = true;
   }
-  const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
+  const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) * ep.groups;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * (sms / 2));
   cfg.blockDim = dim3(kGemmThreads);
@@ -824,13 +838,13 @@ static int launch_gemm_pair(const void* A, const void* B, int M, int N, int K, c
   }
   const int pairs = std::min(tiles, std::min(max_pairs, sms / 2));
   cfg.gridDim = dim3(2 * pairs);
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, M, N, K, ep, GatherB{}, err);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb[0], tb[1], tb[2], M, N, K, ep, GatherB{}, err);
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
 
 // Split tiles (template flag SPLIT): a cluster of SPLIT pairs per 256 x 256 tile, as many clusters as tiles.
 template <int A_MN, int B_MN, int SPLIT>
-static int launch_gemm_split(const void* A, const void* B, int M, int N, int K, const GemmEpilogue& ep, int* err, cudaStream_t st,
+static int launch_gemm_split(const void* A, const void* const* B, int M, int N, int K, const GemmEpilogue& ep, int* err, cudaStream_t st,
                              int* clusters) {
   auto kern = gemm_bf16_kernel<A_MN, B_MN, false, true, SPLIT>;
   cudaLaunchConfig_t cfg = {};
@@ -859,16 +873,19 @@ static int launch_gemm_split(const void* A, const void* B, int M, int N, int K, 
     *clusters = max_clusters;
     return 0;
   }
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tb[3];
   int rc;
   if (A_MN == 0) rc = make_tmap_2d_bf16(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, BM);
   else rc = make_tmap_2d_bf16(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)M * 2, 64, BK);
   if (rc) return rc;
-  if (B_MN == 0) rc = make_tmap_2d_bf16(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, BK, BN / 2);
-  else rc = make_tmap_2d_bf16(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)N * 2, 64, BK);
-  if (rc) return rc;
-  cfg.gridDim = dim3(2 * SPLIT * ((M + 2 * BM - 1) / (2 * BM)) * (N / BN));
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, M, N, K, ep, GatherB{}, err);
+  for (int g = 0; g < 3; ++g) {
+    const void* w = B[g < ep.groups ? g : 0];
+    if (B_MN == 0) rc = make_tmap_2d_bf16(&tb[g], w, (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, BK, BN / 2);   // each CTA loads half the columns
+    else rc = make_tmap_2d_bf16(&tb[g], w, (uint64_t)N, (uint64_t)K, (uint64_t)N * 2, 64, BK);
+    if (rc) return rc;
+  }
+  cfg.gridDim = dim3(2 * SPLIT * ((M + 2 * BM - 1) / (2 * BM)) * (N / BN) * ep.groups);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb[0], tb[1], tb[2], M, N, K, ep, GatherB{}, err);
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
 
@@ -877,8 +894,8 @@ static int launch_gemm_split(const void* A, const void* B, int M, int N, int K, 
 // against 7.0 us of fixed time, 0.3 us a k-block. 512 x 2048 from K = 2048: 18.7 -> 13.9 us, from K = 8192: 46.9 -> 28; 1024 x 1024 from
 // K = 100,352 (the text projection): 460 -> 241 us.
 template <int A_MN, int B_MN>
-static int launch_gemm_any(const void* A, const void* B, int M, int N, int K, const GemmEpilogue& ep, int* err, int sms, cudaStream_t st) {
-  const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN), kb = (K + BK - 1) / BK;
+static int launch_gemm_any(const void* A, const void* const* B, int M, int N, int K, const GemmEpilogue& ep, int* err, int sms, cudaStream_t st) {
+  const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) * ep.groups, kb = (K + BK - 1) / BK;
   const int pairs = sms / 2;
   if (N % BN == 0 && ep.hs.P == 0 && 2 * tiles <= pairs && kb >= 8) {
     constexpr long kExchange = 6;
@@ -912,6 +929,7 @@ extern "C" int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int
                                int* err, int sms, cudaStream_t st) {
   GemmEpilogue ep{};
   ep.C = (bf16*)C;
+  ep.groups = 1;
   ep.pre = (bf16*)pre;
   ep.bias = (const bf16*)bias;
   ep.resid = (const bf16*)resid;
@@ -920,15 +938,35 @@ extern "C" int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int
   ep.act = act;
   ep.L = L > 0 ? L : 1;
   if (cb200_gemm_pair_mode(-1) == 1 && M >= 2 * BM && N % 8 == 0) {
-    if (a_mn == 0 && b_mn == 0) return launch_gemm_any<0, 0>(A, B, M, N, K, ep, err, sms, st);
-    if (a_mn == 0 && b_mn == 1) return launch_gemm_any<0, 1>(A, B, M, N, K, ep, err, sms, st);
-    if (a_mn == 1 && b_mn == 0) return launch_gemm_any<1, 0>(A, B, M, N, K, ep, err, sms, st);
-    return launch_gemm_any<1, 1>(A, B, M, N, K, ep, err, sms, st);
+    if (a_mn == 0 && b_mn == 0) return launch_gemm_any<0, 0>(A, &B, M, N, K, ep, err, sms, st);
+    if (a_mn == 0 && b_mn == 1) return launch_gemm_any<0, 1>(A, &B, M, N, K, ep, err, sms, st);
+    if (a_mn == 1 && b_mn == 0) return launch_gemm_any<1, 0>(A, &B, M, N, K, ep, err, sms, st);
+    return launch_gemm_any<1, 1>(A, &B, M, N, K, ep, err, sms, st);
   }
   if (a_mn == 0 && b_mn == 0) return launch_gemm<0, 0>(A, B, M, N, K, ep, err, sms, st);
   if (a_mn == 0 && b_mn == 1) return launch_gemm<0, 1>(A, B, M, N, K, ep, err, sms, st);
   if (a_mn == 1 && b_mn == 0) return launch_gemm<1, 0>(A, B, M, N, K, ep, err, sms, st);
   return launch_gemm<1, 1>(A, B, M, N, K, ep, err, sms, st);
+}
+
+// C[g] = A @ B[g]^T for `groups` (1 to 3) weights [N, K] in one launch; fewer than 256 rows: one launch each.
+extern "C" int cb200_gemm_bf16_group(const void* A, const void* const* B, void* const* C, int groups, int M, int N, int K, int* err, int sms,
+                                     cudaStream_t st) {
+  if (groups < 1 || groups > 3 || N % 8 != 0) return -41;
+  if (cb200_gemm_pair_mode(-1) != 1 || M < 2 * BM) {
+    for (int g = 0; g < groups; ++g) {
+      const int rc = cb200_gemm_bf16(A, B[g], C[g], M, N, K, 0, 0, nullptr, 0, nullptr, nullptr, nullptr, 0, 1, err, sms, st);
+      if (rc) return rc;
+    }
+    return 0;
+  }
+  GemmEpilogue ep{};
+  ep.C = (bf16*)C[0];
+  ep.C1 = groups > 1 ? (bf16*)C[1] : nullptr;
+  ep.C2 = groups > 2 ? (bf16*)C[2] : nullptr;
+  ep.groups = groups;
+  ep.L = 1;
+  return launch_gemm_any<0, 0>(A, B, M, N, K, ep, err, sms, st);
 }
 
 // C is not written: row (b, s) of A[M = B*S, K] @ W[N = H*128, K]^T is split into heads, each head is RMS-normalised with
@@ -954,7 +992,8 @@ extern "C" int cb200_gemm_bf16_scatter_heads(const void* A, const void* W, int M
   ep.hs.raw = (bf16*)raw;
   ep.hs.rstd_out = rstd_out;
   ep.L = 1;
-  if (cb200_gemm_pair_mode(-1) == 1 && M >= 2 * BM) return launch_gemm_pair<0, 0>(A, W, M, N, K, ep, err, sms, st);
+  ep.groups = 1;
+  if (cb200_gemm_pair_mode(-1) == 1 && M >= 2 * BM) return launch_gemm_pair<0, 0>(A, &W, M, N, K, ep, err, sms, st);
   return launch_gemm<0, 0>(A, W, M, N, K, ep, err, sms, st);
 }
 
