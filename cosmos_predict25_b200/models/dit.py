@@ -535,7 +535,8 @@ def _native_call_ok(x: torch.Tensor) -> bool:
     glob = torch.nn.modules.module
     return (x.is_cuda and x.dtype == torch.bfloat16 and not torch.is_grad_enabled() and not native.forward_mode() and native.available()
             and ops.settings.gemm == "native" and ops.settings.attention == "native" and torch._C._len_torch_dispatch_stack() == 0
-            and torch._C._len_torch_function_stack() == 0 and not torch.compiler.is_compiling()
+            and torch._C._len_torch_function_stack() == 0 and torch._C._functorch.peek_interpreter_stack() is None
+            and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
             and not glob._global_forward_hooks and not glob._global_forward_pre_hooks)
 
 

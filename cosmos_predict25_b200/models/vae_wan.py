@@ -327,8 +327,11 @@ class WanVAE_(nn.Module):
             outs.append(run(x[:, :, 1 + tw * i: 1 + tw * (i + 1)]))
         if (t - 1) % tw:
             outs.append(run(x[:, :, 1 + tw * n_full:]))
-        if cl is not None and clear_encoder_cache:
-            cl.state = None
+        if cl is not None:
+            if clear_encoder_cache:
+                cl.state = None
+            else:
+                cl.state.compact()
         out = torch.cat(outs, 2)
         mu, _log_var = self.conv1(out).chunk(2, dim=1)
         mean, inv_std = scale
@@ -360,6 +363,8 @@ class WanVAE_(nn.Module):
             if clear_decoder_cache:
                 cl.state = None
                 self._dec_state = None
+            else:
+                cl.state.compact()
             return torch.cat(outs, 2)
         outs = [self.decoder(x[:, :, i: i + 1], st) for i in range(z.shape[2])]
         if clear_decoder_cache:

@@ -207,6 +207,10 @@ class _Stream:
     def __init__(self):
         self.store = {}
 
+    def compact(self):
+        """Copies of the cached frames in place of views that keep whole chunks alive: for a stream that waits for its next call."""
+        self.store = {k: v.clone() if isinstance(v, torch.Tensor) else v for k, v in self.store.items()}
+
 
 def _with_cache(conv: ConvCL, x: torch.Tensor, state: _Stream, pad_frames: int = CACHE_T) -> torch.Tensor:
     """[cache | x] along time and the cache update: the convolution's input tensor with its causal padding in front (tensors that the

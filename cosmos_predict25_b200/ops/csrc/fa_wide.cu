@@ -57,8 +57,8 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   uint64_t* r_empty = r_full + kRing;         // [kRing]
   uint64_t* s_full = r_empty + kRing;         // [2] scores of buffer b ready
   uint64_t* p_ready = s_full + 2;             // [2] probabilities of buffer b written
-  uint64_t* o_done = p_ready + 2;             // [1] P.V of the next key tile complete (one phase per tile)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
+  uint64_t* o_done = p_ready + 2;             // [2] P.V from buffer b complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -74,8 +74,8 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1);
       mbar_init(&p_ready[i], 4);
+      mbar_init(&o_done[i], 1);
     }
-    mbar_init(o_done, 1);
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -160,7 +160,7 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         umma_commit_w(&r_empty[slot], leader);
         advance();
       }
-      if (ok) umma_commit_w(o_done, leader);
+      if (ok) umma_commit_w(&o_done[j & 1], leader);
     }
     if (!ok && lane == 0) { atomicCAS(err, 0, 92); *abort_flag = 1; }
   } else {
@@ -173,9 +173,6 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     for (int j = 0; j < n_kv; ++j) {
       const uint32_t tS = tmem_base + kSCol + (j & 1) * BKV + lane_off;
       if (!mbar_wait(&s_full[j & 1], (j >> 1) & 1, abort_flag)) { ok = false; break; }
-      // P.V of tile j - 2 was issued before these scores: this wait is over at once, and it keeps the thread no more than one
-      // phase behind o_done, which its parity alone could not tell apart
-      if (j > 1 && !mbar_wait(o_done, j & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       uint32_t r[2][32];
       tmem_ld32(tS, r[0]);
@@ -203,8 +200,11 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         l *= alpha;
       }
       if (j > 0 && __any_sync(0xffffffffu, need)) {
-        // rescale this warp's output rows; P.V of the previous tile has to be complete (that of this tile waits for p_ready)
-        if (!mbar_wait(o_done, (j - 1) & 1, abort_flag)) { ok = false; break; }
+        // Rescale this warp's output rows; P.V of the previous tile has to be complete. A parity tells two neighbouring phases apart,
+        // so the barrier must be neither a phase ahead (P.V of tile j + 1, the next on this barrier, needs this warp's probabilities
+        // of tile j first) nor one behind (that of tile j - 3 was complete before the scores of tile j - 1 were begun). One barrier
+        // for all tiles would not do: it can be a phase ahead of a warp that is late, which then waits for itself.
+        if (!mbar_wait(&o_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < D / 32; ++c) {
@@ -238,8 +238,7 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_ready[j & 1]);
     }
-    if (ok && n_kv > 1) ok = mbar_wait(o_done, n_kv & 1, abort_flag);
-    if (ok) ok = mbar_wait(o_done, (n_kv - 1) & 1, abort_flag);
+    if (ok) ok = mbar_wait(&o_done[(n_kv - 1) & 1], ((n_kv - 1) >> 1) & 1, abort_flag);
     if (ok) {
       tc_fence_after();
       const float inv_l = 1.f / l;

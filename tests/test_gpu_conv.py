@@ -141,6 +141,24 @@ def test_norm_behind_upsampling_phases():
     _close(n, F.silu(F.normalize(y.float(), dim=-1) * 8 * g), 1e-2, 2e-2, "norm")       # the epilogue normalises before y is rounded
 
 
+def test_wide_attention_waits_end():
+    """Many launches beside a second stream's traffic, which delays single warps: no bounded wait may run out and every result is the
+    same. (A softmax warp that was late once waited for a phase that only itself could bring about.)"""
+    torch.manual_seed(13)
+    qkv = torch.randn(4, 2000, 3, 384, device=DEV).bfloat16()
+    want = native.load().fa_wide(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], 384 ** -0.5)
+    side, noise = torch.cuda.Stream(), torch.randn(64 << 20, device=DEV)
+    outs = []
+    for i in range(200):
+        with torch.cuda.stream(side):
+            noise.mul_(1.0)
+        outs.append(native.load().fa_wide(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], 384 ** -0.5))
+        if len(outs) == 20:
+            assert all(torch.equal(o, want) for o in outs)
+            outs.clear()
+    _no_kernel_error()
+
+
 # queries and keys: below one tile, whole tiles, one row over, an odd and an even number of key tiles; large scores move the reference maximum
 @pytest.mark.parametrize("B,Sq,Skv,gain", [(1, 5, 7, 1.0), (2, 128, 64, 1.0), (1, 129, 65, 4.0), (3, 300, 1000, 8.0), (1, 1024, 1024, 1.0)])
 def test_wide_attention_matches_fp32(B, Sq, Skv, gain):
@@ -221,3 +239,46 @@ def test_channels_last_encoder_matches_torch_encoder():
     scale = want.abs().mean().item()
     assert err.mean().item() < 0.03 * scale + 1e-3 and err.max().item() < 0.5 * want.abs().max().item() + 0.05, \
         f"mean err {err.mean().item():.4g} (signal {scale:.4g}), max err {err.max().item():.4g}"
+
+
+@pytest.mark.parametrize("step_bytes", [1, 2 << 20, 3 << 29])
+def test_frames_per_step_do_not_change_the_result(step_bytes, monkeypatch):
+    """One latent frame / encoder window per step, a few, and all of them; one call and a stream that goes on over several calls."""
+    from cosmos_predict25_b200.models import vae_wan_cl
+    from cosmos_predict25_b200.models.vae_wan import WanVAE_
+    torch.manual_seed(11)
+    vae = WanVAE_(dim=32, z_dim=16).eval().requires_grad_(False).to(DEV).bfloat16()
+    z = torch.randn(1, 16, 6, 9, 20, device=DEV).bfloat16()
+    x = torch.randn(1, 3, 21, 72, 104, device=DEV).clamp(-1, 1).bfloat16()      # 1 frame and 5 windows
+    one = (0.0, 1.0)
+    want = vae.decode(z, one), vae.encode(x, one)
+    monkeypatch.setattr(vae_wan_cl, "STEP_BYTES", step_bytes)
+    got = vae.decode(z, one), vae.encode(x, one)
+    parts = [vae.decode(z[:, :, :1], one, clear_decoder_cache=False), vae.decode(z[:, :, 1:4], one, clear_decoder_cache=False),
+             vae.decode(z[:, :, 4:], one, clear_decoder_cache=False)]
+    vae.clear_cache()
+    vae._dec_cl.reset()
+    _no_kernel_error()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) and torch.equal(torch.cat(parts, 2), want[0])
+
+
+@pytest.mark.parametrize("H,W,T", [(72, 104, 9), (24, 40, 5), (432, 136, 1)])
+def test_ragged_frames_are_encoded_by_the_kernel(H, W, T):
+    """Frames that halve three times but are no whole tiles, against the torch encoder in fp32 (bounds of the whole-tile test above)."""
+    from cosmos_predict25_b200.models.vae_wan import WanVAE_
+    torch.manual_seed(12)
+    vae = WanVAE_(dim=32, z_dim=16).eval().requires_grad_(False).to(DEV)
+    for p in vae.parameters():
+        p.data = p.data.bfloat16().float()
+    x = torch.randn(1, 3, T, H, W, device=DEV).clamp(-1, 1)
+    F_ops.settings.conv = "cudnn"
+    try:
+        want = vae.encode(x, (0.0, 1.0))
+    finally:
+        F_ops.settings.conv = "native"
+    vae16 = vae.to(torch.bfloat16)
+    got = vae16.encode(x.bfloat16(), (0.0, 1.0))
+    _no_kernel_error()
+    assert getattr(vae16, "_enc_cl", None) is not None and got.shape == want.shape
+    err, scale = (got.float() - want).abs(), want.abs().mean().item()
+    assert err.mean().item() < 0.03 * scale + 1e-3 and err.max().item() < 0.5 * want.abs().max().item() + 0.05
