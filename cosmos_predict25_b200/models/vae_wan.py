@@ -317,16 +317,16 @@ class WanVAE_(nn.Module):
             # channels-last encoder on this package's convolution kernel; it keeps its own stream state
             if clear_encoder_cache or cl.state is None:
                 cl.reset()
-            run = cl.step
-            tw *= cl.windows_per_step(x.shape[-2], x.shape[-1], tw)
+            run, step = cl.step, tw * cl.windows_per_step(x.shape[-2], x.shape[-1], tw)
         else:
-            run = lambda chunk: self.encoder(chunk, st)
+            run, step = lambda chunk: self.encoder(chunk, st), tw
         outs = [run(x[:, :, :1])]
-        n_full = (t - 1) // tw
-        for i in range(n_full):
-            outs.append(run(x[:, :, 1 + tw * i: 1 + tw * (i + 1)]))
-        if (t - 1) % tw:
-            outs.append(run(x[:, :, 1 + tw * n_full:]))
+        # only whole windows share a step: a remainder is a chunk of its own, so that whether its frames pass the temporal down-samplers
+        # (and whether the call is refused) does not depend on how many windows a step takes
+        end = 1 + (t - 1) // tw * tw
+        outs += [run(x[:, :, lo: min(lo + step, end)]) for lo in range(1, end, step)]
+        if end < t:
+            outs.append(run(x[:, :, end:]))
         if cl is not None:
             if clear_encoder_cache:
                 cl.state = None

@@ -1,0 +1,39 @@
+"""How the VAE cuts a clip into streaming steps, with the channels-last encoder replaced by a recorder (host logic only)."""
+
+import pytest
+import torch
+
+from cosmos_predict25_b200.models import vae_wan, vae_wan_cl
+
+
+class _Recorder:
+    """Stands for ``EncoderCL``: the chunks it is given, the real rule for windows per step."""
+
+    def __init__(self, base_channels):
+        self.state, self.chunks = None, []
+        self.conv1 = type("C", (), {"cout": base_channels})
+        self.windows_per_step = lambda *a: vae_wan_cl.EncoderCL.windows_per_step(self, *a)
+
+    def reset(self):
+        self.state = object()
+
+    def step(self, x):
+        self.chunks.append(x.shape[2])
+        return torch.zeros(1, 32, max(1, x.shape[2] // 4), x.shape[3] // 8, x.shape[4] // 8)
+
+
+@pytest.mark.parametrize("frames", [1, 4, 5, 7, 8, 9, 25, 27, 29])
+@pytest.mark.parametrize("windows", [1, 2, 6, 100])
+@pytest.mark.parametrize("window", [4, 8, 6])
+def test_only_whole_windows_share_a_step(frames, windows, window, monkeypatch):
+    vae = vae_wan.WanVAE_(dim=8, z_dim=16, num_res_blocks=1, temporal_window=window).eval()
+    rec = _Recorder(8)
+    monkeypatch.setattr(vae, "_kernel_encoder", lambda x: rec)
+    H, W = 16, 24
+    monkeypatch.setattr(vae_wan_cl, "STEP_BYTES", windows * window * H * W * 8 * 2)
+    with torch.no_grad():
+        vae.encode(torch.zeros(1, 3, frames, H, W), (0.0, 1.0))
+    whole, rest = divmod(frames - 1, window)
+    per_step = windows if window % 4 == 0 else 1
+    want = [1] + [min(per_step, whole - i) * window for i in range(0, whole, per_step)] + ([rest] if rest else [])
+    assert rec.chunks == want

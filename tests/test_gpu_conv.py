@@ -262,6 +262,25 @@ def test_frames_per_step_do_not_change_the_result(step_bytes, monkeypatch):
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) and torch.equal(torch.cat(parts, 2), want[0])
 
 
+@pytest.mark.parametrize("step_bytes", [1, 2 << 20, 3 << 29])
+@pytest.mark.parametrize("frames", [4, 7, 8, 27])
+def test_clip_lengths_with_a_remainder_are_refused(frames, step_bytes, monkeypatch):
+    """A clip is one frame and groups of four; what is left over is refused by the kernel encoder as by the torch one, however many
+    windows a step takes."""
+    from cosmos_predict25_b200.models import vae_wan_cl
+    from cosmos_predict25_b200.models.vae_wan import WanVAE_
+    vae = WanVAE_(dim=32, z_dim=16).eval().requires_grad_(False).to(DEV).bfloat16()
+    x = torch.zeros(1, 3, frames, 72, 104, device=DEV).bfloat16()
+    monkeypatch.setattr(vae_wan_cl, "STEP_BYTES", step_bytes)
+    for conv in ("native", "cudnn"):
+        monkeypatch.setattr(F_ops.settings, "conv", conv)
+        with pytest.raises(RuntimeError):
+            vae.encode(x, (0.0, 1.0))
+    monkeypatch.setattr(F_ops.settings, "conv", "native")
+    assert vae.encode(x[:, :, :1].expand(-1, -1, 9, -1, -1), (0.0, 1.0)).shape == (1, 16, 3, 9, 13)
+    _no_kernel_error()
+
+
 @pytest.mark.parametrize("H,W,T", [(72, 104, 9), (24, 40, 5), (432, 136, 1)])
 def test_ragged_frames_are_encoded_by_the_kernel(H, W, T):
     """Frames that halve three times but are no whole tiles, against the torch encoder in fp32 (bounds of the whole-tile test above)."""
