@@ -96,7 +96,8 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   uint64_t* empty = bars + kMaxStages;        // [stages]
   uint64_t* acc_full = bars + 2 * kMaxStages; // [2]
   uint64_t* acc_empty = acc_full + 2;         // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* sums_in = acc_empty + 2;          // [2][4] sums of squares of a lane quarter's two warps written (buffer, quarter)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sums_in + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint8_t* stage_out = smem + p.stages * stage_bytes + 256;
   float* ssq = reinterpret_cast<float*>(stage_out + 8 * kStageOut);      // with a fused norm: sums of squares, then gamma
@@ -119,6 +120,7 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
       mbar_init(&acc_empty[a], 16);           // the even CTA hears from the epilogue warps of both
+      for (int q = 0; q < 4; ++q) mbar_init(&sums_in[a * 4 + q], 2);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -263,7 +265,7 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     int acc = 0;
     uint32_t acc_ph = 0;
     bool ok = true;
-    int ss_buf = 0;
+    int sums = 0;                        // exchanges of sums of squares so far: buffer sums & 1, phase sums >> 1
     const bool vec_ok = ((p.out_C | p.oc_add | p.Cout) & 7) == 0;
     const float* bias = p.bias != nullptr && p.Cout <= kBiasMax ? bias_s : p.bias;
     const uint32_t acc_empty_leader[2] = {mapa_shared(smem_u32(&acc_empty[0]), 0), mapa_shared(smem_u32(&acc_empty[1]), 0)};
@@ -296,7 +298,7 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
             if (off[it] >= 0 && n < p.Cout) res[it] = *reinterpret_cast<const uint4*>(p.resid + off[it] + n);
         };
         if (p.resid != nullptr && c_lo < c_hi) fetch(c_lo);
-        if (!arrived && !mbar_wait(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
+        if (!arrived && !mbar_wait_warp(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
         arrived = true;
         tc_fence_after();
         // this thread's 32 channels of chunk c, staged and stored as 64-byte runs
@@ -380,13 +382,18 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
           if (p.write_raw) emit(p.Y, c, a);
         }
         if (p.Yn != nullptr) {
-          // the two warps of a lane quarter hold half of a voxel's channels each
+          // the two warps of a lane quarter hold half of a voxel's channels each. Two buffers: a warp is at most one tile ahead of its
+          // partner. The partner may have given up, so this wait is bounded like every other (a named barrier is not)
+          const int ss_buf = sums & 1;
           float* mine_s = ssq + (ss_buf * 2 + part) * BM + quarter * 32 + lane;
           const float* other_s = ssq + (ss_buf * 2 + (part ^ 1)) * BM + quarter * 32 + lane;
-          ss_buf ^= 1;                   // two buffers: a warp is at most one tile ahead of its partner
+          uint64_t* bar = &sums_in[ss_buf * 4 + quarter];
           *mine_s = ss;
           tmem_st_wait();
-          asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar);
+          if (!mbar_wait_warp(bar, (sums >> 1) & 1, abort_flag)) { ok = false; break; }
+          ++sums;
           const float total = part == 0 ? ss + *other_s : *other_s + ss;
           const float inv = 1.f / fmaxf(sqrtf(total), 1e-12f);
 #pragma unroll 1
@@ -418,7 +425,7 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         }
       } else {
         const long base = offset(quarter * 32 + lane);
-        if (!arrived && !mbar_wait(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
+        if (!arrived && !mbar_wait_warp(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
         arrived = true;
         tc_fence_after();
 #pragma unroll 1
