@@ -79,6 +79,7 @@ fa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   uint64_t* done = dq_free + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* left = abort_flag + 1;  // [8] per pair of element-wise warps: one of them has given up
 
   // the shuffle makes the warp index (and every role branch below) provably warp-uniform for the compiler
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -101,6 +102,7 @@ fa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
     mbar_init(done, 1);
     *abort_flag = 0;
+    for (int i = 0; i < 8; ++i) left[i] = 0;
     fence_barrier_init();
   }
   if (warp == kMmaWarp) {
@@ -253,12 +255,22 @@ fa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const int sw = row & 7;
     const int pair_bar = 1 + u * 4 + quarter;       // named barrier of the two warps that share these TMEM lanes
     bool ok = true;
+    // A named barrier has no limit. A warp whose bounded wait runs out says so and still arrives at its pair's next meeting; its partner
+    // sees the word at its next sub-tile, ahead of a meeting to which nobody would come.
+    volatile int* pair_left = left + u * 4 + quarter;
+    auto give_up = [&](bool meets_again) {
+      ok = false;
+      *pair_left = 1;
+      __threadfence_block();
+      if (meets_again) asm volatile("bar.arrive %0, 64;" ::"r"(pair_bar) : "memory");
+    };
     for (int i = u; i < n_q; i += 2) {
+      if (*pair_left) { ok = false; break; }
       const uint32_t par = (i >> 1) & 1;
       const int n = 2 * i;                                  // ring sequence number of Q_i
       const int qslot = n % kRing;
-      if (!mbar_wait(&s_full[u], par, abort_flag)) { ok = false; break; }
-      if (!mbar_wait(&r_full[qslot], (n / kRing) & 1, abort_flag)) { ok = false; break; }  // row statistics landed
+      if (!mbar_wait_warp(&s_full[u], par, abort_flag) ||
+          !mbar_wait_warp(&r_full[qslot], (n / kRing) & 1, abort_flag)) { give_up(true); break; }  // row statistics landed
       tc_fence_after();
       const float4* l4 = reinterpret_cast<const float4*>(sStat + qslot * (kStat / 4)) + half * 8;
       const float4* d4 = l4 + 16;
@@ -305,7 +317,7 @@ fa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       if (lane == 0) mbar_arrive(&p_ready[u]);
 
       // ---- read this warp's half of dQ^T back (lane = d) and add it into the fp32 dQ buffer
-      if (!mbar_wait(&dq_full[u], par, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(&dq_full[u], par, abort_flag)) { give_up(i + 2 < n_q); break; }
       tc_fence_after();
       uint32_t a[32];
       tmem_ld32(tST + 64 + half * 32, a);
@@ -327,7 +339,7 @@ fa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           if (j < n_valid) red_add_f32(qrow + j * HD, __uint_as_float(a[j]));
       }
     }
-    if (ok) ok = mbar_wait(done, 0, abort_flag);
+    if (ok) ok = mbar_wait_warp(done, 0, abort_flag);
     if (ok) {
       tc_fence_after();
       // warps 0-7 write dV, warps 8-15 write dK (scaled); the two warps of a lane quarter take 64 columns each

@@ -88,3 +88,50 @@ def test_exchange_of_sums_between_two_epilogue_warps(bounded):
 def test_convolution_warps_meet_at_bounded_waits():
     """The convolution kernel is the bounded variant of the model above: no named barrier."""
     assert "bar.sync" not in (CSRC / "conv3d_cl.cu").read_text()
+
+
+def _meetings(polite):
+    """The two element-wise warps of a lane quarter in the single-pass attention backward: per query tile a bounded wait, a meeting at a
+    named barrier without a limit, another bounded wait. ``polite``: a warp that gives up leaves a word, which its partner reads at the
+    top of every tile, and still arrives at the pair's next meeting; otherwise it just goes. State: the word, per warp (tile, step),
+    arrivals per warp."""
+    TOP, BEFORE, AT, AFTER, OUT = range(5)
+
+    def successors(s):
+        word, warps, came = s
+        for i in (0, 1):
+            tile, step = warps[i]
+            last = tile + 1 == TILES
+
+            def to(step, tile=tile, word=word, arrive=0):
+                return (word, warps[:i] + ((tile, step),) + warps[i + 1:], came[:i] + (came[i] + arrive,) + came[i + 1:])
+
+            if step == TOP:
+                yield to(OUT if polite and word else BEFORE)
+            elif step == BEFORE:
+                yield to(AT, arrive=1)
+                yield to(OUT, word=1, arrive=int(polite))
+            elif step == AT:
+                if sum(came) >= 2 * (tile + 1):
+                    yield to(AFTER)
+            elif step == AFTER:
+                yield to(OUT) if last else to(TOP, tile=tile + 1)
+                yield to(OUT, word=1, arrive=int(polite and not last))
+
+    return (0, ((0, TOP), (0, TOP)), (0, 0)), successors, OUT
+
+
+@pytest.mark.parametrize("polite", [True, False])
+def test_a_warp_that_gives_up_comes_to_the_next_meeting(polite):
+    start, successors, out = _meetings(polite)
+    _, stuck = explore(start, successors)
+    hung = [s for s in stuck if any(w[1] != out for w in s[1])]
+    assert bool(hung) == (not polite)
+
+
+def test_backward_warps_leave_together():
+    """The attention backward is the polite variant: no wait of its element-wise warps just breaks off in front of a meeting."""
+    code = (CSRC / "fa_bwd_fused.cu").read_text()
+    loop = code[code.index("for (int i = u; i < n_q; i += 2)"):code.index("mbar_wait_warp(done")]
+    assert "bar.sync" in loop and "bar.arrive" in code and loop.count("mbar_wait") == 3
+    assert loop.count("give_up(") == 2 and "mbar_wait(" not in loop
