@@ -172,7 +172,7 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     bool ok = true;
     for (int j = 0; j < n_kv; ++j) {
       const uint32_t tS = tmem_base + kSCol + (j & 1) * BKV + lane_off;
-      if (!mbar_wait(&s_full[j & 1], (j >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(&s_full[j & 1], (j >> 1) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       uint32_t r[2][32];
       tmem_ld32(tS, r[0]);
@@ -204,7 +204,7 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         // so the barrier must be neither a phase ahead (P.V of tile j + 1, the next on this barrier, needs this warp's probabilities
         // of tile j first) nor one behind (that of tile j - 3 was complete before the scores of tile j - 1 were begun). One barrier
         // for all tiles would not do: it can be a phase ahead of a warp that is late, which then waits for itself.
-        if (!mbar_wait(&o_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&o_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < D / 32; ++c) {
@@ -238,7 +238,7 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_ready[j & 1]);
     }
-    if (ok) ok = mbar_wait(&o_done[(n_kv - 1) & 1], ((n_kv - 1) >> 1) & 1, abort_flag);
+    if (ok) ok = mbar_wait_warp(&o_done[(n_kv - 1) & 1], ((n_kv - 1) >> 1) & 1, abort_flag);
     if (ok) {
       tc_fence_after();
       const float inv_l = 1.f / l;

@@ -369,7 +369,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       const int grp = CTA2 ? t % tiles_n / tiles_g : 0;
       bf16* const out = CTA2 && grp > 0 ? (grp == 1 ? ep.C1 : ep.C2) : ep.C;
       const int m0 = (t / tiles_n) * TM + (CTA2 ? (int)pair_rank * BM : 0), n0 = (t % tiles_n - grp * tiles_g) * BN;
-      ok = mbar_wait(&acc_full[acc], acc_ph, abort_flag);
+      ok = mbar_wait_warp(&acc_full[acc], acc_ph, abort_flag);
       if (SPLIT == 1 && !ok) break;
       tc_fence_after();
       const int row = m0 + quarter * 32 + lane;

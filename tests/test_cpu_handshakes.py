@@ -135,3 +135,14 @@ def test_backward_warps_leave_together():
     loop = code[code.index("for (int i = u; i < n_q; i += 2)"):code.index("mbar_wait_warp(done")]
     assert "bar.sync" in loop and "bar.arrive" in code and loop.count("mbar_wait") == 3
     assert loop.count("give_up(") == 2 and "mbar_wait(" not in loop
+
+
+@pytest.mark.parametrize("name", ["conv3d_cl.cu", "fa_wide.cu", "gemm_tcgen05.cu"])
+def test_waits_in_front_of_collective_instructions_are_the_warps(name):
+    """A wait may run out for some lanes of a warp only. Loads from tensor memory and cluster barriers need every lane, so outside the
+    producer, which is one lane, a warp waits as a whole."""
+    code = (CSRC / name).read_text().split(" TMA producer\n")[1]
+    producer, rest = code.split("// ----", 1)
+    assert producer.lstrip().startswith(("if (lane == 0)", "// one thread")) and "mbar_wait(" in producer
+    waits = [line for line in rest.splitlines() if "mbar_wait(" in line]
+    assert all("__all_sync(0xffffffffu, mbar_wait(" in line for line in waits), waits
