@@ -109,7 +109,6 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   const uint32_t rank = cluster_ctarank();
   const int tiles_w = (p.W_out + TW - 1) / TW, tiles_h = (p.H_out + TH * STACK - 1) / (TH * STACK);
   const int vox_tiles = p.T_out * tiles_h * tiles_w;
-  const int n_tiles = (vox_tiles + 1) / 2 * p.tiles_n;         // tiles of the pair: two voxel tiles x one N tile
   const int first_tile = (int)(blockIdx.x >> 1), tile_step = (int)(gridDim.x >> 1);
 
   if (threadIdx.x == 0) {
@@ -140,6 +139,10 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     for (int i = threadIdx.x; i < p.Cout; i += kThreads) bias_s[i] = p.bias[i];
   if (p.Yn != nullptr)
     for (int i = threadIdx.x; i < p.Cout; i += kThreads) gamma_s[i] = p.gamma[i] * p.norm_scale;
+  if (threadIdx.x == 0) *abort_flag = *reinterpret_cast<volatile int*>(err);   // an earlier error: drain the grid at once
+  __syncthreads();
+  // tiles of the pair: two voxel tiles x one N tile; after an earlier error none
+  const int n_tiles = *abort_flag != 0 ? 0 : (vox_tiles + 1) / 2 * p.tiles_n;
   __syncthreads();
 
   // pair tile -> N tile and this CTA's voxel tile (a trailing odd tile is computed by both CTAs and stored by the even one);
@@ -457,7 +460,7 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   }
 
   __syncwarp();
-  if (*abort_flag) {
+  if (*abort_flag && n_tiles > 0) {
     // let outstanding bulk copies / MMAs drain before shared memory and TMEM go away
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
   }

@@ -157,7 +157,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
   // A CTA that starts after another one has reported an error leaves at once (the whole grid then drains in microseconds
   // instead of running every CTA into its own wait limit). One thread reads the word so that the decision is CTA-uniform.
-  // It is read ahead of the wait for the kernel in front: only errors of kernels before that one are sure to be seen.
+  // It is read ahead of the wait for the kernel in front: the CTAs that start beside that kernel look again behind the wait (issuer).
   if (threadIdx.x == 0) *abort_flag = *reinterpret_cast<volatile int*>(err);
   __syncthreads();
   if (*abort_flag != 0) {
@@ -233,7 +233,9 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)); };
       constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 128, 0, 0);
       constexpr uint32_t idesc_pv = umma_idesc_bf16(128, 128, 0, 1);
-      bool ok = wait_all(q_full, 0);
+      // an error of the kernel in front: the other roles hear of it through the abort flag (the load is over before the first tile is in)
+      const bool stopped = *reinterpret_cast<volatile int*>(err) != 0;
+      bool ok = wait_all(q_full, 0) && !stopped;
       const uint64_t dQ_km = umma_desc_sw128(smem_u32(sQ), 16, 1024);          // Q tiles as K-major A
       const uint64_t dR_km = umma_desc_sw128(smem_u32(sR), 16, 1024);          // ring slot as K-major B (K)
       const uint64_t dR_mn = umma_desc_sw128(smem_u32(sR), kHalfBytes, 1024);  // ring slot as N-major B (V)

@@ -89,8 +89,13 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();                              // launched with programmatic serialisation (see common.cuh)
   pdl_wait();
+  if (threadIdx.x == 0) *abort_flag = *reinterpret_cast<volatile int*>(err);   // an earlier error: drain the grid at once
+  __syncthreads();
+  const bool stopped = *abort_flag != 0;
+  __syncthreads();
 
-  if (warp == 4) {
+  if (stopped) {
+  } else if (warp == 4) {
     // -------------------------------------------------------------------- TMA producer
     if (lane == 0) {
       prefetch_tmap(&tm_q);
@@ -278,7 +283,7 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   }
 
   __syncwarp();
-  if (*abort_flag) {
+  if (*abort_flag && !stopped) {
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
   }
   tc_fence_before();
