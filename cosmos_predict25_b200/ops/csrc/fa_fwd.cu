@@ -151,8 +151,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int h = blockIdx.y, b = blockIdx.z;
   const int q_base = blockIdx.x * QT * BQ;
-  const int n_kv = NA ? na.kv_cnt[blockIdx.x] : (Skv + BKV - 1) / BKV;
-  const int* kv_list = NA ? na.kv_idx + (size_t)blockIdx.x * na.max_n : nullptr;
   constexpr uint32_t kOBase = QT * 128;    // TMEM: S_t at t * 128, O_t at kOBase + t * 128
 
   // A CTA that starts after another one has reported an error leaves at once (the whole grid then drains in microseconds
@@ -189,6 +187,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();                     // launched with programmatic serialisation (see common.cuh)
   pdl_wait();
+  const int n_kv = NA ? na.kv_cnt[blockIdx.x] : (Skv + BKV - 1) / BKV;
+  const int* kv_list = NA ? na.kv_idx + (size_t)blockIdx.x * na.max_n : nullptr;
 
   // With REGS every role branch starts by re-dividing the registers of its warpgroup (the instruction has to sit inside the
   // branch: the compiler takes the smallest limit that reaches a join point as the limit of everything after it).

@@ -2,6 +2,7 @@
 
 import itertools
 import pathlib
+import re
 
 import pytest
 
@@ -146,3 +147,31 @@ def test_waits_in_front_of_collective_instructions_are_the_warps(name):
     assert producer.lstrip().startswith(("if (lane == 0)", "// one thread")) and "mbar_wait(" in producer
     waits = [line for line in rest.splitlines() if "mbar_wait(" in line]
     assert all("__all_sync(0xffffffffu, mbar_wait(" in line for line in waits), waits
+
+
+def _early_kernels():
+    """(name, parameters, body up to the wait) of every kernel that may start beside the kernel in front of it."""
+    for path in sorted(CSRC.glob("*.cu")):
+        for part in re.split(r"\n__global__ ", path.read_text())[1:]:
+            part = part.split("\n}\n")[0]
+            if "pdl_wait();" in part:
+                head, body = part.split(") {\n", 1)
+                name, params = re.search(r"(\w+_kernel)\((.*)$", head, re.S).groups()
+                yield name, params, body[:body.rindex("pdl_wait();")]
+
+
+def test_kernels_read_no_memory_ahead_of_their_wait():
+    """What the kernel in front writes is visible behind ``pdl_wait()`` only. Ahead of it a kernel touches no memory that its parameters
+    point to, except the device's error word."""
+    kernels = list(_early_kernels())
+    assert len(kernels) >= 6
+    for name, params, ahead in kernels:
+        for p in params.split(","):
+            var = re.search(r"(\w+)\s*$", p).group(1)
+            if var == "err" or "CUtensorMap" in p:
+                continue
+            struct = "*" not in p and re.search(r"\b[A-Z]\w+ (?:p|ep|gb|sc|na)\s*$", p)
+            if "*" in p or struct:
+                reads = rf"\b{var}\.\w+\s*\[" if struct else rf"\b{var}\s*\[|\*\s*{var}\b|\({var}\s*\+"
+                hit = re.search(reads, ahead)
+                assert hit is None, f"{name} reads {var} ahead of the wait: {hit.group(0)}"
