@@ -327,11 +327,8 @@ class WanVAE_(nn.Module):
         outs += [run(x[:, :, lo: min(lo + step, end)]) for lo in range(1, end, step)]
         if end < t:
             outs.append(run(x[:, :, end:]))
-        if cl is not None:
-            if clear_encoder_cache:
-                cl.state = None
-            else:
-                cl.state.compact()
+        if cl is not None and clear_encoder_cache:
+            cl.state = None
         out = torch.cat(outs, 2)
         mu, _log_var = self.conv1(out).chunk(2, dim=1)
         mean, inv_std = scale
@@ -363,8 +360,6 @@ class WanVAE_(nn.Module):
             if clear_decoder_cache:
                 cl.state = None
                 self._dec_state = None
-            else:
-                cl.state.compact()
             return torch.cat(outs, 2)
         outs = [self.decoder(x[:, :, i: i + 1], st) for i in range(z.shape[2])]
         if clear_decoder_cache:

@@ -130,11 +130,11 @@ class ConvCL:
 
 
 def _last_frames(prev: Optional[torch.Tensor], x: torch.Tensor, n: int) -> torch.Tensor:
-    """The last ``n`` frames of [prev | x], or fewer when the stream has not seen as many. A view of ``x`` where that is enough: the
-    stream keeps the chunk's tensor alive instead of copying frames out of it."""
-    if x.shape[0] >= n or prev is None:
-        return x[-n:]
-    return torch.cat([prev, x], 0)[-n:]
+    """The last ``n`` frames of [prev | x], or fewer when the stream has not seen as many. Copied out of a longer chunk: the stream has one
+    such tensor per causal convolution, and a view would keep every chunk of the step alive until the next one."""
+    if x.shape[0] > n:
+        return x[-n:].clone()
+    return x if x.shape[0] == n or prev is None else torch.cat([prev[x.shape[0] - n:], x], 0)
 
 
 def _causal3_taps(kt: int, kh: int, kw: int):
@@ -206,10 +206,6 @@ class _Stream:
 
     def __init__(self):
         self.store = {}
-
-    def compact(self):
-        """Copies of the cached frames in place of views that keep whole chunks alive: for a stream that waits for its next call."""
-        self.store = {k: v.clone() if isinstance(v, torch.Tensor) else v for k, v in self.store.items()}
 
 
 def _with_cache(conv: ConvCL, x: torch.Tensor, state: _Stream, pad_frames: int = CACHE_T) -> torch.Tensor:

@@ -37,3 +37,17 @@ def test_only_whole_windows_share_a_step(frames, windows, window, monkeypatch):
     per_step = windows if window % 4 == 0 else 1
     want = [1] + [min(per_step, whole - i) * window for i in range(0, whole, per_step)] + ([rest] if rest else [])
     assert rec.chunks == want
+
+
+@pytest.mark.parametrize("n", [1, 2])
+@pytest.mark.parametrize("chunks", [(1, 8, 8), (1, 1, 1, 3), (4,), (2, 1), (1, 2)])
+def test_stream_keeps_the_last_frames_only(n, chunks):
+    """What a causal convolution carries to the next chunk: at most its ``n`` last input frames, in storage of that size."""
+    frames = torch.randn(sum(chunks), 3, 5, 4)
+    prev, lo = None, 0
+    for T in chunks:
+        x = frames[lo:lo + T].clone()
+        lo += T
+        prev = vae_wan_cl._last_frames(prev, x, n)
+        assert torch.equal(prev, frames[max(0, lo - n):lo]) and prev.is_contiguous()
+        assert prev.untyped_storage().nbytes() <= n * frames[0].numel() * 4
