@@ -860,13 +860,16 @@ static int launch_gemm_split(const void* A, const void* const* B, int M, int N, 
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.numAttrs = 2;
-  static int max_clusters = 0;       // clusters that the GPU holds at once
-  if (max_clusters == 0) {
+  static int max_clusters = -1;      // clusters that the GPU holds at once; none where it has no room for one (a share of a GPU)
+  if (max_clusters < 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
     if (e != cudaSuccess) return 100 + (int)e;
     int n = 0;
     cfg.gridDim = dim3(2 * SPLIT);
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) return 600;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
     max_clusters = n;
   }
   if (clusters != nullptr) {         // only asked for the capacity
@@ -892,20 +895,33 @@ static int launch_gemm_split(const void* A, const void* const* B, int M, int N, 
 // One tile per pair, or clusters of 2 or 4 pairs per tile: whichever takes fewer k-blocks in a row, waves counted, with kExchange
 // k-blocks' time for the exchange of partial tiles. Six k-blocks: measured 9.1 us
 // against 7.0 us of fixed time, 0.3 us a k-block. 512 x 2048 from K = 2048: 18.7 -> 13.9 us, from K = 8192: 46.9 -> 28; 1024 x 1024 from
-// K = 100,352 (the text projection): 460 -> 241 us.
+// K = 100,352 (the text projection): 460 -> 241 us. `c2`, `c4`: clusters of 2 and 4 pairs that the GPU holds at once; where it holds
+// none the split is not taken.
+extern "C" int cb200_gemm_pairs_per_tile(long tiles, long kb, int pairs, int c2, int c4) {
+  if (2 * tiles > pairs || kb < 8) return 1;
+  constexpr long kExchange = 6;
+  long best = kb;
+  int split = 1;
+  if (c2 > 0 && (tiles + c2 - 1) / c2 * ((kb + 1) / 2 + kExchange) < best) {
+    best = (tiles + c2 - 1) / c2 * ((kb + 1) / 2 + kExchange);
+    split = 2;
+  }
+  if (c4 > 0 && (tiles + c4 - 1) / c4 * ((kb + 3) / 4 + kExchange) < best + (split == 2 ? 1 : 0)) split = 4;
+  return split;
+}
+
 template <int A_MN, int B_MN>
 static int launch_gemm_any(const void* A, const void* const* B, int M, int N, int K, const GemmEpilogue& ep, int* err, int sms, cudaStream_t st) {
   const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) * ep.groups, kb = (K + BK - 1) / BK;
   const int pairs = sms / 2;
-  if (N % BN == 0 && ep.hs.P == 0 && 2 * tiles <= pairs && kb >= 8) {
-    constexpr long kExchange = 6;
+  if (N % BN == 0 && ep.hs.P == 0 && 2 * tiles <= pairs) {
     int c2 = 0, c4 = 0;
     int rc = launch_gemm_split<A_MN, B_MN, 2>(A, B, M, N, K, ep, err, st, &c2);
     if (rc) return rc;
     if ((rc = launch_gemm_split<A_MN, B_MN, 4>(A, B, M, N, K, ep, err, st, &c4))) return rc;
-    const long t1 = kb, t2 = ((tiles + c2 - 1) / c2) * ((kb + 1) / 2 + kExchange), t4 = ((tiles + c4 - 1) / c4) * ((kb + 3) / 4 + kExchange);
-    if (t4 < t1 && t4 <= t2) return launch_gemm_split<A_MN, B_MN, 4>(A, B, M, N, K, ep, err, st, nullptr);
-    if (t2 < t1) return launch_gemm_split<A_MN, B_MN, 2>(A, B, M, N, K, ep, err, st, nullptr);
+    const int split = cb200_gemm_pairs_per_tile(tiles, kb, pairs, c2, c4);
+    if (split == 4) return launch_gemm_split<A_MN, B_MN, 4>(A, B, M, N, K, ep, err, st, nullptr);
+    if (split == 2) return launch_gemm_split<A_MN, B_MN, 2>(A, B, M, N, K, ep, err, st, nullptr);
   }
   return launch_gemm_pair<A_MN, B_MN>(A, B, M, N, K, ep, err, sms, st);
 }
