@@ -27,10 +27,15 @@ inline void check_f32(const Tensor& t, const char* name) {
   TORCH_CHECK(t.is_contiguous(), name, " must be contiguous");
 }
 
-// Rows of a per-frame modulation vector ([frames, D] fp32, e.g. a third of the columns of the modulation MLPs' output) as the
-// kernels read them: 16-byte aligned rows of any stride; anything else is copied.
-inline Tensor mod_rows(const Tensor& t, const char* name) {
-  TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kFloat && t.dim() == 2, name, " must be a 2-D float32 CUDA tensor");
+// Rows of a per-frame modulation vector (fp32 [frames, D], e.g. a third of the columns of the modulation MLPs' output) as the
+// kernels read them: 16-byte aligned rows of any stride; others are copied. Any contiguous tensor of such rows serves too.
+inline Tensor mod_rows(const Tensor& t, int64_t D, const char* name) {
+  TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kFloat, name, " must be a float32 CUDA tensor");
+  TORCH_CHECK(D > 0, "channel dim must not be empty");
+  if (t.dim() != 2 || t.size(1) != D) {
+    TORCH_CHECK(t.is_contiguous() && t.numel() % D == 0, name, " must be contiguous rows of the channel count");
+    return mod_rows(t.view({-1, D}), D, name);
+  }
   const bool ok = t.stride(1) == 1 && t.stride(0) % 4 == 0 && t.stride(0) >= 0 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
   return ok ? t : t.clone(at::MemoryFormat::Contiguous);
 }
@@ -65,10 +70,10 @@ std::tuple<Tensor, Tensor, Tensor> ln_modulate_fwd(const Tensor& x, const Tensor
                                                    double eps) {
   check_bf16(x, "x");
   c10::cuda::CUDAGuard g(x.device());
-  const Tensor sh = mod_rows(shift, "shift"), sc = mod_rows(scale, "scale");
   const int64_t rows = x.size(0), D = x.size(1);
+  const Tensor sh = mod_rows(shift, D, "shift"), sc = mod_rows(scale, D, "scale");
   TORCH_CHECK(D % 8 == 0 && D <= 8192, "channel dim must be a multiple of 8 and <= 8192");
-  TORCH_CHECK(rows % L == 0 && shift.size(0) == rows / L && shift.size(1) == D && scale.sizes() == shift.sizes(), "shift/scale must be [rows/L, D]");
+  TORCH_CHECK(rows % L == 0 && shift.size(0) == rows / L && shift.size(1) == D && sc.size(0) >= rows / L, "shift/scale must be [rows/L, D]");
   Tensor y = at::empty_like(x);
   Tensor mean = at::empty({rows}, x.options().dtype(at::kFloat));
   Tensor rstd = at::empty({rows}, x.options().dtype(at::kFloat));
@@ -82,8 +87,9 @@ std::tuple<Tensor, Tensor, Tensor> ln_modulate_bwd(const Tensor& dy, const Tenso
   check_bf16(dy, "dy");
   check_bf16(x, "x");
   c10::cuda::CUDAGuard g(x.device());
-  const Tensor sc = mod_rows(scale, "scale");
   const int64_t rows = x.size(0), D = x.size(1), frames = rows / L;
+  const Tensor sc = mod_rows(scale, D, "scale");
+  TORCH_CHECK(sc.size(0) >= frames, "scale must be [rows/L, D]");
   Tensor dx = at::empty_like(x);
   Tensor dshift = at::empty({frames, D}, scale.options());
   Tensor dscale = at::empty({frames, D}, scale.options());
@@ -99,8 +105,8 @@ Tensor gate_residual_fwd(const Tensor& x, const Tensor& gate, const Tensor& y, i
   check_bf16(x, "x");
   check_bf16(y, "y");
   c10::cuda::CUDAGuard g(x.device());
-  const Tensor gt = mod_rows(gate, "gate");
   const int64_t rows = x.size(0), D = x.size(1);
+  const Tensor gt = mod_rows(gate, D, "gate");
   TORCH_CHECK(D % 8 == 0 && gate.size(0) == rows / L && gate.size(1) == D, "gate must be [rows/L, D]");
   Tensor out = at::empty_like(x);
   cb200_gate_residual_fwd(x.data_ptr(), gt.data_ptr<float>(), y.data_ptr(), out.data_ptr(), rows, (int)D, (int)L, gt.stride(0), stream());
@@ -111,8 +117,9 @@ std::tuple<Tensor, Tensor> gate_residual_bwd(const Tensor& dout, const Tensor& g
   check_bf16(dout, "dout");
   check_bf16(y, "y");
   c10::cuda::CUDAGuard g(y.device());
-  const Tensor gt = mod_rows(gate, "gate");
   const int64_t rows = y.size(0), D = y.size(1), frames = rows / L;
+  const Tensor gt = mod_rows(gate, D, "gate");
+  TORCH_CHECK(gt.size(0) >= frames, "gate must be [rows/L, D]");
   TORCH_CHECK(D <= 8192, "channel dim must be <= 8192");
   Tensor dy = at::empty_like(y);
   Tensor dgate = at::empty({frames, D}, gate.options());
@@ -345,7 +352,7 @@ Tensor gemm_impl(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& 
   long ld_gate = 0;
   if (resid != nullptr) {
     check_bf16(*resid, "resid");
-    gate_c = mod_rows(*gate, "gate");
+    gate_c = mod_rows(*gate, d.N, "gate");
     ld_gate = gate_c.stride(0);
     TORCH_CHECK(resid->numel() == (int64_t)d.M * d.N && gate->size(-1) == d.N && gate->numel() == (d.M / L) * (int64_t)d.N,
                 "gated-residual epilogue shapes");

@@ -49,6 +49,33 @@ def test_gated_gemm_epilogue_reads_strided_gates():
     assert _max_rel(got, want) < 1.5 * 2.0 ** -9
 
 
+def test_row_operators_take_modulation_rows_of_any_shape():
+    """[frames, D] as [B, T, D], as one flat row and as a strided slice are the same rows; rows that are too few are refused."""
+    torch.manual_seed(4)
+    ops = native.load()
+    B, T, L, D, K = 2, 3, 8, 256, 64
+    x, y = (torch.randn(B * T * L, D, device=DEV).bfloat16() for _ in range(2))
+    h, w = torch.randn(B * T * L, K, device=DEV).bfloat16(), torch.randn(D, K, device=DEV).bfloat16()
+    rows = torch.randn(B * T, D, device=DEV)
+    mean, rstd = ops.ln_modulate_fwd(x, rows, rows, L, 1e-6)[1:]
+    calls = {
+        "gated GEMM": lambda g: ops.gemm_bf16_gate_residual(h, w, x, g, L),
+        "gate": lambda g: ops.gate_residual_bwd(y, g, x, L)[0],
+        "LN": lambda g: ops.ln_modulate_fwd(x, rows, g, L, 1e-6)[0],
+        "LN backward": lambda g: ops.ln_modulate_bwd(y, x, mean, rstd, g, L)[0],
+    }
+    wide = torch.cat([rows, rows, rows], 1)
+    for name, call in calls.items():
+        want = call(rows)
+        for form in (rows.view(B, T, D), rows.view(-1), wide[:, D:2 * D]):
+            if form.dim() != 1 or name != "gated GEMM":          # the epilogue wants D in the last dimension
+                assert torch.equal(call(form), want), (name, form.shape)
+        with pytest.raises(RuntimeError):
+            call(rows[:-1])
+    flat = rows[0]                                                # one frame: a plain [D] vector
+    assert torch.equal(ops.gemm_bf16_gate_residual(h, w, x, flat, B * T * L), ops.gemm_bf16_gate_residual(h, w, x, flat[None], B * T * L))
+
+
 @pytest.mark.parametrize("HD,H,S,B", [(128, 5, 7, 2), (128, 16, 33, 1), (64, 3, 130, 2), (128, 40, 3, 1), (64, 1, 1, 1)])
 @pytest.mark.parametrize("wdtype", [torch.bfloat16, torch.float32])
 def test_rmsnorm_rope_head_counts(HD, H, S, B, wdtype):
