@@ -295,7 +295,6 @@ static int launch_skinny_wide(const SkinnyParams& p, int Z, cudaStream_t st) {
     attr = true;
   }
   dim3 grid((p.N + kFsN - 1) / kFsN, (p.R + RT - 1) / RT, Z * p.ksplit);
-  if (grid.y > 65535) return -1;
   return (int)launch_pdl(skinny_wide_kernel<RT, KFAST>, grid, dim3(kFsThreads), Sh::kSmem, st, p);
 }
 
@@ -316,7 +315,8 @@ extern "C" int cb200_skinny_bgemm(const float* a, long a_z, long a_r, long a_k, 
   if (Z <= 0 || R <= 0 || N <= 0 || K <= 0) return 0;
   if (ksplit < 1 || (long)Z * ksplit > 65535 || (R + kSkTile - 1) / kSkTile > 65535) return -1;
   SkinnyParams p{a, a_z, a_r, a_k, b_ptrs, b_base, b_z, b_n, b_k, c, c_z, ldc, add, ld_add, add_cols, R, N, K, silu_a, silu_b, ksplit};
-  if (cb200_skinny_wide(a_k, b_n, b_k, b_is_bf16, c_is_bf16, silu_b, N, K)) {
+  // (row tiles of 48 reach the grid's limit before those of 64)
+  if (cb200_skinny_wide(a_k, b_n, b_k, b_is_bf16, c_is_bf16, silu_b, N, K) && (R + 47) / 48 <= 65535) {
     // rows per CTA: the smallest that holds them all; with several row tiles the weights are read again from L2
     if (b_k == 1)
       return R <= 4 ? launch_skinny_wide<4, true>(p, Z, st) : R <= 16 ? launch_skinny_wide<16, true>(p, Z, st)

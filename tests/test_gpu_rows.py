@@ -119,3 +119,13 @@ def test_few_row_gemm_tiles(R, K, N, Z):
         da = F_ops._skinny_call(native.load(), Z, R, K, N, dout, R * N, N, 1, F_ops._ptr_table(ws), None, 0, 1, K, True, None, 0, Z, R, K, N,
                                 False, False, False)
         assert _max_rel(da, dout.double() @ torch.stack(ws).double()) < 1e-6
+
+
+def test_few_row_gemm_takes_as_many_rows_as_its_widest_tile():
+    """More rows than the 48-row tiles of the wide kernel can address go to the 64-row tile."""
+    R, K, N = 48 * 65535 + 5, 8, 8
+    torch.manual_seed(5)
+    a, w = torch.randn(R, K, device=DEV), torch.randn(N, K, device=DEV).bfloat16()
+    got = F_ops.skinny_linears(a, [w])
+    want = a.double() @ w.double().t()
+    assert _max_rel(got[0], want) < 1e-6
