@@ -716,7 +716,7 @@ class CosmosDiT(nn.Module):
         if not weights:
             return None
         kv = native.load().dit_context_kv(ctx, weights, eps)
-        native.count_launch((2 if ctx.shape[0] * ctx.shape[1] >= 256 else 3) * len(self.blocks))
+        native.count_launch((1 + native.load().gemm_group_launches(ctx.shape[0] * ctx.shape[1], 2)) * len(self.blocks))
         return list(zip(kv[0::2], kv[1::2]))
 
     def _embed(self, x_B_C_T_H_W, condition_mask, padding_mask):
@@ -800,7 +800,7 @@ class CosmosDiT(nn.Module):
             weights, kvs, eps = plain
             cos, sin = rope.cos_sin() if rope is not None else (None, None)
             x = native.load().dit_blocks(x.contiguous(), all_mods, cos, sin, weights, kvs, 1e-6, eps)
-            native.count_launch((14 if B * T * H * W >= 256 else 16) * len(self.blocks))
+            native.count_launch((13 + native.load().gemm_group_launches(B * T * H * W, 3)) * len(self.blocks))
         for i, block in enumerate(self.blocks if plain is None else ()):
             kv = cross_kv[i] if cross_kv else None
             mods = None if all_mods is None else all_mods[3 * i: 3 * i + 3]

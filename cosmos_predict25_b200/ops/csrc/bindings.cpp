@@ -597,6 +597,8 @@ TORCH_LIBRARY(cosmos_b200, m) {
         [](int64_t tiles, int64_t kb, int64_t pairs, int64_t c2, int64_t c4) {
           return (int64_t)cb200_gemm_pairs_per_tile((long)tiles, (long)kb, (int)pairs, (int)c2, (int)c4);
         });
+  m.def("gemm_group_launches(int rows, int groups) -> int",
+        [](int64_t rows, int64_t groups) { return (int64_t)cb200_gemm_group_launches((int)rows, (int)groups); });
   m.def("gemm_pair_mode(int mode) -> int", &gemm_pair_mode);
   m.def("kernel_error(int device, bool clear) -> int", &kernel_error);
   register_attention_ops(m);

@@ -965,11 +965,14 @@ extern "C" int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int
   return launch_gemm<1, 1>(A, B, M, N, K, ep, err, sms, st);
 }
 
+// launches of cb200_gemm_bf16_group: one, or one for each weight where there is no CTA-pair tile
+extern "C" int cb200_gemm_group_launches(int M, int groups) { return cb200_gemm_pair_mode(-1) == 1 && M >= 2 * BM ? 1 : groups; }
+
 // C[g] = A @ B[g]^T for `groups` (1 to 3) weights [N, K] in one launch; fewer than 256 rows: one launch each.
 extern "C" int cb200_gemm_bf16_group(const void* A, const void* const* B, void* const* C, int groups, int M, int N, int K, int* err, int sms,
                                      cudaStream_t st) {
   if (groups < 1 || groups > 3 || N % 8 != 0) return -41;
-  if (cb200_gemm_pair_mode(-1) != 1 || M < 2 * BM) {
+  if (cb200_gemm_group_launches(M, 2) > 1) {
     for (int g = 0; g < groups; ++g) {
       const int rc = cb200_gemm_bf16(A, B[g], C[g], M, N, K, 0, 0, nullptr, 0, nullptr, nullptr, nullptr, 0, 1, err, sms, st);
       if (rc) return rc;

@@ -25,3 +25,15 @@ def test_split_takes_the_fewest_k_blocks_in_a_row():
             assert got == 1
         else:
             assert cost[got] == min(cost.values()) and not (got > 1 and cost[1] == cost[got]) and not (got == 2 and cost[4] == cost[2])
+
+
+def test_launches_of_several_weights():
+    """One launch from 256 rows on while CTA-pair tiles are on, else one for each weight."""
+    ops = native.load()
+    was = ops.gemm_pair_mode(1)
+    try:
+        assert [ops.gemm_group_launches(m, 3) for m in (8, 255, 256, 5000)] == [3, 3, 1, 1]
+        ops.gemm_pair_mode(0)
+        assert [ops.gemm_group_launches(m, 2) for m in (8, 255, 256, 5000)] == [2, 2, 2, 2]
+    finally:
+        ops.gemm_pair_mode(was)
