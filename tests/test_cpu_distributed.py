@@ -27,6 +27,9 @@ def _worker(rank, world, port, fn_name, tmp, kwargs):
         dist.barrier()
         with open(os.path.join(tmp, f"ok{rank}"), "w") as f:
             f.write("ok")
+    except pytest.skip.Exception as e:           # every rank skips at the same place; the parent passes it on
+        with open(os.path.join(tmp, f"skip{rank}"), "w") as f:
+            f.write(str(e))
     except Exception:
         with open(os.path.join(tmp, f"err{rank}"), "w") as f:
             f.write(traceback.format_exc())
@@ -40,6 +43,9 @@ def run_distributed(fn_name: str, world: int = 2, **kwargs):
         mp.spawn(_worker, args=(world, _free_port(), fn_name, tmp, kwargs), nprocs=world, join=True)
         errs = [open(os.path.join(tmp, f)).read() for f in sorted(os.listdir(tmp)) if f.startswith("err")]
         assert not errs, "\n".join(errs)
+        skips = [open(os.path.join(tmp, f)).read() for f in sorted(os.listdir(tmp)) if f.startswith("skip")]
+        if len(skips) == world:
+            pytest.skip(skips[0])
         assert all(os.path.exists(os.path.join(tmp, f"ok{r}")) for r in range(world))
 
 
