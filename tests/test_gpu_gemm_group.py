@@ -1,0 +1,83 @@
+"""GEMMs over several weights of one input in one launch (the context's keys and values, a block's q, k and v): partial N tiles inside a
+group, ragged rows, and groups whose tiles are few enough that clusters of CTA pairs share their contraction."""
+
+import math
+
+import pytest
+import torch
+
+from cosmos_predict25_b200.models import dit
+from cosmos_predict25_b200.ops import native
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+ROUND = 1.5 * 2.0 ** -9        # one bf16 rounding of the result in the 2-norm
+
+
+def _rel(a, b):
+    return ((a.double() - b).norm() / b.norm()).item()
+
+
+# (batch, tokens, context width, model width, CTA pairs per tile): below one launch; unsplit with whole and partial N tiles; both splits;
+# ragged rows; more tiles than half the pairs. The split is the rule's for the 36 and 16 clusters that a B200 holds at least.
+@pytest.mark.parametrize("B,S,C,D,split", [(2, 40, 512, 256, 1), (1, 256, 512, 256, 1), (2, 512, 512, 1024, 1), (2, 512, 1024, 2048, 1),
+                                           (1, 256, 1024, 2048, 4), (1, 512, 1024, 2048, 2), (1, 264, 1024, 1024, 4), (1, 264, 2048, 384, 1),
+                                           (1, 520, 640, 640, 1), (3, 88, 2112, 256, 4)])
+def test_keys_and_values_of_all_blocks(B, S, C, D, split):
+    torch.manual_seed(0)
+    ops = native.load()
+    tiles = -(-B * S // 256) * -(-D // 256) * 2
+    if D % 256 == 0 and B * S >= 256:
+        assert ops.gemm_pairs_per_tile(tiles, C // 64, 74, 36, 16) == split
+    ctx = torch.randn(B, S, C, device=DEV).bfloat16()
+    widths = (D, 128, D)                                       # blocks of another width between
+    ws = []
+    for d in widths:
+        ws += [(torch.randn(d, C, device=DEV) / math.sqrt(C)).bfloat16() for _ in range(2)] + [(1 + 0.2 * torch.randn(128, device=DEV)).bfloat16()]
+    got, again = ops.dit_context_kv(ctx, ws, 1e-6), ops.dit_context_kv(ctx, ws, 1e-6)
+    torch.cuda.synchronize()
+    assert ops.kernel_error(0, True) == 0
+    for i, d in enumerate(widths):
+        wk, wv, wn = (w.double() for w in ws[3 * i: 3 * i + 3])
+        k = (ctx.double() @ wk.t()).view(B, S, d // 128, 128)
+        k = k * torch.rsqrt(k.pow(2).mean(-1, keepdim=True) + 1e-6) * wn
+        v = (ctx.double() @ wv.t()).view(B, S, d // 128, 128)
+        assert _rel(got[2 * i + 1], v) < ROUND
+        assert _rel(got[2 * i], k) < math.sqrt(2) * ROUND      # the product is rounded, and the normalised keys are
+        assert torch.equal(got[2 * i], again[2 * i]) and torch.equal(got[2 * i + 1], again[2 * i + 1])
+
+
+# 264 to 520 tokens of the 1024-wide network: 12 to 36 tiles of q, k and v over 16 k-blocks, all of them split; 80 prompt rows and 256
+@pytest.mark.parametrize("shape,tokens", [((1, 1, 32, 32), 40), ((2, 1, 32, 32), 128), ((1, 1, 24, 88), 256), ((1, 2, 26, 40), 512)])
+def test_query_key_value_of_few_tiles(shape, tokens):
+    """The native block loop against the module path, whose q, k and v are launches of their own: the same sums in another order, so a few
+    bf16 roundings (2^-9 each) through two blocks."""
+    torch.manual_seed(0)
+    with torch.device(DEV):
+        net = dit.CosmosDiT(dit.dit_mini(num_blocks=2, crossattn_proj_in_channels=512, crossattn_emb_channels=512))
+    net.init_weights()
+    for n, p in net.named_parameters():
+        if "adaln_modulation" in n:
+            torch.nn.init.normal_(p, 0.0, 0.05)
+    net = net.to(torch.bfloat16).eval().requires_grad_(False)
+    B, T, H, W = shape
+    rows, D = B * T * H * W // 4, net.cfg.model_channels
+    assert native.load().gemm_pairs_per_tile(-(-rows // 256) * (D // 256) * 3, D // 64, 74, 36, 16) > 1
+    x, text = torch.randn(B, 16, T, H, W, device=DEV).bfloat16(), torch.randn(B, tokens, 512, device=DEV).bfloat16()
+    t, fps = torch.rand(B, T, device=DEV) * 1000, torch.full((B,), 16.0, device=DEV)
+
+    def run():
+        with torch.no_grad():
+            cache = net.build_context_cache(text)
+            return net(x, t, None, fps=fps, context_cache=cache), cache.cross_kv
+
+    got, kv = run()
+    hooks = [m.register_forward_hook(lambda *a: None) for m in (net.blocks[1].mlp.layer1, net.blocks[0].cross_attn.k_proj)]
+    want, kv_want = run()
+    for h in hooks:
+        h.remove()
+    torch.cuda.synchronize()
+    assert native.load().kernel_error(0, True) == 0
+    assert _rel(got, want.double()) < 4 * 2.0 ** -9
+    for a, b in zip([t for p in kv for t in p], [t for p in kv_want for t in p]):
+        assert _rel(a, b.double()) < 4 * 2.0 ** -9
