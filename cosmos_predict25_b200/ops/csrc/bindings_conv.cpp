@@ -63,6 +63,9 @@ void conv_cl(const Tensor& x, const Tensor& w, int64_t n_tile, int64_t Cout, c10
                     y_norm->numel() >= last && Cout <= n_tile && Cout % 8 == 0 && out_C % 8 == 0 && oc_add % 8 == 0 && gamma->is_cuda() &&
                     gamma->scalar_type() == at::kFloat && gamma->is_contiguous() && gamma->numel() == Cout && gamma->device() == x.device(),
                 "y_norm must cover the output map, gamma be fp32 [Cout], and all channels lie in one N tile");
+  if (((out_C | oc_add | Cout) & 7) == 0)      // voxels move as 16-byte pieces
+    for (const Tensor* t : {(const Tensor*)&y, resid.has_value() ? &*resid : nullptr, y_norm.has_value() ? &*y_norm : nullptr})
+      TORCH_CHECK(t == nullptr || reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "y, resid and y_norm must start on a 16-byte boundary");
   c10::cuda::CUDAGuard g(x.device());
   std::vector<int> tp(taps.begin(), taps.end()), om(out_map.begin(), out_map.end());
   const int dev = x.get_device();
@@ -99,6 +102,7 @@ Tensor fa_wide(const Tensor& q, const Tensor& k, const Tensor& v, double scale) 
     TORCH_CHECK(t->stride(1) % 8 == 0 && t->stride(0) % 8 == 0 && t->stride(1) > 0 && t->stride(0) > 0 &&
                     reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "fa_wide: rows must start on 16-byte boundaries");
   }
+  TORCH_CHECK(scale > 0, "fa_wide: the softmax scale must be positive (the row maximum is taken before it is applied)");
   TORCH_CHECK(k.size(1) == v.size(1) && q.numel() > 0 && k.numel() > 0, "fa_wide: empty input or k / v of different length");
   c10::cuda::CUDAGuard g(q.device());
   Tensor o = at::empty({q.size(0), q.size(1), 384}, q.options());

@@ -129,6 +129,25 @@ def test_norm_in_the_epilogue(Cout, silu, raw, resid):
     _close(n, F.silu(wn) if silu else wn, 4e-3, 1e-2, "norm of the conv")
 
 
+def test_operands_that_the_kernels_cannot_read_are_refused():
+    """Outputs off a 16-byte boundary (they are moved as 16-byte pieces) and a softmax scale that is not positive."""
+    from cosmos_predict25_b200.models import vae_wan_cl
+    cl = vae_wan_cl.ConvCL(torch.randn(64, 1, 64), None, [(0, 0, 0)], DEV)
+    x, g = torch.randn(1, 8, 16, 64, device=DEV).bfloat16(), torch.ones(64, device=DEV)
+    whole, odd = (torch.zeros(1 + x.numel(), device=DEV).bfloat16()[o:o + x.numel()].view_as(x) for o in (0, 1))
+    for y, resid, norm in ((odd, None, None), (whole, odd, None), (whole, None, odd)):
+        with pytest.raises(RuntimeError, match="16-byte"):
+            cl._launch(x, cl.taps, 1, 8, 16, y, None, resid, norm=None if norm is None else (g, True), normed=norm)
+    cl3 = vae_wan_cl.ConvCL(torch.randn(3, 1, 64), None, [(0, 0, 0)], DEV)          # channels that are stored one by one may lie anywhere
+    y = torch.zeros(1 + 128 * 3, device=DEV).bfloat16()[1:].view(1, 8, 16, 3)
+    assert torch.equal(cl3._launch(x, cl3.taps, 1, 8, 16, y, None, None), cl3(x, 1))
+    q = torch.randn(1, 64, 384, device=DEV).bfloat16()
+    for scale in (0.0, -0.1, float("nan")):
+        with pytest.raises(RuntimeError, match="positive"):
+            native.load().fa_wide(q, q, q, scale)
+    _no_kernel_error()
+
+
 def test_norm_behind_upsampling_phases():
     from cosmos_predict25_b200.models import vae_wan, vae_wan_cl
     torch.manual_seed(10)
