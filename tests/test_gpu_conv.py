@@ -129,6 +129,44 @@ def test_norm_in_the_epilogue(Cout, silu, raw, resid):
     _close(n, F.silu(wn) if silu else wn, 4e-3, 1e-2, "norm of the conv")
 
 
+def _band(monkeypatch, whole, lo, hi):
+    """Makes the layers believe that they hold rows [lo, hi) of a frame: the boundary rows come out of ``whole()``, the whole tensor."""
+    from cosmos_predict25_b200.models import vae_parallel
+
+    def exchange_rows(x, dim, n, top=True, bottom=True):
+        f = F.pad(whole(), (0, 0, 0, 0, n, n))
+        return f[:, lo:hi + 2 * n].contiguous()
+
+    monkeypatch.setattr(vae_parallel, "_active", (None, 0, 2))
+    monkeypatch.setattr(vae_parallel, "exchange_rows", exchange_rows)
+
+
+@pytest.mark.parametrize("lo,hi", [(0, 7), (7, 20), (20, 24)])
+def test_row_bands_equal_the_whole_frame(lo, hi, monkeypatch):
+    """A band of rows with its neighbours' boundary rows (row-sharded decoding), chunk by chunk: the cached frames keep theirs. The ranks'
+    exchange is replaced by reading the whole tensor."""
+    from cosmos_predict25_b200.models import vae_wan, vae_wan_cl
+    torch.manual_seed(14)
+    C, H, W = 64, 24, 20
+    w = torch.randn(96, C, 3, 3, 3, device=DEV) / (27 * C) ** 0.5
+    cl = vae_wan_cl.ConvCL(w.permute(0, 2, 3, 4, 1).reshape(96, -1, C), torch.randn(96, device=DEV), vae_wan_cl._causal3_taps(3, 3, 3), DEV)
+    up = vae_wan_cl._UpsampleCL(vae_wan.Resample(C, "upsample2d").to(DEV), DEV)
+    norms = (1 + 0.1 * torch.randn(96, device=DEV), True), (torch.ones(C // 2, device=DEV), True)
+    chunks = [torch.randn(T, H, W, C, device=DEV).bfloat16() for T in (1, 1, 4, 2)]
+    st = vae_wan_cl._Stream()
+    want = [(cl.causal(x, st, norm=norms[0]), up.run(x, st, None, norms[1])) for x in chunks]
+    st, now = vae_wan_cl._Stream(), []
+    _band(monkeypatch, lambda: now[-1], lo, hi)
+    for x, (conv, ups) in zip(chunks, want):
+        now.append(x)
+        band = x[:, lo:hi].contiguous()
+        for got, full in zip(cl.causal(band, st, norm=norms[0]), conv):
+            assert torch.equal(got, full[:, lo:hi])
+        for got, full in zip(up.run(band, st, None, norms[1]), ups):
+            assert torch.equal(got, full[:, 2 * lo:2 * hi])
+    _no_kernel_error()
+
+
 def test_operands_that_the_kernels_cannot_read_are_refused():
     """Outputs off a 16-byte boundary (they are moved as 16-byte pieces) and a softmax scale that is not positive."""
     from cosmos_predict25_b200.models import vae_wan_cl
