@@ -63,6 +63,12 @@ int* cb200_error_word(int device) {
   return words[device];
 }
 
+int cb200_sm_count(int device) {
+  static int counts[64] = {0};
+  if (counts[device] == 0) counts[device] = at::cuda::getDeviceProperties(device)->multiProcessorCount;
+  return counts[device];
+}
+
 namespace {
 inline int* error_word(int device) { return cb200_error_word(device); }
 
@@ -321,12 +327,6 @@ GemmDims gemm_dims(const Tensor& a, const Tensor& b, bool trans_a, bool trans_b)
   return d;
 }
 
-int sm_count(int device) {
-  static int cache[64] = {0};
-  if (cache[device] == 0) cache[device] = at::cuda::getDeviceProperties(device)->multiProcessorCount;
-  return cache[device];
-}
-
 Tensor gemm_impl(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& bias, int64_t act, bool trans_a, bool trans_b,
                  Tensor* pre, const Tensor* resid, const Tensor* gate, int64_t L) {
   check_bf16(a, "a");
@@ -361,7 +361,7 @@ Tensor gemm_impl(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& 
   }
   const int dev = a.get_device();
   const int rc = cb200_gemm_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), d.M, d.N, d.K, trans_a ? 1 : 0, trans_b ? 1 : 0, bias_p,
-                                 (int)act, pre_p, resid_p, gate_p, ld_gate, (int)L, error_word(dev), sm_count(dev), stream());
+                                 (int)act, pre_p, resid_p, gate_p, ld_gate, (int)L, error_word(dev), cb200_sm_count(dev), stream());
   TORCH_CHECK(rc == 0, "tcgen05 GEMM launch failed with code ", rc);
   return c;
 }
@@ -429,7 +429,7 @@ std::tuple<Tensor, Tensor> gemm_scatter_heads_peer(const Tensor& x, const Tensor
   const int dev = x.get_device();
   const int rc = cb200_gemm_bf16_scatter_heads(x.data_ptr(), w.data_ptr(), d.M, d.N, d.K, p.data(), (int)p.size(), (int)rank, (int)S,
                                                wp, wp != nullptr ? is_bf16(wf) : 0, cp, sp, (float)eps, keep_raw ? raw.data_ptr() : nullptr,
-                                               keep_raw ? rstd.data_ptr<float>() : nullptr, error_word(dev), sm_count(dev), stream());
+                                               keep_raw ? rstd.data_ptr<float>() : nullptr, error_word(dev), cb200_sm_count(dev), stream());
   TORCH_CHECK(rc == 0, "tcgen05 GEMM (head-scatter epilogue) launch failed with code ", rc);
   return {raw, rstd};
 }

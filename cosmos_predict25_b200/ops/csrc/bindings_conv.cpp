@@ -11,15 +11,10 @@
 #include "launchers.h"
 
 int* cb200_error_word(int device);
+int cb200_sm_count(int device);
 
 namespace {
 using at::Tensor;
-
-int sm_count(int device) {
-  static int counts[64] = {0};
-  if (counts[device] == 0) counts[device] = at::cuda::getDeviceProperties(device)->multiProcessorCount;
-  return counts[device];
-}
 
 // x [T_in, H_in, W_in, Cin] bf16; w [n_rows, ntaps * ceil(Cin / 64) * 64] bf16 (tap-major, channels zero-padded to 64);
 // taps: ntaps * 3 ints (dt, dh, dw) added to the (strided) output coordinate, dt counted from the first of `pad` frames in front of
@@ -74,7 +69,7 @@ void conv_cl(const Tensor& x, const Tensor& w, int64_t n_tile, int64_t Cout, c10
                                (int)t_stride, (int)hw_stride, w.data_ptr(), (int)w.size(0), (int)n_tile, (int)Cout, tp.data(), (int)ntaps, (int)T_out, (int)H_out, (int)W_out, om.data(), y.data_ptr(),
                                resid.has_value() ? resid->data_ptr() : nullptr, bias.has_value() ? bias->data_ptr<float>() : nullptr,
                                y_norm.has_value() ? y_norm->data_ptr() : nullptr, gamma.has_value() ? gamma->data_ptr<float>() : nullptr,
-                               silu ? 1 : 0, write_raw ? 1 : 0, cb200_error_word(dev), sm_count(dev), at::cuda::getCurrentCUDAStream().stream());
+                               silu ? 1 : 0, write_raw ? 1 : 0, cb200_error_word(dev), cb200_sm_count(dev), at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(rc == 0, "conv_cl launch failed with code ", rc);
 }
 

@@ -19,15 +19,10 @@
 #include "launchers.h"
 
 int* cb200_error_word(int device);
+int cb200_sm_count(int device);
 
 namespace {
 using at::Tensor;
-
-int sm_count(int device) {
-  static int counts[64] = {0};
-  if (counts[device] == 0) counts[device] = at::cuda::getDeviceProperties(device)->multiProcessorCount;
-  return counts[device];
-}
 
 // a weight matrix [rows, cols] as the GEMM reads it
 const void* weight(const Tensor& w, const Tensor& x, int64_t rows, int64_t cols) {
@@ -99,7 +94,7 @@ Tensor dit_blocks(const Tensor& x, const Tensor& mods, const c10::optional<Tenso
                     t.size(3) == 128 && t.size(1) > 0 && t.device() == x.device(), "dit_blocks: keys / values must be contiguous CUDA bf16 [B, S, H, 128]");
   c10::cuda::CUDAGuard guard(x.device());
   const int dev = x.get_device();
-  const Launcher run{cb200_error_word(dev), sm_count(dev), at::cuda::getCurrentCUDAStream().stream()};
+  const Launcher run{cb200_error_word(dev), cb200_sm_count(dev), at::cuda::getCurrentCUDAStream().stream()};
   const auto f32 = x.options().dtype(at::kFloat);
   // two residual streams in turn, the normalised input, and one buffer that is q, k, v, attention output and then the MLP's hidden layer
   Tensor r0 = at::empty({M, D}, x.options()), r1 = at::empty({M, D}, x.options()), h = at::empty({M, D}, x.options());
@@ -160,7 +155,7 @@ std::vector<Tensor> dit_context_kv(const Tensor& context, at::TensorList weights
   TORCH_CHECK((int64_t)weights.size() == 3 * n && C % 64 == 0 && M % 8 == 0, "dit_context_kv: three weights per block, C a multiple of 64, B * S of 8");
   c10::cuda::CUDAGuard guard(context.device());
   const int dev = context.get_device();
-  const Launcher run{cb200_error_word(dev), sm_count(dev), at::cuda::getCurrentCUDAStream().stream()};
+  const Launcher run{cb200_error_word(dev), cb200_sm_count(dev), at::cuda::getCurrentCUDAStream().stream()};
   std::vector<Tensor> out, keep;
   Tensor rstd, raw;
   for (int64_t i = 0; i < n; ++i) {

@@ -11,6 +11,7 @@
 #include "launchers.h"
 
 int* cb200_error_word(int device);
+int cb200_sm_count(int device);
 
 namespace {
 using at::Tensor;
@@ -137,12 +138,6 @@ Tensor a2a_gather_seq_peer(c10::ArrayRef<int64_t> src_ptrs, int64_t B, int64_t S
   return out;
 }
 
-int sm_count_peer(int device) {
-  static int cache[64] = {0};
-  if (cache[device] == 0) cache[device] = at::cuda::getDeviceProperties(device)->multiProcessorCount;
-  return cache[device];
-}
-
 // Small parameters of a unit, all-gathered by peer reads: segs [n, 4] as for the other segment kernels; `full` is the local
 // full-layout buffer that receives every rank's chunk.
 void gather_slots_peer(c10::ArrayRef<int64_t> shard_ptrs, const Tensor& segs, Tensor full) {
@@ -189,7 +184,7 @@ Tensor gemm_bf16_gather(const Tensor& x, Tensor ws, c10::ArrayRef<int64_t> shard
   const int dev = x.get_device();
   const int rc = cb200_gemm_bf16_gather(x.data_ptr(), ws.data_ptr(), c.data_ptr(), (int)M, (int)rows, (int)ld, trans_b ? 1 : 0, p.data(),
                                         (int)p.size(), (int)chunk_rows, counters.data_ptr<int>(), bias_p, (int)act, pre_p,
-                                        cb200_error_word(dev), sm_count_peer(dev), stream());
+                                        cb200_error_word(dev), cb200_sm_count(dev), stream());
   TORCH_CHECK(rc == 0, "gather GEMM launch failed with code ", rc);
   return c;
 }

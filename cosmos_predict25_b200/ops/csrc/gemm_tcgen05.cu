@@ -1,14 +1,14 @@
 // bf16 GEMM on the 5th-generation tensor cores (sm_100a): C[M,N] = epilogue(A x B), fp32 accumulation.
 //
-// Persistent, warp-specialised kernel, one CTA per SM:
-//   warp 0   TMA producer: streams 128x64 A tiles and 256x64 B tiles (128-byte swizzle) through a
-//            4-stage shared-memory ring; completion by mbarrier transaction bytes.
-//   warp 1   MMA issuer: one thread issues tcgen05.mma (UMMA 128x256x16, cta_group::1) from
-//            shared-memory descriptors into one of two 128x256 fp32 accumulators in TMEM
-//            (2 x 256 = all 512 columns), and releases ring slots with tcgen05.commit.
-//   warps 2-5 epilogue: tcgen05.ld the finished accumulator (each warp owns one 32-lane quarter of
-//            TMEM), apply the fused epilogue in registers and store bf16 straight to global memory,
-//            while warp 1 already accumulates the next tile into the other TMEM buffer.
+// Persistent, warp-specialised kernel, one CTA per SM, in three forms:
+//   CTA pairs (from 256 rows on): clusters of two CTAs work on a 256 x 256 tile with cta_group::2 MMAs, six 32 KB stages; a cluster of two
+//            or four pairs shares a tile where there are few of them (see the kernel below);
+//   single CTAs (fewer rows, and the gather mode): 128 x 256 tiles, four 48 KB stages.
+// Roles: warp 0 is the TMA producer (128x64 A tiles and 256x64 B tiles, 128-byte swizzle, through the ring of stages; completion by
+//   mbarrier transaction bytes), warp 1 issues tcgen05.mma from shared-memory descriptors into one of two 128x256 fp32 accumulators
+//   in TMEM (2 x 256 = all 512 columns) and releases ring slots with tcgen05.commit, warps 2-9 are the epilogue: two warps per
+//   32-lane quarter of TMEM, 128 columns each, apply the fused epilogue in registers and store bf16 through a staging block while
+//   warp 1 already accumulates the next tile into the other TMEM buffer.
 //
 // Operand majors are template parameters so the same kernel serves forward (x @ W^T: both K-major),
 // dgrad (dy @ W: B is N-major) and wgrad (dy^T @ x: both MN-major) without transposing in memory.
@@ -791,91 +791,50 @@ static int launch_gemm(const void* A, const void* B, int M, int N, int K, const 
   return (int)cudaGetLastError();
 }
 
-// Same contraction on CTA pairs (template flag CTA2): clusters of two CTAs, one 256 x 256 tile per pair.
-template <int A_MN, int B_MN>
-static int launch_gemm_pair(const void* A, const void* const* B, int M, int N, int K, const GemmEpilogue& ep, int* err, int sms,
-                            cudaStream_t st) {
-  CUtensorMap ta, tb[3];
-  int rc;
-  if (A_MN == 0) rc = make_tmap_2d_bf16(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, BM);
-  else rc = make_tmap_2d_bf16(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)M * 2, 64, BK);
-  if (rc) return rc;
-  for (int g = 0; g < 3; ++g) {
-    const void* w = B[g < ep.groups ? g : 0];
-    if (B_MN == 0) rc = make_tmap_2d_bf16(&tb[g], w, (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, BK, BN / 2);   // each CTA loads half the columns
-    else rc = make_tmap_2d_bf16(&tb[g], w, (uint64_t)N, (uint64_t)K, (uint64_t)N * 2, 64, BK);
-    if (rc) return rc;
-  }
-  static bool attr_set = false;
-  auto kern = gemm_bf16_kernel<A_MN, B_MN, false, true>;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-    if (e != cudaSuccess) return 100 + (int)e;
-    attr_set = true;
-  }
-  const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) * ep.groups;
+// Same contraction on CTA pairs (template flag CTA2): clusters of SPLIT pairs, one 256 x 256 tile per cluster.
+struct PairLaunch {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * (sms / 2));
-  cfg.blockDim = dim3(kGemmThreads);
-  cfg.dynamicSmemBytes = kSmemBytes;
-  cfg.stream = st;
   cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.numAttrs = 2;
-  // A persistent grid must be resident as a whole: the pairs that the GPU can hold at once (a pair lives inside one GPC, so a
-  // GPC with an odd number of free SMs leaves one out) bound the grid, otherwise late pairs would run after the others.
-  static int max_pairs = 0;
-  if (max_pairs == 0) {
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) return 600;
-    max_pairs = n;
+  PairLaunch(int split, int clusters, cudaStream_t st) {
+    cfg.gridDim = dim3(2 * split * clusters);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = kSmemBytes;
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2 * split;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
   }
-  const int pairs = std::min(tiles, std::min(max_pairs, sms / 2));
-  cfg.gridDim = dim3(2 * pairs);
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb[0], tb[1], tb[2], M, N, K, ep, GatherB{}, err);
-  return e == cudaSuccess ? 0 : 500 + (int)e;
-}
+  PairLaunch(const PairLaunch&) = delete;
+};
 
-// Split tiles (template flag SPLIT): a cluster of SPLIT pairs per 256 x 256 tile, as many clusters as tiles.
+// clusters that the GPU holds at once: none where it has no room for one (a share of a GPU)
 template <int A_MN, int B_MN, int SPLIT>
-static int launch_gemm_split(const void* A, const void* const* B, int M, int N, int K, const GemmEpilogue& ep, int* err, cudaStream_t st,
-                             int* clusters) {
-  auto kern = gemm_bf16_kernel<A_MN, B_MN, false, true, SPLIT>;
-  cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(kGemmThreads);
-  cfg.dynamicSmemBytes = kSmemBytes;
-  cfg.stream = st;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2 * SPLIT;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.numAttrs = 2;
-  static int max_clusters = -1;      // clusters that the GPU holds at once; none where it has no room for one (a share of a GPU)
-  if (max_clusters < 0) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+static int resident_clusters(int* clusters) {
+  static int resident = -1;
+  if (resident < 0) {
+    const auto kern = gemm_bf16_kernel<A_MN, B_MN, false, true, SPLIT>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
     if (e != cudaSuccess) return 100 + (int)e;
+    PairLaunch l(SPLIT, 1, nullptr);
     int n = 0;
-    cfg.gridDim = dim3(2 * SPLIT);
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &l.cfg) != cudaSuccess) {
       cudaGetLastError();
       n = 0;
     }
-    max_clusters = n;
+    resident = n;
   }
-  if (clusters != nullptr) {         // only asked for the capacity
-    *clusters = max_clusters;
-    return 0;
-  }
+  *clusters = resident;
+  return 0;
+}
+
+template <int A_MN, int B_MN, int SPLIT>
+static int launch_gemm_pairs(const void* A, const void* const* B, int M, int N, int K, const GemmEpilogue& ep, int clusters, int* err,
+                             cudaStream_t st) {
   CUtensorMap ta, tb[3];
   int rc;
   if (A_MN == 0) rc = make_tmap_2d_bf16(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, BM);
@@ -887,15 +846,16 @@ static int launch_gemm_split(const void* A, const void* const* B, int M, int N, 
     else rc = make_tmap_2d_bf16(&tb[g], w, (uint64_t)N, (uint64_t)K, (uint64_t)N * 2, 64, BK);
     if (rc) return rc;
   }
-  cfg.gridDim = dim3(2 * SPLIT * ((M + 2 * BM - 1) / (2 * BM)) * (N / BN) * ep.groups);
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb[0], tb[1], tb[2], M, N, K, ep, GatherB{}, err);
+  PairLaunch l(SPLIT, clusters, st);
+  const cudaError_t e = cudaLaunchKernelEx(&l.cfg, gemm_bf16_kernel<A_MN, B_MN, false, true, SPLIT>, ta, tb[0], tb[1], tb[2], M, N, K, ep,
+                                           GatherB{}, err);
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
 
 // One tile per pair, or clusters of 2 or 4 pairs per tile: whichever takes fewer k-blocks in a row, waves counted, with kExchange
-// k-blocks' time for the exchange of partial tiles. Six k-blocks: measured 9.1 us
-// against 7.0 us of fixed time, 0.3 us a k-block. 512 x 2048 from K = 2048: 18.7 -> 13.9 us, from K = 8192: 46.9 -> 28; 1024 x 1024 from
-// K = 100,352 (the text projection): 460 -> 241 us. `c2`, `c4`: clusters of 2 and 4 pairs that the GPU holds at once; where it holds
+// k-blocks' time for the exchange of partial tiles. Six k-blocks: measured 9.1 us against 7.0 us of fixed time, 0.3 us a k-block. Launches
+// back to back, one pair per tile and split: 512 x 2048 from K = 2048 18.7 and 13.1 us, from K = 8192 46.9 and 26.7; 1024 x 1024 from
+// K = 100,352 (the text projection) 460 and 229 us. `c2`, `c4`: clusters of 2 and 4 pairs that the GPU holds at once; where it holds
 // none the split is not taken.
 extern "C" int cb200_gemm_pairs_per_tile(long tiles, long kb, int pairs, int c2, int c4) {
   if (2 * tiles > pairs || kb < 8) return 1;
@@ -914,16 +874,18 @@ template <int A_MN, int B_MN>
 static int launch_gemm_any(const void* A, const void* const* B, int M, int N, int K, const GemmEpilogue& ep, int* err, int sms, cudaStream_t st) {
   const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) * ep.groups, kb = (K + BK - 1) / BK;
   const int pairs = sms / 2;
+  int c1 = 0, c2 = 0, c4 = 0, rc;
   if (N % BN == 0 && ep.hs.P == 0 && 2 * tiles <= pairs) {
-    int c2 = 0, c4 = 0;
-    int rc = launch_gemm_split<A_MN, B_MN, 2>(A, B, M, N, K, ep, err, st, &c2);
-    if (rc) return rc;
-    if ((rc = launch_gemm_split<A_MN, B_MN, 4>(A, B, M, N, K, ep, err, st, &c4))) return rc;
+    if ((rc = resident_clusters<A_MN, B_MN, 2>(&c2)) || (rc = resident_clusters<A_MN, B_MN, 4>(&c4))) return rc;
     const int split = cb200_gemm_pairs_per_tile(tiles, kb, pairs, c2, c4);
-    if (split == 4) return launch_gemm_split<A_MN, B_MN, 4>(A, B, M, N, K, ep, err, st, nullptr);
-    if (split == 2) return launch_gemm_split<A_MN, B_MN, 2>(A, B, M, N, K, ep, err, st, nullptr);
+    if (split == 4) return launch_gemm_pairs<A_MN, B_MN, 4>(A, B, M, N, K, ep, (int)tiles, err, st);
+    if (split == 2) return launch_gemm_pairs<A_MN, B_MN, 2>(A, B, M, N, K, ep, (int)tiles, err, st);
   }
-  return launch_gemm_pair<A_MN, B_MN>(A, B, M, N, K, ep, err, sms, st);
+  // A persistent grid must be resident as a whole: the pairs that the GPU can hold at once (a pair lives inside one GPC, so a
+  // GPC with an odd number of free SMs leaves one out) bound the grid, otherwise late pairs would run after the others.
+  if ((rc = resident_clusters<A_MN, B_MN, 1>(&c1))) return rc;
+  if (c1 < 1) return 600;
+  return launch_gemm_pairs<A_MN, B_MN, 1>(A, B, M, N, K, ep, (int)std::min<long>(tiles, std::min(c1, pairs)), err, st);
 }
 
 // 0: single-CTA tiles; 1 (default): CTA pairs where the shape allows (measured 8-45 % faster on the 2B shapes: half the B-operand
@@ -1012,7 +974,7 @@ extern "C" int cb200_gemm_bf16_scatter_heads(const void* A, const void* W, int M
   ep.hs.rstd_out = rstd_out;
   ep.L = 1;
   ep.groups = 1;
-  if (cb200_gemm_pair_mode(-1) == 1 && M >= 2 * BM) return launch_gemm_pair<0, 0>(A, &W, M, N, K, ep, err, sms, st);
+  if (cb200_gemm_pair_mode(-1) == 1 && M >= 2 * BM) return launch_gemm_any<0, 0>(A, &W, M, N, K, ep, err, sms, st);
   return launch_gemm<0, 0>(A, W, M, N, K, ep, err, sms, st);
 }
 
