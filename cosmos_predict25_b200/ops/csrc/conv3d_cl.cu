@@ -23,8 +23,9 @@
 // CTA pairs (tcgen05 cta_group::2): two consecutive voxel tiles share the B operand, each CTA fetches its own A box and half of
 // the B rows, the even CTA issues M = 256 MMAs. What bounds the kernel is the L2 -> shared-memory path of narrow layers: for one
 // (dt, dw) column of a 3 x 3 x 3 convolution with 96 channels a CTA now fetches 20 + 18 KB per channel block instead of
-// 3 x (16 + 12) KB. Decoding 8 latent frames of 720p: 296 ms in this kernel
-// before (one CTA per tile, a box per tap), 224 ms now; a single 640 x 640 image 5.7 -> 2.6 ms.
+// 3 x (16 + 12) KB. Decoding 8 latent frames of 720p: 296 ms in this kernel before (one CTA per tile, a box per tap), 176 ms now, norms
+// included; a single 640 x 640 image 5.7 and 2.1 ms. 96 channels, 27 taps with the norm, 4 frames of 704 x 1280: tensor pipe 75 % busy,
+// 1.35 ms (1,329 TFLOP/s); 192 channels 1,635, 384 channels 1,699 TFLOP/s.
 //
 // Persistent, warp-specialised, one CTA per SM, same skeleton as the GEMM of this package: warp 0 TMA producer (ring of A box + B
 // boxes, as many stages as fit), warp 1 MMA issuer (two TMEM accumulators of n_tile columns), warps 2-9 epilogue (bias, optional
@@ -279,176 +280,176 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       bool arrived = false;              // whether the accumulators of this tile have been waited for
 #pragma unroll 1
       for (int u = 0; u < STACK; ++u, h0 += TH) {
-      // element offset of a voxel of the tile (row r = 16 h + w), or -1 outside the frame
-      auto offset = [&](int r) -> long {
-        const int h = h0 + (r >> 4), w = w0 + (r & 15);
-        if (!mine || h >= p.H_out || w >= p.W_out) return -1;
-        return (((long)(tf * p.ot_mul + p.ot_add) * p.out_H + (h * p.oh_mul + p.oh_add)) * p.out_W + (w * p.ow_mul + p.ow_add)) * p.out_C + p.oc_add;
-      };
-      const uint32_t t_row = tmem_base + acc * 256 + u * 128 + ((uint32_t)(quarter * 32) << 16);
-      if (vec_ok) {
-        const int piece = lane & 3;                       // 16-byte piece of the 64-byte run that this lane moves
-        long off[4];                                      // voxels quarter * 32 + 8 it + lane / 4
-#pragma unroll
-        for (int it = 0; it < 4; ++it) off[it] = offset(quarter * 32 + it * 8 + (lane >> 2));
-        auto slot = [&](int row, int pc) { return stage_warp + row * 64 + ((pc ^ ((row >> 1) & 3)) << 4); };   // no bank conflicts
-        // residual of the first chunk: on its way while the accumulator is still being computed
-        uint4 res[4];
-        auto fetch = [&](int c) {
-          const int n = nt * p.n_tile + c * 32 + piece * 8;
-#pragma unroll
-          for (int it = 0; it < 4; ++it)
-            if (off[it] >= 0 && n < p.Cout) res[it] = *reinterpret_cast<const uint4*>(p.resid + off[it] + n);
+        // element offset of a voxel of the tile (row r = 16 h + w), or -1 outside the frame
+        auto offset = [&](int r) -> long {
+          const int h = h0 + (r >> 4), w = w0 + (r & 15);
+          if (!mine || h >= p.H_out || w >= p.W_out) return -1;
+          return (((long)(tf * p.ot_mul + p.ot_add) * p.out_H + (h * p.oh_mul + p.oh_add)) * p.out_W + (w * p.ow_mul + p.ow_add)) * p.out_C + p.oc_add;
         };
-        if (p.resid != nullptr && c_lo < c_hi) fetch(c_lo);
-        if (!arrived && !mbar_wait_warp(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
-        arrived = true;
-        tc_fence_after();
-        // this thread's 32 channels of chunk c, staged and stored as 64-byte runs
-        auto emit = [&](bf16* dst, int c, const uint32_t (&a)[32]) {
+        const uint32_t t_row = tmem_base + acc * 256 + u * 128 + ((uint32_t)(quarter * 32) << 16);
+        if (vec_ok) {
+          const int piece = lane & 3;                       // 16-byte piece of the 64-byte run that this lane moves
+          long off[4];                                      // voxels quarter * 32 + 8 it + lane / 4
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint4 o;
-            __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
+          for (int it = 0; it < 4; ++it) off[it] = offset(quarter * 32 + it * 8 + (lane >> 2));
+          auto slot = [&](int row, int pc) { return stage_warp + row * 64 + ((pc ^ ((row >> 1) & 3)) << 4); };   // no bank conflicts
+          // residual of the first chunk: on its way while the accumulator is still being computed
+          uint4 res[4];
+          auto fetch = [&](int c) {
+            const int n = nt * p.n_tile + c * 32 + piece * 8;
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-              o2[j] = __floats2bfloat162_rn(__uint_as_float(a[q * 8 + 2 * j]), __uint_as_float(a[q * 8 + 2 * j + 1]));
-            *reinterpret_cast<uint4*>(slot(lane, q)) = o;
-          }
-          __syncwarp();
-          const int n = nt * p.n_tile + c * 32 + piece * 8;
-#pragma unroll
-          for (int it = 0; it < 4; ++it)
-            if (off[it] >= 0 && n < p.Cout && c * 32 + piece * 8 < p.n_tile)
-              *reinterpret_cast<uint4*>(dst + off[it] + n) = *reinterpret_cast<const uint4*>(slot(it * 8 + (lane >> 2), piece));
-          __syncwarp();
-        };
-        float ss = 0.f;
-#pragma unroll 1
-        for (int c = c_lo; c < c_hi; ++c) {
-          const int n0 = nt * p.n_tile + c * 32;
-          uint32_t a[32];
-          tmem_ld32(t_row + c * 32, a);                   // warp-collective; columns past the tile are loaded and not stored
-          tmem_ld_wait();
-          if (bias != nullptr) {
-            if (n0 + 32 <= p.Cout && bias == bias_s) {
-#pragma unroll
-              for (int j = 0; j < 32; j += 4) {
-                const float4 f = *reinterpret_cast<const float4*>(bias_s + n0 + j);
-                a[j] = __float_as_uint(__uint_as_float(a[j]) + f.x);
-                a[j + 1] = __float_as_uint(__uint_as_float(a[j + 1]) + f.y);
-                a[j + 2] = __float_as_uint(__uint_as_float(a[j + 2]) + f.z);
-                a[j + 3] = __float_as_uint(__uint_as_float(a[j + 3]) + f.w);
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (n0 + j < p.Cout) a[j] = __float_as_uint(__uint_as_float(a[j]) + bias[n0 + j]);
-            }
-          }
-          if (p.resid != nullptr) {
-            // the sum is rounded once: the residual comes through the staging block to the thread that owns the voxel
-#pragma unroll
-            for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(slot(it * 8 + (lane >> 2), piece)) = res[it];
-            if (c + 1 < c_hi) fetch(c + 1);
-            __syncwarp();
+            for (int it = 0; it < 4; ++it)
+              if (off[it] >= 0 && n < p.Cout) res[it] = *reinterpret_cast<const uint4*>(p.resid + off[it] + n);
+          };
+          if (p.resid != nullptr && c_lo < c_hi) fetch(c_lo);
+          if (!arrived && !mbar_wait_warp(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
+          arrived = true;
+          tc_fence_after();
+          // this thread's 32 channels of chunk c, staged and stored as 64-byte runs
+          auto emit = [&](bf16* dst, int c, const uint32_t (&a)[32]) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-              const uint4 rr = *reinterpret_cast<const uint4*>(slot(lane, q));
-              const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rr);
+              uint4 o;
+              __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const float2 rf = __bfloat1622float2(r2[j]);
-                a[q * 8 + 2 * j] = __float_as_uint(__uint_as_float(a[q * 8 + 2 * j]) + rf.x);
-                a[q * 8 + 2 * j + 1] = __float_as_uint(__uint_as_float(a[q * 8 + 2 * j + 1]) + rf.y);
+              for (int j = 0; j < 4; ++j)
+                o2[j] = __floats2bfloat162_rn(__uint_as_float(a[q * 8 + 2 * j]), __uint_as_float(a[q * 8 + 2 * j + 1]));
+              *reinterpret_cast<uint4*>(slot(lane, q)) = o;
+            }
+            __syncwarp();
+            const int n = nt * p.n_tile + c * 32 + piece * 8;
+#pragma unroll
+            for (int it = 0; it < 4; ++it)
+              if (off[it] >= 0 && n < p.Cout && c * 32 + piece * 8 < p.n_tile)
+                *reinterpret_cast<uint4*>(dst + off[it] + n) = *reinterpret_cast<const uint4*>(slot(it * 8 + (lane >> 2), piece));
+            __syncwarp();
+          };
+          float ss = 0.f;
+#pragma unroll 1
+          for (int c = c_lo; c < c_hi; ++c) {
+            const int n0 = nt * p.n_tile + c * 32;
+            uint32_t a[32];
+            tmem_ld32(t_row + c * 32, a);                   // warp-collective; columns past the tile are loaded and not stored
+            tmem_ld_wait();
+            if (bias != nullptr) {
+              if (n0 + 32 <= p.Cout && bias == bias_s) {
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) {
+                  const float4 f = *reinterpret_cast<const float4*>(bias_s + n0 + j);
+                  a[j] = __float_as_uint(__uint_as_float(a[j]) + f.x);
+                  a[j + 1] = __float_as_uint(__uint_as_float(a[j + 1]) + f.y);
+                  a[j + 2] = __float_as_uint(__uint_as_float(a[j + 2]) + f.z);
+                  a[j + 3] = __float_as_uint(__uint_as_float(a[j + 3]) + f.w);
+                }
+              } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                  if (n0 + j < p.Cout) a[j] = __float_as_uint(__uint_as_float(a[j]) + bias[n0 + j]);
               }
             }
+            if (p.resid != nullptr) {
+              // the sum is rounded once: the residual comes through the staging block to the thread that owns the voxel
+#pragma unroll
+              for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(slot(it * 8 + (lane >> 2), piece)) = res[it];
+              if (c + 1 < c_hi) fetch(c + 1);
+              __syncwarp();
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const uint4 rr = *reinterpret_cast<const uint4*>(slot(lane, q));
+                const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rr);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const float2 rf = __bfloat1622float2(r2[j]);
+                  a[q * 8 + 2 * j] = __float_as_uint(__uint_as_float(a[q * 8 + 2 * j]) + rf.x);
+                  a[q * 8 + 2 * j + 1] = __float_as_uint(__uint_as_float(a[q * 8 + 2 * j + 1]) + rf.y);
+                }
+              }
+            }
+            if (p.Yn != nullptr) {
+              // the finished values go back to TMEM for the second pass
+              if (n0 + 32 <= p.Cout) {
+                float2 s2[4] = {make_float2(ss, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                  const float2 v = make_float2(__uint_as_float(a[2 * j]), __uint_as_float(a[2 * j + 1]));
+                  s2[j & 3] = fma2(v, v, s2[j & 3]);
+                }
+                const float2 t = add2(add2(s2[0], s2[1]), add2(s2[2], s2[3]));
+                ss = t.x + t.y;
+              } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                  if (n0 + j < p.Cout) ss = fmaf(__uint_as_float(a[j]), __uint_as_float(a[j]), ss);
+              }
+              tmem_st32(t_row + c * 32, a);
+            }
+            if (p.write_raw) emit(p.Y, c, a);
           }
           if (p.Yn != nullptr) {
-            // the finished values go back to TMEM for the second pass
-            if (n0 + 32 <= p.Cout) {
-              float2 s2[4] = {make_float2(ss, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            // the two warps of a lane quarter hold half of a voxel's channels each. Two buffers: a warp is at most one tile ahead of its
+            // partner. The partner may have given up, so this wait is bounded like every other (a named barrier is not)
+            const int ss_buf = sums & 1;
+            float* mine_s = ssq + (ss_buf * 2 + part) * BM + quarter * 32 + lane;
+            const float* other_s = ssq + (ss_buf * 2 + (part ^ 1)) * BM + quarter * 32 + lane;
+            uint64_t* bar = &sums_in[ss_buf * 4 + quarter];
+            *mine_s = ss;
+            tmem_st_wait();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar);
+            if (!mbar_wait_warp(bar, (sums >> 1) & 1, abort_flag)) { ok = false; break; }
+            ++sums;
+            const float total = part == 0 ? ss + *other_s : *other_s + ss;
+            const float inv = 1.f / fmaxf(sqrtf(total), 1e-12f);
+#pragma unroll 1
+            for (int c = c_lo; c < c_hi; ++c) {
+              uint32_t a[32];
+              tmem_ld32(t_row + c * 32, a);
+              tmem_ld_wait();
+              const float2 inv2 = make_float2(inv, inv);
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const float2 v = make_float2(__uint_as_float(a[2 * j]), __uint_as_float(a[2 * j + 1]));
-                s2[j & 3] = fma2(v, v, s2[j & 3]);
+              for (int j = 0; j < 32; j += 4) {
+                // gamma past the last channel is whatever follows it in shared memory: those columns are not stored
+                const float4 g = *reinterpret_cast<const float4*>(gamma_s + c * 32 + j);
+                const float2 z0 = mul2(mul2(make_float2(__uint_as_float(a[j]), __uint_as_float(a[j + 1])), inv2), make_float2(g.x, g.y));
+                const float2 z1 = mul2(mul2(make_float2(__uint_as_float(a[j + 2]), __uint_as_float(a[j + 3])), inv2), make_float2(g.z, g.w));
+                a[j] = __float_as_uint(z0.x);
+                a[j + 1] = __float_as_uint(z0.y);
+                a[j + 2] = __float_as_uint(z1.x);
+                a[j + 3] = __float_as_uint(z1.y);
               }
-              const float2 t = add2(add2(s2[0], s2[1]), add2(s2[2], s2[3]));
-              ss = t.x + t.y;
-            } else {
+              if (p.silu) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (n0 + j < p.Cout) ss = fmaf(__uint_as_float(a[j]), __uint_as_float(a[j]), ss);
+                for (int j = 0; j < 32; ++j) {
+                  const float z = __uint_as_float(a[j]);
+                  a[j] = __float_as_uint(z / (1.f + __expf(-z)));
+                }
+              }
+              emit(p.Yn, c, a);
             }
-            tmem_st32(t_row + c * 32, a);
           }
-          if (p.write_raw) emit(p.Y, c, a);
-        }
-        if (p.Yn != nullptr) {
-          // the two warps of a lane quarter hold half of a voxel's channels each. Two buffers: a warp is at most one tile ahead of its
-          // partner. The partner may have given up, so this wait is bounded like every other (a named barrier is not)
-          const int ss_buf = sums & 1;
-          float* mine_s = ssq + (ss_buf * 2 + part) * BM + quarter * 32 + lane;
-          const float* other_s = ssq + (ss_buf * 2 + (part ^ 1)) * BM + quarter * 32 + lane;
-          uint64_t* bar = &sums_in[ss_buf * 4 + quarter];
-          *mine_s = ss;
-          tmem_st_wait();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar);
-          if (!mbar_wait_warp(bar, (sums >> 1) & 1, abort_flag)) { ok = false; break; }
-          ++sums;
-          const float total = part == 0 ? ss + *other_s : *other_s + ss;
-          const float inv = 1.f / fmaxf(sqrtf(total), 1e-12f);
+        } else {
+          const long base = offset(quarter * 32 + lane);
+          if (!arrived && !mbar_wait_warp(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
+          arrived = true;
+          tc_fence_after();
 #pragma unroll 1
           for (int c = c_lo; c < c_hi; ++c) {
             uint32_t a[32];
             tmem_ld32(t_row + c * 32, a);
             tmem_ld_wait();
-            const float2 inv2 = make_float2(inv, inv);
+            const int n0 = nt * p.n_tile + c * 32;
+            if (base >= 0) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              // gamma past the last channel is whatever follows it in shared memory: those columns are not stored
-              const float4 g = *reinterpret_cast<const float4*>(gamma_s + c * 32 + j);
-              const float2 z0 = mul2(mul2(make_float2(__uint_as_float(a[j]), __uint_as_float(a[j + 1])), inv2), make_float2(g.x, g.y));
-              const float2 z1 = mul2(mul2(make_float2(__uint_as_float(a[j + 2]), __uint_as_float(a[j + 3])), inv2), make_float2(g.z, g.w));
-              a[j] = __float_as_uint(z0.x);
-              a[j + 1] = __float_as_uint(z0.y);
-              a[j + 2] = __float_as_uint(z1.x);
-              a[j + 3] = __float_as_uint(z1.y);
+              for (int j = 0; j < 32; ++j)
+                if (n0 + j < p.Cout && c * 32 + j < p.n_tile) {
+                  float o = __uint_as_float(a[j]);
+                  if (bias != nullptr) o += bias[n0 + j];
+                  if (p.resid != nullptr) o += __bfloat162float(p.resid[base + n0 + j]);
+                  p.Y[base + n0 + j] = __float2bfloat16(o);
+                }
             }
-            if (p.silu) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const float z = __uint_as_float(a[j]);
-                a[j] = __float_as_uint(__fdividef(z, 1.f + __expf(-z)));
-              }
-            }
-            emit(p.Yn, c, a);
           }
         }
-      } else {
-        const long base = offset(quarter * 32 + lane);
-        if (!arrived && !mbar_wait_warp(&acc_full[acc], acc_ph, abort_flag)) { ok = false; break; }
-        arrived = true;
-        tc_fence_after();
-#pragma unroll 1
-        for (int c = c_lo; c < c_hi; ++c) {
-          uint32_t a[32];
-          tmem_ld32(t_row + c * 32, a);
-          tmem_ld_wait();
-          const int n0 = nt * p.n_tile + c * 32;
-          if (base >= 0) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (n0 + j < p.Cout && c * 32 + j < p.n_tile) {
-                float o = __uint_as_float(a[j]);
-                if (bias != nullptr) o += bias[n0 + j];
-                if (p.resid != nullptr) o += __bfloat162float(p.resid[base + n0 + j]);
-                p.Y[base + n0 + j] = __float2bfloat16(o);
-              }
-          }
-        }
-      }
       }
       if (!ok) break;
       tc_fence_before();
