@@ -9,9 +9,8 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-def _set_error():
+def _set_error(flags, lonely):
     """A peer barrier whose flag nobody sets: it gives up after a millisecond and reports 101."""
-    flags, lonely = (torch.zeros(64, dtype=torch.int32, device=DEV) for _ in range(2))
     native.load().peer_barrier([flags.data_ptr(), lonely.data_ptr()], 0, 1, 0, 1000)
 
 
@@ -25,8 +24,8 @@ def _conv():
 
 
 def _wide():
-    qkv = torch.randn(2, 600, 3, 384, device=DEV).bfloat16()
-    return lambda: native.load().fa_wide(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], 384 ** -0.5), 2 * 600 * 384
+    qkv = torch.randn(2, 1500, 3, 384, device=DEV).bfloat16()
+    return lambda: native.load().fa_wide(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], 384 ** -0.5), 2 * 1500 * 384
 
 
 def _attention():
@@ -41,13 +40,14 @@ def test_kernels_behind_an_error_return_at_once(case):
     want = run().clone()
     torch.cuda.synchronize()
     assert native.load().kernel_error(0, True) == 0
+    flags = [torch.zeros(64, dtype=torch.int32, device=DEV) for _ in range(2)]
     torch.cuda.empty_cache()
     marked = torch.full((n,), 7.0, dtype=torch.bfloat16, device=DEV)
     if case is _conv:
         run().fill_(7.0)
     else:
         del marked                                   # the output allocated next lies where the marks are
-    _set_error()
+    _set_error(*flags)
     begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
     begin.record()
     out = run()
