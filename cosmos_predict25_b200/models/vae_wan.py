@@ -317,14 +317,16 @@ class WanVAE_(nn.Module):
             # channels-last encoder on this package's convolution kernel; it keeps its own stream state
             if clear_encoder_cache or cl.state is None:
                 cl.reset()
-            run, step = lambda chunk, last: cl.step(chunk, last=last and clear_encoder_cache), tw * cl.windows_per_step(x.shape[-2], x.shape[-1], tw)
+            run, step = cl.step, tw * cl.windows_per_step(x.shape[-2], x.shape[-1], tw)
         else:
-            run, step = lambda chunk, last: self.encoder(chunk, st), tw
+            run, step = lambda chunk: self.encoder(chunk, st), tw
+        outs = [run(x[:, :, :1])]
         # only whole windows share a step: a remainder is a chunk of its own, so that whether its frames pass the temporal down-samplers
         # (and whether the call is refused) does not depend on how many windows a step takes
         end = 1 + (t - 1) // tw * tw
-        cuts = [0] + list(range(1, end, step)) + [end] + ([t] if end < t else [])
-        outs = [run(x[:, :, lo:hi], hi == t) for lo, hi in zip(cuts[:-1], cuts[1:])]
+        outs += [run(x[:, :, lo: min(lo + step, end)]) for lo in range(1, end, step)]
+        if end < t:
+            outs.append(run(x[:, :, end:]))
         if cl is not None and clear_encoder_cache:
             cl.state = None
         out = torch.cat(outs, 2)
@@ -354,7 +356,7 @@ class WanVAE_(nn.Module):
             # channels-last decoder on this package's convolution kernel; it keeps its own stream state
             if clear_decoder_cache or cl.state is None:
                 cl.reset()
-            outs = [cl.step(x[:, :, lo:hi], last=clear_decoder_cache and hi == z.shape[2]) for lo, hi in cl.steps(*z.shape[2:])]
+            outs = [cl.step(x[:, :, lo:hi]) for lo, hi in cl.steps(*z.shape[2:])]
             if clear_decoder_cache:
                 cl.state = None
                 self._dec_state = None

@@ -30,7 +30,7 @@ from ..ops import native
 from . import vae_parallel
 
 CACHE_T = 2
-STEP_BYTES = 3 << 29       # full-resolution activation of one streaming step (a step holds a handful of them, the stream two frames per layer)
+STEP_BYTES = 3 << 29       # full-resolution activation of one streaming step (a step holds a handful of them; the stream one per layer)
 
 
 def _n_tile(cout: int) -> int:
@@ -125,7 +125,7 @@ class ConvCL:
         prev = state.store.get(id(self))
         fused = norm if self.fuses_norm(x) else None
         y = self._launch(x, taps, t_out, H, W, None, None, resid, prev, pad_frames, fused, None, raw or fused is None)
-        state.keep(id(self), prev, x, pad_frames)
+        state.store[id(self)] = _last_frames(prev, x, pad_frames)
         return y if fused is not None else self._finish(y, norm, raw)
 
 
@@ -206,11 +206,6 @@ class _Stream:
 
     def __init__(self):
         self.store = {}
-        self.ends = False       # the step in progress is the stream's last: nothing is carried on
-
-    def keep(self, key, prev: Optional[torch.Tensor], x: torch.Tensor, n: int):
-        """Leaves the last ``n`` frames of [prev | x] under ``key`` for the next step."""
-        self.store[key] = None if self.ends else _last_frames(prev, x, n)
 
 
 def _with_cache(conv: ConvCL, x: torch.Tensor, state: _Stream, pad_frames: int = CACHE_T) -> torch.Tensor:
@@ -299,7 +294,7 @@ class _UpsampleCL(_Layer):
                 out = torch.empty(2 * T, H, W, C, dtype=x.dtype, device=x.device)
                 for s, conv in enumerate(self.time):
                     conv._launch(x, conv.taps, T, H, W, out, [2, s, 1, 0, 1, 0, H, W, C, 0], None, cache, CACHE_T)
-                state.keep(id(self._key), cache, x, CACHE_T)
+                state.store[id(self._key)] = _last_frames(cache, x, CACHE_T)
                 x = out
                 T = 2 * T
         cout = self.phases[0][0].cout
@@ -357,14 +352,12 @@ class DecoderCL:
         return list(zip(cuts[:-1], cuts[1:]))
 
     @torch.no_grad()
-    def step(self, x: torch.Tensor, last: bool = False) -> torch.Tensor:
-        """x [B=1, z, T, h, w] (already through the 1 x 1 ``conv2``) -> pixels [1, 3, T', 8h, 8w] for this chunk. ``last``: the
-        stream ends with it (the caller drops the state)."""
+    def step(self, x: torch.Tensor) -> torch.Tensor:
+        """x [B=1, z, T, h, w] (already through the 1 x 1 ``conv2``) -> pixels [1, 3, T', 8h, 8w] for this chunk."""
         assert x.shape[0] == 1, "the channels-last decoder runs one video at a time"
         if self.state is None:
             self.reset()
         st = self.state
-        st.ends = last
         T, h, w = x.shape[2:]
         xin = torch.zeros(T, h, w, self.z_pad, dtype=torch.bfloat16, device=self.device)
         xin[..., : self.z_dim] = x[0].permute(1, 2, 3, 0)
@@ -449,14 +442,12 @@ class EncoderCL:
         return max(1, STEP_BYTES // (window * H * W * self.conv1.cout * 2))
 
     @torch.no_grad()
-    def step(self, x: torch.Tensor, last: bool = False) -> torch.Tensor:
-        """x [1, 3, T, H, W] (one chunk) -> [1, 2 z, T', H / 8, W / 8] (input of the 1 x 1 ``conv1`` of the VAE). ``last`` as in the
-        decoder."""
+    def step(self, x: torch.Tensor) -> torch.Tensor:
+        """x [1, 3, T, H, W] (one chunk) -> [1, 2 z, T', H / 8, W / 8] (input of the 1 x 1 ``conv1`` of the VAE)."""
         assert x.shape[0] == 1, "the channels-last encoder runs one video at a time"
         if self.state is None:
             self.reset()
         st = self.state
-        st.ends = last
         T, H, W = x.shape[2:]
         xin = torch.zeros(T, H, W, self.in_pad, dtype=torch.bfloat16, device=self.device)
         xin[..., : self.cin] = x[0].permute(1, 2, 3, 0)
@@ -469,7 +460,7 @@ class EncoderCL:
 def encoder_supported(x: torch.Tensor) -> bool:
     """The kernel encoder serves bf16 CUDA videos, one at a time, whole frames (row-sharded encoding stays on the torch path),
     whose frames halve three times without a remainder (the kernel serves ragged tiles; 29 frames of 768 x 432, which are not whole
-    16 x 8 pixel tiles at the last level: 218 ms on torch convolutions, 44 ms here)."""
+    16 x 8 pixel tiles at the last level: 218 ms on torch convolutions, 69 ms here)."""
     return (x.is_cuda and x.dtype == torch.bfloat16 and x.shape[0] == 1 and x.shape[-2] % 8 == 0 and x.shape[-1] % 8 == 0
             and vae_parallel.active() is None and native.available() and hasattr(native.load(), "conv_cl")
             and not native.forward_mode())

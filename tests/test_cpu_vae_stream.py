@@ -17,29 +17,26 @@ class _Recorder:
     def reset(self):
         self.state = object()
 
-    def step(self, x, last=False):
+    def step(self, x):
         self.chunks.append(x.shape[2])
-        self.last = last
         return torch.zeros(1, 32, max(1, x.shape[2] // 4), x.shape[3] // 8, x.shape[4] // 8)
 
 
 @pytest.mark.parametrize("frames", [1, 4, 5, 7, 8, 9, 25, 27, 29])
 @pytest.mark.parametrize("windows", [1, 2, 6, 100])
 @pytest.mark.parametrize("window", [4, 8, 6])
-@pytest.mark.parametrize("clear", [True, False])
-def test_only_whole_windows_share_a_step(frames, windows, window, clear, monkeypatch):
+def test_only_whole_windows_share_a_step(frames, windows, window, monkeypatch):
     vae = vae_wan.WanVAE_(dim=8, z_dim=16, num_res_blocks=1, temporal_window=window).eval()
     rec = _Recorder(8)
     monkeypatch.setattr(vae, "_kernel_encoder", lambda x: rec)
     H, W = 16, 24
     monkeypatch.setattr(vae_wan_cl, "STEP_BYTES", windows * window * H * W * 8 * 2)
     with torch.no_grad():
-        vae.encode(torch.zeros(1, 3, frames, H, W), (0.0, 1.0), clear_encoder_cache=clear)
+        vae.encode(torch.zeros(1, 3, frames, H, W), (0.0, 1.0))
     whole, rest = divmod(frames - 1, window)
     per_step = windows if window % 4 == 0 else 1
     want = [1] + [min(per_step, whole - i) * window for i in range(0, whole, per_step)] + ([rest] if rest else [])
     assert rec.chunks == want
-    assert rec.last == clear                # a stream that goes on keeps its frames
 
 
 @pytest.mark.parametrize("n", [1, 2])
