@@ -30,7 +30,7 @@ from ..ops import native
 from . import vae_parallel
 
 CACHE_T = 2
-STEP_BYTES = 3 << 29       # full-resolution activation of one streaming step (a step holds a handful of them; the stream one per layer)
+STEP_BYTES = 3 << 29       # full-resolution activation of one streaming step (a step holds a handful of them, the stream two frames per layer)
 
 
 def _n_tile(cout: int) -> int:
@@ -460,7 +460,7 @@ class EncoderCL:
 def encoder_supported(x: torch.Tensor) -> bool:
     """The kernel encoder serves bf16 CUDA videos, one at a time, whole frames (row-sharded encoding stays on the torch path),
     whose frames halve three times without a remainder (the kernel serves ragged tiles; 29 frames of 768 x 432, which are not whole
-    16 x 8 pixel tiles at the last level: 218 ms on torch convolutions, 69 ms here)."""
+    16 x 8 pixel tiles at the last level: 218 ms on torch convolutions, 44 ms here)."""
     return (x.is_cuda and x.dtype == torch.bfloat16 and x.shape[0] == 1 and x.shape[-2] % 8 == 0 and x.shape[-1] % 8 == 0
             and vae_parallel.active() is None and native.available() and hasattr(native.load(), "conv_cl")
             and not native.forward_mode())

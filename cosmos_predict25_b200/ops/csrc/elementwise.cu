@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kThreads) gate_residual_bwd_kernel(
 // offset, so that the rotation partner of every element is in the lane itself and one cosine / sine vector serves both; reductions
 // stay inside the 16-lane half. Token and head of a row are counted along instead of divided out (64-bit divisions per row, a
 // shuffle per element and twice the table loads bound the earlier layout by instruction issue: 46,800 tokens x 16 heads 147 us,
-// now 90 us; the bytes take 59 us).
+// now 95 us; the bytes take 59 us).
 constexpr int kRmsPasses = 4;        // forward: passes (of two rows) whose loads a warp keeps in flight together
 
 template <int P>
