@@ -370,7 +370,7 @@ class WanVAE_(nn.Module):
         """The channels-last kernel encoder for this input, or None when the torch / cuDNN path has to serve it."""
         from ..ops import functional as F_ops
         from . import vae_wan_cl
-        if F_ops.settings.conv != "native" or not vae_wan_cl.encoder_supported(x):
+        if F_ops.settings.conv != "native" or not vae_wan_cl.encoder_supported(x, self.encoder):
             return None
         sig = tuple((p.data_ptr(), p._version) for p in self.encoder.parameters())
         if getattr(self, "_enc_cl", None) is None or self._enc_cl_sig != sig:

@@ -457,10 +457,40 @@ class EncoderCL:
         return y.permute(3, 0, 1, 2).unsqueeze(0)
 
 
-def encoder_supported(x: torch.Tensor) -> bool:
+def _restated(encoder) -> bool:
+    """Whether ``EncoderCL`` computes what the modules of this encoder would: the published layers, unhooked, without active dropout, and
+    channel counts that the kernels take."""
+    from . import vae_wan
+    known = (vae_wan.Encoder3d, vae_wan.ResidualBlock, vae_wan.AttentionBlock, vae_wan.Resample, vae_wan.CausalConv3d, vae_wan.RMS_norm,
+             torch.nn.Sequential, torch.nn.Conv2d, torch.nn.SiLU, torch.nn.Dropout, torch.nn.Identity, torch.nn.ZeroPad2d)
+    for m in encoder.modules():
+        if type(m) not in known or m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
+            return False
+        if isinstance(m, torch.nn.Dropout) and m.training and m.p > 0:
+            return False
+        if isinstance(m, vae_wan.RMS_norm) and (isinstance(m.bias, torch.Tensor) or m.gamma.numel() > 1024):
+            return False
+        if isinstance(m, (torch.nn.Conv2d, torch.nn.Conv3d)) and m is not encoder.conv1 and m.in_channels % 16:
+            return False
+    return True
+
+
+def _only_the_result_is_wanted(x: torch.Tensor, module) -> bool:
+    """No gradient, no functional transform, no tracing and no mode or global hook that would want to see the single operators."""
+    glob = torch.nn.modules.module
+    return (not (torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in module.parameters())))
+            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+            and torch._C._functorch.peek_interpreter_stack() is None and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+            and not glob._global_forward_hooks and not glob._global_forward_pre_hooks)
+
+
+def encoder_supported(x: torch.Tensor, encoder) -> bool:
     """The kernel encoder serves bf16 CUDA videos, one at a time, whole frames (row-sharded encoding stays on the torch path),
     whose frames halve three times without a remainder (the kernel serves ragged tiles; 29 frames of 768 x 432, which are not whole
-    16 x 8 pixel tiles at the last level: 218 ms on torch convolutions, 44 ms here)."""
-    return (x.is_cuda and x.dtype == torch.bfloat16 and x.shape[0] == 1 and x.shape[-2] % 8 == 0 and x.shape[-1] % 8 == 0
+    16 x 8 pixel tiles at the last level: 218 ms on torch convolutions, 44 ms here). Frames that are whole tiles always go there; for
+    the others the torch modules stay where their result can be differentiated, hooked or is made by other layers."""
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and x.shape[0] == 1 and x.shape[-2] % 8 == 0 and x.shape[-1] % 8 == 0
             and vae_parallel.active() is None and native.available() and hasattr(native.load(), "conv_cl")
-            and not native.forward_mode())
+            and not native.forward_mode()):
+        return False
+    return (x.shape[-2] % 64 == 0 and x.shape[-1] % 128 == 0) or (_restated(encoder) and _only_the_result_is_wanted(x, encoder))

@@ -51,3 +51,28 @@ def test_stream_keeps_the_last_frames_only(n, chunks):
         prev = vae_wan_cl._last_frames(prev, x, n)
         assert torch.equal(prev, frames[max(0, lo - n):lo]) and prev.is_contiguous()
         assert prev.untyped_storage().nbytes() <= n * frames[0].numel() * 4
+
+
+def test_what_the_kernel_encoder_restates():
+    """Channel counts, hooks, other layers and active dropout keep the torch modules."""
+    enc = lambda **kw: vae_wan.Encoder3d(dim=kw.pop("dim", 16), z_dim=8, num_res_blocks=1, **kw).eval()
+    ok = vae_wan_cl._restated
+    assert ok(enc()) and ok(enc(dim=96)) and ok(enc(attn_scales=(0.5,))) and ok(enc(dropout=0.1)) and ok(enc(dropout=0.0).train())
+    assert not ok(enc(dim=24)) and not ok(enc(dim=8)) and not ok(enc(dim=272)) and not ok(enc(dropout=0.1).train())
+    e = enc()
+    hook = e.middle[1].register_forward_hook(lambda *a: None)
+    assert not ok(e)
+    hook.remove()
+    assert ok(e)
+    e.head[2].forward = e.head[2].forward
+    assert not ok(e)
+    e = enc()
+    e.middle[0].residual[2] = torch.nn.utils.parametrizations.weight_norm(e.middle[0].residual[2])
+    assert not ok(e)
+    x, want = torch.zeros(1), vae_wan_cl._only_the_result_is_wanted
+    e = enc()
+    assert not want(x, e)
+    with torch.no_grad():
+        assert want(x, e)
+    e.requires_grad_(False)
+    assert want(x, e) and not want(x.clone().requires_grad_(True), e)

@@ -338,6 +338,43 @@ def test_clip_lengths_with_a_remainder_are_refused(frames, step_bytes, monkeypat
     _no_kernel_error()
 
 
+def test_ragged_frames_stay_on_torch_where_more_than_the_result_is_wanted():
+    """Frames that the kernel encoder came to serve last: gradients of pixels and weights, hooks and channel counts that the kernel does not
+    take still go through the torch modules."""
+    from cosmos_predict25_b200.models.vae_wan import WanVAE_
+    torch.manual_seed(15)
+    vae = WanVAE_(dim=16, z_dim=16, num_res_blocks=1).eval().requires_grad_(False).to(DEV).bfloat16()
+    x = torch.randn(1, 3, 5, 24, 40, device=DEV).clamp(-1, 1).bfloat16()
+    plain = vae.encode(x, (0.0, 1.0))
+    assert vae._enc_cl is not None
+    scale = plain.float().norm().item()
+    xg = x.clone().requires_grad_(True)
+    out = vae.encode(xg, (0.0, 1.0))
+    out.float().sum().backward()
+    assert xg.grad is not None and xg.grad.abs().sum().item() > 0
+    vae.requires_grad_(True)
+    vae.encode(x, (0.0, 1.0)).float().sum().backward()
+    assert vae.encoder.conv1.weight.grad is not None
+    vae.requires_grad_(False)
+    seen = []
+    hook = vae.encoder.middle[1].register_forward_hook(lambda m, a, o: seen.append(o.shape))
+    hooked = vae.encode(x, (0.0, 1.0))
+    hook.remove()
+    assert len(seen) == 2                                    # the first frame and one window
+    for y in (out.detach(), hooked):
+        assert (y.float() - plain.float()).norm().item() < 0.05 * scale
+    odd = WanVAE_(dim=24, z_dim=16, num_res_blocks=1).eval().requires_grad_(False).to(DEV).bfloat16()
+    assert odd.encode(x, (0.0, 1.0)).shape == plain.shape and getattr(odd, "_enc_cl", None) is None
+    small = vae.encode(x[..., :8, :8], (0.0, 1.0))           # one latent pixel
+    F_ops.settings.conv = "cudnn"
+    try:
+        want = vae.encode(x[..., :8, :8], (0.0, 1.0))
+    finally:
+        F_ops.settings.conv = "native"
+    assert small.shape == want.shape == (1, 16, 2, 1, 1) and (small.float() - want.float()).norm().item() < 0.05 * want.float().norm().item()
+    _no_kernel_error()
+
+
 @pytest.mark.parametrize("H,W,T", [(72, 104, 9), (24, 40, 5), (432, 136, 1)])
 def test_ragged_frames_are_encoded_by_the_kernel(H, W, T):
     """Frames that halve three times but are no whole tiles, against the torch encoder in fp32 (bounds of the whole-tile test above)."""
