@@ -2,6 +2,7 @@
 group, ragged rows, and groups whose tiles are few enough that clusters of CTA pairs share their contraction."""
 
 import math
+from dataclasses import replace
 
 import pytest
 import torch
@@ -47,14 +48,18 @@ def test_keys_and_values_of_all_blocks(B, S, C, D, split):
         assert torch.equal(got[2 * i], again[2 * i]) and torch.equal(got[2 * i + 1], again[2 * i + 1])
 
 
-# 264 to 520 tokens of the 1024-wide network: 12 to 36 tiles of q, k and v over 16 k-blocks, all of them split; 80 prompt rows and 256
-@pytest.mark.parametrize("shape,tokens", [((1, 1, 32, 32), 40), ((2, 1, 32, 32), 128), ((1, 1, 24, 88), 256), ((1, 2, 26, 40), 512)])
-def test_query_key_value_of_few_tiles(shape, tokens):
+# 256 to 528 tokens: 12 to 36 tiles of q, k and v over 16 k-blocks, all of them split; 80 prompt rows to 1,024. The other widths, the widest
+# with the row kernels for more than 4096 channels: few tokens, split and unsplit.
+@pytest.mark.parametrize("preset,shape,tokens,split", [("mini", (1, 1, 32, 32), 40, 4), ("mini", (2, 1, 32, 32), 128, 2), ("mini", (1, 1, 24, 88), 256, 2),
+                                                       ("mini", (1, 2, 26, 40), 512, 2), ("2b", (1, 1, 32, 32), 512, 2), ("2b", (1, 1, 8, 12), 24, None),
+                                                       ("2b", (2, 3, 32, 36), 40, 1), ("14b", (1, 1, 8, 8), 32, None), ("14b", (1, 3, 24, 32), 256, 1)])
+def test_query_key_value_of_few_tiles(preset, shape, tokens, split):
     """The native block loop against the module path, whose q, k and v are launches of their own: the same sums in another order, so a few
-    bf16 roundings (2^-9 each) through two blocks."""
+    bf16 roundings (2^-9 each) through the blocks."""
     torch.manual_seed(0)
+    make = {"mini": dit.dit_mini, "2b": dit.dit_2b, "14b": dit.dit_14b}[preset]
     with torch.device(DEV):
-        net = dit.CosmosDiT(dit.dit_mini(num_blocks=2, crossattn_proj_in_channels=512, crossattn_emb_channels=512))
+        net = dit.CosmosDiT(replace(make(), num_blocks=2 if preset != "14b" else 1, crossattn_proj_in_channels=512, crossattn_emb_channels=512))
     net.init_weights()
     for n, p in net.named_parameters():
         if "adaln_modulation" in n:
@@ -62,22 +67,29 @@ def test_query_key_value_of_few_tiles(shape, tokens):
     net = net.to(torch.bfloat16).eval().requires_grad_(False)
     B, T, H, W = shape
     rows, D = B * T * H * W // 4, net.cfg.model_channels
-    assert native.load().gemm_pairs_per_tile(-(-rows // 256) * (D // 256) * 3, D // 64, 74, 36, 16) > 1
+    if split is not None:                                       # below 256 rows q, k and v are launches of their own
+        assert native.load().gemm_pairs_per_tile(-(-rows // 256) * (D // 256) * 3, D // 64, 74, 36, 16) == split
     x, text = torch.randn(B, 16, T, H, W, device=DEV).bfloat16(), torch.randn(B, tokens, 512, device=DEV).bfloat16()
     t, fps = torch.rand(B, T, device=DEV) * 1000, torch.full((B,), 16.0, device=DEV)
+    served = []
+    real = dit.native_block_weights
 
     def run():
-        with torch.no_grad():
-            cache = net.build_context_cache(text)
-            return net(x, t, None, fps=fps, context_cache=cache), cache.cross_kv
+        dit.native_block_weights = lambda *a: served.append(real(*a)) or served[-1]
+        try:
+            with torch.no_grad():
+                cache = net.build_context_cache(text)
+                return net(x, t, None, fps=fps, context_cache=cache), cache.cross_kv
+        finally:
+            dit.native_block_weights = real
 
     got, kv = run()
-    hooks = [m.register_forward_hook(lambda *a: None) for m in (net.blocks[1].mlp.layer1, net.blocks[0].cross_attn.k_proj)]
+    hooks = [m.register_forward_hook(lambda *a: None) for m in (net.blocks[-1].mlp.layer1, net.blocks[0].cross_attn.k_proj)]
     want, kv_want = run()
     for h in hooks:
         h.remove()
     torch.cuda.synchronize()
-    assert native.load().kernel_error(0, True) == 0
+    assert native.load().kernel_error(0, True) == 0 and served[0] is not None and served[1] is None
     assert _rel(got, want.double()) < 4 * 2.0 ** -9
     for a, b in zip([t for p in kv for t in p], [t for p in kv_want for t in p]):
         assert _rel(a, b.double()) < 4 * 2.0 ** -9
