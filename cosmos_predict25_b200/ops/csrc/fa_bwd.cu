@@ -240,7 +240,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const float my_delta = (q_row < Sq_pad) ? delta[stat] : 0.f;
     bool ok = true;
     for (int j = 0; j < n_kv; ++j) {
-      if (!mbar_wait(&s_full[t], j & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(&s_full[t], j & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const int n_valid = Skv - j * 64;
       uint32_t pk[2][16];
@@ -270,7 +270,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       __syncwarp();
       if (lane == 0) mbar_arrive(&ds_ready[t]);
     }
-    if (ok) ok = mbar_wait(&s_full[t], n_kv & 1, abort_flag);
+    if (ok) ok = mbar_wait_warp(&s_full[t], n_kv & 1, abort_flag);
     if (ok) {
       tc_fence_after();
       bf16* orow = dQ + (((size_t)b * Sq + q_row) * H + h) * HD;
@@ -462,7 +462,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const float* del_bh = delta + ((size_t)b * H + h) * Sq_pad;
     bool ok = true;
     for (int i = u; i < n_q; i += 2) {
-      if (!mbar_wait(&s_full[u], (i >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(&s_full[u], (i >> 1) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const float4* l4 = reinterpret_cast<const float4*>(lse_bh + i * 64);
       const float4* d4 = reinterpret_cast<const float4*>(del_bh + i * 64);
@@ -503,7 +503,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_ready[u]);
     }
-    if (ok) ok = mbar_wait(done, 0, abort_flag);
+    if (ok) ok = mbar_wait_warp(done, 0, abort_flag);
     if (ok) {
       tc_fence_after();
       // warps 0-3 write dV, warps 4-7 write dK (scaled)

@@ -291,7 +291,7 @@ fa_bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     const uint32_t tY = tmem_base + Y + ((uint32_t)(quarter * 32) << 16);
     bool ok = true;
     for (int i = 0; i < n_q; ++i) {
-      if (!mbar_wait(dq_full, i & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(dq_full, i & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
 #pragma unroll 1
       for (int half = 0; half < 2; ++half) {
@@ -365,8 +365,8 @@ fa_bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           }
         }
       }
-      if (!mbar_wait(&st_full[ss], (i >> 1) & 1, abort_flag)) { ok = false; break; }
-      if (!mbar_wait(s_full, par, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(&st_full[ss], (i >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(s_full, par, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const float4* l4 = reinterpret_cast<const float4*>(sStat + ss * 256 + cg * 32);   // -lse * log2(e)
       const float4* d4 = l4 + 32;                                                       // -delta
@@ -405,7 +405,7 @@ fa_bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       if (lane == 0) mbar_arrive(p_ready);
 
       // ---- phase 2: dS^T = P^T o (dP^T - delta) -> shared memory
-      if (!mbar_wait(dp_full, par, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(dp_full, par, abort_flag)) { ok = false; break; }
       tc_fence_after();
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
@@ -439,7 +439,7 @@ fa_bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         mbar_arrive(&st_empty[ss]);
       }
     }
-    if (ok && n_q > 0) ok = mbar_wait(done, 0, abort_flag);
+    if (ok && n_q > 0) ok = mbar_wait_warp(done, 0, abort_flag);
     if (ok) {
       tc_fence_after();
       // warps with cg 0,1 write dV, cg 2,3 write dK (scaled); the two warps of a lane quarter take 64 columns each

@@ -338,7 +338,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 #pragma unroll
         for (int c = 0; c < 4; ++c) vis[c] = ((mt >> c) & 1u) ? plane : 0u;
       }
-      if (!mbar_wait(&s_full[t], j & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(&s_full[t], j & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       uint32_t r[4][32];
       tmem_ld32(tS, r[0]);
@@ -424,7 +424,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_ready[t]);
     }
-    if (ok) ok = mbar_wait(&s_full[t], n_kv & 1, abort_flag);
+    if (ok) ok = mbar_wait_warp(&s_full[t], n_kv & 1, abort_flag);
     if (ok) {
       tc_fence_after();
       const float inv_l = 1.f / l;

@@ -220,7 +220,7 @@ fa_jvp_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     float mu = 0.f;
     bool ok = true;
     for (int j = u; j < n_kv; j += 2) {
-      if (!mbar_wait(&s_full[u], (j >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(&s_full[u], (j >> 1) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const int kv0 = j * 64;
       const bool ragged = kv0 + 64 > Skv;
@@ -259,7 +259,7 @@ fa_jvp_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     sMu[u * 128 + row] = mu;
     asm volatile("bar.sync 1, 256;" ::: "memory");   // the eight element-wise warps
     const float mu_all = sMu[row] + sMu[128 + row];
-    if (ok) ok = mbar_wait(done, 0, abort_flag);
+    if (ok) ok = mbar_wait_warp(done, 0, abort_flag);
     if (ok) {
       tc_fence_after();
       // group 0 reads out columns [0,64), group 1 [64,128):  to = OT - mu * o

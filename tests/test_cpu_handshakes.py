@@ -138,15 +138,23 @@ def test_backward_warps_leave_together():
     assert loop.count("give_up(") == 2 and "mbar_wait(" not in loop
 
 
-@pytest.mark.parametrize("name", ["conv3d_cl.cu", "fa_wide.cu", "gemm_tcgen05.cu"])
-def test_waits_in_front_of_collective_instructions_are_the_warps(name):
-    """A wait may run out for some lanes of a warp only. Loads from tensor memory and cluster barriers need every lane, so outside the
-    producer, which is one lane, a warp waits as a whole."""
-    code = (CSRC / name).read_text().split(" TMA producer\n")[1]
-    producer, rest = code.split("// ----", 1)
-    assert producer.lstrip().startswith(("if (lane == 0)", "// one thread")) and "mbar_wait(" in producer
-    waits = [line for line in rest.splitlines() if "mbar_wait(" in line]
-    assert all("__all_sync(0xffffffffu, mbar_wait(" in line for line in waits), waits
+@pytest.mark.parametrize("path", [p for p in sorted(CSRC.glob("*.cu")) if "tmem_ld" in p.read_text()], ids=lambda p: p.name)
+def test_waits_in_front_of_collective_instructions_are_the_warps(path):
+    """A wait may run out for some lanes of a warp only. Loads from tensor memory and cluster barriers need every lane, so a warp waits as
+    a whole; a plain wait belongs to code that one lane runs."""
+    lines = path.read_text().splitlines()
+    assert any("mbar_wait" in line for line in lines)
+    for n, line in enumerate(lines):
+        if "mbar_wait(" not in line or "__all_sync(0xffffffffu, mbar_wait(" in line:
+            continue
+        depth = len(line) - len(line.lstrip())
+        for above in reversed(lines[:n]):                       # the statement that opens the nearest enclosing role
+            d = len(above) - len(above.lstrip())
+            if above.strip() and above[0] != "#" and d < depth:
+                depth = d
+                if "lane == 0" in above or "else if (warp" in above or "} else {" in above:
+                    break
+        assert "if (lane == 0) {" in above, f"{path.name}:{n + 1} waits lane by lane"
 
 
 def _early_kernels():
