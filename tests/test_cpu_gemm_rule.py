@@ -2,7 +2,11 @@
 
 import itertools
 
+import pytest
+
 from cosmos_predict25_b200.ops import native
+
+pytestmark = pytest.mark.skipif(not native.available(), reason="the extension is not built")
 
 
 def _rule(*a):
