@@ -557,7 +557,7 @@ extern "C" int cb200_fa_bwd_fused_main(const void* d_o, const void* q, const voi
 extern "C" int cb200_fa_bwd_tile_main(const void* d_o, const void* q, const void* k, const void* v, const float* lse2,
                                       const float* delta, float* dq_acc, void* dk, void* dv, int B, int Sq, int Skv, int H, int S_pad,
                                       float scale, int* err, cudaStream_t st);
-extern "C" void cb200_fa_bwd_dq_convert(const float* acc, void* dq, int B, int S, int H, float scale, cudaStream_t st);
+extern "C" void cb200_fa_bwd_tile_dq_convert(const float* acc, void* dq, int B, int S, int H, float scale, cudaStream_t st);
 
 // variant 0: choose by problem size; 1: two deterministic kernels (7 GEMMs, no atomics); 2: single pass over 128 x 64 sub-tiles with
 // fp32 dQ accumulation (5 GEMMs); 3: single pass over 128 x 128 tiles (5 GEMMs, every MMA N = 128)
@@ -567,7 +567,7 @@ static bool fa_bwd_use_fused(int Skv, int variant) { return fa_bwd_pick(Skv, var
 extern "C" long cb200_fa_bwd_scratch_floats_v(int B, int Sq, int Skv, int H, int variant) {
   const long S_pad = (Sq + 127) / 128 * 128;
   long n = 2L * B * H * S_pad;
-  if (fa_bwd_use_fused(Skv, variant)) n += (long)B * Sq * H * 128;
+  if (fa_bwd_use_fused(Skv, variant)) n += (long)B * H * (fa_bwd_pick(Skv, variant) == 3 ? S_pad : Sq) * 128;
   return n;
 }
 
@@ -604,7 +604,7 @@ extern "C" int cb200_fa_bwd_v(const void* d_o, const void* q, const void* k, con
     float* acc = scratch + 2 * (size_t)B * H * S_pad;
     const int rc = cb200_fa_bwd_tile_main(d_o, q, k, v, lse2, delta, acc, dk, dv, B, Sq, Skv, H, S_pad, scale, err, st);
     if (rc) return rc;
-    cb200_fa_bwd_dq_convert(acc, dq, B, Sq, H, scale, st);
+    cb200_fa_bwd_tile_dq_convert(acc, dq, B, Sq, H, scale, st);
     return (int)cudaGetLastError();
   }
   if (fa_bwd_use_fused(Skv, variant))
@@ -665,6 +665,6 @@ extern "C" int cb200_fa_bwd_na(const void* d_o, const void* q, const void* k, co
   const int rc = cb200_fa_bwd_tile_na(d_o, q, k, v, lse2, delta, acc, dk, dv, B, S, H, scale, q_list, q_cnt, max_n, bt, bh, bw, nT, nH, nW,
                                       err, st);
   if (rc) return rc;
-  cb200_fa_bwd_dq_convert(acc, dq, B, S, H, scale, st);
+  cb200_fa_bwd_tile_dq_convert(acc, dq, B, S, H, scale, st);
   return (int)cudaGetLastError();
 }

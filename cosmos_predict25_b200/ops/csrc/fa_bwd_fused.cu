@@ -409,11 +409,6 @@ __global__ void __launch_bounds__(256) fa_bwd_dq_convert_kernel(const float* __r
 
 using namespace cb200;
 
-extern "C" void cb200_fa_bwd_dq_convert(const float* acc, void* dq, int B, int S, int H, float scale, cudaStream_t st) {
-  const long n8 = (long)B * S * H * 16;
-  fa_bwd_dq_convert_kernel<<<(unsigned)std::min<long>((n8 + 255) / 256, 148 * 16), 256, 0, st>>>(acc, (bf16*)dq, B, S, H, scale);
-}
-
 // Runs after the preprocessing kernel has produced lse2 / delta (padded to S_pad rows per (b, h)).
 // dq_acc: B*Sq*H*128 floats of scratch, zeroed here.
 extern "C" int cb200_fa_bwd_fused_main(const void* d_o, const void* q, const void* k, const void* v, const float* lse2,
