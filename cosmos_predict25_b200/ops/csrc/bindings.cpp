@@ -593,9 +593,9 @@ TORCH_LIBRARY(cosmos_b200, m) {
         });
   m.def("skinny_bgemm(Tensor a, int a_z, int a_r, int a_k, Tensor? b_ptrs, Tensor? b, int b_z, int b_n, int b_k, bool b_bf16, "
         "Tensor? add, int add_cols, int Z, int R, int N, int K, bool silu_a, bool silu_b, bool out_bf16, int ksplit) -> Tensor", &skinny_bgemm);
-  m.def("gemm_pairs_per_tile(int tiles, int k_blocks, int pairs, int clusters2, int clusters4) -> int",
-        [](int64_t tiles, int64_t kb, int64_t pairs, int64_t c2, int64_t c4) {
-          return (int64_t)cb200_gemm_pairs_per_tile((long)tiles, (long)kb, (int)pairs, (int)c2, (int)c4);
+  m.def("gemm_pairs_per_tile(int tiles, int k_blocks, int pairs, int clusters2, int clusters4, int clusters3=0) -> int",
+        [](int64_t tiles, int64_t kb, int64_t pairs, int64_t c2, int64_t c4, int64_t c3) {
+          return (int64_t)cb200_gemm_pairs_per_tile((long)tiles, (long)kb, (int)pairs, (int)c2, (int)c4, (int)c3);
         });
   m.def("gemm_group_launches(int rows, int groups) -> int",
         [](int64_t rows, int64_t groups) { return (int64_t)cb200_gemm_group_launches((int)rows, (int)groups); });

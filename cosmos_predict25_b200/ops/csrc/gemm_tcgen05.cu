@@ -2,7 +2,7 @@
 //
 // Persistent, warp-specialised kernel, one CTA per SM, in three forms:
 //   CTA pairs (from 256 rows on): clusters of two CTAs work on a 256 x 256 tile with cta_group::2 MMAs, six 32 KB stages; a cluster of two
-//            or four pairs shares a tile where there are few of them (see the kernel below);
+//            to four pairs shares a tile where there are few of them (see the kernel below);
 //   single CTAs (fewer rows, and the gather mode): 128 x 256 tiles, four 48 KB stages.
 // Roles: warp 0 is the TMA producer (128x64 A tiles and 256x64 B tiles, 128-byte swizzle, through the ring of stages; completion by
 //   mbarrier transaction bytes), warp 1 issues tcgen05.mma from shared-memory descriptors into one of two 128x256 fp32 accumulators
@@ -45,6 +45,7 @@ constexpr int kABytes = BM * BK * 2;  // 16 KB
 constexpr int kBBytes = BN * BK * 2;  // 32 KB
 constexpr int kStageBytes = kABytes + kBBytes;
 constexpr int kGemmThreads = 320;  // TMA warp, MMA warp, 8 epilogue warps (two per TMEM lane quarter, 128 columns each)
+constexpr int kPrefetchBlocks = 8;    // k-blocks of the first tile's B operand asked into L2 ahead of the wait
 constexpr int kStageOutBytes = 8 * 32 * 128;  // one 32-row x 128-byte staging block per epilogue warp
 constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + 1024 /*alignment slack*/ + 256 /*barriers*/ + kStageOutBytes;
 
@@ -115,7 +116,7 @@ __device__ __forceinline__ void red_release_gpu_add(int* p, int v) {
 // SPLIT > 1: a cluster of SPLIT pairs works on ONE tile, each pair on its share of the contraction dimension, for outputs of so few
 // tiles that most of the GPU would idle while a handful of SMs pull the operands (a 512 x 2048 output is 16 tiles: 32 SMs fetch 1 MB
 // each at K = 2048). The fp32 partial tiles are exchanged through distributed shared memory - pair s receives the SPLIT - 1 other
-// partials of its 256 / SPLIT columns in the shared memory that the operand ring no longer needs - added in a fixed order (the
+// partials of its share of the columns (in units of 64) in the shared memory that the operand ring no longer needs - added in a fixed order (the
 // result is deterministic) and put back into TMEM, from where the ordinary epilogue finishes those columns.
 template <int A_MN, int B_MN, bool GATHER, bool CTA2 = false, int SPLIT = 1>
 __global__ void __launch_bounds__(kGemmThreads + (GATHER ? kGatherWarps * 32 : 0), 1)
@@ -125,7 +126,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   static_assert(!(CTA2 && GATHER), "the gather mode runs on single-CTA tiles");
-  static_assert(SPLIT == 1 || (CTA2 && (SPLIT == 2 || SPLIT == 4)), "split tiles: clusters of two or four pairs");
+  static_assert(SPLIT == 1 || (CTA2 && SPLIT >= 2 && SPLIT <= 4), "split tiles: clusters of two to four pairs");
+  // SPLIT > 1: pair s finishes the 64-column units [unit_first(s), unit_first(s + 1)) of the tile: two each, two / one / one, one each
+  auto unit_first = [](int s) -> int { return SPLIT == 3 ? (s == 0 ? 0 : s + 1) : s * 4 / SPLIT; };
   constexpr int STG = CTA2 ? 6 : kStages;                                   // pipeline stages
   constexpr int STG_BYTES = CTA2 ? (kABytes + kBBytes / 2) : kStageBytes;   // bytes per stage in this CTA
   constexpr int TM = CTA2 ? 2 * BM : BM;                                    // output rows per tile (per pair with CTA2)
@@ -179,6 +182,24 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const uint32_t tmem_base = *tmem_slot;
   if (CTA2) {                        // launched with programmatic serialisation (see common.cuh)
     pdl_trigger();
+    if (warp == 0 && lane == 0) {
+      // The first tile's B operand, as a rule a weight that only HBM holds, on its way into L2 while the kernel in front still runs.
+      prefetch_tmap(&tma_a);
+      prefetch_tmap(&tma_b);
+      const int grp = first_tile % tiles_n / tiles_g;
+      const CUtensorMap* tb = grp > 0 ? (grp == 1 ? &tma_b1 : &tma_b2) : &tma_b;
+      const int n0 = (first_tile % tiles_n - grp * tiles_g) * BN + (int)pair_rank * (BN / 2);
+      const int ahead = min(k_blocks, kPrefetchBlocks);
+      for (int kb = 0; kb < ahead; ++kb) {
+        const int k0 = (kb_first + kb) * BK;
+        if (B_MN == 0) {
+          tma_prefetch_l2_2d(tb, k0, n0);
+        } else {
+#pragma unroll
+          for (int j = 0; j < BN / 128; ++j) tma_prefetch_l2_2d(tb, n0 + j * 64, k0);
+        }
+      }
+    }
     pdl_wait();
   }
 
@@ -363,12 +384,33 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     uint32_t acc_ph = 0;
     bool ok = true;
     const bool vec_ok = (N % 8) == 0;
+    // SPLIT > 1: the 64-column unit of the tile that this warp finishes; the two warps of a lane quarter share the pair's slice
+    constexpr int kSliceMax = SPLIT == 4 ? 64 : 128;
+    const int my_unit = SPLIT > 1 && unit_first(split) + part < unit_first(split + 1) ? unit_first(split) + part : -1;
+    // Gated residual: the rows of the residual that a pass of 64 columns needs are fetched ahead - the first pass's while the tile's
+    // products are still being summed, the next one's while this one is finished - and the gate of 32 columns is one batch of loads.
+    // Loaded where they were used, a tile paid their latency once per 16 bytes: 46,800 x 2048 x 2048 400 us, now 270 (the plain product
+    // 255), 7040 x 2048 x 2048 74 and 51 us, 512 x 2048 x 2048 22.0 and 15.5 us.
+    auto fetch_resid = [&](uint4 (&ahead)[8], int row0, int colbase) {
+#pragma unroll
+      for (int it = 0; it < 8; ++it) {
+        const int r = row0 + it * 4 + (lane >> 3);
+        ahead[it] = make_uint4(0, 0, 0, 0);
+        if (r < M) ahead[it] = *reinterpret_cast<const uint4*>(ep.resid + (size_t)r * N + colbase + (lane & 7) * 8);
+      }
+    };
     const uint32_t acc_empty_leader[2] = {CTA2 ? mapa_shared(smem_u32(&acc_empty[0]), lead_rank) : 0u,
                                           CTA2 ? mapa_shared(smem_u32(&acc_empty[1]), lead_rank) : 0u};
     for (int t = first_tile; t < n_tiles && ok; t += tile_step) {
       const int grp = CTA2 ? t % tiles_n / tiles_g : 0;
       bf16* const out = CTA2 && grp > 0 ? (grp == 1 ? ep.C1 : ep.C2) : ep.C;
       const int m0 = (t / tiles_n) * TM + (CTA2 ? (int)pair_rank * BM : 0), n0 = (t % tiles_n - grp * tiles_g) * BN;
+      const bool whole = vec_ok && n0 + BN <= N;            // a tile of full width: vector accesses through the staging block
+      uint4 ahead[8];
+#pragma unroll
+      for (int it = 0; it < 8; ++it) ahead[it] = make_uint4(0, 0, 0, 0);
+      if (whole && ep.gate != nullptr && ep.hs.P == 0 && (SPLIT == 1 || my_unit >= 0))
+        fetch_resid(ahead, m0 + quarter * 32, n0 + (SPLIT > 1 ? my_unit * 64 : part * 128));
       ok = mbar_wait_warp(&acc_full[acc], acc_ph, abort_flag);
       if (SPLIT == 1 && !ok) break;
       tc_fence_after();
@@ -377,20 +419,20 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       if (SPLIT > 1) {
         // One tile per cluster: this code runs once. Block (src, float4 column g of the slice) of the receiving CTA holds 128 rows x
         // 16 bytes, so that the lanes of a warp write and read 512 contiguous bytes.
-        constexpr int kSlice = BN / SPLIT;
         const int r_tile = quarter * 32 + lane;
         __syncwarp();
         cluster_sync_all();            // every pair's MMAs are complete: the operand rings are free
         if (ok) {
 #pragma unroll 1
           for (int c = part * 4; c < part * 4 + 4; ++c) {
-            const int dst = c * 32 / kSlice;
+            int dst = SPLIT - 1;       // the pair that finishes this 32-column chunk
+            while (unit_first(dst) * 2 > c) --dst;
             if (dst == split) continue;
             uint32_t r[32];
             tmem_ld32(t_row + c * 32, r);
             tmem_ld_wait();
             const uint32_t base = mapa_shared(smem_u32(smem), (uint32_t)(2 * dst) + pair_rank) +
-                                  (uint32_t)((split * (kSlice / 4) + (c * 32 - dst * kSlice) / 4) * (BM * 16) + r_tile * 16);
+                                  (uint32_t)((split * (kSliceMax / 4) + (c * 32 - unit_first(dst) * 64) / 4) * (BM * 16) + r_tile * 16);
 #pragma unroll
             for (int q = 0; q < 8; ++q)
               st_cluster_v4(base + q * (BM * 16), __uint_as_float(r[q * 4]), __uint_as_float(r[q * 4 + 1]), __uint_as_float(r[q * 4 + 2]),
@@ -400,9 +442,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         __syncwarp();
         cluster_sync_all();            // every partial has arrived
         if (!ok) break;
-        if (part != split * kSlice / 128) break;      // the slice's columns belong to the warps of one half
+        if (my_unit < 0) break;        // no unit left for this warp
 #pragma unroll 1
-        for (int c = split * kSlice / 32; c < (split + 1) * kSlice / 32; ++c) {
+        for (int c = my_unit * 2; c < my_unit * 2 + 2; ++c) {
           uint32_t own[32];
           tmem_ld32(t_row + c * 32, own);
           tmem_ld_wait();
@@ -415,7 +457,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 #pragma unroll
               for (int j = 0; j < 32; ++j) sum[j] += __uint_as_float(own[j]);
             } else {
-              const uint8_t* in = smem + (src * (kSlice / 4) + (c * 32 - split * kSlice) / 4) * (BM * 16) + r_tile * 16;
+              const uint8_t* in = smem + (src * (kSliceMax / 4) + (c * 32 - unit_first(split) * 64) / 4) * (BM * 16) + r_tile * 16;
 #pragma unroll
               for (int q = 0; q < 8; ++q) {
                 const float4 f = *reinterpret_cast<const float4*>(in + q * (BM * 16));
@@ -555,7 +597,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         continue;
       }
       const float* gate_row = (ep.gate != nullptr && row < M) ? ep.gate + (size_t)(row / ep.L) * ep.ld_gate : nullptr;
-      if (vec_ok && n0 + BN <= N) {
+      if (whole) {
         // ---- full-width tile: every global access of the epilogue goes through the warp's 4 KB staging block, so that a
         // warp instruction moves four contiguous 128-byte row segments instead of 32 scattered 16-byte pieces (the scattered
         // form made K = 2048 GEMMs epilogue-bound).  This warp owns 128 columns: two passes of 64; TMEM loads stay
@@ -582,9 +624,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           }
         };
 #pragma unroll 1
-        for (int pass = 0; pass < 2; ++pass) {
-          const int coff = part * 128 + pass * 64;              // column offset inside the tile
-          if (SPLIT == 4 && coff != split * 64) continue;       // this pair finishes 64 columns (with SPLIT 2: the 128 of this warp)
+        for (int pass = 0; pass < (SPLIT > 1 ? 1 : 2); ++pass) {
+          const int coff = SPLIT > 1 ? my_unit * 64 : part * 128 + pass * 64;   // column offset inside the tile
           const int colbase = n0 + coff;
           if (ep.pre != nullptr && (ep.act == 1 || ep.gate != nullptr)) {
             // second output first (TMEM is read again below): the pre-activation of a GELU, or the plain product of a
@@ -605,25 +646,24 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             }
             write_out(ep.pre, colbase);
           }
-          if (ep.gate != nullptr) {                             // residual rows in, coalesced
-#pragma unroll 4
+          if (ep.gate != nullptr) {                             // residual rows, fetched coalesced
+#pragma unroll
             for (int it = 0; it < 8; ++it) {
               const int r_src = it * 4 + (lane >> 3), chunk = lane & 7;
-              uint4 v4 = make_uint4(0, 0, 0, 0);
-              if (row0 + r_src < M) v4 = *reinterpret_cast<const uint4*>(ep.resid + (size_t)(row0 + r_src) * N + colbase + chunk * 8);
-              *reinterpret_cast<uint4*>(stage_warp + r_src * 128 + ((chunk ^ (r_src & 7)) << 4)) = v4;
+              *reinterpret_cast<uint4*>(stage_warp + r_src * 128 + ((chunk ^ (r_src & 7)) << 4)) = ahead[it];
             }
             __syncwarp();
+            if (SPLIT == 1 && pass == 0) fetch_resid(ahead, row0, colbase + 64);
           }
 #pragma unroll 1
           for (int c = 0; c < 2; ++c) {
+            const int col0 = colbase + c * 32;
             uint32_t r[32];
             tmem_ld32(t_row + coff + c * 32, r);
             tmem_ld_wait();
             float v[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-            const int col0 = colbase + c * 32;
             if (ep.bias != nullptr) {
 #pragma unroll
               for (int j = 0; j < 32; ++j) v[j] += __bfloat162float(ep.bias[col0 + j]);
@@ -633,16 +673,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
               for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
             }
             if (ep.gate != nullptr) {
+              float4 g4[8];                                     // all of the chunk's gate values at once: one latency
+#pragma unroll
+              for (int q = 0; q < 8; ++q)
+                g4[q] = gate_row != nullptr ? *reinterpret_cast<const float4*>(gate_row + col0 + q * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
               for (int q = 0; q < 4; ++q) {
                 const uint4 rr = *reinterpret_cast<const uint4*>(stage_row + (((c * 4 + q) ^ (lane & 7)) << 4));
                 const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rr);
-                float g[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                if (gate_row != nullptr) {
-                  const float4 g0 = *reinterpret_cast<const float4*>(gate_row + col0 + q * 8);
-                  const float4 g1 = *reinterpret_cast<const float4*>(gate_row + col0 + q * 8 + 4);
-                  g[0] = g0.x; g[1] = g0.y; g[2] = g0.z; g[3] = g0.w; g[4] = g1.x; g[5] = g1.y; g[6] = g1.z; g[7] = g1.w;
-                }
+                const float4 g0 = g4[2 * q], g1 = g4[2 * q + 1];
+                const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                   const float2 rf = __bfloat1622float2(r2[j]);
@@ -852,12 +892,13 @@ static int launch_gemm_pairs(const void* A, const void* const* B, int M, int N, 
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
 
-// One tile per pair, or clusters of 2 or 4 pairs per tile: whichever takes fewer k-blocks in a row, waves counted, with kExchange
-// k-blocks' time for the exchange of partial tiles. Six k-blocks: measured 9.1 us against 7.0 us of fixed time, 0.3 us a k-block. Launches
-// back to back, one pair per tile and split: 512 x 2048 from K = 2048 18.7 and 13.1 us, from K = 8192 46.9 and 26.7; 1024 x 1024 from
-// K = 100,352 (the text projection) 460 and 229 us. `c2`, `c4`: clusters of 2 and 4 pairs that the GPU holds at once; where it holds
-// none the split is not taken.
-extern "C" int cb200_gemm_pairs_per_tile(long tiles, long kb, int pairs, int c2, int c4) {
+// One tile per pair, or clusters of 2 to 4 pairs per tile: whichever takes fewer k-blocks in a row, waves counted, with kExchange
+// k-blocks' time for the exchange of partial tiles, twice that for three pairs (0.27 us a k-block; two pairs 2.4 to 2.9 us, three 4.3).
+// Launches back to back with one, two and three pairs per tile: 512 x 2048 from K = 2048 16.0, 14.1, 14.6 us, from K = 8192 43.8, 29.1,
+// 25.2 us; 1024 x 1024 from K = 100,352 (the text projection) 449, 230, 181 us. A B200 holds 33 clusters of two pairs, 22 of three and 15
+// or 16 of four: for 16 tiles (512 x 2048) four pairs are one wave on some of them and two on the others (38.9 us at K = 8192).
+// `c2`, `c4`, `c3`: clusters of 2, 4 and 3 pairs that the GPU holds at once; where it holds none the split is not taken.
+extern "C" int cb200_gemm_pairs_per_tile(long tiles, long kb, int pairs, int c2, int c4, int c3) {
   if (2 * tiles > pairs || kb < 8) return 1;
   constexpr long kExchange = 6;
   long best = kb;
@@ -865,6 +906,10 @@ extern "C" int cb200_gemm_pairs_per_tile(long tiles, long kb, int pairs, int c2,
   if (c2 > 0 && (tiles + c2 - 1) / c2 * ((kb + 1) / 2 + kExchange) < best) {
     best = (tiles + c2 - 1) / c2 * ((kb + 1) / 2 + kExchange);
     split = 2;
+  }
+  if (c3 > 0 && (tiles + c3 - 1) / c3 * ((kb + 2) / 3 + 2 * kExchange) < best) {
+    best = (tiles + c3 - 1) / c3 * ((kb + 2) / 3 + 2 * kExchange);
+    split = 3;
   }
   if (c4 > 0 && (tiles + c4 - 1) / c4 * ((kb + 3) / 4 + kExchange) < best + (split == 2 ? 1 : 0)) split = 4;
   return split;
@@ -874,11 +919,13 @@ template <int A_MN, int B_MN>
 static int launch_gemm_any(const void* A, const void* const* B, int M, int N, int K, const GemmEpilogue& ep, int* err, int sms, cudaStream_t st) {
   const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) * ep.groups, kb = (K + BK - 1) / BK;
   const int pairs = sms / 2;
-  int c1 = 0, c2 = 0, c4 = 0, rc;
+  int c1 = 0, c2 = 0, c3 = 0, c4 = 0, rc;
   if (N % BN == 0 && ep.hs.P == 0 && 2 * tiles <= pairs) {
-    if ((rc = resident_clusters<A_MN, B_MN, 2>(&c2)) || (rc = resident_clusters<A_MN, B_MN, 4>(&c4))) return rc;
-    const int split = cb200_gemm_pairs_per_tile(tiles, kb, pairs, c2, c4);
+    if ((rc = resident_clusters<A_MN, B_MN, 2>(&c2)) || (rc = resident_clusters<A_MN, B_MN, 3>(&c3)) || (rc = resident_clusters<A_MN, B_MN, 4>(&c4)))
+      return rc;
+    const int split = cb200_gemm_pairs_per_tile(tiles, kb, pairs, c2, c4, c3);
     if (split == 4) return launch_gemm_pairs<A_MN, B_MN, 4>(A, B, M, N, K, ep, (int)tiles, err, st);
+    if (split == 3) return launch_gemm_pairs<A_MN, B_MN, 3>(A, B, M, N, K, ep, (int)tiles, err, st);
     if (split == 2) return launch_gemm_pairs<A_MN, B_MN, 2>(A, B, M, N, K, ep, (int)tiles, err, st);
   }
   // A persistent grid must be resident as a whole: the pairs that the GPU can hold at once (a pair lives inside one GPC, so a

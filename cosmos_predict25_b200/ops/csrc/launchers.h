@@ -58,7 +58,7 @@ int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
                     int act, void* pre, const void* resid, const float* gate, long ld_gate, int L, int* err, int sms, cudaStream_t st);
 int cb200_gemm_bf16_group(const void* A, const void* const* B, void* const* C, int groups, int M, int N, int K, int* err, int sms, cudaStream_t st);
 int cb200_gemm_group_launches(int M, int groups);
-int cb200_gemm_pairs_per_tile(long tiles, long kb, int pairs, int c2, int c4);   // 1, 2 or 4 CTA pairs share a tile's contraction
+int cb200_gemm_pairs_per_tile(long tiles, long kb, int pairs, int c2, int c4, int c3);   // 1 to 4 CTA pairs share a tile's contraction
 int cb200_gemm_pair_mode(int mode);   // 0 / 1 sets, -1 reads; returns the previous mode (1 = CTA-pair tiles where the shape allows)
 int cb200_gemm_bf16_gather(const void* A, void* ws, void* C, int M, int rows, int ld, int b_mn, const int64_t* shard_ptrs, int P,
                            int chunk_rows, int* counters, const void* bias, int act, void* pre, int* err, int sms, cudaStream_t st);
