@@ -716,7 +716,7 @@ class CosmosDiT(nn.Module):
         if not weights:
             return None
         kv = native.load().dit_context_kv(ctx, weights, eps)
-        native.count_launch((1 + native.load().gemm_group_launches(ctx.shape[0] * ctx.shape[1], 2)) * len(self.blocks))
+        native.count_launch(native.load().dit_context_launches(ctx.shape[0] * ctx.shape[1], ctx.shape[2], [w.shape[0] for w in weights[::3]]))
         return list(zip(kv[0::2], kv[1::2]))
 
     def _embed(self, x_B_C_T_H_W, condition_mask, padding_mask):

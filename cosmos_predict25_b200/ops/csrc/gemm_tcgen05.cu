@@ -68,13 +68,23 @@ __device__ __forceinline__ float norm_weight(const HeadScatter& hs, int i) {
   return hs.w_bf16 ? __bfloat162float(reinterpret_cast<const bf16*>(hs.w)[i]) : reinterpret_cast<const float*>(hs.w)[i];
 }
 
+// Products of one A with up to NW weights of the same shape [N, K] in one launch: N tiles [g tiles, (g + 1) tiles) belong to weight g.
+// Three (q, k, v) is what every launch carries; kManyWeights (the context's keys and values of all blocks) is a kernel of its own,
+// since the parameters are copied for each launch.
+constexpr int kManyWeights = 80;
+template <int NW>
+struct GemmWeights {
+  CUtensorMap map[NW];
+  bf16* out[NW];
+  // many weights: per-head RMSNorm weight [128] of the product's heads (fp32, or bf16 where `norm_bf16` says so), or null: plain product
+  const void* norm[NW > 3 ? NW : 1];
+  uint8_t norm_bf16[NW > 3 ? NW : 1];
+};
+
 struct GemmEpilogue {
   HeadScatter hs;     // hs.P == 0: disabled
-  bf16* C;
-  // up to three products of one A with weights of the same shape [N, K] in one launch (q, k, v; the context's k, v): N tiles
-  // [g tiles, (g + 1) tiles) belong to weight g, whose tensor map is tma_b, tma_b1 or tma_b2 and whose product goes to C, C1 or C2
-  bf16 *C1, *C2;
-  int groups;         // 1 to 3; more than one only without bias, activation, residual and head scatter
+  int groups;         // weights; more than one only without bias, activation, residual and head scatter
+  float norm_eps;     // many weights: of their norms
   bf16* pre;          // optional second output: the pre-activation (act == 1) or the product before the gated residual
                       // (full 256-column tiles only)
   const bf16* bias;   // optional [N]
@@ -118,11 +128,10 @@ __device__ __forceinline__ void red_release_gpu_add(int* p, int v) {
 // each at K = 2048). The fp32 partial tiles are exchanged through distributed shared memory - pair s receives the SPLIT - 1 other
 // partials of its share of the columns (in units of 64) in the shared memory that the operand ring no longer needs - added in a fixed order (the
 // result is deterministic) and put back into TMEM, from where the ordinary epilogue finishes those columns.
-template <int A_MN, int B_MN, bool GATHER, bool CTA2 = false, int SPLIT = 1>
+template <int A_MN, int B_MN, bool GATHER, bool CTA2 = false, int SPLIT = 1, int NW = 3>
 __global__ void __launch_bounds__(kGemmThreads + (GATHER ? kGatherWarps * 32 : 0), 1)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                 const __grid_constant__ CUtensorMap tma_b1, const __grid_constant__ CUtensorMap tma_b2, int M, int N, int K,
-                 GemmEpilogue ep, GatherB gb, int* __restrict__ err) {
+gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ GemmWeights<NW> bw, int M, int N, int K, GemmEpilogue ep,
+                 GatherB gb, int* __restrict__ err) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   static_assert(!(CTA2 && GATHER), "the gather mode runs on single-CTA tiles");
@@ -151,6 +160,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int tiles_m = (M + TM - 1) / TM, tiles_g = (N + BN - 1) / BN;
   const int tiles_n = CTA2 ? tiles_g * ep.groups : tiles_g;      // N tiles of all weights
   const int n_tiles = tiles_m * tiles_n;
+  // Tile t's row and column. Neighbours run at the same time and share their row of A, whose columns fit L2 - except with many weights,
+  // which together do not: there neighbours share a weight's columns, so that every weight is read from HBM once.
+  auto tile_row = [&](int t) -> int { return NW > 3 ? t % tiles_m : t / tiles_n; };
+  auto tile_col = [&](int t) -> int { return NW > 3 ? t / tiles_m : t % tiles_n; };
   const int k_all = (K + BK - 1) / BK;
   const int kb_first = SPLIT > 1 ? k_all * split / SPLIT : 0, k_blocks = SPLIT > 1 ? k_all * (split + 1) / SPLIT - kb_first : k_all;
 
@@ -185,10 +198,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     if (warp == 0 && lane == 0) {
       // The first tile's B operand, as a rule a weight that only HBM holds, on its way into L2 while the kernel in front still runs.
       prefetch_tmap(&tma_a);
-      prefetch_tmap(&tma_b);
-      const int grp = first_tile % tiles_n / tiles_g;
-      const CUtensorMap* tb = grp > 0 ? (grp == 1 ? &tma_b1 : &tma_b2) : &tma_b;
-      const int n0 = (first_tile % tiles_n - grp * tiles_g) * BN + (int)pair_rank * (BN / 2);
+      const int grp = tile_col(first_tile) / tiles_g;
+      const CUtensorMap* tb = &bw.map[grp];
+      prefetch_tmap(tb);
+      const int n0 = (tile_col(first_tile) - grp * tiles_g) * BN + (int)pair_rank * (BN / 2);
       const int ahead = min(k_blocks, kPrefetchBlocks);
       for (int kb = 0; kb < ahead; ++kb) {
         const int k0 = (kb_first + kb) * BK;
@@ -206,8 +219,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      prefetch_tmap(&tma_a);
-      prefetch_tmap(&tma_b);
+      if (!CTA2) {
+        prefetch_tmap(&tma_a);
+        prefetch_tmap(&bw.map[0]);
+      }
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -227,10 +242,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       };
       for (int t = first_tile; t < n_tiles && ok; t += tile_step) {
         // with CTA2 this CTA fetches its 128 rows of the pair's A tile and its 128 rows of the B tile
-        const int grp = CTA2 ? t % tiles_n / tiles_g : 0;
-        const CUtensorMap* tb = CTA2 && grp > 0 ? (grp == 1 ? &tma_b1 : &tma_b2) : &tma_b;
-        const int m0 = (t / tiles_n) * TM + (CTA2 ? (int)pair_rank * BM : 0);
-        const int n0 = (t % tiles_n - grp * tiles_g) * BN + (CTA2 ? (int)pair_rank * (BN / 2) : 0);
+        const int grp = CTA2 ? tile_col(t) / tiles_g : 0;
+        const CUtensorMap* tb = &bw.map[grp];
+        const int m0 = tile_row(t) * TM + (CTA2 ? (int)pair_rank * BM : 0);
+        const int n0 = (tile_col(t) - grp * tiles_g) * BN + (CTA2 ? (int)pair_rank * (BN / 2) : 0);
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (GATHER) {
             // rows of the weight this stage reads: an N tile of 256 rows (forward) or 64 rows of the contraction dimension (dgrad)
@@ -267,10 +282,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
               for (int j = 0; j < BM / 64; ++j) tma_load_2d(sa + j * 8192, &tma_a, &full[s], m0 + j * 64, k0);
             }
             if (B_MN == 0) {
-              tma_load_2d(sb, &tma_b, &full[s], k0, n0);
+              tma_load_2d(sb, tb, &full[s], k0, n0);
             } else {
 #pragma unroll
-              for (int j = 0; j < BN / 64; ++j) tma_load_2d(sb + j * 8192, &tma_b, &full[s], n0 + j * 64, k0);
+              for (int j = 0; j < BN / 64; ++j) tma_load_2d(sb + j * 8192, tb, &full[s], n0 + j * 64, k0);
             }
           }
           if (++s == STG) { s = 0; ph ^= 1; }
@@ -402,9 +417,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     const uint32_t acc_empty_leader[2] = {CTA2 ? mapa_shared(smem_u32(&acc_empty[0]), lead_rank) : 0u,
                                           CTA2 ? mapa_shared(smem_u32(&acc_empty[1]), lead_rank) : 0u};
     for (int t = first_tile; t < n_tiles && ok; t += tile_step) {
-      const int grp = CTA2 ? t % tiles_n / tiles_g : 0;
-      bf16* const out = CTA2 && grp > 0 ? (grp == 1 ? ep.C1 : ep.C2) : ep.C;
-      const int m0 = (t / tiles_n) * TM + (CTA2 ? (int)pair_rank * BM : 0), n0 = (t % tiles_n - grp * tiles_g) * BN;
+      const int grp = CTA2 ? tile_col(t) / tiles_g : 0;
+      bf16* const out = bw.out[grp];
+      const int m0 = tile_row(t) * TM + (CTA2 ? (int)pair_rank * BM : 0), n0 = (tile_col(t) - grp * tiles_g) * BN;
       const bool whole = vec_ok && n0 + BN <= N;            // a tile of full width: vector accesses through the staging block
       uint4 ahead[8];
 #pragma unroll
@@ -623,6 +638,25 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             *reinterpret_cast<uint4*>(stage_row + (((c * 4 + q) ^ (lane & 7)) << 4)) = o;
           }
         };
+        // many weights: this warp's 128 columns are one head, this thread's accumulator row all of it: the norm needs no exchange
+        const void* const norm_w = NW > 3 ? bw.norm[NW > 3 ? grp : 0] : nullptr;
+        float rstd = 1.f;
+        if (NW > 3 && norm_w != nullptr) {
+          float2 ss[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            uint32_t r[32];
+            tmem_ld32(t_row + part * 128 + c * 32, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const float2 v = make_float2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+              ss[j & 1] = fma2(v, v, ss[j & 1]);
+            }
+          }
+          const float2 t2 = add2(ss[0], ss[1]);
+          rstd = rsqrtf((t2.x + t2.y) * (1.f / 128.f) + ep.norm_eps);
+        }
 #pragma unroll 1
         for (int pass = 0; pass < (SPLIT > 1 ? 1 : 2); ++pass) {
           const int coff = SPLIT > 1 ? my_unit * 64 : part * 128 + pass * 64;   // column offset inside the tile
@@ -664,6 +698,27 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             float v[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+            if (NW > 3) {
+              if (norm_w != nullptr) {
+                const int i0 = pass * 64 + c * 32;          // channel of the head
+                const bool wb = bw.norm_bf16[NW > 3 ? grp : 0] != 0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                  float w8[8];
+                  if (wb) {
+                    unpack8(*reinterpret_cast<const bf16x8*>(reinterpret_cast<const bf16*>(norm_w) + i0 + q * 8), w8);
+                  } else {
+                    const float4* w4 = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(norm_w) + i0 + q * 8);
+                    const float4 f0 = w4[0], f1 = w4[1];
+                    w8[0] = f0.x; w8[1] = f0.y; w8[2] = f0.z; w8[3] = f0.w; w8[4] = f1.x; w8[5] = f1.y; w8[6] = f1.z; w8[7] = f1.w;
+                  }
+#pragma unroll
+                  for (int j = 0; j < 8; ++j) v[q * 8 + j] = v[q * 8 + j] * rstd * w8[j];
+                }
+              }
+              stage_chunk(c, v);
+              continue;
+            }
             if (ep.bias != nullptr) {
 #pragma unroll
               for (int j = 0; j < 32; ++j) v[j] += __bfloat162float(ep.bias[col0 + j]);
@@ -806,9 +861,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 using namespace cb200;
 
 template <int A_MN, int B_MN, bool GATHER = false>
-static int launch_gemm(const void* A, const void* B, int M, int N, int K, const GemmEpilogue& ep, int* err, int sms,
+static int launch_gemm(const void* A, const void* B, bf16* C, int M, int N, int K, const GemmEpilogue& ep, int* err, int sms,
                        cudaStream_t st, const GatherB& gb = GatherB{}) {
-  CUtensorMap ta, tb;
+  CUtensorMap ta;
+  GemmWeights<3> bw{};
+  CUtensorMap& tb = bw.map[0];
   int rc;
   // A: K-major [M,K] -> dims {K, M}, box {64, 128};  MN-major stored [K,M] -> dims {M, K}, box {64, 64}
   if (A_MN == 0) rc = make_tmap_2d_bf16(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, BM);
@@ -817,6 +874,7 @@ static int launch_gemm(const void* A, const void* B, int M, int N, int K, const 
   if (B_MN == 0) rc = make_tmap_2d_bf16(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, BK, BN);
   else rc = make_tmap_2d_bf16(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)N * 2, 64, BK);
   if (rc) return rc;
+  bw.out[0] = C;
   static bool attr_set = false;      // one flag per template instantiation
   auto kern = gemm_bf16_kernel<A_MN, B_MN, GATHER>;
   if (!attr_set) {
@@ -827,7 +885,7 @@ static int launch_gemm(const void* A, const void* B, int M, int N, int K, const 
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   // with a gather every SM takes part (its gather warps work even when it has no tile): the grid is the whole machine
   const int grid = GATHER ? sms : (tiles < sms ? tiles : sms);
-  kern<<<grid, kGemmThreads + (GATHER ? kGatherWarps * 32 : 0), kSmemBytes, st>>>(ta, tb, tb, tb, M, N, K, ep, gb, err);
+  kern<<<grid, kGemmThreads + (GATHER ? kGatherWarps * 32 : 0), kSmemBytes, st>>>(ta, bw, M, N, K, ep, gb, err);
   return (int)cudaGetLastError();
 }
 
@@ -853,11 +911,11 @@ struct PairLaunch {
 };
 
 // clusters that the GPU holds at once: none where it has no room for one (a share of a GPU)
-template <int A_MN, int B_MN, int SPLIT>
+template <int A_MN, int B_MN, int SPLIT, int NW = 3>
 static int resident_clusters(int* clusters) {
   static int resident = -1;
   if (resident < 0) {
-    const auto kern = gemm_bf16_kernel<A_MN, B_MN, false, true, SPLIT>;
+    const auto kern = gemm_bf16_kernel<A_MN, B_MN, false, true, SPLIT, NW>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
     if (e != cudaSuccess) return 100 + (int)e;
     PairLaunch l(SPLIT, 1, nullptr);
@@ -872,23 +930,27 @@ static int resident_clusters(int* clusters) {
   return 0;
 }
 
-template <int A_MN, int B_MN, int SPLIT>
-static int launch_gemm_pairs(const void* A, const void* const* B, int M, int N, int K, const GemmEpilogue& ep, int clusters, int* err,
-                             cudaStream_t st) {
-  CUtensorMap ta, tb[3];
+template <int A_MN, int B_MN, int SPLIT, int NW = 3>
+static int launch_gemm_pairs(const void* A, const void* const* B, void* const* C, int M, int N, int K, const GemmEpilogue& ep, int clusters,
+                             int* err, cudaStream_t st, const void* const* norm = nullptr, const uint8_t* norm_bf16 = nullptr) {
+  CUtensorMap ta;
+  GemmWeights<NW> bw{};
   int rc;
   if (A_MN == 0) rc = make_tmap_2d_bf16(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, BM);
   else rc = make_tmap_2d_bf16(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)M * 2, 64, BK);
   if (rc) return rc;
-  for (int g = 0; g < 3; ++g) {
-    const void* w = B[g < ep.groups ? g : 0];
-    if (B_MN == 0) rc = make_tmap_2d_bf16(&tb[g], w, (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, BK, BN / 2);   // each CTA loads half the columns
-    else rc = make_tmap_2d_bf16(&tb[g], w, (uint64_t)N, (uint64_t)K, (uint64_t)N * 2, 64, BK);
+  for (int g = 0; g < ep.groups; ++g) {
+    if (B_MN == 0) rc = make_tmap_2d_bf16(&bw.map[g], B[g], (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, BK, BN / 2);   // each CTA loads half the columns
+    else rc = make_tmap_2d_bf16(&bw.map[g], B[g], (uint64_t)N, (uint64_t)K, (uint64_t)N * 2, 64, BK);
     if (rc) return rc;
+    bw.out[g] = (bf16*)C[g];
+    if (NW > 3 && norm != nullptr) {
+      bw.norm[NW > 3 ? g : 0] = norm[g];
+      bw.norm_bf16[NW > 3 ? g : 0] = norm_bf16[g];
+    }
   }
   PairLaunch l(SPLIT, clusters, st);
-  const cudaError_t e = cudaLaunchKernelEx(&l.cfg, gemm_bf16_kernel<A_MN, B_MN, false, true, SPLIT>, ta, tb[0], tb[1], tb[2], M, N, K, ep,
-                                           GatherB{}, err);
+  const cudaError_t e = cudaLaunchKernelEx(&l.cfg, gemm_bf16_kernel<A_MN, B_MN, false, true, SPLIT, NW>, ta, bw, M, N, K, ep, GatherB{}, err);
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
 
@@ -916,7 +978,8 @@ extern "C" int cb200_gemm_pairs_per_tile(long tiles, long kb, int pairs, int c2,
 }
 
 template <int A_MN, int B_MN>
-static int launch_gemm_any(const void* A, const void* const* B, int M, int N, int K, const GemmEpilogue& ep, int* err, int sms, cudaStream_t st) {
+static int launch_gemm_any(const void* A, const void* const* B, void* const* C, int M, int N, int K, const GemmEpilogue& ep, int* err, int sms,
+                          cudaStream_t st) {
   const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) * ep.groups, kb = (K + BK - 1) / BK;
   const int pairs = sms / 2;
   int c1 = 0, c2 = 0, c3 = 0, c4 = 0, rc;
@@ -924,15 +987,15 @@ static int launch_gemm_any(const void* A, const void* const* B, int M, int N, in
     if ((rc = resident_clusters<A_MN, B_MN, 2>(&c2)) || (rc = resident_clusters<A_MN, B_MN, 3>(&c3)) || (rc = resident_clusters<A_MN, B_MN, 4>(&c4)))
       return rc;
     const int split = cb200_gemm_pairs_per_tile(tiles, kb, pairs, c2, c4, c3);
-    if (split == 4) return launch_gemm_pairs<A_MN, B_MN, 4>(A, B, M, N, K, ep, (int)tiles, err, st);
-    if (split == 3) return launch_gemm_pairs<A_MN, B_MN, 3>(A, B, M, N, K, ep, (int)tiles, err, st);
-    if (split == 2) return launch_gemm_pairs<A_MN, B_MN, 2>(A, B, M, N, K, ep, (int)tiles, err, st);
+    if (split == 4) return launch_gemm_pairs<A_MN, B_MN, 4>(A, B, C, M, N, K, ep, (int)tiles, err, st);
+    if (split == 3) return launch_gemm_pairs<A_MN, B_MN, 3>(A, B, C, M, N, K, ep, (int)tiles, err, st);
+    if (split == 2) return launch_gemm_pairs<A_MN, B_MN, 2>(A, B, C, M, N, K, ep, (int)tiles, err, st);
   }
   // A persistent grid must be resident as a whole: the pairs that the GPU can hold at once (a pair lives inside one GPC, so a
   // GPC with an odd number of free SMs leaves one out) bound the grid, otherwise late pairs would run after the others.
   if ((rc = resident_clusters<A_MN, B_MN, 1>(&c1))) return rc;
   if (c1 < 1) return 600;
-  return launch_gemm_pairs<A_MN, B_MN, 1>(A, B, M, N, K, ep, (int)std::min<long>(tiles, std::min(c1, pairs)), err, st);
+  return launch_gemm_pairs<A_MN, B_MN, 1>(A, B, C, M, N, K, ep, (int)std::min<long>(tiles, std::min(c1, pairs)), err, st);
 }
 
 // 0: single-CTA tiles; 1 (default): CTA pairs where the shape allows (measured 8-45 % faster on the 2B shapes: half the B-operand
@@ -953,7 +1016,6 @@ extern "C" int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int
                                const void* bias, int act, void* pre, const void* resid, const float* gate, long ld_gate, int L,
                                int* err, int sms, cudaStream_t st) {
   GemmEpilogue ep{};
-  ep.C = (bf16*)C;
   ep.groups = 1;
   ep.pre = (bf16*)pre;
   ep.bias = (const bf16*)bias;
@@ -963,15 +1025,15 @@ extern "C" int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int
   ep.act = act;
   ep.L = L > 0 ? L : 1;
   if (cb200_gemm_pair_mode(-1) == 1 && M >= 2 * BM && N % 8 == 0) {
-    if (a_mn == 0 && b_mn == 0) return launch_gemm_any<0, 0>(A, &B, M, N, K, ep, err, sms, st);
-    if (a_mn == 0 && b_mn == 1) return launch_gemm_any<0, 1>(A, &B, M, N, K, ep, err, sms, st);
-    if (a_mn == 1 && b_mn == 0) return launch_gemm_any<1, 0>(A, &B, M, N, K, ep, err, sms, st);
-    return launch_gemm_any<1, 1>(A, &B, M, N, K, ep, err, sms, st);
+    if (a_mn == 0 && b_mn == 0) return launch_gemm_any<0, 0>(A, &B, &C, M, N, K, ep, err, sms, st);
+    if (a_mn == 0 && b_mn == 1) return launch_gemm_any<0, 1>(A, &B, &C, M, N, K, ep, err, sms, st);
+    if (a_mn == 1 && b_mn == 0) return launch_gemm_any<1, 0>(A, &B, &C, M, N, K, ep, err, sms, st);
+    return launch_gemm_any<1, 1>(A, &B, &C, M, N, K, ep, err, sms, st);
   }
-  if (a_mn == 0 && b_mn == 0) return launch_gemm<0, 0>(A, B, M, N, K, ep, err, sms, st);
-  if (a_mn == 0 && b_mn == 1) return launch_gemm<0, 1>(A, B, M, N, K, ep, err, sms, st);
-  if (a_mn == 1 && b_mn == 0) return launch_gemm<1, 0>(A, B, M, N, K, ep, err, sms, st);
-  return launch_gemm<1, 1>(A, B, M, N, K, ep, err, sms, st);
+  if (a_mn == 0 && b_mn == 0) return launch_gemm<0, 0>(A, B, (bf16*)C, M, N, K, ep, err, sms, st);
+  if (a_mn == 0 && b_mn == 1) return launch_gemm<0, 1>(A, B, (bf16*)C, M, N, K, ep, err, sms, st);
+  if (a_mn == 1 && b_mn == 0) return launch_gemm<1, 0>(A, B, (bf16*)C, M, N, K, ep, err, sms, st);
+  return launch_gemm<1, 1>(A, B, (bf16*)C, M, N, K, ep, err, sms, st);
 }
 
 // launches of cb200_gemm_bf16_group: one, or one for each weight where there is no CTA-pair tile
@@ -989,12 +1051,34 @@ extern "C" int cb200_gemm_bf16_group(const void* A, const void* const* B, void* 
     return 0;
   }
   GemmEpilogue ep{};
-  ep.C = (bf16*)C[0];
-  ep.C1 = groups > 1 ? (bf16*)C[1] : nullptr;
-  ep.C2 = groups > 2 ? (bf16*)C[2] : nullptr;
   ep.groups = groups;
   ep.L = 1;
-  return launch_gemm_any<0, 0>(A, B, M, N, K, ep, err, sms, st);
+  return launch_gemm_any<0, 0>(A, B, C, M, N, K, ep, err, sms, st);
+}
+
+// Weights that one launch of cb200_gemm_bf16_many takes for this shape: none where fewer than 256 rows, a partial N tile or half a head
+// rule out the tiles it is made of, or where all of the weights together are less than a wave of tiles, which the grouped launches
+// above split over clusters.
+extern "C" int cb200_gemm_many_weights(int n, int M, int N, int K, int sms) {
+  const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * (N / BN) * n;
+  return cb200_gemm_pair_mode(-1) == 1 && M >= 2 * BM && N % BN == 0 && K % 8 == 0 && tiles >= sms / 2 ? kManyWeights : 0;
+}
+
+// C[i] = A @ B[i]^T for n <= kManyWeights weights [N, K] in one launch, heads of 128 columns RMS-normalised with norm[i] where that is
+// not null (fp32, or bf16 with norm_bf16[i]; 16-byte aligned).
+extern "C" int cb200_gemm_bf16_many(const void* A, const void* const* B, void* const* C, const void* const* norm, const uint8_t* norm_bf16,
+                                    int n, int M, int N, int K, float eps, int* err, int sms, cudaStream_t st) {
+  if (n < 1 || n > kManyWeights || M < 2 * BM || N % BN != 0 || K % 8 != 0) return -43;
+  GemmEpilogue ep{};
+  ep.groups = n;
+  ep.norm_eps = eps;
+  ep.L = 1;
+  int c1 = 0;
+  const int rc = resident_clusters<0, 0, 1, kManyWeights>(&c1);
+  if (rc) return rc;
+  if (c1 < 1) return 600;
+  const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * (N / BN) * n;
+  return launch_gemm_pairs<0, 0, 1, kManyWeights>(A, B, C, M, N, K, ep, (int)std::min<long>(tiles, std::min(c1, sms / 2)), err, st, norm, norm_bf16);
 }
 
 // C is not written: row (b, s) of A[M = B*S, K] @ W[N = H*128, K]^T is split into heads, each head is RMS-normalised with
@@ -1021,8 +1105,9 @@ extern "C" int cb200_gemm_bf16_scatter_heads(const void* A, const void* W, int M
   ep.hs.rstd_out = rstd_out;
   ep.L = 1;
   ep.groups = 1;
-  if (cb200_gemm_pair_mode(-1) == 1 && M >= 2 * BM) return launch_gemm_any<0, 0>(A, &W, M, N, K, ep, err, sms, st);
-  return launch_gemm<0, 0>(A, W, M, N, K, ep, err, sms, st);
+  void* none = nullptr;
+  if (cb200_gemm_pair_mode(-1) == 1 && M >= 2 * BM) return launch_gemm_any<0, 0>(A, &W, &none, M, N, K, ep, err, sms, st);
+  return launch_gemm<0, 0>(A, W, nullptr, M, N, K, ep, err, sms, st);
 }
 
 // C = epilogue(A @ op(W)) where W [rows, ld] is sharded by rows over P ranks (rank r: shard_ptrs[r] holds rows [r * chunk_rows, ...)).
@@ -1033,7 +1118,6 @@ extern "C" int cb200_gemm_bf16_gather(const void* A, void* ws, void* C, int M, i
                                       cudaStream_t st) {
   if (P < 1 || P > 8 || chunk_rows < 1 || (long)chunk_rows * P < rows || ld % 8 != 0) return -31;
   GemmEpilogue ep{};
-  ep.C = (bf16*)C;
   ep.pre = (bf16*)pre;
   ep.bias = (const bf16*)bias;
   ep.act = act;
@@ -1050,6 +1134,6 @@ extern "C" int cb200_gemm_bf16_gather(const void* A, void* ws, void* C, int M, i
   gb.slices = sms / n_groups < 1 ? 1 : (sms / n_groups > 16 ? 16 : sms / n_groups);
   cudaError_t e = cudaMemsetAsync(counters, 0, (size_t)n_groups * sizeof(int), st);
   if (e != cudaSuccess) return 400 + (int)e;
-  if (b_mn == 0) return launch_gemm<0, 0, true>(A, ws, M, rows, ld, ep, err, sms, st, gb);
-  return launch_gemm<0, 1, true>(A, ws, M, ld, rows, ep, err, sms, st, gb);
+  if (b_mn == 0) return launch_gemm<0, 0, true>(A, ws, (bf16*)C, M, rows, ld, ep, err, sms, st, gb);
+  return launch_gemm<0, 1, true>(A, ws, (bf16*)C, M, ld, rows, ep, err, sms, st, gb);
 }

@@ -56,6 +56,9 @@ int cb200_skinny_wide(long a_k, long b_n, long b_k, int b_is_bf16, int c_is_bf16
 // gemm_tcgen05.cu
 int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int b_mn, const void* bias,
                     int act, void* pre, const void* resid, const float* gate, long ld_gate, int L, int* err, int sms, cudaStream_t st);
+int cb200_gemm_many_weights(int n, int M, int N, int K, int sms);   // weights a launch of cb200_gemm_bf16_many takes, or 0
+int cb200_gemm_bf16_many(const void* A, const void* const* B, void* const* C, const void* const* norm, const uint8_t* norm_bf16, int n, int M,
+                         int N, int K, float eps, int* err, int sms, cudaStream_t st);
 int cb200_gemm_bf16_group(const void* A, const void* const* B, void* const* C, int groups, int M, int N, int K, int* err, int sms, cudaStream_t st);
 int cb200_gemm_group_launches(int M, int groups);
 int cb200_gemm_pairs_per_tile(long tiles, long kb, int pairs, int c2, int c4, int c3);   // 1 to 4 CTA pairs share a tile's contraction

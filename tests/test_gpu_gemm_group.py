@@ -93,3 +93,29 @@ def test_query_key_value_of_few_tiles(preset, shape, tokens, split):
     assert _rel(got, want.double()) < 4 * 2.0 ** -9
     for a, b in zip([t for p in kv for t in p], [t for p in kv_want for t in p]):
         assert _rel(a, b.double()) < 4 * 2.0 ** -9
+
+
+# Blocks of one width: every key and value in one launch (several from 40 blocks on), tiles by weight, the keys normalised in the epilogue.
+# Ragged rows, contraction that is no whole k-block count of the ring, a width of many N tiles, more blocks than a launch takes.
+@pytest.mark.parametrize("B,S,C,D,blocks", [(2, 512, 1024, 2048, 5), (1, 264, 1024, 1024, 10), (3, 88, 576, 512, 20), (1, 77 * 8, 1024, 5120, 2),
+                                            (1, 512, 512, 256, 41)])
+@pytest.mark.parametrize("norm_dtype", [torch.bfloat16, torch.float32])
+def test_all_blocks_in_one_launch(B, S, C, D, blocks, norm_dtype):
+    torch.manual_seed(1)
+    ops = native.load()
+    assert ops.dit_context_launches(B * S, C, [D] * blocks) == -(-blocks // 40)
+    assert ops.dit_context_launches(B * S, C, [D, D + 256]) == 4 and ops.dit_context_launches(248, C, [D] * blocks) == 3 * blocks
+    ctx = torch.randn(B, S, C, device=DEV).bfloat16()
+    ws = []
+    for _ in range(blocks):
+        ws += [(torch.randn(D, C, device=DEV) / math.sqrt(C)).bfloat16() for _ in range(2)] + [(1 + 0.2 * torch.randn(128, device=DEV)).to(norm_dtype)]
+    got, again = ops.dit_context_kv(ctx, ws, 1e-6), ops.dit_context_kv(ctx, ws, 1e-6)
+    torch.cuda.synchronize()
+    assert ops.kernel_error(0, True) == 0 and len(got) == 2 * blocks
+    for i in range(blocks):
+        wk, wv, wn = (w.double() for w in ws[3 * i: 3 * i + 3])
+        k = (ctx.double() @ wk.t()).view(B, S, D // 128, 128)
+        k = k * torch.rsqrt(k.pow(2).mean(-1, keepdim=True) + 1e-6) * wn
+        v = (ctx.double() @ wv.t()).view(B, S, D // 128, 128)
+        assert _rel(got[2 * i], k) < ROUND and _rel(got[2 * i + 1], v) < ROUND       # one rounding each
+        assert torch.equal(got[2 * i], again[2 * i]) and torch.equal(got[2 * i + 1], again[2 * i + 1])

@@ -57,3 +57,36 @@ def test_epilogues(M, N, K):
     assert _rel(pre, pre_want) < ROUND and _rel(y, torch.nn.functional.gelu(pre_want)) < ROUND
     sum_want = resid.double() + gate.double().repeat_interleave(L, 0) * prod
     assert _rel(p, prod) < ROUND and _rel(out, sum_want) < ROUND and torch.equal(out, only)
+
+
+# 18 and 20 tiles: no room for clusters of four pairs in one wave, so three pairs share a tile; shares of 13 to 15 and 43 k-blocks, ragged rows
+@pytest.mark.parametrize("M,N,K", [(768, 1536, 8256), (1000, 1280, 2624), (904, 1280, 2752)])
+def test_three_pairs(M, N, K):
+    torch.manual_seed(2)
+    ops = native.load()
+    assert ops.gemm_pairs_per_tile(-(-M // 256) * (N // 256), K // 64, 74, 33, 16, 22) == 3
+    a = torch.randn(M, K, device=DEV).bfloat16()
+    b = (torch.randn(N, K, device=DEV) / math.sqrt(K)).bfloat16()
+    L = 8
+    gate = torch.randn(M // L, 3 * N, device=DEV)[:, N:2 * N]
+    resid = torch.randn(M, N, device=DEV).bfloat16()
+    prod = a.double() @ b.double().t()
+    got, again = ops.gemm_bf16(a, b, None, 0, False, False), ops.gemm_bf16(a, b, None, 0, False, False)
+    out, p = ops.gemm_bf16_gate_residual_pre(a, b, resid, gate, L)
+    _check()
+    assert _rel(got, prod) < ROUND and torch.equal(got, again) and torch.equal(p, got)
+    assert _rel(out, resid.double() + gate.double().repeat_interleave(L, 0) * prod) < ROUND
+
+
+# The gated residual of several tiles per pair: the rows of the next tile are fetched while this one is finished; gates that change
+# inside a warp's rows, a last row tile that is mostly empty
+@pytest.mark.parametrize("M,N,K,L", [(7040, 2048, 128, 3520), (19208, 1024, 192, 8), (20000, 1024, 64, 40)])
+def test_gated_tiles_in_a_row(M, N, K, L):
+    torch.manual_seed(3)
+    a = torch.randn(M, K, device=DEV).bfloat16()
+    b = (torch.randn(N, K, device=DEV) / math.sqrt(K)).bfloat16()
+    gate = torch.randn(M // L, 3 * N, device=DEV)[:, 2 * N:]
+    resid = torch.randn(M, N, device=DEV).bfloat16()
+    got = native.load().gemm_bf16_gate_residual(a, b, resid, gate, L)
+    _check()
+    assert _rel(got, resid.double() + gate.double().repeat_interleave(L, 0) * (a.double() @ b.double().t())) < ROUND
