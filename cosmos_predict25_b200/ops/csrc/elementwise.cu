@@ -14,6 +14,8 @@
 
 #include "common.cuh"
 #include "launchers.h"
+#include <algorithm>
+
 #include "sm100.cuh"   // packed fp32x2 arithmetic
 
 namespace cb200 {
@@ -58,147 +60,234 @@ __device__ __forceinline__ void store_f8(float* p, const float (&f)[8]) {
 // ------------------------------------------------------------------------------------------------
 // LayerNorm + modulate, forward: one CTA per token row
 // ------------------------------------------------------------------------------------------------
-template <int MV>
-__global__ void __launch_bounds__(kThreads) ln_modulate_fwd_kernel(
+// For few rows and short frames. Few rows are bound by latency: the row and its modulation vectors
+// are loaded together, a thread holds NV pieces of 16 bytes, and each of the two sums is one barrier. With a warp per row, its two
+// reductions and then its loads of the modulation in a row, 512 rows of 2048 took 5.6 us in a row of launches, now 3.5 (1024 rows 7.1
+// and 3.7; a launch that does nothing about 2).
+template <int NV, int THREADS>
+__global__ void __launch_bounds__(THREADS) ln_modulate_fwd_row_kernel(
     const bf16* __restrict__ x, const float* __restrict__ shift, const float* __restrict__ scale,
     bf16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int D, int L, long ld_shift, long ld_scale,
     float eps) {
-  __shared__ float red[64];
+  __shared__ float red[2][THREADS / 32];
+  pdl_trigger();                     // launched with programmatic serialisation (see common.cuh)
+  pdl_wait();
   const long row = blockIdx.x;
   const long frame = row / L;
-  const int nvec = D >> 3;
+  const int nvec = D >> 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + row * D);
-  float v[MV][8];
-  float s = 0.f;
+  const float* sh = shift + frame * ld_shift;
+  const float* sc = scale + frame * ld_scale;
+  bf16x8 v[NV];
+  float a[NV][8], b[NV][8];
 #pragma unroll
-  for (int i = 0; i < MV; ++i) {
-    const int c = threadIdx.x + i * kThreads;
+  for (int i = 0; i < NV; ++i) {
+    const int c = threadIdx.x + i * THREADS;
+    v[i] = c < nvec ? xr[c] : bf16x8{};
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = threadIdx.x + i * THREADS;
     if (c < nvec) {
-      unpack8(xr[c], v[i]);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) s += v[i][j];
+      load_f8(sh + c * 8, a[i]);
+      load_f8(sc + c * 8, b[i]);
     }
   }
-  const float mean = block_sum(s, red) / D;
-  float q = 0.f;
+  auto total = [&](float2 s2, float* slots) -> float {
+    const float s = warp_sum(s2.x + s2.y);
+    if (lane == 0) slots[warp] = s;
+    __syncthreads();
+    float t = 0.f;
 #pragma unroll
-  for (int i = 0; i < MV; ++i) {
-    const int c = threadIdx.x + i * kThreads;
-    if (c < nvec) {
+    for (int w = 0; w < THREADS / 32; ++w) t += slots[w];
+    return t;
+  };
+  float2 s2 = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float d = v[i][j] - mean;
-        q += d * d;
+  for (int i = 0; i < NV; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s2 = add2(s2, __bfloat1622float2(v[i].v[j]));
+  const float mean = total(s2, red[0]) / D;
+  const float2 nm = make_float2(-mean, -mean);
+  float2 q2 = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < NV; ++i)
+    if (threadIdx.x + i * THREADS < nvec) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 d = add2(__bfloat1622float2(v[i].v[j]), nm);
+        q2 = fma2(d, d, q2);
       }
     }
-  }
-  const float rstd = rsqrtf(block_sum(q, red) / D + eps);
+  const float rstd = rsqrtf(total(q2, red[1]) / D + eps);
   if (threadIdx.x == 0) {
     mean_out[row] = mean;
     rstd_out[row] = rstd;
   }
-  bf16x8* yr = reinterpret_cast<bf16x8*>(y + row * D);
-  const float* sh = shift + frame * ld_shift;
-  const float* sc = scale + frame * ld_scale;
+  const float2 one2 = make_float2(1.f, 1.f), rs2 = make_float2(rstd, rstd);
 #pragma unroll
-  for (int i = 0; i < MV; ++i) {
-    const int c = threadIdx.x + i * kThreads;
+  for (int i = 0; i < NV; ++i) {
+    const int c = threadIdx.x + i * THREADS;
     if (c < nvec) {
-      float a[8], b[8], o[8];
-      load_f8(sh + c * 8, a);
-      load_f8(sc + c * 8, b);
+      bf16x8 o;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = (v[i][j] - mean) * rstd * (1.f + b[j]) + a[j];
-      yr[c] = pack8(o);
+      for (int j = 0; j < 4; ++j) {
+        const float2 t = fma2(mul2(add2(__bfloat1622float2(v[i].v[j]), nm), rs2), add2(CB200_P2(b[i], j), one2), CB200_P2(a[i], j));
+        o.v[j] = __floats2bfloat162_rn(t.x, t.y);
+      }
+      reinterpret_cast<bf16x8*>(y + row * D)[c] = o;
     }
   }
 }
 
-// Same operator for D <= 256 NV: a warp owns R rows of one frame, all of whose 16-byte pieces are in flight together (kept packed),
-// and reduces them with shuffles alone. Bound by memory; with a CTA per four rows the two block-wide reductions (four barriers) kept
-// the memory pipe idle. The modulation vectors are four times a row's bytes and come from L1, whose bandwidth is the next limit: a
-// pair of rows shares them. Inside a denoising step: 46,800 rows of 2048 174 us before, 125 us now (155 with a row per warp); 512
-// rows 22 us before, 6.9 us with a row per warp (8.2 with pairs): a row per warp while the pairs would not fill the GPU.
-// shift / scale rows are `ld_*` apart: slices of the modulation MLPs' output serve as they lie.
-constexpr int kLnWarps = 4;
-template <int NV, int R>
-__global__ void __launch_bounds__(kLnWarps * 32) ln_modulate_fwd_warp_kernel(
+// Same operator for many rows: a CTA walks over `rows_per_cta` rows of one frame, four at a time, and a thread keeps the modulation of its
+// NV pieces of 16 bytes in registers (read for every row or pair of rows they are four or two times its bytes). The loads of the
+// next four rows are in flight while four are reduced; each warp reduces its part of a row to a sum and a sum of squares about
+// its own mean, and the parts are put together behind one barrier.
+// Bound by memory: 46,800 rows of 2048 (383 MB) 107 us with a pair of rows per warp, now 84 (4.6 TB/s; the bytes take 59 us), 7040 rows
+// in L2 13.5 and 13.2, 46,800 rows of 5120 325 (a CTA per row) and 238, 46,800 rows of 1024 51 and 42. Two rows at a time are a tenth
+// slower at 2048 channels, from 2056 channels on four spill registers. A spill costs more than a CTA more on the SM gives.
+// sums over the warp of R values a lane (two or four): lane l receives the total of value l / (32 / R)
+template <int R>
+__device__ __forceinline__ float warp_sums(const float (&v)[R], int lane) {
+  static_assert(R == 2 || R == 4, "two or four values");
+  const bool hi = lane & 16, odd = lane & 8;
+  float k;
+  if constexpr (R == 4) {
+    const float k0 = (hi ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], 16);
+    const float k1 = (hi ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], 16);
+    k = (odd ? k1 : k0) + __shfl_xor_sync(0xffffffffu, odd ? k0 : k1, 8);
+  } else {
+    k = (hi ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[1], 16);
+    k += __shfl_xor_sync(0xffffffffu, k, 8);
+  }
+  k += __shfl_xor_sync(0xffffffffu, k, 4);
+  k += __shfl_xor_sync(0xffffffffu, k, 2);
+  k += __shfl_xor_sync(0xffffffffu, k, 1);
+  return k;
+}
+
+template <int NV, int MAXT, int kLnRows, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) ln_modulate_fwd_rows_kernel(
     const bf16* __restrict__ x, const float* __restrict__ shift, const float* __restrict__ scale,
-    bf16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, long groups, int D, int L, int groups_per_frame,
+    bf16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int D, int L, int rows_per_cta, int groups_per_frame,
     long ld_shift, long ld_scale, float eps) {
+  static_assert(MAXT <= 512, "sixteen warps");
+  constexpr int G = 32 / kLnRows;            // lanes that put the parts of one row together, 16 / G parts each
+  constexpr bool two = G == 8;
+  __shared__ float2 red[2][kLnRows][16];     // (sum, squares about the warp's mean) of row r in warp w; two sets in turn
   pdl_trigger();                     // launched with programmatic serialisation (see common.cuh)
   pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const long group = (long)blockIdx.x * kLnWarps + (threadIdx.x >> 5);
-  if (group >= groups) return;
-  const long frame = group / groups_per_frame;
-  const int r_in = (int)(group - frame * groups_per_frame) * R, n_here = min(R, L - r_in);
-  const long row0 = frame * L + r_in;
-  const int nvec = D >> 3;
-  bf16x8 v[R][NV];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, T = blockDim.x, nw = T >> 5, nvec = D >> 3;
+  const long frame = blockIdx.x / groups_per_frame;
+  const int r0 = (int)(blockIdx.x % groups_per_frame) * rows_per_cta, r1 = min(r0 + rows_per_cta, L);
+  const bf16* xf = x + frame * L * D;
+  bf16* yf = y + frame * L * D;
+  bf16x8 nx[kLnRows][NV];
+  auto fetch = [&](int r) {
 #pragma unroll
-  for (int r = 0; r < R; ++r)
+    for (int k = 0; k < kLnRows; ++k)
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      if (r < n_here && lane + i * 32 < nvec) v[r][i] = reinterpret_cast<const bf16x8*>(x + (row0 + r) * D)[lane + i * 32];
-      else v[r][i] = bf16x8{};
-    }
-  float mean[R], rstd[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    float2 s2 = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int i = 0; i < NV; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) s2 = add2(s2, __bfloat1622float2(v[r][i].v[j]));
-    mean[r] = s2.x + s2.y;
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r) mean[r] = warp_sum(mean[r]) / D;
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const float2 nm = make_float2(-mean[r], -mean[r]);
-    float2 q2 = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int i = 0; i < NV; ++i)
-      if (lane + i * 32 < nvec) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 d = add2(__bfloat1622float2(v[r][i].v[j]), nm);
-          q2 = fma2(d, d, q2);
-        }
+      for (int i = 0; i < NV; ++i) {
+        const int c = threadIdx.x + i * T;
+        nx[k][i] = r + k < r1 && c < nvec ? reinterpret_cast<const bf16x8*>(xf + (long)(r + k) * D)[c] : bf16x8{};
       }
-    rstd[r] = q2.x + q2.y;
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    rstd[r] = rsqrtf(warp_sum(rstd[r]) / D + eps);
-    if (lane == 0 && r < n_here) {
-      mean_out[row0 + r] = mean[r];
-      rstd_out[row0 + r] = rstd[r];
-    }
-  }
-  const float* sh = shift + frame * ld_shift;
-  const float* sc = scale + frame * ld_scale;
-  const float2 one2 = make_float2(1.f, 1.f);
+  };
+  fetch(r0);
+  float a[NV][8], b[NV][8];
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    const int c = lane + i * 32;
+    const int c = threadIdx.x + i * T;
     if (c < nvec) {
-      float a[8], b[8];
-      load_f8(sh + c * 8, a);
-      load_f8(sc + c * 8, b);
+      load_f8(shift + frame * ld_shift + c * 8, a[i]);
+      load_f8(scale + frame * ld_scale + c * 8, b[i]);
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        if (r < n_here) {
-          const float2 nm = make_float2(-mean[r], -mean[r]), rs2 = make_float2(rstd[r], rstd[r]);
+      for (int j = 0; j < 8; ++j) b[i][j] += 1.f;
+    }
+  }
+  // channels of a row that warp w holds
+  auto channels = [&](int w) -> float {
+    int n = 0;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) n += 8 * max(0, min(32, nvec - (w * 32 + i * T)));
+    return (float)n;
+  };
+  const float inv_own = 1.f / channels(warp);
+  const int w0 = lane % G, w1 = w0 + 8, row_in = lane / G;       // the parts of a row that this lane puts together
+  const float n0 = w0 < nw ? channels(w0) : 0.f, n1 = two && w1 < nw ? channels(w1) : 0.f;
+  const float i0 = n0 > 0.f ? 1.f / n0 : 0.f, i1 = n1 > 0.f ? 1.f / n1 : 0.f, inv_d = 1.f / D;
+  int set = 0;
+  for (int r = r0; r < r1; r += kLnRows, set ^= 1) {
+    bf16x8 v[kLnRows][NV];
+#pragma unroll
+    for (int k = 0; k < kLnRows; ++k)
+#pragma unroll
+      for (int i = 0; i < NV; ++i) v[k][i] = nx[k][i];
+    if (r + kLnRows < r1) fetch(r + kLnRows);
+    float part[kLnRows];
+#pragma unroll
+    for (int k = 0; k < kLnRows; ++k) {
+      float2 s2 = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < NV; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s2 = add2(s2, __bfloat1622float2(v[k][i].v[j]));
+      part[k] = s2.x + s2.y;
+    }
+    const float sum = warp_sums(part, lane);
+    const float own_mean = sum * inv_own;
+#pragma unroll
+    for (int k = 0; k < kLnRows; ++k) {
+      const float m = __shfl_sync(0xffffffffu, own_mean, k * G);
+      const float2 nm = make_float2(-m, -m);
+      float2 q2 = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < NV; ++i)
+        if (threadIdx.x + i * T < nvec) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 d = add2(__bfloat1622float2(v[k][i].v[j]), nm);
+            q2 = fma2(d, d, q2);
+          }
+        }
+      part[k] = q2.x + q2.y;
+    }
+    const float squares = warp_sums(part, lane);
+    if (w0 == 0) red[set][row_in][warp] = make_float2(sum, squares);
+    __syncthreads();
+    const float2 p0 = w0 < nw ? red[set][row_in][w0] : make_float2(0.f, 0.f), p1 = two && w1 < nw ? red[set][row_in][w1] : make_float2(0.f, 0.f);
+    float mean = p0.x + p1.x;
+    if (!two) mean += __shfl_xor_sync(0xffffffffu, mean, 8);
+    mean += __shfl_xor_sync(0xffffffffu, mean, 4);
+    mean += __shfl_xor_sync(0xffffffffu, mean, 2);
+    mean += __shfl_xor_sync(0xffffffffu, mean, 1);
+    mean *= inv_d;
+    const float d0 = p0.x * i0 - mean, d1 = p1.x * i1 - mean;
+    float var = p0.y + p1.y + n0 * d0 * d0 + n1 * d1 * d1;
+    if (!two) var += __shfl_xor_sync(0xffffffffu, var, 8);
+    var += __shfl_xor_sync(0xffffffffu, var, 4);
+    var += __shfl_xor_sync(0xffffffffu, var, 2);
+    var += __shfl_xor_sync(0xffffffffu, var, 1);
+    const float rstd = rsqrtf(var * inv_d + eps);
+    if (warp == 0 && w0 == 0 && r + row_in < r1) {
+      mean_out[frame * L + r + row_in] = mean;
+      rstd_out[frame * L + r + row_in] = rstd;
+    }
+#pragma unroll
+    for (int k = 0; k < kLnRows; ++k) {
+      const float m = __shfl_sync(0xffffffffu, mean, k * G), rs = __shfl_sync(0xffffffffu, rstd, k * G);
+      const float2 nm = make_float2(-m, -m), rs2 = make_float2(rs, rs);
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int c = threadIdx.x + i * T;
+        if (r + k < r1 && c < nvec) {
           bf16x8 o;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const float2 t = fma2(mul2(add2(__bfloat1622float2(v[r][i].v[j]), nm), rs2), add2(CB200_P2(b, j), one2), CB200_P2(a, j));
+            const float2 t = fma2(mul2(add2(__bfloat1622float2(v[k][i].v[j]), nm), rs2), CB200_P2(b[i], j), CB200_P2(a[i], j));
             o.v[j] = __floats2bfloat162_rn(t.x, t.y);
           }
-          reinterpret_cast<bf16x8*>(y + (row0 + r) * D)[c] = o;
+          reinterpret_cast<bf16x8*>(yf + (long)(r + k) * D)[c] = o;
         }
       }
     }
@@ -423,10 +512,22 @@ __global__ void __launch_bounds__(kThreads) gate_residual_bwd_kernel(
 // Sixteen lanes per (token, head) row, two rows per warp pass. A lane holds P = HD / 32 elements of each half of the row, at the same
 // offset, so that the rotation partner of every element is in the lane itself and one cosine / sine vector serves both; reductions
 // stay inside the 16-lane half. Token and head of a row are counted along instead of divided out (64-bit divisions per row, a
-// shuffle per element and twice the table loads bound the earlier layout by instruction issue: 46,800 tokens x 16 heads 147 us,
-// now 95 us; the bytes take 59 us).
+// shuffle per element and twice the table loads bound the first layout by instruction issue). Bound by memory and by the warps in flight:
+// the rows of later passes wait as bf16 (72 registers a thread before, 62 now: four CTAs on an SM for three) and the table's row is
+// loaded with the first ones and again only when the token changes. 46,800 tokens x 16 heads 88 us before, 68 now, without rotation
+// 67 and 57 (the bytes take 59 us; part of them are in L2); 7040 tokens 10.4 and 8.0, 46,800 tokens x 40 heads 209 and 156.
 constexpr int kRmsPasses = 4;        // forward: passes (of two rows) whose loads a warp keeps in flight together
 
+template <int P>
+__device__ __forceinline__ void load_raw(const bf16* p, __nv_bfloat162 (&v)[P / 2]) {
+  if constexpr (P == 4) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    v[0] = *reinterpret_cast<const __nv_bfloat162*>(&raw.x);
+    v[1] = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+  } else {
+    v[0] = *reinterpret_cast<const __nv_bfloat162*>(p);
+  }
+}
 template <int P>
 __device__ __forceinline__ void load_part(const bf16* p, float2 (&v)[P / 2]) {
   if constexpr (P == 4) {
@@ -489,7 +590,7 @@ struct RowCursor {
   }
 };
 
-template <int HD>
+template <int HD, bool ROPE>
 __global__ void __launch_bounds__(256) rmsnorm_rope_fwd_kernel(
     const bf16* __restrict__ x, const void* __restrict__ w, int w_bf16, const float* __restrict__ cosv,
     const float* __restrict__ sinv, bf16* __restrict__ y, float* __restrict__ rstd_out, long n_rows, int S, int H,
@@ -500,53 +601,67 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_fwd_kernel(
   pdl_wait();
   const int lane = threadIdx.x & 31, sub = lane & 15, half = lane >> 4;
   const long row0 = ((long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (2 * U) + half;   // this lane's rows: row0 + 2u
-  float2 lo[U][Q], hi[U][Q];
+  __nv_bfloat162 raw_lo[U][Q], raw_hi[U][Q];        // as bf16 until their pass: half the registers, one CTA more on an SM
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     if (row0 + 2 * u < n_rows) {
       const bf16* xr = x + (row0 + 2 * u) * HD + sub * P;
-      load_part<P>(xr, lo[u]);
-      load_part<P>(xr + HD / 2, hi[u]);
+      load_raw<P>(xr, raw_lo[u]);
+      load_raw<P>(xr + HD / 2, raw_hi[u]);
     } else {
 #pragma unroll
-      for (int j = 0; j < Q; ++j) lo[u][j] = hi[u][j] = make_float2(0.f, 0.f);
+      for (int j = 0; j < Q; ++j) raw_lo[u][j] = raw_hi[u][j] = __floats2bfloat162_rn(0.f, 0.f);
     }
   }
   float2 wl[Q], wh[Q];
   load_weight_part<P>(w, w_bf16, sub * P, wl);
   load_weight_part<P>(w, w_bf16, HD / 2 + sub * P, wh);
   RowCursor at(row0 < n_rows ? row0 : 0, S, H);
+  float2 c[Q], sn[Q];                         // of token `table_s`: a lane's rows are heads of one token as a rule
+  int table_s = at.s;
+  if (ROPE) {
+    load_f32_part<P>(cosv + (long)at.s * (HD / 2) + sub * P, c);
+    load_f32_part<P>(sinv + (long)at.s * (HD / 2) + sub * P, sn);
+  }
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const long row = row0 + 2 * u;
     const bool valid = row < n_rows;          // both halves run every shuffle; only the accesses are predicated
+    float2 lo[Q], hi[Q];
+#pragma unroll
+    for (int j = 0; j < Q; ++j) {
+      lo[j] = __bfloat1622float2(raw_lo[u][j]);
+      hi[j] = __bfloat1622float2(raw_hi[u][j]);
+    }
     float2 ss2 = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int j = 0; j < Q; ++j) ss2 = fma2(hi[u][j], hi[u][j], fma2(lo[u][j], lo[u][j], ss2));
+    for (int j = 0; j < Q; ++j) ss2 = fma2(hi[j], hi[j], fma2(lo[j], lo[j], ss2));
     const float ss = half_warp_sum(ss2.x + ss2.y);
     const float rstd = rsqrtf(ss / HD + eps);
     if (sub == 0 && valid) rstd_out[row] = rstd;
     const float2 rs2 = make_float2(rstd, rstd);
 #pragma unroll
     for (int j = 0; j < Q; ++j) {
-      lo[u][j] = mul2(mul2(lo[u][j], rs2), wl[j]);
-      hi[u][j] = mul2(mul2(hi[u][j], rs2), wh[j]);
+      lo[j] = mul2(mul2(lo[j], rs2), wl[j]);
+      hi[j] = mul2(mul2(hi[j], rs2), wh[j]);
     }
-    if (cosv != nullptr && valid) {
-      float2 c[Q], sn[Q];
-      load_f32_part<P>(cosv + (long)at.s * (HD / 2) + sub * P, c);
-      load_f32_part<P>(sinv + (long)at.s * (HD / 2) + sub * P, sn);
+    if (ROPE && valid) {
+      if (at.s != table_s) {
+        load_f32_part<P>(cosv + (long)at.s * (HD / 2) + sub * P, c);
+        load_f32_part<P>(sinv + (long)at.s * (HD / 2) + sub * P, sn);
+        table_s = at.s;
+      }
 #pragma unroll
       for (int j = 0; j < Q; ++j) {
-        const float2 a = lo[u][j], b = hi[u][j], ns = make_float2(-sn[j].x, -sn[j].y);
-        lo[u][j] = fma2(b, ns, mul2(a, c[j]));
-        hi[u][j] = fma2(a, sn[j], mul2(b, c[j]));
+        const float2 a = lo[j], b = hi[j], ns = make_float2(-sn[j].x, -sn[j].y);
+        lo[j] = fma2(b, ns, mul2(a, c[j]));
+        hi[j] = fma2(a, sn[j], mul2(b, c[j]));
       }
     }
     if (valid) {
       bf16* yr = y + row * HD + sub * P;
-      store_part<P>(yr, lo[u]);
-      store_part<P>(yr + HD / 2, hi[u]);
+      store_part<P>(yr, lo);
+      store_part<P>(yr + HD / 2, hi);
     }
     at.advance(2, S, H);
   }
@@ -776,14 +891,26 @@ int cb200_ln_groups_per_frame(int L, int rows_per_cta) { return (L + rows_per_ct
 
 void cb200_ln_modulate_fwd(const void* x, const float* shift, const float* scale, void* y, float* mean, float* rstd,
                            long rows, int D, int L, long ld_shift, long ld_scale, float eps, cudaStream_t st) {
-#define LAUNCH(MV) ln_modulate_fwd_kernel<MV><<<(unsigned)rows, kThreads, 0, st>>>((const bf16*)x, shift, scale, (bf16*)y, mean, rstd, D, L, ld_shift, ld_scale, eps)
-#define LAUNCH_WARP(NV, R) launch_pdl(ln_modulate_fwd_warp_kernel<NV, R>, dim3((unsigned)((rows / L * ((L + R - 1) / R) + kLnWarps - 1) / kLnWarps)), dim3(kLnWarps * 32), 0, st, (const bf16*)x, shift, scale, (bf16*)y, mean, rstd, rows / L * ((L + R - 1) / R), D, L, (L + R - 1) / R, ld_shift, ld_scale, eps)
-  const bool pairs = rows >= 2 * 148 * 3 * kLnWarps && L > 1;      // three CTAs of pairs on every SM
-  if (D <= 1024) { if (pairs) LAUNCH_WARP(4, 2); else LAUNCH_WARP(4, 1); }
-  else if (D <= 2048) { if (pairs) LAUNCH_WARP(8, 2); else LAUNCH_WARP(8, 1); }
-  else if (D <= 4096) LAUNCH(2); else LAUNCH(4);
-#undef LAUNCH_WARP
-#undef LAUNCH
+  // Few rows (or frames of fewer rows than a CTA takes at a time): a CTA for each. The line: 2048 rows of 2048 6.4 us that way and 6.2 us in
+  // batches, 1024 rows 3.7 and 4.4; 1024 rows of 5120 8.6 and 6.9, 512 rows 4.9 and 6.3.
+  if (rows < (D <= 2048 ? 2048 : 1024) || L < 4) {
+#define LAUNCH_ROW(NV, T) launch_pdl(ln_modulate_fwd_row_kernel<NV, T>, dim3((unsigned)rows), dim3(T), 0, st, (const bf16*)x, shift, scale, (bf16*)y, mean, rstd, D, L, ld_shift, ld_scale, eps)
+    if (D <= 1024) LAUNCH_ROW(1, 128); else if (D <= 2048) LAUNCH_ROW(2, 128); else if (D <= 4096) LAUNCH_ROW(2, 256); else LAUNCH_ROW(4, 256);
+#undef LAUNCH_ROW
+    return;
+  }
+  // rows of a CTA: two waves of CTAs while they are few, at most 20 (longer walks leave the last wave emptier)
+  const int resident = 148 * (D <= 512 ? 12 : D <= 1024 ? 6 : D <= 2048 ? 3 : 2);
+  const int per = (int)std::min<long>((rows / (2 * resident) + 4) / 4 * 4, 20);
+  const int groups = (L + per - 1) / per, nvec = D / 8;
+  auto launch = [&](auto kern, int nv) {
+    const int threads = ((nvec + nv - 1) / nv + 31) / 32 * 32;
+    launch_pdl(kern, dim3((unsigned)(rows / L * groups)), dim3(threads), 0, st, (const bf16*)x, shift, scale, (bf16*)y, mean, rstd, D, L, per, groups,
+               ld_shift, ld_scale, eps);
+  };
+  if (D <= 2048) launch(ln_modulate_fwd_rows_kernel<1, 256, 4, 3>, 1);
+  else if (D <= 5120) launch(ln_modulate_fwd_rows_kernel<2, 320, 2, 2>, 2);
+  else launch(ln_modulate_fwd_rows_kernel<2, 512, 2, 1>, 2);
 }
 
 void cb200_ln_modulate_bwd(const void* dy, const void* x, const float* mean, const float* rstd, const float* scale,
@@ -817,10 +944,9 @@ void cb200_gate_residual_bwd(const void* dout, const float* gate, const void* y,
 void cb200_rmsnorm_rope_fwd(const void* x, const void* w, int w_bf16, const float* cosv, const float* sinv, void* y, float* rstd,
                             long n_rows, int S, int H, int HD, float eps, cudaStream_t st) {
   const unsigned blocks = (unsigned)((n_rows + 16 * kRmsPasses - 1) / (16 * kRmsPasses));   // 8 warps x 2 rows x passes per CTA
-  if (HD == 128)
-    launch_pdl(rmsnorm_rope_fwd_kernel<128>, dim3(blocks), dim3(256), 0, st, (const bf16*)x, w, w_bf16, cosv, sinv, (bf16*)y, rstd, n_rows, S, H, eps);
-  else
-    launch_pdl(rmsnorm_rope_fwd_kernel<64>, dim3(blocks), dim3(256), 0, st, (const bf16*)x, w, w_bf16, cosv, sinv, (bf16*)y, rstd, n_rows, S, H, eps);
+  auto launch = [&](auto kern) { launch_pdl(kern, dim3(blocks), dim3(256), 0, st, (const bf16*)x, w, w_bf16, cosv, sinv, (bf16*)y, rstd, n_rows, S, H, eps); };
+  if (HD == 128) cosv != nullptr ? launch(rmsnorm_rope_fwd_kernel<128, true>) : launch(rmsnorm_rope_fwd_kernel<128, false>);
+  else cosv != nullptr ? launch(rmsnorm_rope_fwd_kernel<64, true>) : launch(rmsnorm_rope_fwd_kernel<64, false>);
 }
 
 long cb200_rmsnorm_bwd_blocks(long n_rows, int rows_per_warp) {

@@ -36,6 +36,24 @@ def test_modulation_slices_are_read_in_place(D, L, T, offset):
     assert _max_rel(dg.view(1, T, D), (dout.double() * y.double()).sum(2)) < 1e-5
 
 
+# a CTA per row (few rows, short frames) and batches of rows per CTA: partial warps and partial last pieces of a row, frames that end
+# inside a batch, the row counts where the kernel changes, every instantiation
+@pytest.mark.parametrize("D,L,T", [(8, 700, 3), (520, 4, 520), (1024, 2047, 1), (2048, 2048, 1), (2040, 41, 53), (2048, 3, 700), (2056, 1023, 1),
+                                   (2056, 26, 41), (4104, 513, 2), (5120, 1041, 1), (5128, 130, 8), (8192, 7, 150), (8192, 5, 3)])
+def test_layernorm_row_counts_and_widths(D, L, T):
+    torch.manual_seed(6)
+    x = (torch.randn(T * L, D, device=DEV) * 2 + 3 * torch.randn(T * L, 1, device=DEV)).bfloat16()
+    mod = torch.randn(T, 2 * D, device=DEV)
+    y, mean, rstd = native.load().ln_modulate_fwd(x, mod[:, :D], mod[:, D:], L, 1e-6)
+    xd = x.double()
+    want_mean, want_rstd = xd.mean(1), torch.rsqrt(xd.var(1, unbiased=False) + 1e-6)
+    frame = torch.arange(T * L, device=DEV) // L
+    want = (xd - want_mean[:, None]) * want_rstd[:, None] * (1 + mod[:, D:].double()[frame]) + mod[:, :D].double()[frame]
+    assert _max_rel(y, want) < 1.5 * 2.0 ** -9
+    # fp32 sums of at most 8192 terms in parts of 64 and a tree: a handful of roundings of 2^-24
+    assert _max_rel(mean, want_mean) < 1e-6 and _max_rel(rstd, want_rstd) < 1e-6
+
+
 def test_gated_gemm_epilogue_reads_strided_gates():
     torch.manual_seed(1)
     B, T, L, D, K = 1, 3, 88, 256, 128
