@@ -11,6 +11,7 @@
 #include "launchers.h"
 
 int* cb200_error_word(int device);
+int cb200_sm_count(int device);
 
 namespace {
 using at::Tensor;
@@ -31,7 +32,7 @@ std::tuple<Tensor, Tensor> fa_fwd_variant(const Tensor& q, const Tensor& k, cons
   Tensor o = at::empty_like(q);
   Tensor lse = at::empty({B, H, Sq}, q.options().dtype(at::kFloat));
   const int rc = cb200_fa_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), B, Sq, Skv, H,
-                              (float)scale, (int)variant, cb200_error_word(q.get_device()),
+                              (float)scale, (int)variant, cb200_sm_count(q.get_device()), cb200_error_word(q.get_device()),
                               at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(rc == 0, "fa_fwd launch failed with code ", rc);
   return {o, lse};

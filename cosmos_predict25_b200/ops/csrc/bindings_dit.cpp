@@ -58,7 +58,7 @@ struct Launcher {
     TORCH_CHECK(rc == 0, "tcgen05 GEMM (several weights) launch failed with code ", rc);
   }
   void attention(const void* q, const void* k, const void* v, void* o, float* lse, int64_t B, int64_t Sq, int64_t Skv, int64_t H) const {
-    const int rc = cb200_fa_fwd(q, k, v, o, lse, (int)B, (int)Sq, (int)Skv, (int)H, (float)(1.0 / std::sqrt(128.0)), 0, err, st);
+    const int rc = cb200_fa_fwd(q, k, v, o, lse, (int)B, (int)Sq, (int)Skv, (int)H, (float)(1.0 / std::sqrt(128.0)), 0, sms, err, st);
     TORCH_CHECK(rc == 0, "fa_fwd launch failed with code ", rc);
   }
 };

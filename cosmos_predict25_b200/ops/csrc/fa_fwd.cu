@@ -25,7 +25,8 @@
 //   * SPLITP = 2 or 4: the probabilities are published in halves / quarters of the key tile on their own barriers, so P.V of
 //     the first keys runs while the rest of the row is still being exponentiated.
 // QT = 1 is the shape for short key sequences (cross-attention, 512 keys): one query tile, 192 threads, 97 KB of shared memory and 256
-// TMEM columns per CTA, so that two CTAs share an SM and fill each other's prologue / epilogue gaps.
+// TMEM columns per CTA, so that two CTAs share an SM and fill each other's prologue / epilogue gaps. Where there are no more CTAs than
+// SMs it has an SM to itself and a ring of five slots (DEEP).
 //
 // Online softmax keeps a reference maximum per row that is only moved when the running maximum grows
 // by more than 2^8; the output accumulator is rescaled in TMEM only then (rare after the first tiles).
@@ -47,22 +48,24 @@ constexpr int BQ = 128;          // query rows per tile (two tiles per CTA)
 constexpr int BKV = 128;         // keys per tile
 constexpr int kTileBytes = 128 * HD * 2;  // 32 KB
 constexpr int kHalfBytes = kTileBytes / 2;
+constexpr int kAheadTiles = 4;            // key tiles asked into L2 ahead of the wait (DEEP)
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 // shape of a CTA with QT query tiles: 4 softmax warps per tile, then the TMA warp and the MMA warp
 // REGS: the CTA is padded to whole warpgroups (12 warps) and re-divides its registers at start: the warpgroup of the TMA / MMA warps
 // gives registers back (setmaxnreg.dec) and the softmax warpgroups take them (setmaxnreg.inc), which removes the spills of the
 // 128-value score row. The padding also pays for a second MMA issuer: each query tile gets its own issuing warp, so a wait
 // on one tile's probabilities never delays the other tile's MMAs.
-template <int QT, bool REGS = false>
+// DEEP: one query tile in a CTA that has its SM to itself: the ring takes the shared memory that a second CTA would have
+template <int QT, bool REGS = false, bool DEEP = false>
 struct Shape {
-  static constexpr int kRing = QT == 2 ? 5 : 2;           // K/V ring slots
+  static constexpr int kRing = QT == 2 || DEEP ? 5 : 2;   // K/V ring slots
   static constexpr int kTmaWarp = 4 * QT, kMmaWarp = 4 * QT + 1;
   static constexpr int kIssuers = REGS ? QT : 1;          // MMA issuer warps kMmaWarp .. kMmaWarp + kIssuers - 1
   static constexpr int kThreads = REGS ? (4 * QT + 4) * 32 : (4 * QT + 2) * 32;
   // register re-division: launched with kRegsLaunch per thread (12 warps); the CTA can only re-divide that allocation
   static constexpr int kRegsLaunch = 168, kRegsSoftmax = 224, kRegsOther = 56;
   static_assert(!REGS || (8 * kRegsSoftmax + 4 * kRegsOther <= 12 * kRegsLaunch), "setmaxnreg budget: increases must be covered by decreases");
-  static constexpr int kMinCtas = QT == 2 ? 1 : 2;
+  static constexpr int kMinCtas = QT == 2 || DEEP ? 1 : 2;
   static constexpr uint32_t kTmemCols = 256 * QT;
   static constexpr size_t kSmem = (QT + kRing) * (size_t)kTileBytes + 1024 + 256;
 };
@@ -124,13 +127,13 @@ struct NaParams {
   int max_n, nT, nH, nW;
 };
 
-template <int QT, int EXPM, int SPLITP, bool NA, bool REGS>
-__global__ void __launch_bounds__(fa::Shape<QT, REGS>::kThreads, fa::Shape<QT, REGS>::kMinCtas)
+template <int QT, int EXPM, int SPLITP, bool NA, bool REGS, bool DEEP>
+__global__ void __launch_bounds__(fa::Shape<QT, REGS, DEEP>::kThreads, fa::Shape<QT, REGS, DEEP>::kMinCtas)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, bf16* __restrict__ O, float* __restrict__ LSE, int Sq, int Skv, int H,
               float scale_log2, SeqScatter sc, NaParams na, int* __restrict__ err) {
   using namespace fa;
-  using Sh = Shape<QT, REGS>;
+  using Sh = Shape<QT, REGS, DEEP>;
   constexpr int kRing = Sh::kRing, kMmaWarp = Sh::kMmaWarp, kTmaWarp = Sh::kTmaWarp;
   static_assert(!REGS || QT == 2, "register re-division needs whole warpgroups per role");
   extern __shared__ uint8_t smem_raw[];
@@ -186,6 +189,19 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();                     // launched with programmatic serialisation (see common.cuh)
+  if (DEEP && warp == kTmaWarp && lane == 0) {
+    // The first keys and values, of a context as a rule ones that only HBM holds, on their way into L2 while the kernel in front still
+    // runs (a hint: where that kernel writes them, the loads below see what it wrote).
+    prefetch_tmap(&tm_q);
+    prefetch_tmap(&tm_k);
+    prefetch_tmap(&tm_v);
+    const int ahead = min((Skv + BKV - 1) / BKV, kAheadTiles);
+    for (int n = 0; n < ahead; ++n)
+      for (int c = 0; c < 2; ++c) {
+        tma_prefetch_l2_4d(&tm_k, c * 64, h, n * BKV, b);
+        tma_prefetch_l2_4d(&tm_v, c * 64, h, n * BKV, b);
+      }
+  }
   pdl_wait();
   const int n_kv = NA ? na.kv_cnt[blockIdx.x] : (Skv + BKV - 1) / BKV;
   const int* kv_list = NA ? na.kv_idx + (size_t)blockIdx.x * na.max_n : nullptr;
@@ -196,9 +212,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     // -------------------------------------------------------------------- TMA producer
     if (REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Sh::kRegsOther));
     if (lane == 0) {
-      prefetch_tmap(&tm_q);
-      prefetch_tmap(&tm_k);
-      prefetch_tmap(&tm_v);
+      if (!DEEP) {
+        prefetch_tmap(&tm_q);
+        prefetch_tmap(&tm_k);
+        prefetch_tmap(&tm_v);
+      }
       mbar_arrive_expect_tx(q_full, QT * kTileBytes);
       // neighbourhood mode: tile index -> coordinates of its 5-D box (w0, h0, b * T + t0)
       auto load_tile = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int tile) {
@@ -497,13 +515,13 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
 using namespace cb200;
 
-template <int QT, int EXPM, int SPLITP, bool NA = false, bool REGS = false>
+template <int QT, int EXPM, int SPLITP, bool NA = false, bool REGS = false, bool DEEP = false>
 static int launch_fa_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* o, float* lse, int B, int Sq,
                          int Skv, int H, float scale, const SeqScatter& sc, int* err, cudaStream_t st,
                          const NaParams& na = NaParams{}) {
   using namespace fa;
-  using Sh = Shape<QT, REGS>;
-  auto kern = fa_fwd_kernel<QT, EXPM, SPLITP, NA, REGS>;
+  using Sh = Shape<QT, REGS, DEEP>;
+  auto kern = fa_fwd_kernel<QT, EXPM, SPLITP, NA, REGS, DEEP>;
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::kSmem);
@@ -529,7 +547,7 @@ constexpr int kShortKeys = 1024;   // at most this many keys: the one-tile shape
 // variant: 0 = default; 1..: tuning variants (all produce the same result within rounding)
 static int fa_fwd_dispatch(const void* q, const void* k, const void* v, void* o, float* lse, int B, int Sq, int Skv, int H,
                            float scale, int variant, const SeqScatter& sc, int* err, cudaStream_t st,
-                           const NaParams* na = nullptr) {
+                           const NaParams* na = nullptr, int sms = 0) {
   using namespace fa;
   CUtensorMap tq, tk, tv;
   auto make = [&](CUtensorMap* m, const void* p, int S) {
@@ -566,14 +584,19 @@ static int fa_fwd_dispatch(const void* q, const void* k, const void* v, void* o,
     case 11: return launch_fa_fwd<2, 0, 4, false, true>(tq, tk, tv, o, lse, B, Sq, Skv, H, scale, sc, err, st);
     default: break;
   }
+  // No more CTAs than SMs: two on an SM would leave others idle. With five ring slots for two the next keys are loaded while a tile is in
+  // softmax, and the first four tiles' come from L2: 2 x 256 queries x 16 heads from 512 keys 11.4 us before, now 9.5, from 256 keys 8.0
+  // and 6.4, 500 x 16 from 1024 18.3 and 15.3; with more CTAs two on an SM are the faster ones (160 CTAs 13.6).
+  if (sc.P == 0 && Skv <= kShortKeys && (long)((Sq + BQ - 1) / BQ) * H * B <= sms)
+    return launch_fa_fwd<1, kDefaultExpm, kDefaultSplit, false, false, true>(tq, tk, tv, o, lse, B, Sq, Skv, H, scale, sc, err, st);
   if (sc.P == 0 && Skv <= kShortKeys) return launch_fa_fwd<1, kDefaultExpm, kDefaultSplit>(tq, tk, tv, o, lse, B, Sq, Skv, H, scale, sc, err, st);
   return launch_fa_fwd<2, kDefaultExpm, kDefaultSplit, false, true>(tq, tk, tv, o, lse, B, Sq, Skv, H, scale, sc, err, st);
 }
 
 extern "C" int cb200_fa_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int B, int Sq, int Skv, int H,
-                            float scale, int variant, int* err, cudaStream_t st) {
+                            float scale, int variant, int sms, int* err, cudaStream_t st) {
   SeqScatter sc{};
-  return fa_fwd_dispatch(q, k, v, o, lse, B, Sq, Skv, H, scale, variant, sc, err, st);
+  return fa_fwd_dispatch(q, k, v, o, lse, B, Sq, Skv, H, scale, variant, sc, err, st, nullptr, sms);
 }
 
 // Attention whose output rows are scattered to the P ranks' sequence shards (out_ptrs[r]: [B, Sq / P, P*H, 128] bf16 on rank r).

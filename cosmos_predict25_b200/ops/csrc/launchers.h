@@ -84,7 +84,7 @@ int cb200_fa_bwd_na(const void* d_o, const void* q, const void* k, const void* v
                     void* dv, float* scratch, int B, int S, int H, float scale, const int* q_list, const int* q_cnt, int max_n,
                     const uint8_t* bt, const uint8_t* bh, const uint8_t* bw, int nT, int nH, int nW, int* err, cudaStream_t st);
 int cb200_fa_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int B, int Sq, int Skv, int H, float scale,
-                 int variant, int* err, cudaStream_t st);
+                 int variant, int sms, int* err, cudaStream_t st);
 }
 
 extern "C" {

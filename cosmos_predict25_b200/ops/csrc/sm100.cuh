@@ -121,6 +121,11 @@ __device__ __forceinline__ void tma_load_5d(void* smem_dst, const CUtensorMap* m
 __device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* m, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y) : "memory");
 }
+__device__ __forceinline__ void tma_prefetch_l2_4d(const CUtensorMap* m, int x, int y, int z, int w) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global [%0, {%1, %2, %3, %4}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(z),
+               "r"(w)
+               : "memory");
+}
 // Untiled bulk copy global -> shared (both addresses 16-byte aligned, bytes a multiple of 16), same completion rule.
 __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"

@@ -294,6 +294,21 @@ def test_flash_attention_fwd_variants(B, Sq, Skv, H, variant):
     _close(o, orf, 2e-2, 2e-2, "o")
 
 
+# short key sequences: as many query tiles as a B200 has SMs and one more (a CTA with the SM to itself, two on an SM), key tiles around
+# the ring's five slots
+@pytest.mark.parametrize("Sq", [128 * 37, 128 * 37 + 1])
+@pytest.mark.parametrize("Skv", [1, 256, 300, 1024])
+def test_flash_attention_fwd_short_keys(Sq, Skv):
+    torch.manual_seed(11)
+    q, k, v = (torch.randn(1, S, 4, 128, device=DEV).bfloat16() for S in (Sq, Skv, Skv))
+    scale = 1.0 / math.sqrt(128)
+    o, lse = _ops().fa_fwd(q, k, v, scale)
+    _no_kernel_error()
+    orf, lser = ref.attention(q.float(), k.float(), v.float(), scale)
+    _close(lse, lser, 2e-2, 1e-3, "lse")
+    _close(o, orf, 2e-2, 2e-2, "o")
+
+
 def test_forward_kernels_are_bitwise_repeatable():
     """The forward has no atomics: two runs on the same inputs must agree bit for bit (default shape choice for long and for
     short key sequences)."""
