@@ -800,7 +800,7 @@ class CosmosDiT(nn.Module):
             weights, kvs, eps = plain
             cos, sin = rope.cos_sin() if rope is not None else (None, None)
             x = native.load().dit_blocks(x.contiguous(), all_mods, cos, sin, weights, kvs, 1e-6, eps)
-            native.count_launch((13 + native.load().gemm_group_launches(B * T * H * W, 3)) * len(self.blocks))
+            native.count_launch((12 + native.load().gemm_group_launches(B * T * H * W, 3)) * len(self.blocks))
         for i, block in enumerate(self.blocks if plain is None else ()):
             kv = cross_kv[i] if cross_kv else None
             mods = None if all_mods is None else all_mods[3 * i: 3 * i + 3]

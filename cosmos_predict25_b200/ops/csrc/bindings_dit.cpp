@@ -1,6 +1,6 @@
 // The sampling-time path of the DiT in native code: all transformer blocks of a denoising step (and the cross-attention keys / values
 // of all blocks for a prompt) as ONE operator each, which launches the package's kernels back to back. A block is 16 launches
-// (14 here: q, k and v are one GEMM over three weights);
+// (13 here: q, k and v are one GEMM over three weights, the norms of q and k one launch);
 // issued one by one through Python and the dispatcher they cost about 25 us of host time each, more than most of them take on the GPU
 // for an image of 256 x 256 (512 tokens with guidance): 12.9 ms a step, 8.0 ms with this loop when it was written, 6.1 ms with the
 // kernels of today (4.3 ms of it host time). The kernels are those of models/dit.py:
@@ -99,7 +99,7 @@ Tensor dit_blocks(const Tensor& x, const Tensor& mods, const c10::optional<Tenso
   // two residual streams in turn, the normalised input, and one buffer that is q, k, v, attention output and then the MLP's hidden layer
   Tensor r0 = at::empty({M, D}, x.options()), r1 = at::empty({M, D}, x.options()), h = at::empty({M, D}, x.options());
   Tensor wide = at::empty({std::max(4 * D, F) * M}, x.options());
-  Tensor stats = at::empty({2 * M}, f32), rstd = at::empty({M * H}, f32), lse = at::empty({B * H * S}, f32);
+  Tensor stats = at::empty({2 * M}, f32), rstd = at::empty({2 * M * H}, f32), lse = at::empty({B * H * S}, f32);
   auto part = [&](int64_t i) { return static_cast<void*>(static_cast<char*>(wide.data_ptr()) + i * M * D * 2); };
   void *q = part(0), *k = part(1), *v = part(2), *o = part(3), *hp = h.data_ptr();
   float *mean = stats.data_ptr<float>(), *rs = mean + M, *rn = rstd.data_ptr<float>(), *lp = lse.data_ptr<float>();
@@ -129,8 +129,15 @@ Tensor dit_blocks(const Tensor& x, const Tensor& mods, const c10::optional<Tenso
     ln(0);
     // the attention output's and the next residual stream's places hold the raw projections meanwhile
     run.gemms(hp, {weight(w[0], x, D, D), weight(w[1], x, D, D), weight(w[2], x, D, D)}, {o, nxt, v}, M, D, D);
-    rms(o, norm(w[4], x, keep), cp, sp, q);
-    rms(nxt, norm(w[5], x, keep), cp, sp, k);
+    {
+      // both in one launch: a launch of its own took k 3.9 us at 512 tokens, bound by its start
+      const Norm nq = norm(w[4], x, keep), nk = norm(w[5], x, keep);
+      const void *raw[2] = {o, nxt}, *nw[2] = {nq.p, nk.p};
+      const int nb[2] = {nq.bf16, nk.bf16};
+      void* dst[2] = {q, k};
+      float* rr[2] = {rn, rn + M * H};
+      cb200_rmsnorm_rope_fwd_pair(raw, nw, nb, cp, sp, dst, rr, M * H, (int)S, (int)H, 128, (float)rms_eps, run.st);
+    }
     run.attention(q, k, v, o, lp, B, S, S, H);
     add(0, o, weight(w[3], x, D, D), D);
     ln(1);

@@ -590,15 +590,28 @@ struct RowCursor {
   }
 };
 
+// One tensor or two of the same shape (q and k of a self-attention) in a launch: tensor blockIdx.y.
+struct RmsTensors {
+  const bf16* x[2];
+  const void* w[2];
+  int w_bf16[2];
+  bf16* y[2];
+  float* rstd[2];
+};
+
 template <int HD, bool ROPE>
 __global__ void __launch_bounds__(256) rmsnorm_rope_fwd_kernel(
-    const bf16* __restrict__ x, const void* __restrict__ w, int w_bf16, const float* __restrict__ cosv,
-    const float* __restrict__ sinv, bf16* __restrict__ y, float* __restrict__ rstd_out, long n_rows, int S, int H,
+    const __grid_constant__ RmsTensors tensors, const float* __restrict__ cosv, const float* __restrict__ sinv, long n_rows, int S, int H,
     float eps) {
   constexpr int P = HD / 32, Q = P / 2;
   constexpr int U = kRmsPasses;
   pdl_trigger();                     // launched with programmatic serialisation (see common.cuh)
   pdl_wait();
+  const bf16* __restrict__ x = tensors.x[blockIdx.y];
+  const void* __restrict__ w = tensors.w[blockIdx.y];
+  const int w_bf16 = tensors.w_bf16[blockIdx.y];
+  bf16* __restrict__ y = tensors.y[blockIdx.y];
+  float* __restrict__ rstd_out = tensors.rstd[blockIdx.y];
   const int lane = threadIdx.x & 31, sub = lane & 15, half = lane >> 4;
   const long row0 = ((long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (2 * U) + half;   // this lane's rows: row0 + 2u
   __nv_bfloat162 raw_lo[U][Q], raw_hi[U][Q];        // as bf16 until their pass: half the registers, one CTA more on an SM
@@ -941,12 +954,23 @@ void cb200_gate_residual_bwd(const void* dout, const float* gate, const void* y,
   reduce_partials_kernel<<<grid, 256, 0, st>>>(partials, dgate, nullptr, D, G, 1);
 }
 
-void cb200_rmsnorm_rope_fwd(const void* x, const void* w, int w_bf16, const float* cosv, const float* sinv, void* y, float* rstd,
-                            long n_rows, int S, int H, int HD, float eps, cudaStream_t st) {
-  const unsigned blocks = (unsigned)((n_rows + 16 * kRmsPasses - 1) / (16 * kRmsPasses));   // 8 warps x 2 rows x passes per CTA
-  auto launch = [&](auto kern) { launch_pdl(kern, dim3(blocks), dim3(256), 0, st, (const bf16*)x, w, w_bf16, cosv, sinv, (bf16*)y, rstd, n_rows, S, H, eps); };
+static void launch_rmsnorm_rope_fwd(const RmsTensors& tensors, int n, const float* cosv, const float* sinv, long n_rows, int S, int H, int HD,
+                                    float eps, cudaStream_t st) {
+  const dim3 blocks((unsigned)((n_rows + 16 * kRmsPasses - 1) / (16 * kRmsPasses)), n);   // 8 warps x 2 rows x passes per CTA
+  auto launch = [&](auto kern) { launch_pdl(kern, blocks, dim3(256), 0, st, tensors, cosv, sinv, n_rows, S, H, eps); };
   if (HD == 128) cosv != nullptr ? launch(rmsnorm_rope_fwd_kernel<128, true>) : launch(rmsnorm_rope_fwd_kernel<128, false>);
   else cosv != nullptr ? launch(rmsnorm_rope_fwd_kernel<64, true>) : launch(rmsnorm_rope_fwd_kernel<64, false>);
+}
+
+void cb200_rmsnorm_rope_fwd(const void* x, const void* w, int w_bf16, const float* cosv, const float* sinv, void* y, float* rstd,
+                            long n_rows, int S, int H, int HD, float eps, cudaStream_t st) {
+  launch_rmsnorm_rope_fwd({{(const bf16*)x}, {w}, {w_bf16}, {(bf16*)y}, {rstd}}, 1, cosv, sinv, n_rows, S, H, HD, eps, st);
+}
+
+void cb200_rmsnorm_rope_fwd_pair(const void* const* x, const void* const* w, const int* w_bf16, const float* cosv, const float* sinv,
+                                 void* const* y, float* const* rstd, long n_rows, int S, int H, int HD, float eps, cudaStream_t st) {
+  launch_rmsnorm_rope_fwd({{(const bf16*)x[0], (const bf16*)x[1]}, {w[0], w[1]}, {w_bf16[0], w_bf16[1]}, {(bf16*)y[0], (bf16*)y[1]},
+                           {rstd[0], rstd[1]}}, 2, cosv, sinv, n_rows, S, H, HD, eps, st);
 }
 
 long cb200_rmsnorm_bwd_blocks(long n_rows, int rows_per_warp) {

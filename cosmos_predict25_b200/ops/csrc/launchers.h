@@ -21,6 +21,9 @@ void cb200_gate_residual_bwd(const void* dout, const float* gate, const void* y,
                              long frames, int D, int L, int rows_per_cta, long ld_gate, cudaStream_t st);
 void cb200_rmsnorm_rope_fwd(const void* x, const void* w, int w_bf16, const float* cosv, const float* sinv, void* y, float* rstd,
                             long n_rows, int S, int H, int HD, float eps, cudaStream_t st);
+// two tensors of one shape in one launch
+void cb200_rmsnorm_rope_fwd_pair(const void* const* x, const void* const* w, const int* w_bf16, const float* cosv, const float* sinv,
+                                 void* const* y, float* const* rstd, long n_rows, int S, int H, int HD, float eps, cudaStream_t st);
 long cb200_rmsnorm_bwd_blocks(long n_rows, int rows_per_warp);
 void cb200_rmsnorm_rope_bwd(const void* dy, const void* x, const void* w, int w_bf16, const float* rstd, const float* cosv,
                             const float* sinv, void* dx, float* dw, float* partials, long n_rows, int S, int H, int HD,
