@@ -95,7 +95,35 @@ struct GemmEpilogue {
   int L;              // rows per gate vector
 };
 
-__device__ __forceinline__ float gelu_erf(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
+// Exact GELU of a pair of values: x Phi(x) = (x + |x|) / 2 - |x| Phi(-|x|), and Phi(-a) = exp(-a^2 / 2) R(a), where R = erfcx(a / sqrt 2) / 2
+// falls smoothly from 1/2: a degree-11 polynomial in a scaled to [-1, 1] on [0, 5.5], fitted for the relative error (4.2e-6; a thousandth
+// of a bf16 rounding). a R(a) hardly changes beyond 5.5, where the product is below 1e-7: a is held there. The difference 1 + erff
+// that stood here loses its digits for x below -3, and took twice the instructions, which an epilogue has to itself when a CTA has one tile:
+// 512 x 8192 x 2048 with GELU 20.6 us before, now 18.6 (without GELU 16.1).
+// Coefficients are negated: the sum is a fused multiply-add. Infinities and NaN give what the product x Phi(x) gives.
+__device__ __forceinline__ float2 gelu2(float2 x) {
+  constexpr float kC[12] = {-0.130724221f,  0.108487532f,  -0.0841316134f, 0.0614620969f,  -0.0422496423f, 0.0284217875f,
+                            -0.0201631337f, 0.0114772478f, -0.00272275996f, 0.00254054717f, -0.00517878076f, 0.00243854383f};
+  const float2 a = make_float2(fabsf(x.x), fabsf(x.y));
+  const float2 held = make_float2(fminf(a.x, 5.5f), fminf(a.y, 5.5f));
+  const float2 u = fma2(held, make_float2(2.f / 5.5f, 2.f / 5.5f), make_float2(-1.f, -1.f));
+  float2 r = make_float2(kC[11], kC[11]);
+#pragma unroll
+  for (int k = 10; k >= 0; --k) r = fma2(r, u, make_float2(kC[k], kC[k]));
+  constexpr float kHalfLog2e = -0.72134752044448171f;
+  const float2 t = mul2(mul2(x, x), make_float2(kHalfLog2e, kHalfLog2e));
+  const float2 q = mul2(make_float2(exp2f(t.x), exp2f(t.y)), r);
+  const float2 half = make_float2(0.5f, 0.5f);
+  return fma2(held, q, fma2(x, half, mul2(a, half)));
+}
+__device__ __forceinline__ void gelu32(float (&v)[32]) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const float2 g = gelu2(make_float2(v[2 * j], v[2 * j + 1]));
+    v[2 * j] = g.x;
+    v[2 * j + 1] = g.y;
+  }
+}
 
 // Row-sharded B operand gathered inside the kernel (see the header comment).
 constexpr int kGatherWarps = 2;   // with the 10 GEMM warps: three warpgroups, 168 registers per thread (four more warps
@@ -723,10 +751,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 #pragma unroll
               for (int j = 0; j < 32; ++j) v[j] += __bfloat162float(ep.bias[col0 + j]);
             }
-            if (ep.act == 1) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
-            }
+            if (ep.act == 1) gelu32(v);
             if (ep.gate != nullptr) {
               float4 g4[8];                                     // all of the chunk's gate values at once: one latency
 #pragma unroll
@@ -791,8 +816,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 for (int j = 0; j < 32 && col0 + j < N; ++j) ep.pre[off + j] = __float2bfloat16(v[j]);
               }
             }
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
+            gelu32(v);
           }
           if (gate_row != nullptr) {
             if (full_chunk) {

@@ -213,6 +213,36 @@ def test_linear_autograd_matches_reference():
     _close(w.grad, wr.grad, 0.3, 3e-2, "dw")
 
 
+# full tiles and the ragged path; the identity as weight leaves the values as they are in the accumulator
+@pytest.mark.parametrize("M,N", [(512, 512), (300, 200), (128, 72)])
+@pytest.mark.parametrize("spread", [0.1, 1.0, 4.0, 50.0])
+def test_gelu_epilogue_is_as_exact_as_its_rounding(M, N, spread):
+    torch.manual_seed(12)
+    x = (torch.randn(M, N, device=DEV) * spread).bfloat16()
+    y = _ops().gemm_bf16(x, torch.eye(N, device=DEV).bfloat16(), None, 1, False, False)
+    _no_kernel_error()
+    xd = x.double()
+    want = xd * torch.special.ndtr(xd)
+    # one rounding to bf16 (2^-8 relative at most, with the 1e-5 of the approximation beside it), to |x| = 5.4; below 1e-7 beyond on the left
+    near = xd > -5.4
+    assert ((y.double() - want).abs()[near] <= want.abs()[near] * (2.0 ** -8 + 1e-5)).all()
+    assert (y.double() - want).abs()[~near].max().item() < 2e-7 if (~near).any() else True
+
+
+def test_gelu_epilogue_special_values():
+    v = torch.tensor([float("inf"), -float("inf"), float("nan"), 0.0, 3e38, -3e38, 1e-30, -1e-30], device=DEV).bfloat16()   # results below 1.2e-38 have no relative bound in bf16
+    x = torch.zeros(512, 64, device=DEV).bfloat16()
+    x[:8, 0] = v
+    w = torch.zeros(256, 64, device=DEV).bfloat16()
+    w[:, 0] = 1
+    y = _ops().gemm_bf16(x, w, None, 1, False, False)[:8, 0]
+    want = torch.nn.functional.gelu(v.float())
+    _no_kernel_error()
+    assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(torch.isinf(y), torch.isinf(want))
+    ok = torch.isfinite(want)
+    assert torch.allclose(y[ok].float(), want[ok], rtol=2.0 ** -8, atol=0)
+
+
 @pytest.mark.parametrize("B,Sq,Skv,H", [(1, 256, 256, 2), (2, 512, 384, 3), (1, 1000, 999, 2), (1, 300, 15, 4), (1, 2048, 4096, 2)])
 def test_flash_attention_fwd(B, Sq, Skv, H):
     torch.manual_seed(8)
