@@ -475,6 +475,14 @@ class Block(nn.Module):
     def adaln_mlps(self) -> Tuple[nn.Sequential, nn.Sequential, nn.Sequential]:
         return self.adaln_modulation_self_attn, self.adaln_modulation_cross_attn, self.adaln_modulation_mlp
 
+    def keeps_attention_itself(self, x: torch.Tensor) -> bool:
+        """Whether every attention call of ``forward`` is ``ops.attention`` on the native kernel, so that a checkpointed run can keep the
+        results there (``ops.AttentionResults``). Other blocks are looked through operator by operator."""
+        return (type(self) is Block and type(self.self_attn) is Attention and type(self.cross_attn) is Attention and x.is_cuda
+                and x.dtype == torch.bfloat16 and self.self_attn.head_dim == 128 and self.cross_attn.head_dim == 128
+                and self.self_attn.sparse_op is None and self.self_attn.cp_group is None and self.cross_attn.cp_group is None
+                and ops.settings.attention == "native" and ops.settings.attention_bwd == "native" and not native.forward_mode())
+
     def init_weights(self):
         self.self_attn.init_weights()
         self.cross_attn.init_weights()

@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import math
 import os
+import threading
 from dataclasses import dataclass
 from typing import Optional, Sequence, Tuple
 
@@ -290,13 +291,57 @@ def rmsnorm_rope(x: torch.Tensor, weight: torch.Tensor, rope: Optional[RopeTable
 # --------------------------------------------------------------------------------------
 # attention
 # --------------------------------------------------------------------------------------
+class AttentionResults:
+    """Attention outputs and statistics of one checkpointed region: kept while the forward pass runs, handed out again, in the same order,
+    while the region is recomputed. Only the thread that is inside a ``with`` of ``keep()`` or ``reuse()`` sees it (the recomputation runs in
+    a thread of the autograd engine)."""
+
+    _active = threading.local()
+
+    def __init__(self):
+        self._kept = []
+
+    class _Scope:
+        def __init__(self, results, reuse: bool):
+            self.results, self.reuse, self.outer = results, reuse, []
+
+        def __enter__(self):
+            self.outer.append(getattr(AttentionResults._active, "scope", None))
+            AttentionResults._active.scope = self
+
+        def __exit__(self, *exc):
+            AttentionResults._active.scope = self.outer.pop()
+
+    def keep(self):
+        return self._Scope(self, False)
+
+    def reuse(self):
+        return self._Scope(self, True)
+
+    @classmethod
+    def forward(cls, q, k, v, scale):
+        """(o, lse) of the native forward kernel, or the kept ones."""
+        scope = getattr(cls._active, "scope", None)
+        kept = None if scope is None else scope.results._kept
+        if scope is not None and scope.reuse:
+            if not kept:
+                raise RuntimeError("the attention results of this checkpointed region have been used: backward can run through it only once")
+            (o, lse), version = kept.pop(0)
+            if o._version != version:
+                raise RuntimeError("an attention output kept for the recomputation of a checkpointed region was modified in place")
+            return o.detach(), lse
+        o, lse = native.load().fa_fwd(q, k, v, scale)
+        native.count_launch()
+        if kept is not None:
+            kept.append(((o.detach(), lse), o._version))
+        return o, lse
+
+
 class _FlashAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, scale):
-        ops = native.load()
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        o, lse = ops.fa_fwd(q, k, v, scale)
-        native.count_launch()
+        o, lse = AttentionResults.forward(q, k, v, scale)
         ctx.save_for_backward(q, k, v, o, lse)
         ctx.scale = scale
         return o

@@ -88,3 +88,54 @@ def test_seeded_training_losses_repeat():
     assert a == b, (a, b)
     c = _three_losses(12)
     assert a != c
+
+
+def _block_step(mode, selective_by_operator=False):
+    """Output, input gradients and weight gradients of one checkpointed block; launches counted on the way."""
+    from cosmos_predict25_b200.models import checkpointing
+    from cosmos_predict25_b200.models.dit import Block
+    from cosmos_predict25_b200.ops import native
+
+    torch.manual_seed(3)
+    block = Block(dit_mini(model_channels=512, num_heads=4, crossattn_emb_channels=256)).to("cuda", torch.bfloat16).train()
+    block.init_weights()
+    for m in block.adaln_mlps():
+        torch.nn.init.normal_(m[-1].weight, std=0.02)
+    if selective_by_operator:
+        block.keeps_attention_itself = lambda x: False
+    x = torch.randn(1, 2, 96, 512, device="cuda").bfloat16().requires_grad_(True)
+    emb = torch.randn(1, 2, 512, device="cuda").requires_grad_(True)
+    ctx = torch.randn(1, 40, 256, device="cuda").bfloat16().requires_grad_(True)
+    before = native.launches()
+    y = checkpointing.run_block(block, mode, x, emb, ctx, None, None)
+    return block, y, (x, emb, ctx), before
+
+
+def test_kept_attention_results_give_the_gradients_of_the_other_modes():
+    from cosmos_predict25_b200.ops import native
+
+    got = []
+    for mode, by_operator in (("none", False), ("save_attention", False), ("save_attention", True)):
+        block, y, inputs, before = _block_step(mode, by_operator)
+        y.float().pow(2).sum().backward()
+        got.append(([y.detach()] + [t.grad for t in inputs] + [p.grad for p in block.parameters()], native.launches() - before))
+    for other, _ in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0][0], other))
+    assert got[1][1] == got[2][1]           # both count the attention kernels once
+
+
+def test_kept_attention_results_are_used_once_and_unchanged():
+    block, y, _, _ = _block_step("save_attention")
+    y.sum().backward(retain_graph=True)
+    with pytest.raises(RuntimeError, match="only once"):
+        y.sum().backward()
+    # a second region inside the first one's backward, and a region that is dropped, leave nothing behind
+    from cosmos_predict25_b200.ops.functional import AttentionResults
+    assert getattr(AttentionResults._active, "scope", None) is None
+    q = torch.randn(1, 64, 1, 128, device="cuda").bfloat16()
+    results = AttentionResults()
+    with results.keep():
+        o, _ = AttentionResults.forward(q, q, q, 0.1)
+    o.add_(1)
+    with results.reuse(), pytest.raises(RuntimeError, match="in place"):
+        AttentionResults.forward(q, q, q, 0.1)
