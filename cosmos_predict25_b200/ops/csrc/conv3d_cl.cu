@@ -8,12 +8,14 @@
 //   weights    W [N_pad, taps, C_pad]        (K-major; C_pad = C_in rounded up to 64, N_pad = C_out rounded up to the N tile)
 //   output     Y[t, h, w, n] = bias[n] + sum_{tap, c} X[t + dt(tap), h + dh(tap), w + dw(tap), c] * W[n, tap, c]  (+ residual)
 //
-// There is no im2col buffer: an output tile is 128 voxels = 8 rows x 16 columns of one frame, and the A operand of taps
-// (dt, dh .. dh + n - 1, dw), channel block kb is ONE TMA box {64 channels, 16 w, 7 + n h, 1 t} at coordinates
-// (64 kb, w0 + dw, h0 + dh, t + dt) of the activation tensor itself. It lands in shared memory as rows of 64 channels with 128-byte
-// swizzle, K-major, which is what the MMA wants; a step of one tap down is 16 rows = 2,048 bytes, a whole number of swizzle atoms,
-// so the n taps of a column read the same box at shifted start addresses. Coordinates outside the tensor read zeros: that IS the
-// zero padding of the convolution (the channel coordinate stays a multiple of 64, so the 16-byte alignment rule of TMA holds).
+// There is no im2col buffer: an output tile is 128 voxels = 16 lines of 8 of one frame, and the A operand of ALL n x n spatial taps of one
+// frame offset, channel block kb, is ONE TMA box {64 channels, 7 + n, 15 + n, 1 t} of the activation tensor itself. It lands in shared
+// memory as rows of 64 channels with 128-byte swizzle, K-major, which is what the MMA wants: eight voxels of a line are one 8-row group, the
+// groups are a line of the box apart, and tap (dy, dx) reads the same box from dy lines and dx rows on. The swizzle goes by the address, so
+// neither the start of a tap nor the distance of the groups has to be a whole number of 1,024-byte atoms (checked for every shift and
+// distance used here against a plain copy of the rows). Coordinates outside the tensor read zeros: that IS the zero padding of the
+// convolution (the channel coordinate stays a multiple of 64, so the 16-byte alignment rule of TMA holds).
+// The eight voxels run along the width or along the height, whichever leaves fewer tiles over the frame's edge.
 //
 // The causal time padding is either the leading frames of the input tensor (pad = 0), or `pad` frames in a tensor of their own
 // (the stream cache of the previous chunk) of which the oldest may be missing = zeros: taps whose frame lies in zero padding for
@@ -21,14 +23,14 @@
 // down-sampling) step the frame coordinate, and the pixel coordinates through the tensor map's element strides.
 //
 // CTA pairs (tcgen05 cta_group::2): two consecutive voxel tiles share the B operand, each CTA fetches its own A box and half of
-// the B rows, the even CTA issues M = 256 MMAs. What bounds the kernel is the L2 -> shared-memory path of narrow layers: for one
-// (dt, dw) column of a 3 x 3 x 3 convolution with 96 channels a CTA now fetches 20 + 18 KB per channel block instead of
-// 3 x (16 + 12) KB. Decoding 8 latent frames of 720p: 296 ms in this kernel before (one CTA per tile, a box per tap), 176 ms now, norms
-// included; a single 640 x 640 image 5.7 and 2.1 ms. 96 channels, 27 taps with the norm, 4 frames of 704 x 1280: tensor pipe 75 % busy,
-// 1.35 ms (1,329 TFLOP/s); 192 channels 1,635, 384 channels 1,699 TFLOP/s.
+// the B rows, the even CTA issues M = 256 MMAs. A and B have a ring each: a box serves n columns of B boxes. What bounds the kernel is the
+// L2 -> shared-memory path of narrow layers and, on long runs, the card's power, to which that traffic adds: 128 voxels of a
+// 3 x 3 x 3 convolution with 96 channels took 498 KB with a box for each column of taps, now 290 (with 192 channels 1,035 and 800).
+// Decoding 8 latent frames of 720p 196 and 189 ms, encoding 29 frames of 768 x 432 46 and 44, an image of 640 x 640 2.31 and 2.25.
+// Two boxes in flight and the rest for B columns is the best split: three boxes the same, four (two columns of B left) 5 % slower.
 //
-// Persistent, warp-specialised, one CTA per SM, same skeleton as the GEMM of this package: warp 0 TMA producer (ring of A box + B
-// boxes, as many stages as fit), warp 1 MMA issuer (two TMEM accumulators of n_tile columns), warps 2-9 epilogue (bias, optional
+// Persistent, warp-specialised, one CTA per SM, same skeleton as the GEMM of this package: warp 0 TMA producer (a ring of A boxes and
+// one of B boxes), warp 1 MMA issuer (two TMEM accumulators of n_tile columns), warps 2-9 epilogue (bias, optional
 // residual, bf16 store through a per-voxel output mapping that also expresses the phase interleave of the up-sampling
 // convolutions and the frame interleave of the temporal up-sampler). All waits are bounded and report through `err`.
 
@@ -45,29 +47,30 @@ namespace cb200 {
 using namespace sm100;
 
 namespace cv {
-constexpr int BM = 128, BK = 64, TH = 8, TW = 16;
+constexpr int BM = 128, BK = 64, TX = 8, TY = 16;   // a tile: TY lines of TX voxels
 constexpr int kThreads = 320;                 // TMA warp, MMA warp, 8 epilogue warps
-constexpr int kMaxTaps = 27, kMaxRun = 3;     // taps, and taps of one column that share a box
-constexpr int kMaxStages = 8;
+constexpr int kMaxTaps = 27, kMaxRun = 3;     // taps, and lines / columns of taps that share a box
+constexpr int kMaxSlots = 8;                  // of each ring
+constexpr int kBarBytes = 512;
 constexpr int kStageOut = 32 * 64;            // staging block of an epilogue warp: 32 voxels x 32 channels
 constexpr int kBiasMax = 1024;                // channels whose bias is kept in shared memory
-constexpr int kSmemMax = 227 * 1024, kSmemFixed = 1024 /*alignment slack*/ + 256 /*barriers*/ + 8 * kStageOut;
+constexpr int kSmemMax = 227 * 1024, kSmemFixed = 1024 /*alignment slack*/ + kBarBytes + 8 * kStageOut;
 constexpr int kSumSq = 2 * 2 * BM * 4;       // partial sums of squares: buffer, column half, row
 }  // namespace cv
 
 struct ConvParams {
-  int T_out, H_out, W_out;      // output grid walked by the tiles
+  int T_out, X_out, Y_out;      // output grid walked by the tiles; X, Y: width and height, or height and width
   int Cin, Cout;
   int n_tile, tiles_n;          // N per tile (multiple of 16, <= 256) and number of N tiles
-  int ngroups, kblocks;         // K loop: groups of RUN vertically adjacent taps (by ascending dt) x 64-channel blocks
-  int stages;                   // ring depth
+  int npanels, kblocks;         // K loop: panels of RUN x RUN taps of one frame offset (by ascending dt) x 64-channel blocks
+  int a_slots, b_slots;         // ring depths
   int pad, cache_frames;        // frames of causal padding in front of X; tm_c holds the last `cache_frames` of them, the rest is zero
-  int t_stride, hw_stride;      // input coordinate = output coordinate x stride + offset
-  int8_t dt[cv::kMaxTaps], dh[cv::kMaxTaps], dw[cv::kMaxTaps];   // per group: input coordinate = output coordinate + offset
-  int8_t tap[cv::kMaxTaps][cv::kMaxRun];                         // weight column block of each tap of the group
-  // element offset of output voxel (t, h, w), channel n:
-  //   (((t * ot_mul + ot_add) * out_H + h * oh_mul + oh_add) * out_W + w * ow_mul + ow_add) * out_C + oc_add + n
-  int ot_mul, ot_add, oh_mul, oh_add, ow_mul, ow_add, out_H, out_W, out_C, oc_add;
+  int t_stride, xy_stride;      // input coordinate = output coordinate x stride + offset
+  int8_t dt[cv::kMaxTaps], dx[cv::kMaxTaps], dy[cv::kMaxTaps];   // per panel: input coordinate = output coordinate + offset
+  int8_t tap[cv::kMaxTaps][cv::kMaxRun][cv::kMaxRun];            // weight column block of the panel's tap in column i (width), row j (height)
+  // element offset of output voxel (t, x, y), channel n: out_at + t * out_t + x * out_x + y * out_y + n
+  long out_at, out_t, out_x, out_y;
+  int vec;                      // voxels can be moved as 16-byte pieces
   bf16* Y;
   const bf16* resid;            // optional, same addressing as Y
   const float* bias;            // optional [Cout]
@@ -79,10 +82,11 @@ struct ConvParams {
   int silu, write_raw;          // write_raw 0: only Yn is stored
 };
 
-// STACK = 2 (narrow layers, N tile <= 128): a CTA owns two voxel tiles, one below the other, with an accumulator each; their A box is
-// one of 16 + RUN - 1 rows and every B row in shared memory serves both: 486 instead of 684 KB per 128 voxels of a 3 x 3 x 3
-// convolution with 96 channels. 4 frames of 704 x 1280: 1637 -> 1366 us (1,315 TFLOP/s).
-template <int RUN, int STACK>
+// STACK = 2 (narrow layers, N tile <= 128): a CTA owns two voxel tiles side by side, 16 x 16 voxels, with an accumulator each; their A
+// box is one of 18 x 18 voxels and every B row in shared memory serves both.
+// BY_HEIGHT: X is the frame's height. The order of a sum - columns of taps along the width, their rows, channels - is the same either way, so that
+// a band of rows gives the bits of the whole frame.
+template <int RUN, int STACK, bool BY_HEIGHT>
 __global__ void __launch_bounds__(cv::kThreads, 1)
 conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_w,
                const __grid_constant__ ConvParams p, int* __restrict__ err) {
@@ -90,17 +94,22 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int b_half = p.n_tile * (BK * 2 / 2);                  // bytes of one tap's B rows in this CTA (half of the N tile)
-  constexpr int a_bytes = (TH * STACK + RUN - 1) * TW * BK * 2;
-  const int stage_bytes = a_bytes + RUN * b_half;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + p.stages * stage_bytes);
-  uint64_t* full = bars;                      // [stages], the even CTA's count the bytes of both
-  uint64_t* empty = bars + kMaxStages;        // [stages]
-  uint64_t* acc_full = bars + 2 * kMaxStages; // [2]
+  constexpr int kLine = TX * STACK + RUN - 1;                  // voxels of a line of the A box
+  constexpr int kBoxBytes = kLine * (TY + RUN - 1) * BK * 2, kASlot = (kBoxBytes + 1023) / 1024 * 1024;
+  const int b_slot = RUN * b_half;                             // the taps of one column
+  uint8_t* const ring_b = smem + p.a_slots * kASlot;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ring_b + p.b_slots * b_slot);
+  uint64_t* a_full = bars;                    // [a_slots], the even CTA's count the bytes of both
+  uint64_t* a_empty = bars + kMaxSlots;       // [a_slots]
+  uint64_t* b_full = bars + 2 * kMaxSlots;    // [b_slots]
+  uint64_t* b_empty = bars + 3 * kMaxSlots;   // [b_slots]
+  uint64_t* acc_full = bars + 4 * kMaxSlots;  // [2]
   uint64_t* acc_empty = acc_full + 2;         // [2]
   uint64_t* sums_in = acc_empty + 2;          // [2][4] sums of squares of a lane quarter's two warps written (buffer, quarter)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sums_in + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint8_t* stage_out = smem + p.stages * stage_bytes + 256;
+  static_assert((4 * kMaxSlots + 2 + 2 + 8) * 8 + 8 <= kBarBytes, "barriers, tensor-memory address and flag");
+  uint8_t* stage_out = reinterpret_cast<uint8_t*>(bars) + kBarBytes;
   float* ssq = reinterpret_cast<float*>(stage_out + 8 * kStageOut);      // with a fused norm: sums of squares, then gamma
   float* gamma_s = ssq + kSumSq / 4;
   float* bias_s = p.Yn != nullptr ? gamma_s + 256 : ssq;   // [Cout] when Cout <= kBiasMax
@@ -108,14 +117,18 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   // the shuffle makes the warp index (and every role branch below) provably warp-uniform for the compiler
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
-  const int tiles_w = (p.W_out + TW - 1) / TW, tiles_h = (p.H_out + TH * STACK - 1) / (TH * STACK);
-  const int vox_tiles = p.T_out * tiles_h * tiles_w;
+  const int tiles_x = (p.X_out + TX * STACK - 1) / (TX * STACK), tiles_y = (p.Y_out + TY - 1) / TY;
+  const int vox_tiles = p.T_out * tiles_y * tiles_x;
   const int first_tile = (int)(blockIdx.x >> 1), tile_step = (int)(gridDim.x >> 1);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < p.stages; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
+    for (int s = 0; s < p.a_slots; ++s) {
+      mbar_init(&a_full[s], 1);
+      mbar_init(&a_empty[s], 1);
+    }
+    for (int s = 0; s < p.b_slots; ++s) {
+      mbar_init(&b_full[s], 1);
+      mbar_init(&b_empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
@@ -148,22 +161,22 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
 
   // pair tile -> N tile and this CTA's voxel tile (a trailing odd tile is computed by both CTAs and stored by the even one);
   // N tiles of one voxel pair are neighbours so that they run at the same time and share the activation boxes through L2
-  auto decode = [&](int t, int& nt, int& w0, int& h0, int& tf, bool& mine) {
+  auto decode = [&](int t, int& nt, int& x0, int& y0, int& tf, bool& mine) {
     nt = t % p.tiles_n;
     int v = t / p.tiles_n * 2 + (int)rank;
     mine = v < vox_tiles;
     v = min(v, vox_tiles - 1);
-    w0 = (v % tiles_w) * TW;
-    v /= tiles_w;
-    h0 = (v % tiles_h) * (TH * STACK);
-    tf = v / tiles_h;
+    x0 = (v % tiles_x) * (TX * STACK);
+    v /= tiles_x;
+    y0 = (v % tiles_y) * TY;
+    tf = v / tiles_y;
   };
-  // groups whose frame is zero padding for both tiles of the pair are left out: the later tile's frame decides, and the groups
+  // panels whose frame is zero padding for both tiles of the pair are left out: the later tile's frame decides, and the panels
   // are in the order of their frames
-  auto first_group = [&](int t) {
-    const int tf_last = min(t / p.tiles_n * 2 + 1, vox_tiles - 1) / (tiles_h * tiles_w);
+  auto first_panel = [&](int t) {
+    const int tf_last = min(t / p.tiles_n * 2 + 1, vox_tiles - 1) / (tiles_y * tiles_x);
     int g = 0;
-    while (g < p.ngroups - 1 && tf_last * p.t_stride + p.dt[g] < p.pad - p.cache_frames) ++g;
+    while (g < p.npanels - 1 && tf_last * p.t_stride + p.dt[g] < p.pad - p.cache_frames) ++g;
     return g;
   };
 
@@ -173,30 +186,35 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       prefetch_tmap(&tm_x);
       prefetch_tmap(&tm_c);
       prefetch_tmap(&tm_w);
-      int s = 0;
-      uint32_t ph = 0;
+      int as = 0, bs = 0;
+      uint32_t aph = 0, bph = 0;
       bool ok = true;
       for (int t = first_tile; t < n_tiles && ok; t += tile_step) {
-        int nt, w0, h0, tf;
+        int nt, x0, y0, tf;
         bool mine;
-        decode(t, nt, w0, h0, tf, mine);
+        decode(t, nt, x0, y0, tf, mine);
         const int n0 = nt * p.n_tile + (int)rank * (p.n_tile / 2);
-        for (int g = first_group(t); g < p.ngroups && ok; ++g) {
+        for (int g = first_panel(t); g < p.npanels && ok; ++g) {
           const int tx = tf * p.t_stride + p.dt[g] - p.pad;          // frame of X; negative: a cached frame or padding
           const bool cached = tx < 0 && p.cache_frames > 0;
           const CUtensorMap* tm = cached ? &tm_c : &tm_x;
           const int tc = cached ? tx + p.cache_frames : tx;
-          const int xw = w0 * p.hw_stride + p.dw[g], xh = h0 * p.hw_stride + p.dh[g];
-          for (int kb = 0; kb < p.kblocks; ++kb) {
-            if (!mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-            uint8_t* sa = smem + s * stage_bytes;
-            if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * stage_bytes);
-            const uint32_t bar = mapa_shared(smem_u32(&full[s]), 0);
-            tma_load_4d_pair(sa, tm, bar, kb * BK, xw, xh, tc);
+          const int xx = x0 * p.xy_stride + p.dx[g], xy = y0 * p.xy_stride + p.dy[g];
+          for (int kb = 0; kb < p.kblocks && ok; ++kb) {
+            if (!mbar_wait(&a_empty[as], aph ^ 1, abort_flag)) { ok = false; break; }
+            if (rank == 0) mbar_arrive_expect_tx(&a_full[as], 2 * kBoxBytes);
+            tma_load_4d_pair(smem + as * kASlot, tm, mapa_shared(smem_u32(&a_full[as]), 0), kb * BK, xx, xy, tc);
+            if (++as == p.a_slots) { as = 0; aph ^= 1; }
 #pragma unroll
-            for (int j = 0; j < RUN; ++j)
-              tma_load_2d_pair(sa + a_bytes + j * b_half, &tm_w, bar, (p.tap[g][j] * p.kblocks + kb) * BK, n0);
-            if (++s == p.stages) { s = 0; ph ^= 1; }
+            for (int i = 0; i < RUN; ++i) {
+              if (!mbar_wait(&b_empty[bs], bph ^ 1, abort_flag)) { ok = false; break; }
+              if (rank == 0) mbar_arrive_expect_tx(&b_full[bs], 2 * b_slot);
+              const uint32_t bar = mapa_shared(smem_u32(&b_full[bs]), 0);
+#pragma unroll
+              for (int j = 0; j < RUN; ++j)
+                tma_load_2d_pair(ring_b + bs * b_slot + j * b_half, &tm_w, bar, (p.tap[g][i][j] * p.kblocks + kb) * BK, n0);
+              if (++bs == p.b_slots) { bs = 0; bph ^= 1; }
+            }
           }
         }
       }
@@ -207,10 +225,10 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     const uint32_t leader = elect_one() ? 1u : 0u;
     auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)); };
     const uint32_t idesc = umma_idesc_bf16(2 * BM, p.n_tile, 0, 0);
-    const uint64_t da0 = umma_desc_sw128(smem_u32(smem), 16, 1024);
-    const uint64_t db0 = umma_desc_sw128(smem_u32(smem) + a_bytes, 16, 1024);
-    int s = 0;
-    uint32_t ph = 0;
+    const uint64_t da0 = umma_desc_sw128(smem_u32(smem), 16, kLine * BK * 2);
+    const uint64_t db0 = umma_desc_sw128(smem_u32(ring_b), 16, 1024);
+    int as = 0, bs = 0;
+    uint32_t aph = 0, bph = 0;
     int acc = 0;
     uint32_t acc_ph = 0;
     bool ok = true;
@@ -219,37 +237,45 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + acc * 256;
       uint32_t first = 0;
-      for (int g = first_group(t); g < p.ngroups && ok; ++g) {
-        for (int kb = 0; kb < p.kblocks; ++kb) {
-          if (!wait_all(&full[s], ph)) { ok = false; break; }
-          tc_fence_after();
-          const uint64_t da_s = da0 + (uint64_t)(s * (stage_bytes >> 4)), db_s = db0 + (uint64_t)(s * (stage_bytes >> 4));
+      for (int g = first_panel(t); g < p.npanels && ok; ++g) {
+        for (int kb = 0; kb < p.kblocks && ok; ++kb) {
+          if (!wait_all(&a_full[as], aph)) { ok = false; break; }
+          const uint64_t da_s = da0 + (uint64_t)(as * (kASlot >> 4));
           const int ksteps = (p.Cin - kb * BK) / 16;   // below 4 in the last block of, e.g., C_in = 96: 32 real channels
-          // straight-line issue: one warp issues every MMA of the pair, and a narrow MMA (N = 96: 48 clocks) is over before a
-          // loop with descriptor arithmetic gets to the next one (64 -> 16 channels, 27 taps: 6.8 us a tile as loops, 4.4 us)
-          auto issue = [&](int j, int k) {
-            const uint64_t db = db_s + (uint32_t)(j * (b_half >> 4) + k * 2);
 #pragma unroll
-            for (int u = 0; u < STACK; ++u)
-              umma_ss_pair_w(d_tmem + u * 128, da_s + (uint32_t)(((u * TH + j) * TW * 128 + k * 32) >> 4), db, idesc, (j | k) ? 1u : first, leader);
-          };
-          if (ksteps >= 4) {
+          for (int i = 0; i < RUN; ++i) {
+            if (!wait_all(&b_full[bs], bph)) { ok = false; break; }
+            tc_fence_after();
+            const uint64_t db_s = db0 + (uint64_t)(bs * (b_slot >> 4));
+            // straight-line issue: one warp issues every MMA of the pair, and a narrow MMA (N = 96: 48 clocks) is over before a
+            // loop with descriptor arithmetic gets to the next one (64 -> 16 channels, 27 taps: 6.8 us a tile as loops, 4.4 us)
+            auto issue = [&](int j, int k) {
+              const uint64_t db = db_s + (uint32_t)(j * (b_half >> 4) + k * 2);
 #pragma unroll
-            for (int j = 0; j < RUN; ++j)
+              for (int u = 0; u < STACK; ++u)
+                umma_ss_pair_w(d_tmem + u * 128, da_s + (uint32_t)((((BY_HEIGHT ? i * kLine + j : j * kLine + i) + u * TX) * BK * 2 + k * 32) >> 4), db, idesc,
+                               (i | j | k) ? 1u : first, leader);
+            };
+            if (ksteps >= 4) {
 #pragma unroll
-              for (int k = 0; k < 4; ++k) issue(j, k);
-          } else if (ksteps == 2) {
+              for (int j = 0; j < RUN; ++j)
 #pragma unroll
-            for (int j = 0; j < RUN; ++j)
+                for (int k = 0; k < 4; ++k) issue(j, k);
+            } else if (ksteps == 2) {
 #pragma unroll
-              for (int k = 0; k < 2; ++k) issue(j, k);
-          } else {
-            for (int j = 0; j < RUN; ++j)
-              for (int k = 0; k < ksteps; ++k) issue(j, k);
+              for (int j = 0; j < RUN; ++j)
+#pragma unroll
+                for (int k = 0; k < 2; ++k) issue(j, k);
+            } else {
+              for (int j = 0; j < RUN; ++j)
+                for (int k = 0; k < ksteps; ++k) issue(j, k);
+            }
+            umma_commit_pair_w(&b_empty[bs], leader);  // slot reusable in both CTAs once these MMAs have read it
+            if (++bs == p.b_slots) { bs = 0; bph ^= 1; }
           }
           first = 1u;
-          umma_commit_pair_w(&empty[s], leader);  // slot reusable in both CTAs once these MMAs have read it
-          if (++s == p.stages) { s = 0; ph ^= 1; }
+          umma_commit_pair_w(&a_empty[as], leader);
+          if (++as == p.a_slots) { as = 0; aph ^= 1; }
         }
       }
       if (!ok) break;
@@ -270,21 +296,21 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     uint32_t acc_ph = 0;
     bool ok = true;
     int sums = 0;                        // exchanges of sums of squares so far: buffer sums & 1, phase sums >> 1
-    const bool vec_ok = ((p.out_C | p.oc_add | p.Cout) & 7) == 0;
+    const bool vec_ok = p.vec != 0;
     const float* bias = p.bias != nullptr && p.Cout <= kBiasMax ? bias_s : p.bias;
     const uint32_t acc_empty_leader[2] = {mapa_shared(smem_u32(&acc_empty[0]), 0), mapa_shared(smem_u32(&acc_empty[1]), 0)};
     for (int t = first_tile; t < n_tiles && ok; t += tile_step) {
-      int nt, w0, h0, tf;
+      int nt, x0, y0, tf;
       bool mine;
-      decode(t, nt, w0, h0, tf, mine);
+      decode(t, nt, x0, y0, tf, mine);
       bool arrived = false;              // whether the accumulators of this tile have been waited for
 #pragma unroll 1
-      for (int u = 0; u < STACK; ++u, h0 += TH) {
-        // element offset of a voxel of the tile (row r = 16 h + w), or -1 outside the frame
+      for (int u = 0; u < STACK; ++u, x0 += TX) {
+        // element offset of a voxel of the tile (row r = 8 y + x), or -1 outside the frame
         auto offset = [&](int r) -> long {
-          const int h = h0 + (r >> 4), w = w0 + (r & 15);
-          if (!mine || h >= p.H_out || w >= p.W_out) return -1;
-          return (((long)(tf * p.ot_mul + p.ot_add) * p.out_H + (h * p.oh_mul + p.oh_add)) * p.out_W + (w * p.ow_mul + p.ow_add)) * p.out_C + p.oc_add;
+          const int x = x0 + (r & 7), y = y0 + (r >> 3);
+          if (!mine || x >= p.X_out || y >= p.Y_out) return -1;
+          return p.out_at + tf * p.out_t + x * p.out_x + y * p.out_y;
         };
         const uint32_t t_row = tmem_base + acc * 256 + u * 128 + ((uint32_t)(quarter * 32) << 16);
         if (vec_ok) {
@@ -530,12 +556,12 @@ __global__ void __launch_bounds__(256) rmsnorm_silu_cl_kernel(const bf16* __rest
 
 using namespace cb200;
 
-// As in the GEMM: the persistent grid is bounded by the pairs that the GPU can hold at once. One CTA per SM whatever the ring depth
-// (every ring is over half of the shared memory), so the figure for the largest shared-memory size holds for all.
-template <int RUN, int STACK>
+// As in the GEMM: the persistent grid is bounded by the pairs that the GPU can hold at once. One CTA per SM whatever the ring depths
+// (the rings are over half of the shared memory), so the figure for the largest shared-memory size holds for all.
+template <int RUN, int STACK, bool BY_HEIGHT>
 static int launch_conv(cudaLaunchConfig_t& cfg, long tiles, int sms, const CUtensorMap& tx, const CUtensorMap& tc,
                        const CUtensorMap& tw, const ConvParams& p, int* err) {
-  const auto kern = conv_cl_kernel<RUN, STACK>;
+  const auto kern = conv_cl_kernel<RUN, STACK, BY_HEIGHT>;
   static int max_pairs = 0;
   if (max_pairs == 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cv::kSmemMax);
@@ -564,8 +590,6 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
     return -51;
   ConvParams p{};
   p.T_out = T_out;
-  p.H_out = H_out;
-  p.W_out = W_out;
   p.Cin = Cin;
   p.Cout = Cout;
   p.n_tile = n_tile;
@@ -574,7 +598,7 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
   p.pad = pad;
   p.cache_frames = cache != nullptr ? cache_frames : 0;
   p.t_stride = t_stride;
-  p.hw_stride = hw_stride;
+  p.xy_stride = hw_stride;
   int max_dt = -128;
   for (int i = 0; i < ntaps; ++i) {
     const int dt = taps[3 * i], dh = taps[3 * i + 1], dw = taps[3 * i + 2];
@@ -582,64 +606,90 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
     max_dt = std::max(max_dt, dt);
   }
   if (pad > 0 && max_dt < pad) return -52;      // the newest tap has to read X itself: otherwise a frame could be all padding
-  // Columns of taps: for `run` = 3, 2 the whole list has to fall into (dt, dw) columns of exactly `run` adjacent rows, else 1.
+  // Panels of taps: for run = 3, 2 the whole list has to fall into squares of run x run taps of one frame offset, else each tap is its own
   // (with a spatial stride neighbouring taps do not share rows of a strided box)
   int order[kMaxTaps], run = 1;
   for (int i = 0; i < ntaps; ++i) order[i] = i;
   std::stable_sort(order, order + ntaps, [&](int a, int b) { return taps[3 * a] < taps[3 * b]; });
+  int panel_dh[kMaxTaps], panel_dw[kMaxTaps], square[kMaxTaps][kMaxRun][kMaxRun];       // [panel][dh][dw] -> tap
   for (run = hw_stride == 1 ? kMaxRun : 1; run >= 1; --run) {
     bool used[kMaxTaps] = {};
-    int ng = 0;
-    bool fits = ntaps % run == 0;
+    int np = 0;
+    bool fits = ntaps % (run * run) == 0;
     for (int q = 0; q < ntaps && fits; ++q) {
       const int i = order[q];
       if (used[i]) continue;
-      const int dt = taps[3 * i], dw = taps[3 * i + 2];
-      int dh0 = taps[3 * i + 1];
+      // the corner of the panel: the first row among the frame offset's unused taps, and the first column of that row
+      int dh0 = taps[3 * i + 1], dw0 = taps[3 * i + 2];
       if (run > 1)
         for (int k = 0; k < ntaps; ++k)
-          if (!used[k] && taps[3 * k] == dt && taps[3 * k + 2] == dw) dh0 = std::min(dh0, taps[3 * k + 1]);
-      for (int j = 0; j < run && fits; ++j) {
+          if (!used[k] && taps[3 * k] == taps[3 * i] && (taps[3 * k + 1] < dh0 || (taps[3 * k + 1] == dh0 && taps[3 * k + 2] < dw0))) {
+            dh0 = taps[3 * k + 1];
+            dw0 = taps[3 * k + 2];
+          }
+      for (int j = 0; j < run * run && fits; ++j) {
         int found = run > 1 ? -1 : i;
         for (int k = 0; k < ntaps && found < 0; ++k)
-          if (!used[k] && taps[3 * k] == dt && taps[3 * k + 2] == dw && taps[3 * k + 1] == dh0 + j) found = k;
+          if (!used[k] && taps[3 * k] == taps[3 * i] && taps[3 * k + 1] == dh0 + j / run && taps[3 * k + 2] == dw0 + j % run) found = k;
         fits = found >= 0;
         if (fits) {
           used[found] = true;
-          p.tap[ng][j] = (int8_t)found;
+          square[np][j / run][j % run] = found;
         }
       }
-      p.dt[ng] = (int8_t)dt;
-      p.dh[ng] = (int8_t)dh0;
-      p.dw[ng] = (int8_t)dw;
-      ++ng;
+      p.dt[np] = (int8_t)taps[3 * i];
+      panel_dh[np] = dh0;
+      panel_dw[np] = dw0;
+      ++np;
     }
     if (fits) {
-      p.ngroups = ng;
+      p.npanels = np;
       break;
     }
   }
-  // two stacked tiles per CTA for narrow layers, unless the frame's last rows would leave more than a fifth of them empty
-  const int rows8 = (H_out + TH - 1) / TH, rows16 = (H_out + 2 * TH - 1) / (2 * TH);
-  const int stack = run == 3 && n_tile <= 128 && rows16 * 10 <= rows8 * 6 ? 2 : 1;
-  const int box_rows = TH * stack + run - 1;
-  const int stage_bytes = box_rows * TW * BK * 2 + run * n_tile * BK;
+  // Voxels of a line along the width, or along the height where that leaves fewer tiles; two tiles side by side for narrow layers, unless
+  // 16 x 16 voxels leave more than a fifth over.
+  auto up = [](int a, int b) -> long { return (a + b - 1) / b; };
+  const long along_w = up(W_out, TX) * up(H_out, TY), along_h = up(H_out, TX) * up(W_out, TY), pairs = 2 * up(W_out, 2 * TX) * up(H_out, TY);
+  const int stack = run == 3 && n_tile <= 128 && pairs * 10 <= std::min(along_w, along_h) * 12 ? 2 : 1;
+  const bool by_height = stack == 1 && along_h < along_w;
+  p.X_out = by_height ? H_out : W_out;
+  p.Y_out = by_height ? W_out : H_out;
+  for (int g = 0; g < p.npanels; ++g) {
+    p.dx[g] = (int8_t)(by_height ? panel_dh[g] : panel_dw[g]);
+    p.dy[g] = (int8_t)(by_height ? panel_dw[g] : panel_dh[g]);
+    for (int i = 0; i < run; ++i)
+      for (int j = 0; j < run; ++j) p.tap[g][i][j] = (int8_t)square[g][j][i];
+  }
+  const int box_x = TX * stack + run - 1, box_y = TY + run - 1;
+  const int a_slot = (box_x * box_y * BK * 2 + 1023) / 1024 * 1024, b_slot = run * n_tile * BK;
   const int fixed = kSmemFixed + (Cout <= kBiasMax ? (Cout * 4 + 15) / 16 * 16 : 0) + (y_norm != nullptr ? kSumSq + 256 * 4 : 0);
-  p.stages = std::min(kMaxStages, (kSmemMax - fixed) / stage_bytes);
-  p.ot_mul = out_map[0];
-  p.ot_add = out_map[1];
-  p.oh_mul = out_map[2];
-  p.oh_add = out_map[3];
-  p.ow_mul = out_map[4];
-  p.ow_add = out_map[5];
-  p.out_H = out_map[6];
-  p.out_W = out_map[7];
-  p.out_C = out_map[8];
-  p.oc_add = out_map[9];
+  // ring depths: as many columns of taps ahead as both rings hold
+  int ahead = 0;
+  for (int a = 1; a <= kMaxSlots; ++a) {
+    const int b = std::min(kMaxSlots, (kSmemMax - fixed - a * a_slot) / b_slot);
+    const int cols = std::min(a * run, b);
+    if (b >= 1 && (cols > ahead || (cols == ahead && a == 2))) {       // a second box even where it does not reach further
+      ahead = cols;
+      p.a_slots = a;
+      p.b_slots = b;
+    }
+  }
+  if (ahead == 0) return -57;
+  {
+    const long ot_mul = out_map[0], ot_add = out_map[1], oh_mul = out_map[2], oh_add = out_map[3], ow_mul = out_map[4], ow_add = out_map[5],
+               out_H = out_map[6], out_W = out_map[7], out_C = out_map[8], oc_add = out_map[9];
+    p.out_t = ot_mul * out_H * out_W * out_C;
+    const long per_h = oh_mul * out_W * out_C, per_w = ow_mul * out_C;
+    p.out_x = by_height ? per_h : per_w;
+    p.out_y = by_height ? per_w : per_h;
+    p.out_at = ((ot_add * out_H + oh_add) * out_W + ow_add) * out_C + oc_add;
+    p.vec = ((out_C | oc_add | Cout) & 7) == 0;
+  }
   p.Y = (bf16*)y;
   p.resid = (const bf16*)resid;
   p.bias = bias;
-  if (y_norm != nullptr && (p.tiles_n != 1 || gamma == nullptr || ((p.out_C | p.oc_add | Cout) & 7) != 0)) return -55;
+  if (y_norm != nullptr && (p.tiles_n != 1 || gamma == nullptr || !p.vec)) return -55;
   if (y_norm == nullptr && !write_raw) return -55;
   p.Yn = (bf16*)y_norm;
   p.gamma = gamma;
@@ -647,16 +697,18 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
   p.silu = silu;
   p.write_raw = write_raw;
   CUtensorMap tx, tc, tw;
-  const uint64_t strides[3] = {(uint64_t)Cin * 2, (uint64_t)W_in * Cin * 2, (uint64_t)H_in * W_in * Cin * 2};
-  const uint32_t hw = (uint32_t)hw_stride, box[4] = {BK, TW * hw, (uint32_t)box_rows * hw, 1}, step[4] = {1, hw, hw, 1};
+  const uint64_t per_w = (uint64_t)Cin * 2, per_h = (uint64_t)W_in * Cin * 2;
+  const uint64_t strides[3] = {by_height ? per_h : per_w, by_height ? per_w : per_h, (uint64_t)H_in * W_in * Cin * 2};
+  const uint64_t in_x = (uint64_t)(by_height ? H_in : W_in), in_y = (uint64_t)(by_height ? W_in : H_in);
+  const uint32_t hw = (uint32_t)hw_stride, box[4] = {BK, (uint32_t)box_x * hw, (uint32_t)box_y * hw, 1}, step[4] = {1, hw, hw, 1};
   {
-    const uint64_t dims[4] = {(uint64_t)Cin, (uint64_t)W_in, (uint64_t)H_in, (uint64_t)T_in};
+    const uint64_t dims[4] = {(uint64_t)Cin, in_x, in_y, (uint64_t)T_in};
     const int rc = make_tmap_bf16(&tx, x, 4, dims, strides, box, 1, step);
     if (rc) return rc;
   }
   tc = tx;
   if (p.cache_frames > 0) {
-    const uint64_t dims[4] = {(uint64_t)Cin, (uint64_t)W_in, (uint64_t)H_in, (uint64_t)p.cache_frames};
+    const uint64_t dims[4] = {(uint64_t)Cin, in_x, in_y, (uint64_t)p.cache_frames};
     const int rc = make_tmap_bf16(&tc, cache, 4, dims, strides, box, 1, step);
     if (rc) return rc;
   }
@@ -665,13 +717,13 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
     const int rc = make_tmap_2d_bf16(&tw, w, kdim, (uint64_t)n_rows, kdim * 2, BK, (uint32_t)(n_tile / 2));
     if (rc) return rc;
   }
-  const long vox = (long)T_out * (stack == 2 ? rows16 : rows8) * ((W_out + TW - 1) / TW);
+  const long vox = (long)T_out * up(p.X_out, TX * stack) * up(p.Y_out, TY);
   const long tiles = (vox + 1) / 2 * p.tiles_n;
   if (tiles <= 0 || 2 * tiles > 0x7fffffffL) return -53;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * (sms / 2));
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = (size_t)p.stages * stage_bytes + fixed;
+  cfg.dynamicSmemBytes = (size_t)p.a_slots * a_slot + (size_t)p.b_slots * b_slot + fixed;
   cfg.stream = st;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -682,10 +734,11 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.numAttrs = 2;
-  return stack == 2 ? launch_conv<3, 2>(cfg, tiles, sms, tx, tc, tw, p, err)
-       : run == 3   ? launch_conv<3, 1>(cfg, tiles, sms, tx, tc, tw, p, err)
-       : run == 2   ? launch_conv<2, 1>(cfg, tiles, sms, tx, tc, tw, p, err)
-                    : launch_conv<1, 1>(cfg, tiles, sms, tx, tc, tw, p, err);
+  // (with one tap per panel both orders of the axes run the same code)
+  if (stack == 2) return launch_conv<3, 2, false>(cfg, tiles, sms, tx, tc, tw, p, err);
+  if (run == 1) return launch_conv<1, 1, false>(cfg, tiles, sms, tx, tc, tw, p, err);
+  if (run == 2) return by_height ? launch_conv<2, 1, true>(cfg, tiles, sms, tx, tc, tw, p, err) : launch_conv<2, 1, false>(cfg, tiles, sms, tx, tc, tw, p, err);
+  return by_height ? launch_conv<3, 1, true>(cfg, tiles, sms, tx, tc, tw, p, err) : launch_conv<3, 1, false>(cfg, tiles, sms, tx, tc, tw, p, err);
 }
 
 extern "C" int cb200_rmsnorm_silu_cl(const void* x, const float* gamma, void* y, long n_vox, int C, int silu, cudaStream_t st) {

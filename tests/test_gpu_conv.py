@@ -50,6 +50,34 @@ def test_causal_conv3d_matches_torch(T, H, W, Cin, Cout):
     _close(got, ref, 2e-2 * (27 * Cin) ** 0.5 / 8, 2e-2, "conv3d")
 
 
+# voxel lines along the width or the height (whichever leaves fewer tiles), frames around the 8 x 16 and 16 x 16 tiles, one and two tiles per
+# CTA, channel blocks of 16, 64 and 64 + 32; squares of taps in any order, and lists that are no squares (a box for each tap)
+_LISTS = {"3x3": [(0, i, j) for i in (-1, 0, 1) for j in (-1, 0, 1)], "2x2": [(0, i, j) for j in (0, 1) for i in (-1, 0)],
+          "3x3x2": [(t, i, j) for j in (-1, 0, 1) for t in (1, 0) for i in (-1, 0, 1)], "rows": [(0, i, 0) for i in (-1, 0, 1)],
+          "columns": [(0, 0, j) for j in (1, 0, -1)], "3x2": [(0, i, j) for i in (-1, 0, 1) for j in (0, 1)], "one": [(0, 1, -2)]}
+
+
+@pytest.mark.parametrize("H,W", [(8, 16), (16, 8), (7, 33), (40, 9), (17, 17), (33, 31)])
+@pytest.mark.parametrize("taps", sorted(_LISTS))
+@pytest.mark.parametrize("Cin,Cout", [(16, 24), (96, 96), (64, 192), (96, 256)])
+def test_taps_read_one_box(H, W, taps, Cin, Cout):
+    from cosmos_predict25_b200.models import vae_wan_cl
+    torch.manual_seed(15)
+    lst = _LISTS[taps]
+    w = (torch.randn(Cout, len(lst), Cin, device=DEV) / (len(lst) * Cin) ** 0.5).bfloat16()
+    cl = vae_wan_cl.ConvCL(w, torch.randn(Cout, device=DEV), lst, DEV)
+    x = torch.randn(3, H, W, Cin, device=DEV).bfloat16()
+    got = cl(x, 2)
+    _no_kernel_error()
+    pad = F.pad(x.double(), (0, 0, 2, 2, 1, 1, 0, 0))
+    want = cl.bias.double().expand(2, H, W, Cout).clone()
+    for n, (dt, dh, dw) in enumerate(lst):
+        want += pad[dt:dt + 2, 1 + dh:1 + dh + H, 2 + dw:2 + dw + W] @ w[:, n].double().t()
+    # one rounding to bf16; the fp32 sums of at most 1,728 products stay far below it
+    assert ((got.double() - want).norm() / want.norm()).item() < 1.5 * 2.0 ** -9
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
+
+
 def test_upsample_phase_convolutions_match_nearest_then_conv():
     from cosmos_predict25_b200.models import vae_wan, vae_wan_cl
     torch.manual_seed(1)
