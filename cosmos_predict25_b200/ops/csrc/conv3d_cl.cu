@@ -480,7 +480,7 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       if (!ok) break;
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(acc_empty_leader[acc]);
+      if (lane == 0) mbar_arrive_cluster_tmem(acc_empty_leader[acc]);
       if (++acc == 2) { acc = 0; acc_ph ^= 1; }
     }
     if (!ok && lane == 0) { atomicCAS(err, 0, 63); *abort_flag = 1; }

@@ -633,7 +633,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
-          if (CTA2) mbar_arrive_cluster(acc_empty_leader[acc]);
+          if (CTA2) mbar_arrive_cluster_tmem(acc_empty_leader[acc]);
           else mbar_arrive(&acc_empty[acc]);
         }
         if (++acc == 2) { acc = 0; acc_ph ^= 1; }
@@ -778,7 +778,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
-          if (CTA2) mbar_arrive_cluster(acc_empty_leader[acc]);
+          if (CTA2) mbar_arrive_cluster_tmem(acc_empty_leader[acc]);
           else mbar_arrive(&acc_empty[acc]);
         }
         if (++acc == 2) { acc = 0; acc_ph ^= 1; }
@@ -856,7 +856,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-          if (CTA2) mbar_arrive_cluster(acc_empty_leader[acc]);
+          if (CTA2) mbar_arrive_cluster_tmem(acc_empty_leader[acc]);
           else mbar_arrive(&acc_empty[acc]);
         }
       if (++acc == 2) { acc = 0; acc_ph ^= 1; }

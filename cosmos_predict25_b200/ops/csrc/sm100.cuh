@@ -349,8 +349,12 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t local_smem_addr, uint32
 __device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, float a, float b, float c, float d) {
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+// Arrive on an mbarrier of the pair (shared::cluster address) when all that the arrival announces is that this warp is done with tensor
+// memory (its loads or stores waited for, and tcgen05.fence::before_thread_sync): no write to shared or global memory has to be visible to
+// the other CTA. A release at cluster scope would put a memory barrier in front that waits for the warp's global stores: the convolution's
+// epilogue 3 % of the decoding of a 640 x 640 image (2.25 and 2.18 ms), the attention of CTA pairs 40 % (10.3 and 7.2 ms).
+__device__ __forceinline__ void mbar_arrive_cluster_tmem(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // 2-D tile load into this CTA's shared memory whose completion bytes go to an mbarrier given as a shared::cluster address
 // (the pair leader's barrier)
@@ -387,6 +391,19 @@ __device__ __forceinline__ void umma_ss_pair_w(uint32_t tmem_d, uint64_t desc_a,
       "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
       "}\n"
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(leader)
+      : "memory");
+}
+// the same with A in tensor memory: each CTA's 128 rows lie in its own
+__device__ __forceinline__ void umma_ts_pair_w(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate,
+                                               uint32_t leader) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "}\n"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
 // arrive on the mbarrier at this shared-memory offset in BOTH CTAs of the pair when the MMAs issued so far have completed;
