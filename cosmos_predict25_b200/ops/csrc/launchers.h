@@ -86,6 +86,7 @@ long cb200_fa_bwd_na_scratch_floats(int B, int S, int H);
 int cb200_fa_bwd_na(const void* d_o, const void* q, const void* k, const void* v, const void* o, const float* lse, void* dq, void* dk,
                     void* dv, float* scratch, int B, int S, int H, float scale, const int* q_list, const int* q_cnt, int max_n,
                     const uint8_t* bt, const uint8_t* bh, const uint8_t* bw, int nT, int nH, int nW, int* err, cudaStream_t st);
+int cb200_fa_fwd_pairs(int Sq, int H, int B, int sms);
 int cb200_fa_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int B, int Sq, int Skv, int H, float scale,
                  int variant, int sms, int* err, cudaStream_t st);
 }

@@ -339,6 +339,26 @@ def test_flash_attention_fwd_short_keys(Sq, Skv):
     _close(o, orf, 2e-2, 2e-2, "o")
 
 
+# CTA pairs: an odd number of query blocks (the last CTA has no rows, or one tile of them), key sequences of a tile, of half a tile more, of
+# more tiles than the ring's slots; growing scores move the reference maxima of the two CTAs at different tiles
+@pytest.mark.parametrize("B,Sq,Skv,H", [(1, 512, 128, 2), (2, 257, 192, 3), (1, 1281, 1300, 3), (1, 130, 65, 1), (1, 640, 2900, 2), (2, 2048, 1, 1)])
+@pytest.mark.parametrize("grow", [False, True])
+def test_flash_attention_fwd_pairs_equal_single_ctas(B, Sq, Skv, H, grow):
+    torch.manual_seed(13)
+    q, k, v = (torch.randn(B, S, H, 128, device=DEV) for S in (Sq, Skv, Skv))
+    if grow:
+        k = k * torch.linspace(0.2, 6.0, Skv, device=DEV).view(1, -1, 1, 1)
+        q = q * torch.linspace(0.5, 2.0, Sq, device=DEV).view(1, -1, 1, 1)
+    q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    scale = 1.0 / math.sqrt(128)
+    o, lse = _ops().fa_fwd_variant(q, k, v, scale, 12)
+    single, lse_single = _ops().fa_fwd_variant(q, k, v, scale, 4)
+    _no_kernel_error()
+    assert torch.equal(o, single) and torch.equal(lse, lse_single)
+    orf, _ = ref.attention(q.double(), k.double(), v.double(), scale)
+    assert ((o.double() - orf).norm() / orf.norm()).item() < 2.0 ** -7
+
+
 def test_forward_kernels_are_bitwise_repeatable():
     """The forward has no atomics: two runs on the same inputs must agree bit for bit (default shape choice for long and for
     short key sequences)."""
