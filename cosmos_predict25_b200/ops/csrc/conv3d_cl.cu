@@ -144,7 +144,7 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();                         // the other CTA's barriers exist before anything signals them
+  cluster_sync_relaxed();                     // the other CTA's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();                              // launched with programmatic serialisation (see common.cuh)
@@ -493,7 +493,7 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();                  // neither CTA leaves (or frees TMEM) while the other may still signal it or read its tiles
+  cluster_sync_relaxed();              // neither CTA leaves (or frees TMEM) while the other may still signal it or read its tiles
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, 512);

@@ -212,7 +212,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   }
   tc_fence_before();
   __syncthreads();
-  if (PAIR) cluster_sync_all();      // the other CTA's barriers exist before anything signals them
+  if (PAIR) cluster_sync_relaxed();  // the other CTA's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();                     // launched with programmatic serialisation (see common.cuh)
@@ -556,7 +556,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   }
   tc_fence_before();
   __syncthreads();
-  if (PAIR) cluster_sync_all();      // neither CTA leaves (or frees TMEM) while the other may still signal it or read its tiles
+  if (PAIR) cluster_sync_relaxed();  // neither CTA leaves (or frees TMEM) while the other may still signal it or read its tiles
   if (warp == kMmaWarp) {
     tc_fence_after();
     if (PAIR) tmem_dealloc_pair(tmem_base, Sh::kTmemCols);

@@ -218,7 +218,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   }
   tc_fence_before();
   __syncthreads();
-  if (CTA2) cluster_sync_all();      // the other CTA's barriers exist before anything signals them
+  if (CTA2) cluster_sync_relaxed();  // the other CTA's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   if (CTA2) {                        // launched with programmatic serialisation (see common.cuh)
@@ -323,7 +323,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     }
     if (SPLIT > 1) {                 // the two exchange barriers of the epilogue warps below take every warp of the cluster
       __syncwarp();
-      cluster_sync_all();
+      cluster_sync_relaxed();
       cluster_sync_all();
     }
   } else if (warp == 1) {
@@ -371,7 +371,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     }
     if (SPLIT > 1) {
       __syncwarp();
-      cluster_sync_all();
+      cluster_sync_relaxed();
       cluster_sync_all();
     }
   } else if (GATHER && warp >= 10) {
@@ -464,7 +464,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         // 16 bytes, so that the lanes of a warp write and read 512 contiguous bytes.
         const int r_tile = quarter * 32 + lane;
         __syncwarp();
-        cluster_sync_all();            // every pair's MMAs are complete: the operand rings are free
+        cluster_sync_relaxed();        // every pair's MMAs are complete: the operand rings are free
         if (ok) {
 #pragma unroll 1
           for (int c = part * 4; c < part * 4 + 4; ++c) {
@@ -872,7 +872,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   }
   tc_fence_before();
   __syncthreads();
-  if (CTA2) cluster_sync_all();      // neither CTA leaves (or frees TMEM) while the other may still signal it or read its tiles
+  if (CTA2) cluster_sync_relaxed();  // neither CTA leaves (or frees TMEM) while the other may still signal it or read its tiles
   if (warp == 1) {
     tc_fence_after();
     if (CTA2) tmem_dealloc_pair(tmem_base, 512);

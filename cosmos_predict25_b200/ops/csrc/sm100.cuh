@@ -339,6 +339,12 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same where no write of one CTA has to be visible to another behind it: barriers set up (fence_barrier_init), operand rings read for the
+// last time, nothing left that would signal a CTA that leaves. Without the release no warp waits for its global stores here: denoising
+// step of a 256 x 256 image (168 products of one tile per cluster) 4.91 and 4.77 ms.
+__device__ __forceinline__ void cluster_sync_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 // shared::cluster address of `local_smem_addr` (a shared::cta address of this CTA) in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t mapa_shared(uint32_t local_smem_addr, uint32_t rank) {
   uint32_t r;
