@@ -268,6 +268,16 @@ def test_rmsnorm_silu_widths(C):
         _close(native.load().rmsnorm_silu_cl(x, g, silu), F.silu(want) if silu else want, 4e-3, 8e-3, f"rmsnorm {C}")
 
 
+@pytest.mark.parametrize("C,n", [(384, 444 * 16 * 2 + 5), (192, 444 * 32 + 1), (96, 444 * 64 * 3 - 1), (32, 444 * 128 + 77), (1024, 444 * 8 * 2 + 3)])
+def test_rmsnorm_silu_of_more_voxels_than_one_pass(C, n):
+    """Lanes go on from voxel to voxel: every voxel's result is the one it has in a call of its own few."""
+    torch.manual_seed(16)
+    x, g = torch.randn(n, C, device=DEV).bfloat16(), 1 + 0.1 * torch.randn(C, device=DEV)
+    got = native.load().rmsnorm_silu_cl(x, g, True)
+    for lo in (0, 444 * 256 // max(C // 8, 1) // 8 * 8, n // 2, max(n - 40, 0)):
+        assert torch.equal(got[lo:lo + 40], native.load().rmsnorm_silu_cl(x[lo:lo + 40].contiguous(), g, True))
+
+
 def test_rmsnorm_silu_channels_last():
     torch.manual_seed(2)
     x = torch.randn(5, 7, 9, 96, device=DEV).bfloat16()
