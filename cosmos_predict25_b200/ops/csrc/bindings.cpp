@@ -360,8 +360,12 @@ Tensor gemm_impl(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& 
     gate_p = gate_c.data_ptr<float>();
   }
   const int dev = a.get_device();
+  const long need = cb200_gemm_stream_floats((int)d.M, (int)d.N, (int)d.K, trans_a ? 1 : 0, trans_b ? 1 : 0, resid != nullptr, cb200_sm_count(dev));
+  Tensor scratch;
+  if (need > 0) scratch = at::empty({need}, a.options().dtype(at::kFloat));
   const int rc = cb200_gemm_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), d.M, d.N, d.K, trans_a ? 1 : 0, trans_b ? 1 : 0, bias_p,
-                                 (int)act, pre_p, resid_p, gate_p, ld_gate, (int)L, error_word(dev), cb200_sm_count(dev), stream());
+                                 (int)act, pre_p, resid_p, gate_p, ld_gate, (int)L, error_word(dev), cb200_sm_count(dev), stream(),
+                                 need > 0 ? scratch.data_ptr<float>() : nullptr);
   TORCH_CHECK(rc == 0, "tcgen05 GEMM launch failed with code ", rc);
   return c;
 }

@@ -880,6 +880,216 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   }
 }
 
+// Few tiles of a very long contraction (the projection of a prompt: 100,352 deep, 4 to 74 tiles). Clusters of pairs per tile leave SMs idle
+// where the tiles times a whole number of pairs do not fill the GPU, and take four pairs at most. Here `per_tile` pairs share a tile's k-blocks
+// in turn, all tiles in step, so that what neighbouring tiles have in common comes from L2; pairs left over share the last `tail` k-blocks of
+// all tiles, tile by tile. Each pair writes its sums as fp32 partial tiles to global memory and gemm_stream_finish_kernel adds them in a fixed
+// order: no CTA waits for another pair's work. (With equal shares of all tiles' k-blocks in a row no two pairs were at the same k-block, and
+// 1024 x 1024 read 1.6 GB instead of 0.4: 215 us.) Both operands K-major, N a multiple of 256.
+// ws: [slot][64 column quadruples][256 rows] float4; slots: pair turn * tiles + tile, then three for each pair of the tail.
+// From K = 100,352 to 1024 columns, before and now: 256 rows 125 and 72 us, 512 127 and 83, 768 133 and 115, 1024 174 and 154, 1536 251 and 206,
+// 3072 490 and 441; 2048 rows (32 tiles, two pairs each) would go from 282 to 332 and stay with clusters; 1024 rows from K = 32,768 80 and 72,
+// from K = 16,384 the same.
+struct StreamPlan {
+  int tiles, tiles_n, k_all;
+  int per_tile, extra, tail;     // pairs a tile, pairs of the tail, k-blocks of a tile that are theirs
+};
+constexpr int kStreamSlots = 3;  // tiles that a pair of the tail can touch: at most two tiles' worth of tails (see stream_plan)
+__host__ __device__ inline int stream_tail_first(const StreamPlan& pl, int e) { return (int)((long)e * pl.tiles * pl.tail / pl.extra); }
+
+__global__ void __launch_bounds__(kGemmThreads, 1)
+gemm_stream_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, float* __restrict__ ws, StreamPlan pl,
+                   int* __restrict__ err) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  constexpr int STG = 6, STG_BYTES = kABytes + kBBytes / 2, TM = 2 * BM;
+  const uint32_t rank = cluster_ctarank();
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STG * STG_BYTES);
+  uint64_t* full = bars;                    // [STG]
+  uint64_t* empty = bars + STG;             // [STG]
+  uint64_t* acc_full = bars + 2 * STG;      // [2]
+  uint64_t* acc_empty = acc_full + 2;       // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int pair = (int)blockIdx.x >> 1, tail_pair = pair - pl.per_tile * pl.tiles;
+  const int g0 = tail_pair >= 0 ? stream_tail_first(pl, tail_pair) : 0, g1 = tail_pair >= 0 ? stream_tail_first(pl, tail_pair + 1) : 0;
+  const int t0 = tail_pair >= 0 ? g0 / pl.tail : pair % pl.tiles, n_seg = tail_pair < 0 ? 1 : g1 > g0 ? (g1 - 1) / pl.tail - t0 + 1 : 0;
+  const int slot0 = tail_pair < 0 ? pair : pl.per_tile * pl.tiles + tail_pair * kStreamSlots;
+  const int head = pl.k_all - pl.tail;             // k-blocks that the pairs of a tile share
+  // k-blocks lo, lo + step, ... below hi of segment s, which lies in tile t0 + s
+  const int step = tail_pair < 0 ? pl.per_tile : 1;
+  auto range = [&](int s, int& lo, int& hi) {
+    if (tail_pair < 0) {
+      lo = pair / pl.tiles;
+      hi = head;
+    } else {
+      lo = head + max(g0 - (t0 + s) * pl.tail, 0);
+      hi = head + min(g1 - (t0 + s) * pl.tail, pl.tail);
+    }
+  };
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STG; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&acc_full[a], 1);
+      mbar_init(&acc_empty[a], 16);         // the even CTA hears from the epilogue warps of both
+    }
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(tmem_slot, 512);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_relaxed();            // the other CTA's barriers exist before anything signals them
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();                     // launched with programmatic serialisation (see common.cuh)
+  pdl_wait();
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      prefetch_tmap(&tma_a);
+      prefetch_tmap(&tma_b);
+      int st = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int s = 0; s < n_seg && ok; ++s) {
+        int lo, hi;
+        range(s, lo, hi);
+        const int m0 = (t0 + s) / pl.tiles_n * TM + (int)rank * BM, n0 = (t0 + s) % pl.tiles_n * BN + (int)rank * (BN / 2);
+        for (int kb = lo; kb < hi; kb += step) {
+          if (!mbar_wait(&empty[st], ph ^ 1, abort_flag)) { ok = false; break; }
+          uint8_t* sa = smem + st * STG_BYTES;
+          if (rank == 0) mbar_arrive_expect_tx(&full[st], 2 * STG_BYTES);
+          const uint32_t bar = mapa_shared(smem_u32(&full[st]), 0);
+          tma_load_2d_pair(sa, &tma_a, bar, kb * BK, m0);
+          tma_load_2d_pair(sa + kABytes, &tma_b, bar, kb * BK, n0);
+          if (++st == STG) { st = 0; ph ^= 1; }
+        }
+      }
+      if (!ok) { atomicCAS(err, 0, 4); *abort_flag = 1; }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer (warp-uniform; the elected lane issues)
+    const uint32_t leader = elect_one() ? 1u : 0u;
+    auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)); };
+    constexpr uint32_t idesc = umma_idesc_bf16(TM, BN, 0, 0);
+    const uint64_t da0 = umma_desc_sw128(smem_u32(smem), 16, 1024), db0 = umma_desc_sw128(smem_u32(smem) + kABytes, 16, 1024);
+    int st = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int s = 0; s < n_seg && ok && rank == 0; ++s) {     // only the even CTA issues
+      int lo, hi;
+      range(s, lo, hi);
+      if (!wait_all(&acc_empty[s & 1], ((s >> 1) & 1) ^ 1)) { ok = false; break; }
+      tc_fence_after();
+      for (int kb = lo; kb < hi; kb += step) {
+        if (!wait_all(&full[st], ph)) { ok = false; break; }
+        tc_fence_after();
+        const uint64_t da = da0 + (uint64_t)(st * (STG_BYTES >> 4)), db = db0 + (uint64_t)(st * (STG_BYTES >> 4));
+#pragma unroll
+        for (int k = 0; k < BK / UK; ++k)
+          umma_ss_pair_w(tmem_base + (s & 1) * BN, da + (uint32_t)((k * UK * 2) >> 4), db + (uint32_t)((k * UK * 2) >> 4), idesc,
+                         (kb > lo || k > 0) ? 1u : 0u, leader);
+        umma_commit_pair_w(&empty[st], leader);
+        if (++st == STG) { st = 0; ph ^= 1; }
+      }
+      if (ok) umma_commit_pair_w(&acc_full[s & 1], leader);
+    }
+    if (!ok && lane == 0) { atomicCAS(err, 0, 5); *abort_flag = 1; }
+  } else {
+    // ------------------------------------------------------------------ epilogue warps: 32 rows x 128 columns of each partial tile
+    const int quarter = warp & 3, part = (warp - 2) >> 2;
+    bool ok = true;
+    for (int s = 0; s < n_seg && ok; ++s) {
+      ok = mbar_wait_warp(&acc_full[s & 1], (s >> 1) & 1, abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      float4* dst = reinterpret_cast<float4*>(ws) + ((size_t)(slot0 + s) * (BN / 4)) * TM + rank * BM + quarter * 32 + lane;
+#pragma unroll 1
+      for (int c = part * 4; c < part * 4 + 4; ++c) {
+        uint32_t r[32];
+        tmem_ld32(tmem_base + (s & 1) * BN + ((uint32_t)(quarter * 32) << 16) + c * 32, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          dst[(size_t)(c * 8 + q) * TM] = make_float4(__uint_as_float(r[q * 4]), __uint_as_float(r[q * 4 + 1]), __uint_as_float(r[q * 4 + 2]),
+                                                      __uint_as_float(r[q * 4 + 3]));
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster_tmem(mapa_shared(smem_u32(&acc_empty[s & 1]), 0));
+    }
+    if (!ok && lane == 0) { atomicCAS(err, 0, 6); *abort_flag = 1; }
+  }
+
+  __syncwarp();
+  if (*abort_flag) {
+    // let outstanding bulk copies / MMAs drain before shared memory and TMEM go away
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_relaxed();            // neither CTA leaves (or frees TMEM) while the other may still signal it or read its tiles
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, 512);
+  }
+}
+
+// C = act(sum of the partial tiles + bias), optionally also the value in front of the activation. A CTA takes 32 rows x 64 columns of a tile, a
+// warp 8 of the columns.
+__global__ void __launch_bounds__(256) gemm_stream_finish_kernel(const float* __restrict__ ws, bf16* __restrict__ C, bf16* __restrict__ pre,
+                                                                 const bf16* __restrict__ bias, int act, int M, int N, StreamPlan pl) {
+  pdl_trigger();                     // launched with programmatic serialisation (see common.cuh)
+  pdl_wait();
+  constexpr int TM = 2 * BM;
+  const int tile = (int)blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r = (int)(blockIdx.x >> 2) * 32 + lane, c8 = (int)(blockIdx.x & 3) * 8 + warp;        // row and 8-column group of the tile
+  const int row = tile / pl.tiles_n * TM + r, col = tile % pl.tiles_n * BN + c8 * 8;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+  auto add = [&](int slot) {
+    const float4* src = reinterpret_cast<const float4*>(ws) + ((size_t)slot * (BN / 4) + c8 * 2) * TM + r;
+    const float4 u = src[0], v = src[TM];
+    a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
+    b.x += v.x; b.y += v.y; b.z += v.z; b.w += v.w;
+  };
+#pragma unroll 4
+  for (int i = 0; i < pl.per_tile; ++i) add(i * pl.tiles + tile);
+  if (pl.tail > 0) {
+    // the pairs of the tail whose range [first, next) meets this tile's [tile * tail, (tile + 1) * tail)
+    for (int e = 0; e < pl.extra; ++e) {
+      const int g0 = stream_tail_first(pl, e), g1 = stream_tail_first(pl, e + 1);
+      if (g0 < (tile + 1) * pl.tail && g1 > tile * pl.tail && g1 > g0)
+        add(pl.per_tile * pl.tiles + e * kStreamSlots + tile - g0 / pl.tail);
+    }
+  }
+  if (row >= M) return;
+  float o[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  if (bias != nullptr) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o[j] += __bfloat162float(bias[col + j]);
+  }
+  if (act == 1) {
+    if (pre != nullptr) *reinterpret_cast<bf16x8*>(pre + (size_t)row * N + col) = pack8(o);
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      const float2 g = gelu2(make_float2(o[j], o[j + 1]));
+      o[j] = g.x;
+      o[j + 1] = g.y;
+    }
+  }
+  *reinterpret_cast<bf16x8*>(C + (size_t)row * N + col) = pack8(o);
+}
+
 }  // namespace cb200
 
 using namespace cb200;
@@ -933,6 +1143,8 @@ struct PairLaunch {
   }
   PairLaunch(const PairLaunch&) = delete;
 };
+
+extern "C" int cb200_gemm_pair_mode(int mode);
 
 // clusters that the GPU holds at once: none where it has no room for one (a share of a GPU)
 template <int A_MN, int B_MN, int SPLIT, int NW = 3>
@@ -1001,6 +1213,74 @@ extern "C" int cb200_gemm_pairs_per_tile(long tiles, long kb, int pairs, int c2,
   return split;
 }
 
+// How gemm_stream_kernel would share out `tiles` tiles of `kb` k-blocks over `pairs` pairs. The tail's pairs take equal parts of its k-blocks, two
+// tiles' worth at most (three tiles touched); where they are too few for that there is no tail.
+static StreamPlan stream_plan(int tiles, int tiles_n, int kb, int pairs) {
+  StreamPlan pl{tiles, tiles_n, kb, pairs / tiles, 0, 0};
+  pl.extra = pairs - pl.per_tile * tiles;
+  pl.tail = 2 * pl.extra >= tiles ? (int)((long)kb * pl.extra / pairs) : 0;
+  if (pl.tail == 0) pl.extra = 0;
+  return pl;
+}
+// Whether that takes less time, in k-blocks of a pair: its share, and kStream for writing the partial tiles (256 KB each) and adding them in a
+// launch of its own (12 us); against the rule above or whole waves of tiles.
+extern "C" int cb200_gemm_stream(long tiles, long kb, int pairs, int c2, int c4, int c3) {
+  constexpr long kStream = 45, kExchange = 6;
+  if (tiles < 1 || tiles > pairs || kb < pairs) return 0;
+  const int split = cb200_gemm_pairs_per_tile(tiles, kb, pairs, c2, c4, c3);
+  const long now = split == 2   ? (tiles + c2 - 1) / c2 * ((kb + 1) / 2 + kExchange)
+                   : split == 3 ? (tiles + c3 - 1) / c3 * ((kb + 2) / 3 + 2 * kExchange)
+                   : split == 4 ? (tiles + c4 - 1) / c4 * ((kb + 3) / 4 + kExchange)
+                                : kb;
+  const StreamPlan pl = stream_plan((int)tiles, 1, (int)kb, pairs);
+  return (kb - pl.tail + pl.per_tile - 1) / pl.per_tile + kStream < now ? 1 : 0;
+}
+
+// pairs that the GPU holds at once for gemm_stream_kernel
+static int stream_pairs(int sms, int* pairs) {
+  static int resident = -1;
+  if (resident < 0) {
+    const cudaError_t e = cudaFuncSetAttribute(gemm_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+    if (e != cudaSuccess) return 100 + (int)e;
+    PairLaunch l(1, 1, nullptr);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_stream_kernel, &l.cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    resident = n;
+  }
+  *pairs = std::min(resident, sms / 2);
+  return 0;
+}
+
+// fp32 values of scratch with which cb200_gemm_bf16 can share out the k-blocks of this product, 0: it would not
+extern "C" long cb200_gemm_stream_floats(int M, int N, int K, int a_mn, int b_mn, int gated, int sms) {
+  if (a_mn || b_mn || gated || M < 2 * BM || N % BN != 0 || K % 8 != 0 || K < 64 * BK || cb200_gemm_pair_mode(-1) != 1) return 0;
+  int pairs = 0, c2 = 0, c3 = 0, c4 = 0;
+  if (stream_pairs(sms, &pairs) || resident_clusters<0, 0, 2>(&c2) || resident_clusters<0, 0, 3>(&c3) || resident_clusters<0, 0, 4>(&c4)) return 0;
+  const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * (N / BN);
+  if (!cb200_gemm_stream(tiles, (K + BK - 1) / BK, pairs, c2, c4, c3)) return 0;
+  const StreamPlan pl = stream_plan((int)tiles, N / BN, (K + BK - 1) / BK, pairs);
+  return (long)(pl.per_tile * pl.tiles + pl.extra * kStreamSlots) * 2 * BM * BN;
+}
+
+static int launch_gemm_stream(const void* A, const void* B, void* C, int M, int N, int K, const GemmEpilogue& ep, float* ws, int* err, int sms,
+                              cudaStream_t st) {
+  CUtensorMap ta, tb;
+  int pairs = 0, rc;
+  if ((rc = stream_pairs(sms, &pairs))) return rc;
+  if ((rc = make_tmap_2d_bf16(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, BM))) return rc;
+  if ((rc = make_tmap_2d_bf16(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, BK, BN / 2))) return rc;
+  const int tiles = (M + 2 * BM - 1) / (2 * BM) * (N / BN);
+  const StreamPlan pl = stream_plan(tiles, N / BN, (K + BK - 1) / BK, pairs);
+  PairLaunch l(1, pl.per_tile * tiles + pl.extra, st);
+  cudaError_t e = cudaLaunchKernelEx(&l.cfg, gemm_stream_kernel, ta, tb, ws, pl, err);
+  if (e != cudaSuccess) return 500 + (int)e;
+  e = launch_pdl(gemm_stream_finish_kernel, dim3(2 * BM / 32 * 4, tiles), dim3(256), 0, st, ws, (bf16*)C, ep.pre, ep.bias, ep.act, M, N, pl);
+  return e == cudaSuccess ? 0 : 500 + (int)e;
+}
+
 template <int A_MN, int B_MN>
 static int launch_gemm_any(const void* A, const void* const* B, void* const* C, int M, int N, int K, const GemmEpilogue& ep, int* err, int sms,
                           cudaStream_t st) {
@@ -1038,7 +1318,7 @@ extern "C" int cb200_gemm_pair_mode(int mode) {
 
 extern "C" int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int b_mn,
                                const void* bias, int act, void* pre, const void* resid, const float* gate, long ld_gate, int L,
-                               int* err, int sms, cudaStream_t st) {
+                               int* err, int sms, cudaStream_t st, float* ws) {
   GemmEpilogue ep{};
   ep.groups = 1;
   ep.pre = (bf16*)pre;
@@ -1048,6 +1328,8 @@ extern "C" int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int
   ep.ld_gate = ld_gate;
   ep.act = act;
   ep.L = L > 0 ? L : 1;
+  if (ws != nullptr && cb200_gemm_stream_floats(M, N, K, a_mn, b_mn, gate != nullptr, sms) > 0)
+    return launch_gemm_stream(A, B, C, M, N, K, ep, ws, err, sms, st);
   if (cb200_gemm_pair_mode(-1) == 1 && M >= 2 * BM && N % 8 == 0) {
     if (a_mn == 0 && b_mn == 0) return launch_gemm_any<0, 0>(A, &B, &C, M, N, K, ep, err, sms, st);
     if (a_mn == 0 && b_mn == 1) return launch_gemm_any<0, 1>(A, &B, &C, M, N, K, ep, err, sms, st);

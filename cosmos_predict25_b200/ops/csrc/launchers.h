@@ -57,8 +57,10 @@ int cb200_skinny_bgemm(const float* a, long a_z, long a_r, long a_k, const long 
 int cb200_skinny_wide(long a_k, long b_n, long b_k, int b_is_bf16, int c_is_bf16, int silu_b, int N, int K);   // 1: 256-column tiles
 
 // gemm_tcgen05.cu
+// ws: cb200_gemm_stream_floats fp32 values of scratch, or nullptr
 int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int b_mn, const void* bias,
-                    int act, void* pre, const void* resid, const float* gate, long ld_gate, int L, int* err, int sms, cudaStream_t st);
+                    int act, void* pre, const void* resid, const float* gate, long ld_gate, int L, int* err, int sms, cudaStream_t st, float* ws = nullptr);
+long cb200_gemm_stream_floats(int M, int N, int K, int a_mn, int b_mn, int gated, int sms);
 int cb200_gemm_many_weights(int n, int M, int N, int K, int sms);   // weights a launch of cb200_gemm_bf16_many takes, or 0
 int cb200_gemm_bf16_many(const void* A, const void* const* B, void* const* C, const void* const* norm, const uint8_t* norm_bf16, int n, int M,
                          int N, int K, float eps, int* err, int sms, cudaStream_t st);

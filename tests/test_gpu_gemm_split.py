@@ -90,3 +90,32 @@ def test_gated_tiles_in_a_row(M, N, K, L):
     got = native.load().gemm_bf16_gate_residual(a, b, resid, gate, L)
     _check()
     assert _rel(got, resid.double() + gate.double().repeat_interleave(L, 0) * (a.double() @ b.double().t())) < ROUND
+
+
+# tiles whose k-blocks are shared out over all pairs: one tile for all of them, several pairs a tile with none left over for the tail, a tail
+# whose pairs reach into two and three tiles, more tiles than half of the pairs; ragged rows, a last k-block of 8
+@pytest.mark.parametrize("M,N,K", [(256, 256, 16384), (300, 512, 16384), (1000, 1024, 32768), (2500, 1024, 32768), (2304, 1024, 16384), (520, 768, 32776)])
+@pytest.mark.parametrize("bias,act", [(False, 0), (True, 0), (True, 1)])
+def test_long_contractions_are_shared_over_all_pairs(M, N, K, bias, act):
+    ops = native.load()
+    torch.manual_seed(5)
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    w = (torch.randn(N, K, device=DEV) / K ** 0.5).bfloat16()
+    store = torch.randn(N + 1, device=DEV).bfloat16()
+    b = store[1:] if bias else None                     # two bytes off a 16-byte boundary
+    y = ops.gemm_bf16(x, w, b, act, False, False)
+    again = ops.gemm_bf16(x, w, b, act, False, False)
+    torch.cuda.synchronize()
+    assert ops.kernel_error(torch.cuda.current_device(), True) == 0
+    assert torch.equal(y, again)
+    want = x.double() @ w.double().t()
+    if bias:
+        want = want + b.double()
+    pre = want
+    if act:
+        want = torch.nn.functional.gelu(want)
+    # one rounding to bf16; fp32 sums of 32,776 products of unit variance over sqrt(K) stay at 1e-6 of it
+    assert ((y.double() - want).norm() / want.norm()).item() < 1.5 * 2.0 ** -9
+    if act:
+        y2, got_pre = ops.gemm_bf16_gelu_pre(x, w, b)
+        assert torch.equal(y2, y) and ((got_pre.double() - pre).norm() / pre.norm()).item() < 1.5 * 2.0 ** -9
