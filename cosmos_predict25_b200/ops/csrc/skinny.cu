@@ -14,6 +14,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "common.cuh"
@@ -298,9 +299,119 @@ static int launch_skinny_wide(const SkinnyParams& p, int Z, cudaStream_t st) {
   return (int)launch_pdl(skinny_wide_kernel<RT, KFAST>, grid, dim3(kFsThreads), Sh::kSmem, st, p);
 }
 
+// ------------------------------------------------------------------------------------------------------------------------------
+// The same for up to four rows and K <= 2048 (the modulation MLPs of an image with its negative prompt): the weights, read once, are all that
+// counts. A lane keeps its eight elements of the rows in registers for good and takes one 16-byte piece of eight weight rows at a time, the
+// next eight in flight; WK warps of 256 elements each make up a weight row, their sums of 32 lanes meet in shared memory. No stages of
+// weights in shared memory and no split of the reduction over CTAs (whose sums took a launch more).
+// @ROWS_FIGURES@
+constexpr int kRowsN = 8;                // weight rows of a warp at a time
+template <int RT>
+__global__ void __launch_bounds__(256) skinny_rows_kernel(SkinnyParams p, int wk, int per_cta) {
+  __shared__ float part[2][8][kRowsN * RT];      // two sets in turn: [warp][weight row, row]
+  pdl_trigger();                       // launched with programmatic serialisation (see common.cuh)
+  pdl_wait();
+  constexpr int V = kRowsN * RT;       // sums of a warp: 8, 16 or 32
+  const int z = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kpart = warp % wk, npart = warp / wk, wn = 8 / wk, k = kpart * 256 + lane * 8;
+  const float* A = p.a + (long)z * p.a_z;
+  const __nv_bfloat16* B = p.b_ptrs ? reinterpret_cast<const __nv_bfloat16*>(p.b_ptrs[z])
+                                    : reinterpret_cast<const __nv_bfloat16*>(p.b_base) + (long)z * p.b_z;
+  // a weight that does not start on a 16-byte boundary (a slice of a larger buffer) is read element by element
+  const bool vec = (reinterpret_cast<uintptr_t>(B) & 15) == 0;
+  const int n_lo = (int)blockIdx.x * per_cta, n_hi = min(p.N, n_lo + per_cta);
+  float a[RT][8];
+#pragma unroll
+  for (int r = 0; r < RT; ++r)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float v = r < p.R && k + j < p.K ? A[(long)r * p.a_r + k + j] : 0.f;
+      a[r][j] = p.silu_a ? silu_f(v) : v;
+    }
+  bf16x8 next[kRowsN];
+  auto fetch = [&](int n0) {
+#pragma unroll
+    for (int i = 0; i < kRowsN; ++i) {
+      const int n = n0 + i;
+      next[i] = bf16x8{};
+      if (n < n_hi && k < p.K) {                       // K is a multiple of 8
+        const __nv_bfloat16* src = B + (long)n * p.b_n + k;
+        if (vec) {
+          next[i] = *reinterpret_cast<const bf16x8*>(src);
+        } else {
+          __nv_bfloat16 e[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) e[j] = src[j];
+          next[i] = *reinterpret_cast<const bf16x8*>(e);
+        }
+      }
+    }
+  };
+  float* C = reinterpret_cast<float*>(p.c) + (long)z * p.c_z;
+  const int stride = wn * kRowsN;
+  fetch(n_lo + npart * kRowsN);
+  int set = 0;
+  for (int n0 = n_lo; n0 < n_hi; n0 += stride, set ^= 1) {
+    float sum[V];
+#pragma unroll
+    for (int i = 0; i < kRowsN; ++i) {
+      float w[8];
+      unpack8(next[i], w);
+#pragma unroll
+      for (int r = 0; r < RT; ++r) {
+        float s = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s = fmaf(w[j], a[r][j], s);
+        sum[i * RT + r] = s;
+      }
+    }
+    fetch(n0 + stride + npart * kRowsN);
+    // halves of the values change hands until every lane holds one: value v lies in the lanes whose top bits spell it
+#pragma unroll
+    for (int half = V / 2, d = 16; half >= 1; half /= 2, d /= 2) {
+      const bool up = (lane & d) != 0;
+#pragma unroll
+      for (int i = 0; i < half; ++i) {
+        const float mine = up ? sum[i + half] : sum[i], other = up ? sum[i] : sum[i + half];
+        sum[i] = mine + __shfl_xor_sync(0xffffffffu, other, d);
+      }
+    }
+#pragma unroll
+    for (int d = 16 / V; d >= 1; d /= 2) sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], d);
+    if (lane % (32 / V) == 0) part[set][warp][lane / (32 / V)] = sum[0];
+    __syncthreads();
+    // one thread per value of the CTA's `stride` weight rows; the parts of a row in the order of its elements
+    for (int v = threadIdx.x; v < wn * V; v += 256) {
+      const int np = v / V, i = v % V, n = n0 + np * kRowsN + i / RT, r = i % RT;
+      if (n < n_hi && r < p.R) {
+        float t = 0.f;
+        for (int q = 0; q < wk; ++q) t += part[set][np * wk + q][i];
+        if (p.add != nullptr && n < p.add_cols) t += p.add[(long)r * p.ld_add + n];
+        C[(long)r * p.ldc + n] = t;
+      }
+    }
+  }
+}
+
+template <int RT>
+static int launch_skinny_rows(const SkinnyParams& p, int Z, cudaStream_t st) {
+  int wk = 1;
+  while (wk * 256 < p.K) wk *= 2;
+  // weight rows of a CTA: about four CTAs on every SM over all problems, whole steps of the CTA
+  const int step = 8 / wk * kRowsN;
+  const long want = ((long)p.N * Z + 148 * 4 - 1) / (148 * 4);
+  const int per_cta = (int)std::min<long>((p.N + step - 1) / step, std::max<long>(1, (want + step - 1) / step)) * step;
+  return (int)launch_pdl(skinny_rows_kernel<RT>, dim3((p.N + per_cta - 1) / per_cta, Z), dim3(256), 0, st, p, wk, per_cta);
+}
+
 }  // namespace cb200
 
 using namespace cb200;
+
+// whether a call goes to the kernel for a few rows, which does not split reductions
+extern "C" int cb200_skinny_rows(long a_k, long b_n, long b_k, int b_is_bf16, int c_is_bf16, int silu_b, int R, int N, int K) {
+  return b_is_bf16 && !c_is_bf16 && !silu_b && a_k == 1 && b_k == 1 && b_n % 8 == 0 && K % 8 == 0 && K <= 2048 && R <= 4 && N >= 1 ? 1 : 0;
+}
 
 // whether a call goes to the wide kernel (the split of long reductions counts its tiles): bf16 weights with one contiguous index and
 // 8-element rows, row-major A, fp32 result
@@ -315,6 +426,8 @@ extern "C" int cb200_skinny_bgemm(const float* a, long a_z, long a_r, long a_k, 
   if (Z <= 0 || R <= 0 || N <= 0 || K <= 0) return 0;
   if (ksplit < 1 || (long)Z * ksplit > 65535 || (R + kSkTile - 1) / kSkTile > 65535) return -1;
   SkinnyParams p{a, a_z, a_r, a_k, b_ptrs, b_base, b_z, b_n, b_k, c, c_z, ldc, add, ld_add, add_cols, R, N, K, silu_a, silu_b, ksplit};
+  if (ksplit == 1 && Z <= 65535 && cb200_skinny_rows(a_k, b_n, b_k, b_is_bf16, c_is_bf16, silu_b, R, N, K))
+    return R == 1 ? launch_skinny_rows<1>(p, Z, st) : R == 2 ? launch_skinny_rows<2>(p, Z, st) : launch_skinny_rows<4>(p, Z, st);
   // (row tiles of 48 reach the grid's limit before those of 64)
   if (cb200_skinny_wide(a_k, b_n, b_k, b_is_bf16, c_is_bf16, silu_b, N, K) && (R + 47) / 48 <= 65535) {
     // rows per CTA: the smallest that holds them all; with several row tiles the weights are read again from L2

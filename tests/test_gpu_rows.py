@@ -139,6 +139,25 @@ def test_few_row_gemm_tiles(R, K, N, Z):
         assert _max_rel(da, dout.double() @ torch.stack(ws).double()) < 1e-6
 
 
+# up to four rows: every number of warps to a weight row (K to 2048) and one element more than that kernel takes; columns around a warp's eight
+# and a CTA's steps; weights off the 16-byte boundary; an added term for some of the columns
+@pytest.mark.parametrize("R", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("K,N,Z", [(8, 1, 1), (256, 1543, 3), (264, 70, 2), (1032, 33, 2), (2048, 257, 84), (2056, 64, 1)])
+def test_few_row_gemm_of_up_to_four_rows(R, K, N, Z):
+    torch.manual_seed(7)
+    store = torch.randn(Z * N * K + 1, device=DEV).bfloat16() / math.sqrt(K)
+    for off in (0, 1):
+        ws = [store[off + z * N * K: off + (z + 1) * N * K].view(N, K) for z in range(Z)]
+        add = torch.randn(R, max(N // 2, 1), device=DEV)
+        for a in (torch.randn(Z, R, K, device=DEV), torch.randn(R, K, device=DEV)):
+            for silu in (False, True):
+                got = F_ops.skinny_linears(a, ws, silu=silu, add=add)
+                x = torch.nn.functional.silu(a.double()) if silu else a.double()
+                want = x @ torch.stack(ws).double().transpose(1, 2)
+                want[..., :add.shape[1]] += add.double()
+                assert _max_rel(got, want) < 1e-6
+
+
 def test_few_row_gemm_takes_as_many_rows_as_its_widest_tile():
     """More rows than the 48-row tiles of the wide kernel can address go to the 64-row tile."""
     R, K, N = 48 * 65535 + 5, 8, 8
