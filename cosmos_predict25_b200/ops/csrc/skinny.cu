@@ -339,10 +339,8 @@ __global__ void __launch_bounds__(256) skinny_rows_kernel(SkinnyParams p, int wk
         if (vec) {
           next[i] = *reinterpret_cast<const bf16x8*>(src);
         } else {
-          __nv_bfloat16 e[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) e[j] = src[j];
-          next[i] = *reinterpret_cast<const bf16x8*>(e);
+          for (int j = 0; j < 4; ++j) next[i].v[j] = __halves2bfloat162(src[2 * j], src[2 * j + 1]);
         }
       }
     }

@@ -183,3 +183,28 @@ def test_kernels_read_no_memory_ahead_of_their_wait():
                 reads = rf"\b{var}\.\w+\s*\[" if struct else rf"\b{var}\s*\[|\*\s*{var}\b|\({var}\s*\+"
                 hit = re.search(reads, ahead)
                 assert hit is None, f"{name} reads {var} ahead of the wait: {hit.group(0)}"
+
+
+_SIZES = {"char": 1, "uint8_t": 1, "int8_t": 1, "bf16": 2, "__nv_bfloat16": 2, "half": 2, "float": 4, "int": 4, "uint32_t": 4, "int32_t": 4,
+          "__nv_bfloat162": 4, "float2": 8, "uint2": 8, "int2": 8, "long": 8, "double": 8, "int64_t": 8, "uint64_t": 8, "float4": 16, "uint4": 16,
+          "int4": 16, "bf16x8": 16}
+
+
+def _wider_accesses(code):
+    """(line, array, its type, type it is accessed as) where a cast reads an array as a type that asks for more alignment than the array has."""
+    for cast in re.finditer(r"reinterpret_cast<(?:const )?(\w+)\*>\(&?(\w+)(?:\[[^\]]*\])?\)", code):
+        wide, var = cast.groups()
+        found = [d for d in re.finditer(rf"^[ \t]*([^\n;(){{}}]*?\b)(\w+) {var}(?:\[[^\]]*\])+ *(?=[=;,{{])", code, re.M) if d.start() < cast.start()]
+        if not found or wide not in _SIZES or found[-1].group(2) not in _SIZES:
+            continue
+        qualifiers, narrow = found[-1].groups()
+        if _SIZES[wide] > _SIZES[narrow] and "align" not in qualifiers and "align" not in found[-1].group(0):
+            yield code[:cast.start()].count("\n") + 1, var, narrow, wide
+
+
+def test_arrays_are_aligned_for_the_accesses_to_them():
+    """An array that is read or written through a wider type is declared with that type's alignment: in local memory the access faults."""
+    assert list(_wider_accesses("  bf16 e[8];\n  x = *reinterpret_cast<const bf16x8*>(e);\n")) == [(2, "e", "bf16", "bf16x8")]
+    assert not list(_wider_accesses("  alignas(16) bf16 e[8];\n  x = *reinterpret_cast<const bf16x8*>(e);\n"))
+    for path in sorted([*CSRC.glob("*.cu"), *CSRC.glob("*.cuh")]):
+        assert list(_wider_accesses(path.read_text())) == [], path.name
