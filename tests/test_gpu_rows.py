@@ -155,7 +155,15 @@ def test_few_row_gemm_of_up_to_four_rows(R, K, N, Z):
                 x = torch.nn.functional.silu(a.double()) if silu else a.double()
                 want = x @ torch.stack(ws).double().transpose(1, 2)
                 want[..., :add.shape[1]] += add.double()
-                assert _max_rel(got, want) < 1e-6
+                if R > 4 or K > 2048:                  # the other kernels
+                    assert _max_rel(got, want) < 1e-6
+                    continue
+                # Sums of terms of either sign: the bound is relative to the sum of their magnitudes. Roundings on the way of a term: 8 in
+                # a lane, 5 over the warp, 7 over the warps, 1 for the added term, 2^-24 each. SiLU: the fast exponential is off by at
+                # most 2 + 1.173 |a| = 7 units of 2^-23, the sum 1 + e by 2^-24, the fast division by 2 units of 2^-23: 19 x 2^-24.
+                terms = x.abs() @ torch.stack(ws).double().abs().transpose(1, 2)
+                terms[..., :add.shape[1]] += add.double().abs()
+                assert a.abs().max() < 5.1 and ((got.double() - want).abs() <= (22 + 19 * silu) * 2.0 ** -24 * terms).all()
 
 
 def test_few_row_gemm_takes_as_many_rows_as_its_widest_tile():
