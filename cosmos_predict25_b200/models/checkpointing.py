@@ -83,8 +83,9 @@ def _make_policy(mode: str):
     def policy(ctx, op, *args, **kwargs):
         d = decide(ctx, op)
         if d == CheckpointPolicy.MUST_SAVE and ctx.is_recompute and op in own:
-            # the recompute pass takes this result from the cache: the front-end still counted a launch that never happens
-            native.count_launch(-1)
+            # the recompute pass takes this result from the cache: the front-end still counts launches that never happen
+            plain = "gemm_bf16_gelu_pre" in str(op) or ("gemm_bf16.default" in str(op) and not args[4] and not args[5])
+            native.count_launch(-ops.gemm_launches(args[0], args[1]) if plain else -1)
         return d
 
     return policy

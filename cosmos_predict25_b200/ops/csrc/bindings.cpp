@@ -605,6 +605,24 @@ TORCH_LIBRARY(cosmos_b200, m) {
         [](int64_t tiles, int64_t kb, int64_t pairs, int64_t c2, int64_t c4, int64_t c3) {
           return (int64_t)cb200_gemm_pairs_per_tile((long)tiles, (long)kb, (int)pairs, (int)c2, (int)c4, (int)c3);
         });
+  m.def("gemm_stream_plan(int tiles, int k_blocks, int pairs, int clusters2, int clusters4, int clusters3) -> (bool, int, int, int)",
+        [](int64_t tiles, int64_t kb, int64_t pairs, int64_t c2, int64_t c4, int64_t c3) {
+          int per_tile = 0, extra = 0, tail = 0;
+          const int rc = cb200_gemm_stream((long)tiles, (long)kb, (int)pairs, (int)c2, (int)c4, (int)c3, &per_tile, &extra, &tail);
+          return std::tuple<bool, int64_t, int64_t, int64_t>(rc != 0, per_tile, extra, tail);
+        });
+  m.def("gemm_clusters(int device) -> int[]", [](int64_t device) {
+    c10::cuda::CUDAGuard g(static_cast<c10::DeviceIndex>(device));
+    int pairs = 0, c2 = 0, c4 = 0, c3 = 0;
+    const int rc = cb200_gemm_clusters(cb200_sm_count((int)device), &pairs, &c2, &c4, &c3);
+    TORCH_CHECK(rc == 0, "no count of the clusters that the GPU holds: code ", rc);
+    return std::vector<int64_t>{pairs, c2, c4, c3};
+  });
+  // kernels that gemm_bf16 (with K-major operands) and gemm_bf16_gelu_pre launch on the current device
+  m.def("gemm_launches(int M, int N, int K) -> int", [](int64_t M, int64_t N, int64_t K) {
+    const long need = cb200_gemm_stream_floats((int)M, (int)N, (int)K, 0, 0, 0, cb200_sm_count(at::cuda::current_device()));
+    return (int64_t)(need > 0 ? 2 : 1);
+  });
   m.def("gemm_group_launches(int rows, int groups) -> int",
         [](int64_t rows, int64_t groups) { return (int64_t)cb200_gemm_group_launches((int)rows, (int)groups); });
   m.def("gemm_pair_mode(int mode) -> int", &gemm_pair_mode);

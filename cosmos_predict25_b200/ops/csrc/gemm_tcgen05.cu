@@ -1222,10 +1222,14 @@ static StreamPlan stream_plan(int tiles, int tiles_n, int kb, int pairs) {
   if (pl.tail == 0) pl.extra = 0;
   return pl;
 }
-// Whether that takes less time, in k-blocks of a pair: its share, and kStream for writing the partial tiles (256 KB each) and adding them in a
-// launch of its own (12 us); against the rule above or whole waves of tiles.
-extern "C" int cb200_gemm_stream(long tiles, long kb, int pairs, int c2, int c4, int c3) {
-  constexpr long kStream = 45, kExchange = 6;
+// Whether that takes less time than the rule above or whole waves of tiles. In units of 10 ns, fitted to launches back to back from K = 8192 to
+// 100,352: k-blocks in a row of clusters take 5.5 us + 0.31 us each (within 3 %); shared out, a pair's k-block takes 0.43 us (all pairs draw
+// on L2 at once), and the second launch 10 us and what it adds up one after another: 0.55 us for each pair of a tile and 0.33 us for each
+// pair of the tail. 256 x 256, where 74 partial tiles are added, takes 46 us from any K up to 32,768 and clusters 22 us from 12,288;
+// 256 x 768 from 12,288 28.4 and 22.4, from 32,768 33.5 and 45.5; 4096 x 768 (26 pairs of the tail) from 12,288 74.6 and 65.5, from 32,768
+// 163 and 167.
+extern "C" int cb200_gemm_stream(long tiles, long kb, int pairs, int c2, int c4, int c3, int* per_tile, int* extra, int* tail) {
+  constexpr long kExchange = 6;
   if (tiles < 1 || tiles > pairs || kb < pairs) return 0;
   const int split = cb200_gemm_pairs_per_tile(tiles, kb, pairs, c2, c4, c3);
   const long now = split == 2   ? (tiles + c2 - 1) / c2 * ((kb + 1) / 2 + kExchange)
@@ -1233,7 +1237,11 @@ extern "C" int cb200_gemm_stream(long tiles, long kb, int pairs, int c2, int c4,
                    : split == 4 ? (tiles + c4 - 1) / c4 * ((kb + 3) / 4 + kExchange)
                                 : kb;
   const StreamPlan pl = stream_plan((int)tiles, 1, (int)kb, pairs);
-  return (kb - pl.tail + pl.per_tile - 1) / pl.per_tile + kStream < now ? 1 : 0;
+  if (per_tile != nullptr) *per_tile = pl.per_tile;
+  if (extra != nullptr) *extra = pl.extra;
+  if (tail != nullptr) *tail = pl.tail;
+  const long share = (kb - pl.tail + pl.per_tile - 1) / pl.per_tile;
+  return 1000 + 43 * share + 55 * pl.per_tile + 33 * pl.extra < 550 + 31 * now ? 1 : 0;
 }
 
 // pairs that the GPU holds at once for gemm_stream_kernel
@@ -1254,13 +1262,20 @@ static int stream_pairs(int sms, int* pairs) {
   return 0;
 }
 
+// what the rules above count with on this GPU: pairs of gemm_stream_kernel, clusters of 2, 4 and 3 pairs (K-major operands) held at once
+extern "C" int cb200_gemm_clusters(int sms, int* pairs, int* c2, int* c4, int* c3) {
+  int rc;
+  if ((rc = stream_pairs(sms, pairs)) || (rc = resident_clusters<0, 0, 2>(c2)) || (rc = resident_clusters<0, 0, 4>(c4))) return rc;
+  return resident_clusters<0, 0, 3>(c3);
+}
+
 // fp32 values of scratch with which cb200_gemm_bf16 can share out the k-blocks of this product, 0: it would not
 extern "C" long cb200_gemm_stream_floats(int M, int N, int K, int a_mn, int b_mn, int gated, int sms) {
   if (a_mn || b_mn || gated || M < 2 * BM || N % BN != 0 || K % 8 != 0 || K < 64 * BK || cb200_gemm_pair_mode(-1) != 1) return 0;
   int pairs = 0, c2 = 0, c3 = 0, c4 = 0;
-  if (stream_pairs(sms, &pairs) || resident_clusters<0, 0, 2>(&c2) || resident_clusters<0, 0, 3>(&c3) || resident_clusters<0, 0, 4>(&c4)) return 0;
+  if (cb200_gemm_clusters(sms, &pairs, &c2, &c4, &c3)) return 0;
   const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * (N / BN);
-  if (!cb200_gemm_stream(tiles, (K + BK - 1) / BK, pairs, c2, c4, c3)) return 0;
+  if (!cb200_gemm_stream(tiles, (K + BK - 1) / BK, pairs, c2, c4, c3, nullptr, nullptr, nullptr)) return 0;
   const StreamPlan pl = stream_plan((int)tiles, N / BN, (K + BK - 1) / BK, pairs);
   return (long)(pl.per_tile * pl.tiles + pl.extra * kStreamSlots) * 2 * BM * BN;
 }

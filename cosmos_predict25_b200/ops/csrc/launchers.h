@@ -61,6 +61,8 @@ int cb200_skinny_wide(long a_k, long b_n, long b_k, int b_is_bf16, int c_is_bf16
 // ws: cb200_gemm_stream_floats fp32 values of scratch, or nullptr
 int cb200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int b_mn, const void* bias,
                     int act, void* pre, const void* resid, const float* gate, long ld_gate, int L, int* err, int sms, cudaStream_t st, float* ws = nullptr);
+int cb200_gemm_stream(long tiles, long kb, int pairs, int c2, int c4, int c3, int* per_tile, int* extra, int* tail);   // 1: k-blocks go over all pairs
+int cb200_gemm_clusters(int sms, int* pairs, int* c2, int* c4, int* c3);
 long cb200_gemm_stream_floats(int M, int N, int K, int a_mn, int b_mn, int gated, int sms);
 int cb200_gemm_many_weights(int n, int M, int N, int K, int sms);   // weights a launch of cb200_gemm_bf16_many takes, or 0
 int cb200_gemm_bf16_many(const void* A, const void* const* B, void* const* C, const void* const* norm, const uint8_t* norm_bf16, int n, int M,

@@ -135,20 +135,15 @@ def _linear_fm(x, w, bias, act):
     p2 = p2 if p2.is_contiguous() else p2.contiguous()
     M = p2.shape[0]
     if tx is None:
-        y = ops.gemm_bf16(p2, w, bias, _ACT_CODE[act], False, False)
-        native.count_launch()
-        return y.view(*lead, N)
+        return gemm_nt(p2, w, bias, act).view(*lead, N)
     t2 = tx.reshape(-1, tx.shape[-1])
     t2 = t2 if t2.is_contiguous() else t2.contiguous()
     both = _stacked_rows(p2, t2)
     if both is not None:
-        out = ops.gemm_bf16(both, w, None, 0, False, False)
-        native.count_launch()
+        out = gemm_nt(both, w)
         pre, tpre = out[:M], out[M:]
     else:
-        pre = ops.gemm_bf16(p2, w, None, 0, False, False)
-        tpre = ops.gemm_bf16(t2, w, None, 0, False, False)
-        native.count_launch(2)
+        pre, tpre = gemm_nt(p2, w), gemm_nt(t2, w)
     if bias is not None:
         pre += bias
     if act == "gelu":
@@ -463,6 +458,16 @@ def _native_gemm_ok(x2d: torch.Tensor, w: torch.Tensor) -> bool:
     return K % 64 == 0 and N % 8 == 0 and M >= 1
 
 
+def gemm_launches(a: torch.Tensor, b: torch.Tensor) -> int:
+    """Kernels of ``gemm_bf16`` / ``gemm_bf16_gelu_pre`` on a [M, K] and b [N, K]: two where the contraction of few tiles (no more than
+    the GPU has CTA pairs) goes over all pairs. The conditions in front are necessary and spare ordinary products the question."""
+    M, K = a.shape
+    N = b.shape[0]
+    if K < 4096 or M < 256 or N % 256 or M * N > 74 << 16:
+        return 1
+    return native.load().gemm_launches(M, N, K)
+
+
 def gemm_nt(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None, act: str = "none",
             trans_a: bool = False, trans_b: bool = False) -> torch.Tensor:
     """C[M,N] = op(A) @ op(B)^T-style contraction on the tcgen05 GEMM.
@@ -472,7 +477,7 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = Non
     """
     ops = native.load()
     out = ops.gemm_bf16(a, b, bias, _ACT_CODE[act], trans_a, trans_b)
-    native.count_launch()
+    native.count_launch(1 if trans_a or trans_b else gemm_launches(a, b))
     return out
 
 
@@ -484,7 +489,7 @@ class _Linear(torch.autograd.Function):
             x2d = x2d.contiguous()
         if act == "gelu":
             y, pre = native.load().gemm_bf16_gelu_pre(x2d, w, bias)
-            native.count_launch()
+            native.count_launch(gemm_launches(x2d, w))
             ctx.save_for_backward(x2d, w, pre)
         else:
             y = gemm_nt(x2d, w, bias, "none")

@@ -19,17 +19,23 @@ def _rel(a, b):
     return ((a.double() - b).norm() / b.norm()).item()
 
 
-# (batch, tokens, context width, model width, CTA pairs per tile): below one launch; unsplit with whole and partial N tiles; both splits;
-# ragged rows; more tiles than half the pairs. The split is the rule's for the 36 and 16 clusters that a B200 holds at least.
+def _split(tiles, k_blocks):
+    """CTA pairs per tile for the clusters that this GPU holds."""
+    _, c2, c4, c3 = native.load().gemm_clusters(torch.cuda.current_device())
+    return native.load().gemm_pairs_per_tile(tiles, k_blocks, 74, c2, c4, c3)
+
+
+# (batch, tokens, context width, model width, CTA pairs per tile): below one launch; unsplit with whole and partial N tiles; every split;
+# ragged rows; more tiles than half the pairs.
 @pytest.mark.parametrize("B,S,C,D,split", [(2, 40, 512, 256, 1), (1, 256, 512, 256, 1), (2, 512, 512, 1024, 1), (2, 512, 1024, 2048, 1),
-                                           (1, 256, 1024, 2048, 4), (1, 512, 1024, 2048, 2), (1, 264, 1024, 1024, 4), (1, 264, 2048, 384, 1),
+                                           (1, 256, 1024, 1024, 4), (1, 512, 1024, 2048, 2), (1, 264, 1024, 512, 4), (1, 264, 2048, 384, 1),
                                            (1, 520, 640, 640, 1), (3, 88, 2112, 256, 4)])
 def test_keys_and_values_of_all_blocks(B, S, C, D, split):
     torch.manual_seed(0)
     ops = native.load()
     tiles = -(-B * S // 256) * -(-D // 256) * 2
     if D % 256 == 0 and B * S >= 256:
-        assert ops.gemm_pairs_per_tile(tiles, C // 64, 74, 36, 16) == split
+        assert _split(tiles, C // 64) == split
     ctx = torch.randn(B, S, C, device=DEV).bfloat16()
     widths = (D, 128, D)                                       # blocks of another width between
     ws = []
@@ -48,10 +54,10 @@ def test_keys_and_values_of_all_blocks(B, S, C, D, split):
         assert torch.equal(got[2 * i], again[2 * i]) and torch.equal(got[2 * i + 1], again[2 * i + 1])
 
 
-# 256 to 528 tokens: 12 to 36 tiles of q, k and v over 16 k-blocks, all of them split; 80 prompt rows to 1,024. The other widths, the widest
+# 256 to 528 tokens: 12 to 36 tiles of q, k and v over 16 k-blocks, split up to as many tiles as clusters of two pairs fit; 80 prompt rows to 1,024. The other widths, the widest
 # with the row kernels for more than 4096 channels: few tokens, split and unsplit.
-@pytest.mark.parametrize("preset,shape,tokens,split", [("mini", (1, 1, 32, 32), 40, 4), ("mini", (2, 1, 32, 32), 128, 2), ("mini", (1, 1, 24, 88), 256, 2),
-                                                       ("mini", (1, 2, 26, 40), 512, 2), ("2b", (1, 1, 32, 32), 512, 2), ("2b", (1, 1, 8, 12), 24, None),
+@pytest.mark.parametrize("preset,shape,tokens,split", [("mini", (1, 1, 32, 32), 40, 4), ("mini", (2, 1, 32, 32), 128, 2), ("mini", (1, 1, 24, 44), 256, 2),
+                                                       ("mini", (1, 2, 26, 40), 512, 1), ("2b", (1, 1, 32, 32), 512, 2), ("2b", (1, 1, 8, 12), 24, None),
                                                        ("2b", (2, 3, 32, 36), 40, 1), ("14b", (1, 1, 8, 8), 32, None), ("14b", (1, 3, 24, 32), 256, 1)])
 def test_query_key_value_of_few_tiles(preset, shape, tokens, split):
     """The native block loop against the module path, whose q, k and v are launches of their own: the same sums in another order, so a few
@@ -68,7 +74,7 @@ def test_query_key_value_of_few_tiles(preset, shape, tokens, split):
     B, T, H, W = shape
     rows, D = B * T * H * W // 4, net.cfg.model_channels
     if split is not None:                                       # below 256 rows q, k and v are launches of their own
-        assert native.load().gemm_pairs_per_tile(-(-rows // 256) * (D // 256) * 3, D // 64, 74, 36, 16) == split
+        assert _split(-(-rows // 256) * (D // 256) * 3, D // 64) == split
     x, text = torch.randn(B, 16, T, H, W, device=DEV).bfloat16(), torch.randn(B, tokens, 512, device=DEV).bfloat16()
     t, fps = torch.rand(B, T, device=DEV) * 1000, torch.full((B,), 16.0, device=DEV)
     served = []

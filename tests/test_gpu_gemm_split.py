@@ -6,6 +6,7 @@ import math
 import pytest
 import torch
 
+from cosmos_predict25_b200.ops import functional as F_ops
 from cosmos_predict25_b200.ops import native
 
 pytestmark = pytest.mark.gpu
@@ -15,6 +16,11 @@ ROUND = 1.5 * 2.0 ** -9        # one bf16 rounding of the result in the 2-norm
 
 def _rel(a, b):
     return ((a.double() - b).norm() / b.norm()).item()
+
+
+def _clusters():
+    """Pairs, and clusters of two, four and three pairs, that this GPU holds at once."""
+    return native.load().gemm_clusters(torch.cuda.current_device())
 
 
 def _check():
@@ -64,7 +70,8 @@ def test_epilogues(M, N, K):
 def test_three_pairs(M, N, K):
     torch.manual_seed(2)
     ops = native.load()
-    assert ops.gemm_pairs_per_tile(-(-M // 256) * (N // 256), K // 64, 74, 33, 16, 22) == 3
+    _, c2, c4, c3 = _clusters()
+    assert ops.gemm_pairs_per_tile(-(-M // 256) * (N // 256), K // 64, 74, c2, c4, c3) == 3
     a = torch.randn(M, K, device=DEV).bfloat16()
     b = (torch.randn(N, K, device=DEV) / math.sqrt(K)).bfloat16()
     L = 8
@@ -92,12 +99,19 @@ def test_gated_tiles_in_a_row(M, N, K, L):
     assert _rel(got, resid.double() + gate.double().repeat_interleave(L, 0) * (a.double() @ b.double().t())) < ROUND
 
 
-# tiles whose k-blocks are shared out over all pairs: one tile for all of them, several pairs a tile with none left over for the tail, a tail
-# whose pairs reach into two and three tiles, more tiles than half of the pairs; ragged rows, a last k-block of 8
-@pytest.mark.parametrize("M,N,K", [(256, 256, 16384), (300, 512, 16384), (1000, 1024, 32768), (2500, 1024, 32768), (2304, 1024, 16384), (520, 768, 32776)])
+# Tiles whose k-blocks are shared out over all pairs: one tile for all of them, several pairs a tile with none left over for the tail, a tail
+# whose pairs reach into two and three tiles, more tiles than half of the pairs; ragged rows, a last k-block of 8. `shared`: what the rule says
+# for every GPU that holds 70 pairs and more; None: it depends on the clusters that the GPU holds.
+@pytest.mark.parametrize("M,N,K,shared", [(256, 256, 65536, True), (300, 512, 32768, True), (1000, 1024, 65536, None), (2500, 1024, 65536, None),
+                                          (1280, 2304, 32768, True), (520, 768, 32776, True), (256, 256, 16384, False), (2304, 1024, 16384, None)])
 @pytest.mark.parametrize("bias,act", [(False, 0), (True, 0), (True, 1)])
-def test_long_contractions_are_shared_over_all_pairs(M, N, K, bias, act):
+def test_long_contractions_are_shared_over_all_pairs(M, N, K, shared, bias, act):
     ops = native.load()
+    pairs, c2, c4, c3 = _clusters()
+    taken = ops.gemm_stream_plan(-(-M // 256) * (N // 256), -(-K // 64), pairs, c2, c4, c3)[0]
+    if shared is not None:
+        assert taken == shared
+    assert ops.gemm_launches(M, N, K) == (2 if taken else 1)
     torch.manual_seed(5)
     x = torch.randn(M, K, device=DEV).bfloat16()
     w = (torch.randn(N, K, device=DEV) / K ** 0.5).bfloat16()
@@ -114,8 +128,19 @@ def test_long_contractions_are_shared_over_all_pairs(M, N, K, bias, act):
     pre = want
     if act:
         want = torch.nn.functional.gelu(want)
-    # one rounding to bf16; fp32 sums of 32,776 products of unit variance over sqrt(K) stay at 1e-6 of it
+    # one rounding to bf16; fp32 sums of 65,536 products of unit variance over sqrt(K) stay at 1e-6 of it
     assert ((y.double() - want).norm() / want.norm()).item() < 1.5 * 2.0 ** -9
     if act:
         y2, got_pre = ops.gemm_bf16_gelu_pre(x, w, b)
         assert torch.equal(y2, y) and ((got_pre.double() - pre).norm() / pre.norm()).item() < 1.5 * 2.0 ** -9
+
+
+def test_shared_contraction_counts_both_kernels():
+    """The sums of all pairs are added by a kernel of its own, which the launch count includes; ordinary products are one launch."""
+    for M, N, K, act in ((512, 512, 65536, "none"), (512, 512, 65536, "gelu"), (512, 512, 1024, "none"), (512, 512, 8192, "gelu")):
+        x = torch.randn(M, K, device=DEV).bfloat16().requires_grad_(act == "gelu")
+        w = torch.randn(N, K, device=DEV).bfloat16()
+        before = native.launches()
+        F_ops.linear(x, w, None, act)
+        assert native.launches() - before == (2 if K == 65536 else 1)
+    _check()
