@@ -591,9 +591,9 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("ln_modulate_jvp(Tensor x, Tensor tx, Tensor shift, Tensor scale, Tensor? tshift, Tensor? tscale, int L, float eps) -> "
         "(Tensor, Tensor)", &ln_modulate_jvp);
   m.def("rmsnorm_rope_jvp(Tensor x, Tensor tx, Tensor w, Tensor? cos, Tensor? sin, float eps) -> (Tensor, Tensor)", &rmsnorm_rope_jvp);
-  m.def("skinny_rows(int a_k, int b_n, int b_k, bool b_bf16, bool out_bf16, bool silu_b, int R, int N, int K) -> bool",
-        [](int64_t a_k, int64_t b_n, int64_t b_k, bool b_bf16, bool out_bf16, bool silu_b, int64_t R, int64_t N, int64_t K) {
-          return cb200_skinny_rows(a_k, b_n, b_k, b_bf16, out_bf16, silu_b, (int)std::min<int64_t>(R, 1 << 20), (int)N, (int)K) != 0;
+  m.def("skinny_rows(int a_k, int b_n, int b_k, bool b_bf16, bool out_bf16, bool silu_b, int Z, int R, int N, int K) -> bool",
+        [](int64_t a_k, int64_t b_n, int64_t b_k, bool b_bf16, bool out_bf16, bool silu_b, int64_t Z, int64_t R, int64_t N, int64_t K) {
+          return cb200_skinny_rows(a_k, b_n, b_k, b_bf16, out_bf16, silu_b, (int)Z, (int)std::min<int64_t>(R, 1 << 20), (int)N, (int)K) != 0;
         });
   m.def("skinny_wide(int a_k, int b_n, int b_k, bool b_bf16, bool out_bf16, bool silu_b, int N, int K) -> bool",
         [](int64_t a_k, int64_t b_n, int64_t b_k, bool b_bf16, bool out_bf16, bool silu_b, int64_t N, int64_t K) {

@@ -54,7 +54,7 @@ int cb200_skinny_bgemm(const float* a, long a_z, long a_r, long a_k, const long 
                        long b_k, int b_is_bf16, void* c, long c_z, int ldc, int c_is_bf16, const float* add, int ld_add, int add_cols,
                        int Z, int R, int N, int K, int silu_a, int silu_b, int ksplit, cudaStream_t st);
 
-int cb200_skinny_rows(long a_k, long b_n, long b_k, int b_is_bf16, int c_is_bf16, int silu_b, int R, int N, int K);
+int cb200_skinny_rows(long a_k, long b_n, long b_k, int b_is_bf16, int c_is_bf16, int silu_b, int Z, int R, int N, int K);   // 1: the few-row kernel
 int cb200_skinny_wide(long a_k, long b_n, long b_k, int b_is_bf16, int c_is_bf16, int silu_b, int N, int K);   // 1: 256-column tiles
 
 // gemm_tcgen05.cu

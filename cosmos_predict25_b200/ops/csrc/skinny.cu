@@ -300,11 +300,11 @@ static int launch_skinny_wide(const SkinnyParams& p, int Z, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------------------------------------------------------------------
-// The same for up to four rows and K <= 2048 (the modulation MLPs of an image with its negative prompt): the weights, read once, are all that
-// counts. A lane keeps its eight elements of the rows in registers for good and takes one 16-byte piece of eight weight rows at a time, the
-// next eight in flight; WK warps of 256 elements each make up a weight row, their sums of 32 lanes meet in shared memory. No stages of
-// weights in shared memory and no split of the reduction over CTAs (whose sums took a launch more).
-// @ROWS_FIGURES@
+// The same for up to four rows and K <= 2048: the weights, read once, are what counts, then the sums over the lanes. A lane keeps its eight
+// elements of the rows in registers for good (which is what ends at 2048: eight warps of 256 elements to a weight row) and takes one 16-byte
+// piece of eight weight rows at a time, the next eight in flight; the warps' sums of 32 lanes meet in shared memory. No stages of weights
+// in shared memory and no split of the reduction over CTAs (whose sums took a launch more). Times and the rule: cb200_skinny_rows below.
+// 88 MB of weights (84 x 256 x 2048) go at 3.9 TB/s with one row, 2.9 with two.
 constexpr int kRowsN = 8;                // weight rows of a warp at a time
 template <int RT>
 __global__ void __launch_bounds__(256) skinny_rows_kernel(SkinnyParams p, int wk, int per_cta) {
@@ -406,9 +406,32 @@ static int launch_skinny_rows(const SkinnyParams& p, int Z, cudaStream_t st) {
 
 using namespace cb200;
 
-// whether a call goes to the kernel for a few rows, which does not split reductions
-extern "C" int cb200_skinny_rows(long a_k, long b_n, long b_k, int b_is_bf16, int c_is_bf16, int silu_b, int R, int N, int K) {
-  return b_is_bf16 && !c_is_bf16 && !silu_b && a_k == 1 && b_k == 1 && b_n % 8 == 0 && K % 8 == 0 && K <= 2048 && R <= 4 && N >= 1 ? 1 : 0;
+// Whether a call goes to the kernel for a few rows, which does not split reductions. Its time goes with E, the weight elements with a row
+// padded to its warps (256, 512, 1024 or 2048), times the rows; the wide kernel takes about 9 us as soon as it splits, since the sums are a
+// launch more (from K = 256 on, up to 296 tiles of 256 columns), and 256 columns' time for few columns. us of the wide kernel and of this
+// one, launches back to back with the weights in L2 as far as they fit, and behind a flush of L2 (two layers of 28 blocks' modulation are
+// 84 x 256 x 2048 and 84 x 6144 x 256; a network's weights come from HBM):
+//   rows                  1                         2                         4
+//   1 x 256 x 2048     9.9  3.6, 17.8 10.2      10.4  4.2, 19.5 10.2      11.2  5.1, 21.5 10.2
+//   1 x 4096 x 256     8.9  3.8, 17.4 10.2       9.2  4.6, 17.4 10.2      10.4  6.1, 19.4 12.3
+//   84 x 64 x 2048    32.1 10.8, 37.9 14.4      32.2  9.8, 39.8 16.4      32.6 14.1, 40.0 20.5
+//   84 x 256 x 2048   32.9 22.5, 46.0 28.7      33.7 30.2, 46.1 37.8      34.7 33.1, 48.1 39.9
+//   84 x 6144 x 256   68.6 54.7, 77.8 65.6      70.5 72.0, 79.9 84.0      74.3 90.3, 84.0 97.3     unsplit: one row only
+//   1 x 6144 x 2048   12.5 10.8, 21.5 14.4      13.0 10.4, 23.6 16.4      13.3 17.8, 25.6 20.5
+//   3 x 6144 x 1032   15.8 13.8, 25.7 20.5      16.4 20.2, 27.6 27.5      17.2 23.7, 29.7 30.7     half of the lanes idle
+//   84 x 768 x 64      5.3  8.4, 10.3 14.3       5.6 10.9, 12.3 18.4       6.4 14.9, 13.2 20.5     most of the lanes idle: to 4096 columns
+extern "C" int cb200_skinny_rows(long a_k, long b_n, long b_k, int b_is_bf16, int c_is_bf16, int silu_b, int Z, int R, int N, int K) {
+  if (!(b_is_bf16 && !c_is_bf16 && !silu_b && a_k == 1 && b_k == 1 && b_n % 8 == 0 && K % 8 == 0 && K <= 2048 && R <= 4 && N >= 1)) return 0;
+  long padded = 256;
+  while (padded < K) padded *= 2;
+  const long cols = (long)Z * N, E = cols * padded;
+  const bool split = K >= 256 && (long)Z * ((N + 255) / 256) <= 296, full = K * 5 >= padded * 4;
+  if (K < 128) return cols <= 4096;
+  if (R == 1 && (split || full || (K >= 256 && K * 3 >= padded * 2))) return 1;
+  if (K < 256) return cols <= 16384;
+  if (N <= 128 || E <= 6L << 20) return 1;
+  if (!split || R == 1) return 0;
+  return full || (R == 2 && E <= 14L << 20);
 }
 
 // whether a call goes to the wide kernel (the split of long reductions counts its tiles): bf16 weights with one contiguous index and
@@ -424,7 +447,7 @@ extern "C" int cb200_skinny_bgemm(const float* a, long a_z, long a_r, long a_k, 
   if (Z <= 0 || R <= 0 || N <= 0 || K <= 0) return 0;
   if (ksplit < 1 || (long)Z * ksplit > 65535 || (R + kSkTile - 1) / kSkTile > 65535) return -1;
   SkinnyParams p{a, a_z, a_r, a_k, b_ptrs, b_base, b_z, b_n, b_k, c, c_z, ldc, add, ld_add, add_cols, R, N, K, silu_a, silu_b, ksplit};
-  if (ksplit == 1 && Z <= 65535 && cb200_skinny_rows(a_k, b_n, b_k, b_is_bf16, c_is_bf16, silu_b, R, N, K))
+  if (ksplit == 1 && Z <= 65535 && cb200_skinny_rows(a_k, b_n, b_k, b_is_bf16, c_is_bf16, silu_b, Z, R, N, K))
     return R == 1 ? launch_skinny_rows<1>(p, Z, st) : R == 2 ? launch_skinny_rows<2>(p, Z, st) : launch_skinny_rows<4>(p, Z, st);
   // (row tiles of 48 reach the grid's limit before those of 64)
   if (cb200_skinny_wide(a_k, b_n, b_k, b_is_bf16, c_is_bf16, silu_b, N, K) && (R + 47) / 48 <= 65535) {

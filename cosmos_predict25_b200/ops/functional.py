@@ -687,7 +687,7 @@ def _skinny_split(Z: int, R: int, N: int, K: int, wide: bool) -> int:
 def _skinny_call(ops, Z, R, N, K, *args):
     """args = the operator's arguments up to ``out_bf16``; splits long reductions and adds the partial sums."""
     _, _, _, a_k, _, _, _, b_n, b_k, bf16, _, _, _, _, _, _, _, silu_b, out_bf16 = args
-    if out_bf16 or ops.skinny_rows(a_k, b_n, b_k, bf16, out_bf16, silu_b, R, N, K):
+    if out_bf16 or ops.skinny_rows(a_k, b_n, b_k, bf16, out_bf16, silu_b, Z, R, N, K):
         S = 1
     else:
         S = _skinny_split(Z, R, N, K, ops.skinny_wide(a_k, b_n, b_k, bf16, out_bf16, silu_b, N, K))

@@ -94,3 +94,24 @@ def test_launches_of_several_weights():
         assert [ops.gemm_group_launches(m, 2) for m in (8, 255, 256, 5000)] == [2, 2, 2, 2]
     finally:
         ops.gemm_pair_mode(was)
+
+
+def _few_rows(Z, R, N, K):
+    return native.load().skinny_rows(1, K, 1, True, False, False, Z, R, N, K)
+
+
+def test_few_row_kernel_is_taken_where_it_is_faster():
+    """Measured slower there and back with the wide kernel: the second layer of 28 blocks' modulation from two rows on, weights of up to 64
+    elements a row with many columns, half-empty lanes. Measured faster with the weights from HBM: the first layer, few columns, calls whose
+    reduction the wide kernel splits."""
+    for Z, R, N, K in ((84, 2, 6144, 256), (84, 4, 6144, 256), (84, 2, 2048, 256), (84, 4, 256, 64), (84, 1, 768, 8), (84, 2, 6144, 64), (6, 2, 6144, 64),
+                       (84, 2, 2048, 512), (28, 2, 3072, 264), (3, 2, 6144, 1032), (28, 1, 6144, 264), (84, 3, 256, 128), (84, 1, 1024, 192)):
+        assert not _few_rows(Z, R, N, K), (Z, R, N, K)
+    for Z, R, N, K in ((84, 1, 256, 2048), (84, 2, 256, 2048), (84, 4, 256, 2048), (84, 1, 6144, 256), (1, 1, 4096, 256), (1, 2, 4096, 256), (1, 4, 4096, 256),
+                       (1, 4, 256, 2048), (1, 2, 6144, 2048), (84, 4, 64, 2048), (84, 4, 64, 256), (1, 4, 4096, 64), (1, 1, 1, 8), (12, 2, 1024, 520),
+                       (84, 2, 768, 1024), (84, 1, 3072, 248), (12, 4, 3072, 2048), (84, 3, 768, 1024)):
+        assert _few_rows(Z, R, N, K), (Z, R, N, K)
+    ops = native.load()
+    assert not ops.skinny_rows(1, 2056, 1, True, False, False, 1, 1, 8, 2056) and not _few_rows(1, 5, 64, 2048)
+    assert not ops.skinny_rows(1, 264, 1, True, True, False, 1, 1, 8, 256) and not ops.skinny_rows(2, 256, 1, True, False, False, 1, 1, 8, 256)
+    assert not ops.skinny_rows(1, 260, 1, True, False, False, 1, 1, 8, 256) and not ops.skinny_rows(1, 1, 256, True, False, False, 1, 1, 8, 256)

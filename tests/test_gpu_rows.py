@@ -145,6 +145,7 @@ def test_few_row_gemm_tiles(R, K, N, Z):
 @pytest.mark.parametrize("K,N,Z", [(8, 1, 1), (256, 1543, 3), (264, 70, 2), (1032, 33, 2), (2048, 257, 84), (2056, 64, 1)])
 def test_few_row_gemm_of_up_to_four_rows(R, K, N, Z):
     torch.manual_seed(7)
+    assert native.load().skinny_rows(1, K, 1, True, False, False, Z, R, N, K) == (R <= 4 and K <= 2048)
     store = torch.randn(Z * N * K + 1, device=DEV).bfloat16() / math.sqrt(K)
     for off in (0, 1):
         ws = [store[off + z * N * K: off + (z + 1) * N * K].view(N, K) for z in range(Z)]
