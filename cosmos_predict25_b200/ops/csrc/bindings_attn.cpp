@@ -204,6 +204,7 @@ void register_attention_ops(torch::Library& m) {
         &fa_fwd_scatter_seq_peer);
   m.def("fa_bwd(Tensor do, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, float scale) -> (Tensor, Tensor, Tensor)");
   m.def("fa_fwd_variant(Tensor q, Tensor k, Tensor v, float scale, int variant) -> (Tensor, Tensor)");
+  m.def("fa_bwd_kernel(int queries, int keys) -> int", [](int64_t queries, int64_t keys) { return (int64_t)cb200_fa_bwd_pick((int)queries, (int)keys, 0); });
   m.def("fa_jvp(Tensor q, Tensor k, Tensor v, Tensor tq, Tensor tk, Tensor tv, float scale) -> (Tensor, Tensor, Tensor)");
   m.def("fa_jvp_tangent(Tensor q, Tensor k, Tensor v, Tensor tq, Tensor tk, Tensor tv, Tensor o, Tensor lse, float scale) -> Tensor");
   m.def("fa_bwd_variant(Tensor do, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, float scale, int variant) -> (Tensor, Tensor, Tensor)");

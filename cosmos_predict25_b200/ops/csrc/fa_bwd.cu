@@ -560,14 +560,16 @@ extern "C" int cb200_fa_bwd_tile_main(const void* d_o, const void* q, const void
 extern "C" void cb200_fa_bwd_tile_dq_convert(const float* acc, void* dq, int B, int S, int H, float scale, cudaStream_t st);
 
 // variant 0: choose by problem size; 1: two deterministic kernels (7 GEMMs, no atomics); 2: single pass over 128 x 64 sub-tiles with
-// fp32 dQ accumulation (5 GEMMs); 3: single pass over 128 x 128 tiles (5 GEMMs, every MMA N = 128)
-static int fa_bwd_pick(int Skv, int variant) { return variant != 0 ? variant : (Skv >= 2048 ? kFaBwdDefaultLong : 1); }
-static bool fa_bwd_use_fused(int Skv, int variant) { return fa_bwd_pick(Skv, variant) >= 2; }
+// fp32 dQ accumulation (5 GEMMs); 3: single pass over 128 x 128 tiles (5 GEMMs, every MMA N = 128). Up to 256 queries a CTA of the third has
+// one or two tiles, in whose time its bulk reductions of dQ do not hide: 128 queries x 16 heads from 4096 keys 42.8 (2) and 45 us (3), 1
+// query 36.8 and 45, 200 from 2100 31.5 and 32.8, 256 from 8192 101 and 102; 384 x 40 heads from 2048 97 and 93.
+extern "C" int cb200_fa_bwd_pick(int Sq, int Skv, int variant) { return variant != 0 ? variant : Skv < 2048 ? 1 : Sq <= 256 ? 2 : kFaBwdDefaultLong; }
+static bool fa_bwd_use_fused(int Sq, int Skv, int variant) { return cb200_fa_bwd_pick(Sq, Skv, variant) >= 2; }
 
 extern "C" long cb200_fa_bwd_scratch_floats_v(int B, int Sq, int Skv, int H, int variant) {
   const long S_pad = (Sq + 127) / 128 * 128;
   long n = 2L * B * H * S_pad;
-  if (fa_bwd_use_fused(Skv, variant)) n += (long)B * H * (fa_bwd_pick(Skv, variant) == 3 ? S_pad : Sq) * 128;
+  if (fa_bwd_use_fused(Sq, Skv, variant)) n += (long)B * H * (cb200_fa_bwd_pick(Sq, Skv, variant) == 3 ? S_pad : Sq) * 128;
   return n;
 }
 
@@ -598,16 +600,16 @@ extern "C" int cb200_fa_bwd_v(const void* d_o, const void* q, const void* k, con
   {
     const long rows = (long)B * H * S_pad;
     fa_bwd_prep_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>((const bf16*)o, (const bf16*)d_o, lse, delta, lse2, B, Sq, H, S_pad,
-                                                                   fa_bwd_use_fused(Skv, variant) ? -1.f : 1.f);
+                                                                   fa_bwd_use_fused(Sq, Skv, variant) ? -1.f : 1.f);
   }
-  if (fa_bwd_pick(Skv, variant) == 3) {
+  if (cb200_fa_bwd_pick(Sq, Skv, variant) == 3) {
     float* acc = scratch + 2 * (size_t)B * H * S_pad;
     const int rc = cb200_fa_bwd_tile_main(d_o, q, k, v, lse2, delta, acc, dk, dv, B, Sq, Skv, H, S_pad, scale, err, st);
     if (rc) return rc;
     cb200_fa_bwd_tile_dq_convert(acc, dq, B, Sq, H, scale, st);
     return (int)cudaGetLastError();
   }
-  if (fa_bwd_use_fused(Skv, variant))
+  if (fa_bwd_use_fused(Sq, Skv, variant))
     return cb200_fa_bwd_fused_main(d_o, q, k, v, lse2, delta, scratch + 2 * (size_t)B * H * S_pad, dq, dk, dv, B, Sq, Skv, H, S_pad, scale,
                                    0, err, st);
   auto make = [&](CUtensorMap* m, const void* p, int S, int box_rows) {

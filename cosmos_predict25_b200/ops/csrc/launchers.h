@@ -120,6 +120,7 @@ int cb200_fa_jvp(const void* q, const void* k, const void* v, const void* tq, co
 
 // fa_bwd.cu
 int cb200_fa_bwd_scratch_floats(int B, int Sq, int H);
+int cb200_fa_bwd_pick(int Sq, int Skv, int variant);   // the kernel that variant 0 stands for
 long cb200_fa_bwd_scratch_floats_v(int B, int Sq, int Skv, int H, int variant);
 int cb200_fa_bwd_v(const void* d_o, const void* q, const void* k, const void* v, const void* o, const float* lse, void* dq, void* dk,
                    void* dv, float* scratch, int B, int Sq, int Skv, int H, float scale, int variant, int* err, cudaStream_t st);
