@@ -113,6 +113,13 @@ void register_conv_ops(torch::Library& m) {
   m.def("conv_cl(Tensor x, Tensor w, int n_tile, int Cout, int[] taps, int T_out, int H_out, int W_out, int[] out_map, Tensor(a!) y, "
         "Tensor? resid, Tensor? bias, Tensor? cache=None, int pad=0, int t_stride=1, int hw_stride=1, "
         "Tensor(b!)? y_norm=None, Tensor? gamma=None, bool silu=True, bool write_raw=True) -> ()", &conv_cl);
+  m.def("conv_panels(int[] taps, int hw_stride, int Cin, int n_tile) -> int[]", [](c10::ArrayRef<int64_t> taps, int64_t hw_stride, int64_t Cin, int64_t n_tile) {
+    TORCH_CHECK(taps.size() % 3 == 0 && taps.size() >= 3 && taps.size() <= 81, "taps: 1..27 triples");
+    const std::vector<int> tp(taps.begin(), taps.end());
+    int out[3 + 27 * 6];
+    const int n = cb200_conv_panels(tp.data(), (int)tp.size() / 3, (int)hw_stride, (int)Cin, (int)n_tile, out);
+    return std::vector<int64_t>(out, out + n);
+  });
   m.def("fa_wide(Tensor q, Tensor k, Tensor v, float scale) -> Tensor", &fa_wide);
   m.def("rmsnorm_silu_cl(Tensor x, Tensor gamma, bool silu) -> Tensor", &rmsnorm_silu_cl);
 }

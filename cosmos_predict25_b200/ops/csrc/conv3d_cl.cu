@@ -13,7 +13,8 @@
 // memory as rows of 64 channels with 128-byte swizzle, K-major, which is what the MMA wants: eight voxels of a line are one 8-row group, the
 // groups are a line of the box apart, and tap (dy, dx) reads the same box from dy lines and dx rows on. The swizzle goes by the address, so
 // neither the start of a tap nor the distance of the groups has to be a whole number of 1,024-byte atoms (checked for every shift and
-// distance used here against a plain copy of the rows). Coordinates outside the tensor read zeros: that IS the zero padding of the
+// distance used here against a plain copy of the rows). Layers of 16 input or output channels take a box for each column of taps, as wide
+// as the tile (see tap_panels). Coordinates outside the tensor read zeros: that IS the zero padding of the
 // convolution (the channel coordinate stays a multiple of 64, so the 16-byte alignment rule of TMA holds).
 // The eight voxels run along the width or along the height, whichever leaves fewer tiles over the frame's edge.
 //
@@ -23,7 +24,9 @@
 // down-sampling) step the frame coordinate, and the pixel coordinates through the tensor map's element strides.
 //
 // CTA pairs (tcgen05 cta_group::2): two consecutive voxel tiles share the B operand, each CTA fetches its own A box and half of
-// the B rows, the even CTA issues M = 256 MMAs. A and B have a ring each: a box serves n columns of B boxes. What bounds the kernel is the
+// the B rows, the even CTA issues M = 256 MMAs. A and B have a ring each: a box serves n columns of B boxes. Where a box serves one column only (single taps
+// among them) they are one stage on one barrier: a step of a 3 x 1 x 1 convolution is four MMAs, whose issue a second wait and commit
+// made up a third of (384 to 768 channels, 4 frames of 120 x 208: 144 us with one barrier, 187 with two). What bounds the kernel is the
 // L2 -> shared-memory path of narrow layers and, on long runs, the card's power, to which that traffic adds: 128 voxels of a
 // 3 x 3 x 3 convolution with 96 channels took 498 KB with a box for each column of taps, now 290 (with 192 channels 1,035 and 800).
 // Decoding 8 latent frames of 720p 196 and 189 ms, encoding 29 frames of 768 x 432 46 and 44, an image of 640 x 640 2.31 and 2.25.
@@ -86,7 +89,9 @@ struct ConvParams {
 // box is one of 18 x 18 voxels and every B row in shared memory serves both.
 // BY_HEIGHT: X is the frame's height. The order of a sum - columns of taps along the width, their rows, channels - is the same either way, so that
 // a band of rows gives the bits of the whole frame.
-template <int RUN, int STACK, bool BY_HEIGHT>
+// COLS: columns of taps that an A box serves: all RUN of a square, or 1, a column of RUN rows and a box as wide as the tile. Then the box and its
+// taps' B rows are one stage on one barrier (JOINT; always so with single taps).
+template <int RUN, int STACK, bool BY_HEIGHT, int COLS>
 __global__ void __launch_bounds__(cv::kThreads, 1)
 conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_w,
                const __grid_constant__ ConvParams p, int* __restrict__ err) {
@@ -94,7 +99,9 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int b_half = p.n_tile * (BK * 2 / 2);                  // bytes of one tap's B rows in this CTA (half of the N tile)
-  constexpr int kLine = TX * STACK + RUN - 1;                  // voxels of a line of the A box
+  static_assert(COLS == RUN || (COLS == 1 && !BY_HEIGHT), "a box of one column lies along the width");
+  constexpr bool JOINT = COLS == 1;
+  constexpr int kLine = TX * STACK + COLS - 1;                 // voxels of a line of the A box
   constexpr int kBoxBytes = kLine * (TY + RUN - 1) * BK * 2, kASlot = (kBoxBytes + 1023) / 1024 * 1024;
   const int b_slot = RUN * b_half;                             // the taps of one column
   uint8_t* const ring_b = smem + p.a_slots * kASlot;
@@ -201,15 +208,18 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
           const int tc = cached ? tx + p.cache_frames : tx;
           const int xx = x0 * p.xy_stride + p.dx[g], xy = y0 * p.xy_stride + p.dy[g];
           for (int kb = 0; kb < p.kblocks && ok; ++kb) {
-            if (!mbar_wait(&a_empty[as], aph ^ 1, abort_flag)) { ok = false; break; }
-            if (rank == 0) mbar_arrive_expect_tx(&a_full[as], 2 * kBoxBytes);
-            tma_load_4d_pair(smem + as * kASlot, tm, mapa_shared(smem_u32(&a_full[as]), 0), kb * BK, xx, xy, tc);
-            if (++as == p.a_slots) { as = 0; aph ^= 1; }
+            if (!JOINT) {
+              if (!mbar_wait(&a_empty[as], aph ^ 1, abort_flag)) { ok = false; break; }
+              if (rank == 0) mbar_arrive_expect_tx(&a_full[as], 2 * kBoxBytes);
+              tma_load_4d_pair(smem + as * kASlot, tm, mapa_shared(smem_u32(&a_full[as]), 0), kb * BK, xx, xy, tc);
+              if (++as == p.a_slots) { as = 0; aph ^= 1; }
+            }
 #pragma unroll
-            for (int i = 0; i < RUN; ++i) {
+            for (int i = 0; i < COLS; ++i) {
               if (!mbar_wait(&b_empty[bs], bph ^ 1, abort_flag)) { ok = false; break; }
-              if (rank == 0) mbar_arrive_expect_tx(&b_full[bs], 2 * b_slot);
+              if (rank == 0) mbar_arrive_expect_tx(&b_full[bs], 2 * (b_slot + (JOINT ? kBoxBytes : 0)));
               const uint32_t bar = mapa_shared(smem_u32(&b_full[bs]), 0);
+              if (JOINT) tma_load_4d_pair(smem + bs * kASlot, tm, bar, kb * BK, xx, xy, tc);
 #pragma unroll
               for (int j = 0; j < RUN; ++j)
                 tma_load_2d_pair(ring_b + bs * b_slot + j * b_half, &tm_w, bar, (p.tap[g][i][j] * p.kblocks + kb) * BK, n0);
@@ -239,11 +249,11 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       uint32_t first = 0;
       for (int g = first_panel(t); g < p.npanels && ok; ++g) {
         for (int kb = 0; kb < p.kblocks && ok; ++kb) {
-          if (!wait_all(&a_full[as], aph)) { ok = false; break; }
-          const uint64_t da_s = da0 + (uint64_t)(as * (kASlot >> 4));
+          if (!JOINT && !wait_all(&a_full[as], aph)) { ok = false; break; }
+          const uint64_t da_s = da0 + (uint64_t)((JOINT ? bs : as) * (kASlot >> 4));
           const int ksteps = (p.Cin - kb * BK) / 16;   // below 4 in the last block of, e.g., C_in = 96: 32 real channels
 #pragma unroll
-          for (int i = 0; i < RUN; ++i) {
+          for (int i = 0; i < COLS; ++i) {
             if (!wait_all(&b_full[bs], bph)) { ok = false; break; }
             tc_fence_after();
             const uint64_t db_s = db0 + (uint64_t)(bs * (b_slot >> 4));
@@ -274,8 +284,10 @@ conv_cl_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
             if (++bs == p.b_slots) { bs = 0; bph ^= 1; }
           }
           first = 1u;
-          umma_commit_pair_w(&a_empty[as], leader);
-          if (++as == p.a_slots) { as = 0; aph ^= 1; }
+          if (!JOINT) {
+            umma_commit_pair_w(&a_empty[as], leader);
+            if (++as == p.a_slots) { as = 0; aph ^= 1; }
+          }
         }
       }
       if (!ok) break;
@@ -578,10 +590,10 @@ using namespace cb200;
 
 // As in the GEMM: the persistent grid is bounded by the pairs that the GPU can hold at once. One CTA per SM whatever the ring depths
 // (the rings are over half of the shared memory), so the figure for the largest shared-memory size holds for all.
-template <int RUN, int STACK, bool BY_HEIGHT>
+template <int RUN, int STACK, bool BY_HEIGHT, int COLS>
 static int launch_conv(cudaLaunchConfig_t& cfg, long tiles, int sms, const CUtensorMap& tx, const CUtensorMap& tc,
                        const CUtensorMap& tw, const ConvParams& p, int* err) {
-  const auto kern = conv_cl_kernel<RUN, STACK, BY_HEIGHT>;
+  const auto kern = conv_cl_kernel<RUN, STACK, BY_HEIGHT, COLS>;
   static int max_pairs = 0;
   if (max_pairs == 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cv::kSmemMax);
@@ -595,6 +607,93 @@ static int launch_conv(cudaLaunchConfig_t& cfg, long tiles, int sms, const CUten
   cfg.gridDim = dim3(2 * (unsigned)std::min<long>(tiles, std::min(max_pairs, sms / 2)));
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tx, tc, tw, p, err);
   return e == cudaSuccess ? 0 : 500 + (int)e;
+}
+
+// The K loop of a list of taps: panels of one frame offset, run rows x cols columns each, by ascending frame.
+struct TapPanels {
+  int run, cols, n;
+  int dt[cv::kMaxTaps], dh[cv::kMaxTaps], dw[cv::kMaxTaps];      // of a panel's first row and column
+  int tap[cv::kMaxTaps][cv::kMaxRun][cv::kMaxRun];               // [panel][column][row] -> index in the list
+};
+
+// The whole list has to fall into squares of 3 x 3 or 2 x 2 taps or columns of three or two rows, tried in that order, else each tap is its own
+// (with a spatial stride neighbouring taps do not share rows of a strided box).
+static TapPanels tap_panels(const int* taps, int ntaps, int hw_stride, int Cin, int n_tile) {
+  using namespace cv;
+  constexpr int kShapes[5][2] = {{3, 3}, {3, 1}, {2, 2}, {2, 1}, {1, 1}};
+  TapPanels tp{};
+  int order[kMaxTaps];
+  for (int i = 0; i < ntaps; ++i) order[i] = i;
+  std::stable_sort(order, order + ntaps, [&](int a, int b) { return taps[3 * a] < taps[3 * b]; });
+  for (int shape = hw_stride == 1 ? 0 : 4; shape < 5; ++shape) {
+    const int run = kShapes[shape][0], cols = kShapes[shape][1];
+    bool used[kMaxTaps] = {};
+    bool fits = ntaps % (run * cols) == 0;
+    tp.n = 0;
+    for (int q = 0; q < ntaps && fits; ++q) {
+      const int i = order[q];
+      if (used[i]) continue;
+      // the corner of the panel: the first row among the frame offset's unused taps (of the tap's column, for columns), and the first
+      // column of that row
+      int dh0 = taps[3 * i + 1], dw0 = taps[3 * i + 2];
+      if (run > 1)
+        for (int k = 0; k < ntaps; ++k)
+          if (!used[k] && taps[3 * k] == taps[3 * i] && (cols > 1 || taps[3 * k + 2] == taps[3 * i + 2]) &&
+              (taps[3 * k + 1] < dh0 || (taps[3 * k + 1] == dh0 && taps[3 * k + 2] < dw0))) {
+            dh0 = taps[3 * k + 1];
+            dw0 = taps[3 * k + 2];
+          }
+      for (int j = 0; j < run * cols && fits; ++j) {
+        int found = run > 1 ? -1 : i;
+        for (int k = 0; k < ntaps && found < 0; ++k)
+          if (!used[k] && taps[3 * k] == taps[3 * i] && taps[3 * k + 1] == dh0 + j / cols && taps[3 * k + 2] == dw0 + j % cols) found = k;
+        fits = found >= 0;
+        if (fits) {
+          used[found] = true;
+          tp.tap[tp.n][j % cols][j / cols] = found;
+        }
+      }
+      tp.dt[tp.n] = taps[3 * i];
+      tp.dh[tp.n] = dh0;
+      tp.dw[tp.n] = dw0;
+      ++tp.n;
+    }
+    tp.run = run;
+    tp.cols = cols;
+    if (fits) break;
+  }
+  // Squares go column by column where a shared box costs more than it saves. 16 output channels: an MMA is over as soon as its A rows are
+  // read, and rows that do not start on 1,024 bytes are read slower (96 to 3 channels, 704 x 1280: 9 taps 114 us with one box, 88 by
+  // columns, 27 taps 231 and 217). 16 input channels: a column is three MMAs, in whose time the wait for another barrier does not hide (16 to
+  // 384, 27 taps, 88 x 160 16.9 and 15.2 us, 352 x 640 143 and 132). With 32 channels on either side the shared box is as fast or faster.
+  // (The frame's size has no say: a band of rows has to give the bits of the whole frame.)
+  if (tp.cols == 3 && (Cin == 16 || (n_tile == 16 && Cin > 32))) {
+    const TapPanels square = tp;
+    tp.cols = 1;
+    tp.n = square.n * 3;
+    for (int c = 0; c < tp.n; ++c) {
+      const int g = c / 3, i = c % 3;
+      tp.dt[c] = square.dt[g];
+      tp.dh[c] = square.dh[g];
+      tp.dw[c] = square.dw[g] + i;
+      for (int j = 0; j < 3; ++j) tp.tap[c][0][j] = square.tap[g][i][j];
+    }
+  }
+  return tp;
+}
+
+// rows and columns of the panels, their number, then of each panel: dt, dh, dw and its taps by column and row; returns the number of values
+extern "C" int cb200_conv_panels(const int* taps, int ntaps, int hw_stride, int Cin, int n_tile, int* out) {
+  if (ntaps < 1 || ntaps > cv::kMaxTaps) return 0;
+  const TapPanels tp = tap_panels(taps, ntaps, hw_stride, Cin, n_tile);
+  int n = 0;
+  for (int v : {tp.run, tp.cols, tp.n}) out[n++] = v;
+  for (int g = 0; g < tp.n; ++g) {
+    for (int v : {tp.dt[g], tp.dh[g], tp.dw[g]}) out[n++] = v;
+    for (int i = 0; i < tp.cols; ++i)
+      for (int j = 0; j < tp.run; ++j) out[n++] = tp.tap[g][i][j];
+  }
+  return n;
 }
 
 // x [T_in, H_in, W_in, Cin] bf16; cache [cache_frames <= pad, H_in, W_in, Cin] or null; w [n_rows, ntaps * kblocks * 64] bf16 with
@@ -626,71 +725,34 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
     max_dt = std::max(max_dt, dt);
   }
   if (pad > 0 && max_dt < pad) return -52;      // the newest tap has to read X itself: otherwise a frame could be all padding
-  // Panels of taps: for run = 3, 2 the whole list has to fall into squares of run x run taps of one frame offset, else each tap is its own
-  // (with a spatial stride neighbouring taps do not share rows of a strided box)
-  int order[kMaxTaps], run = 1;
-  for (int i = 0; i < ntaps; ++i) order[i] = i;
-  std::stable_sort(order, order + ntaps, [&](int a, int b) { return taps[3 * a] < taps[3 * b]; });
-  int panel_dh[kMaxTaps], panel_dw[kMaxTaps], square[kMaxTaps][kMaxRun][kMaxRun];       // [panel][dh][dw] -> tap
-  for (run = hw_stride == 1 ? kMaxRun : 1; run >= 1; --run) {
-    bool used[kMaxTaps] = {};
-    int np = 0;
-    bool fits = ntaps % (run * run) == 0;
-    for (int q = 0; q < ntaps && fits; ++q) {
-      const int i = order[q];
-      if (used[i]) continue;
-      // the corner of the panel: the first row among the frame offset's unused taps, and the first column of that row
-      int dh0 = taps[3 * i + 1], dw0 = taps[3 * i + 2];
-      if (run > 1)
-        for (int k = 0; k < ntaps; ++k)
-          if (!used[k] && taps[3 * k] == taps[3 * i] && (taps[3 * k + 1] < dh0 || (taps[3 * k + 1] == dh0 && taps[3 * k + 2] < dw0))) {
-            dh0 = taps[3 * k + 1];
-            dw0 = taps[3 * k + 2];
-          }
-      for (int j = 0; j < run * run && fits; ++j) {
-        int found = run > 1 ? -1 : i;
-        for (int k = 0; k < ntaps && found < 0; ++k)
-          if (!used[k] && taps[3 * k] == taps[3 * i] && taps[3 * k + 1] == dh0 + j / run && taps[3 * k + 2] == dw0 + j % run) found = k;
-        fits = found >= 0;
-        if (fits) {
-          used[found] = true;
-          square[np][j / run][j % run] = found;
-        }
-      }
-      p.dt[np] = (int8_t)taps[3 * i];
-      panel_dh[np] = dh0;
-      panel_dw[np] = dw0;
-      ++np;
-    }
-    if (fits) {
-      p.npanels = np;
-      break;
-    }
-  }
+  const TapPanels tp = tap_panels(taps, ntaps, hw_stride, Cin, n_tile);
+  const int run = tp.run, cols = tp.cols;
+  p.npanels = tp.n;
   // Voxels of a line along the width, or along the height where that leaves fewer tiles; two tiles side by side for narrow layers, unless
   // 16 x 16 voxels leave more than a fifth over.
   auto up = [](int a, int b) -> long { return (a + b - 1) / b; };
   const long along_w = up(W_out, TX) * up(H_out, TY), along_h = up(H_out, TX) * up(W_out, TY), pairs = 2 * up(W_out, 2 * TX) * up(H_out, TY);
   const int stack = run == 3 && n_tile <= 128 && pairs * 10 <= std::min(along_w, along_h) * 12 ? 2 : 1;
-  const bool by_height = stack == 1 && along_h < along_w;
+  const bool by_height = stack == 1 && along_h < along_w && (cols > 1 || run == 1);
   p.X_out = by_height ? H_out : W_out;
   p.Y_out = by_height ? W_out : H_out;
   for (int g = 0; g < p.npanels; ++g) {
-    p.dx[g] = (int8_t)(by_height ? panel_dh[g] : panel_dw[g]);
-    p.dy[g] = (int8_t)(by_height ? panel_dw[g] : panel_dh[g]);
-    for (int i = 0; i < run; ++i)
-      for (int j = 0; j < run; ++j) p.tap[g][i][j] = (int8_t)square[g][j][i];
+    p.dt[g] = (int8_t)tp.dt[g];
+    p.dx[g] = (int8_t)(by_height ? tp.dh[g] : tp.dw[g]);
+    p.dy[g] = (int8_t)(by_height ? tp.dw[g] : tp.dh[g]);
+    for (int i = 0; i < cols; ++i)
+      for (int j = 0; j < run; ++j) p.tap[g][i][j] = (int8_t)tp.tap[g][i][j];
   }
-  const int box_x = TX * stack + run - 1, box_y = TY + run - 1;
+  const int box_x = TX * stack + cols - 1, box_y = TY + run - 1;
   const int a_slot = (box_x * box_y * BK * 2 + 1023) / 1024 * 1024, b_slot = run * n_tile * BK;
   const int fixed = kSmemFixed + (Cout <= kBiasMax ? (Cout * 4 + 15) / 16 * 16 : 0) + (y_norm != nullptr ? kSumSq + 256 * 4 : 0);
   // ring depths: as many columns of taps ahead as both rings hold
   int ahead = 0;
   for (int a = 1; a <= kMaxSlots; ++a) {
-    const int b = std::min(kMaxSlots, (kSmemMax - fixed - a * a_slot) / b_slot);
-    const int cols = std::min(a * run, b);
-    if (b >= 1 && (cols > ahead || (cols == ahead && a == 2))) {       // a second box even where it does not reach further
-      ahead = cols;
+    const int b = cols == 1 ? (a * (a_slot + b_slot) <= kSmemMax - fixed ? a : 0) : std::min(kMaxSlots, (kSmemMax - fixed - a * a_slot) / b_slot);
+    const int reach = std::min(a * cols, b);
+    if (b >= 1 && (reach > ahead || (reach == ahead && a == 2))) {       // a second box even where it does not reach further
+      ahead = reach;
       p.a_slots = a;
       p.b_slots = b;
     }
@@ -755,10 +817,13 @@ extern "C" int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Ci
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.numAttrs = 2;
   // (with one tap per panel both orders of the axes run the same code)
-  if (stack == 2) return launch_conv<3, 2, false>(cfg, tiles, sms, tx, tc, tw, p, err);
-  if (run == 1) return launch_conv<1, 1, false>(cfg, tiles, sms, tx, tc, tw, p, err);
-  if (run == 2) return by_height ? launch_conv<2, 1, true>(cfg, tiles, sms, tx, tc, tw, p, err) : launch_conv<2, 1, false>(cfg, tiles, sms, tx, tc, tw, p, err);
-  return by_height ? launch_conv<3, 1, true>(cfg, tiles, sms, tx, tc, tw, p, err) : launch_conv<3, 1, false>(cfg, tiles, sms, tx, tc, tw, p, err);
+  auto go = [&](auto launch) { return launch(cfg, tiles, sms, tx, tc, tw, p, err); };
+  if (run == 1) return go(launch_conv<1, 1, false, 1>);
+  if (run == 2 && cols == 1) return go(launch_conv<2, 1, false, 1>);
+  if (run == 2) return by_height ? go(launch_conv<2, 1, true, 2>) : go(launch_conv<2, 1, false, 2>);
+  if (cols == 1) return stack == 2 ? go(launch_conv<3, 2, false, 1>) : go(launch_conv<3, 1, false, 1>);
+  if (stack == 2) return go(launch_conv<3, 2, false, 3>);
+  return by_height ? go(launch_conv<3, 1, true, 3>) : go(launch_conv<3, 1, false, 3>);
 }
 
 extern "C" int cb200_rmsnorm_silu_cl(const void* x, const float* gamma, void* y, long n_vox, int C, int silu, cudaStream_t st) {

@@ -130,6 +130,7 @@ int cb200_fa_bwd(const void* d_o, const void* q, const void* k, const void* v, c
 
 extern "C" {
 // conv3d_cl.cu
+int cb200_conv_panels(const int* taps, int ntaps, int hw_stride, int Cin, int n_tile, int* out);   // out: up to 3 + 27 * 6 values
 int cb200_conv_cl(const void* x, int T_in, int H_in, int W_in, int Cin, const void* cache, int cache_frames, int pad, int t_stride,
                   int hw_stride, const void* w, int n_rows, int n_tile, int Cout, const int* taps, int ntaps, int T_out, int H_out, int W_out, const int* out_map, void* y, const void* resid,
                   const float* bias, void* y_norm, const float* gamma, int silu, int write_raw, int* err, int sms, cudaStream_t st);

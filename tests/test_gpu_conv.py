@@ -78,6 +78,31 @@ def test_taps_read_one_box(H, W, taps, Cin, Cout):
     assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
 
 
+# a box for each column of taps: squares of a layer of 16 output channels, columns of three and two rows; one and two tiles per CTA
+_COLUMNS = {"3x3": _LISTS["3x3"], "3x3x2": _LISTS["3x3x2"], "3x2": _LISTS["3x2"], "2x1": [(t, i, 1) for t in (0, 1) for i in (0, -1)]}
+
+
+@pytest.mark.parametrize("H,W", [(17, 33), (40, 9), (32, 48)])
+@pytest.mark.parametrize("taps", sorted(_COLUMNS))
+def test_columns_of_taps_read_one_box(H, W, taps):
+    from cosmos_predict25_b200.models import vae_wan_cl
+    torch.manual_seed(17)
+    lst = _COLUMNS[taps]
+    w = (torch.randn(16, len(lst), 96, device=DEV) / (len(lst) * 96) ** 0.5).bfloat16()
+    cl = vae_wan_cl.ConvCL(w, torch.randn(16, device=DEV), lst, DEV)
+    assert native.load().conv_panels(cl.taps, 1, 96, cl.n_tile)[:2] == [2 if taps == "2x1" else 3, 1]
+    x = torch.randn(3, H, W, 96, device=DEV).bfloat16()
+    got = cl(x, 2)
+    _no_kernel_error()
+    pad = F.pad(x.double(), (0, 0, 2, 2, 1, 1, 0, 0))
+    want = cl.bias.double().expand(2, H, W, 16).clone()
+    for n, (dt, dh, dw) in enumerate(lst):
+        want += pad[dt:dt + 2, 1 + dh:1 + dh + H, 2 + dw:2 + dw + W] @ w[:, n].double().t()
+    # one rounding to bf16; the fp32 sums of at most 1,728 products stay far below it
+    assert ((got.double() - want).norm() / want.norm()).item() < 1.5 * 2.0 ** -9
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
+
+
 def test_upsample_phase_convolutions_match_nearest_then_conv():
     from cosmos_predict25_b200.models import vae_wan, vae_wan_cl
     torch.manual_seed(1)
