@@ -833,11 +833,15 @@ extern "C" int cb200_rmsnorm_silu_cl(const void* x, const float* gamma, void* y,
     const int per_block = 256 / lanes;
     launch_pdl(kern, dim3((unsigned)std::min<long>((n_vox + per_block - 1) / per_block, kRmsCtas)), dim3(256), 0, st, (const bf16*)x, gamma, (bf16*)y, n_vox, C, scale, silu);
   };
-  // three pieces per lane while that fills the lanes (C = 96, 192, 384: no idle lane); the widest rows take four
-  if (C <= 48) run(rmsnorm_silu_cl_kernel<2, 3>, 2);
+  // three pieces per lane while that fills the lanes (C = 96, 192, 384, 768: no idle lane), never more than the row has: a lane keeps gamma for
+  // all of its pieces, and with four pieces for 512 channels the kernel was slower than without (25,600 voxels 13.1 and 17.3 us)
+  if (C <= 16) run(rmsnorm_silu_cl_kernel<2, 1>, 2);
+  else if (C <= 48) run(rmsnorm_silu_cl_kernel<2, 3>, 2);
   else if (C <= 96) run(rmsnorm_silu_cl_kernel<4, 3>, 4);
   else if (C <= 192) run(rmsnorm_silu_cl_kernel<8, 3>, 8);
   else if (C <= 384) run(rmsnorm_silu_cl_kernel<16, 3>, 16);
+  else if (C <= 512) run(rmsnorm_silu_cl_kernel<32, 2>, 32);
+  else if (C <= 768) run(rmsnorm_silu_cl_kernel<32, 3>, 32);
   else run(rmsnorm_silu_cl_kernel<32, 4>, 32);
   return (int)cudaGetLastError();
 }

@@ -282,7 +282,7 @@ def test_wide_attention_matches_fp32(B, Sq, Skv, gain):
     _close(got, want, 1e-2, 1e-2, "attention of width 384")
 
 
-@pytest.mark.parametrize("C", [8, 32, 48, 56, 96, 160, 192, 384, 392, 1024])
+@pytest.mark.parametrize("C", [8, 16, 24, 32, 48, 56, 96, 160, 192, 384, 392, 512, 520, 768, 776, 1024])
 def test_rmsnorm_silu_widths(C):
     torch.manual_seed(7)
     x = torch.randn(3, 5, 7, C, device=DEV).bfloat16()
@@ -293,7 +293,8 @@ def test_rmsnorm_silu_widths(C):
         _close(native.load().rmsnorm_silu_cl(x, g, silu), F.silu(want) if silu else want, 4e-3, 8e-3, f"rmsnorm {C}")
 
 
-@pytest.mark.parametrize("C,n", [(384, 444 * 16 * 2 + 5), (192, 444 * 32 + 1), (96, 444 * 64 * 3 - 1), (32, 444 * 128 + 77), (1024, 444 * 8 * 2 + 3)])
+@pytest.mark.parametrize("C,n", [(384, 444 * 16 * 2 + 5), (192, 444 * 32 + 1), (96, 444 * 64 * 3 - 1), (32, 444 * 128 + 77), (1024, 444 * 8 * 2 + 3), (16, 444 * 128 + 5),
+                                 (512, 444 * 8 + 3), (768, 444 * 8 * 2 + 1)])
 def test_rmsnorm_silu_of_more_voxels_than_one_pass(C, n):
     """Lanes go on from voxel to voxel: every voxel's result is the one it has in a call of its own few."""
     torch.manual_seed(16)
