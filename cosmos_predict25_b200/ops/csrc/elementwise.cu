@@ -63,16 +63,21 @@ __device__ __forceinline__ void store_f8(float* p, const float (&f)[8]) {
 // For few rows and short frames. Few rows are bound by latency: the row and its modulation vectors
 // are loaded together, a thread holds NV pieces of 16 bytes, and each of the two sums is one barrier. With a warp per row, its two
 // reductions and then its loads of the modulation in a row, 512 rows of 2048 took 5.6 us in a row of launches, now 3.5 (1024 rows 7.1
-// and 3.7; a launch that does nothing about 2).
-template <int NV, int THREADS>
-__global__ void __launch_bounds__(THREADS) ln_modulate_fwd_row_kernel(
+// and 3.7; a launch that does nothing about 2). Thousands of rows that a warp holds are bound by the start of CTAs: ROWS rows to a CTA then,
+// a warp each (8192 frames of one row of 256 9.2 us with a CTA a row, now 4.2; 2048 frames of three rows of 512 7.7 and 5.3; 64 frames of 64
+// rows of 256 in batches 3.7, now 3.4).
+template <int NV, int THREADS, int ROWS>
+__global__ void __launch_bounds__(THREADS * ROWS) ln_modulate_fwd_row_kernel(
     const bf16* __restrict__ x, const float* __restrict__ shift, const float* __restrict__ scale,
-    bf16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int D, int L, long ld_shift, long ld_scale,
+    bf16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, long rows, int D, int L, long ld_shift, long ld_scale,
     float eps) {
+  static_assert(ROWS == 1 || THREADS == 32, "several rows in a CTA: a warp each");
   __shared__ float red[2][THREADS / 32];
   pdl_trigger();                     // launched with programmatic serialisation (see common.cuh)
   pdl_wait();
-  const long row = blockIdx.x;
+  const unsigned tid = ROWS == 1 ? threadIdx.x : threadIdx.x & 31;
+  const long row = ROWS == 1 ? (long)blockIdx.x : (long)blockIdx.x * ROWS + (threadIdx.x >> 5);
+  if (ROWS > 1 && row >= rows) return;
   const long frame = row / L;
   const int nvec = D >> 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + row * D);
@@ -82,12 +87,12 @@ __global__ void __launch_bounds__(THREADS) ln_modulate_fwd_row_kernel(
   float a[NV][8], b[NV][8];
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    const int c = threadIdx.x + i * THREADS;
+    const int c = tid + i * THREADS;
     v[i] = c < nvec ? xr[c] : bf16x8{};
   }
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    const int c = threadIdx.x + i * THREADS;
+    const int c = tid + i * THREADS;
     if (c < nvec) {
       load_f8(sh + c * 8, a[i]);
       load_f8(sc + c * 8, b[i]);
@@ -95,6 +100,7 @@ __global__ void __launch_bounds__(THREADS) ln_modulate_fwd_row_kernel(
   }
   auto total = [&](float2 s2, float* slots) -> float {
     const float s = warp_sum(s2.x + s2.y);
+    if (THREADS == 32) return s;
     if (lane == 0) slots[warp] = s;
     __syncthreads();
     float t = 0.f;
@@ -112,7 +118,7 @@ __global__ void __launch_bounds__(THREADS) ln_modulate_fwd_row_kernel(
   float2 q2 = make_float2(0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < NV; ++i)
-    if (threadIdx.x + i * THREADS < nvec) {
+    if (tid + i * THREADS < nvec) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 d = add2(__bfloat1622float2(v[i].v[j]), nm);
@@ -120,14 +126,14 @@ __global__ void __launch_bounds__(THREADS) ln_modulate_fwd_row_kernel(
       }
     }
   const float rstd = rsqrtf(total(q2, red[1]) / D + eps);
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     mean_out[row] = mean;
     rstd_out[row] = rstd;
   }
   const float2 one2 = make_float2(1.f, 1.f), rs2 = make_float2(rstd, rstd);
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    const int c = threadIdx.x + i * THREADS;
+    const int c = tid + i * THREADS;
     if (c < nvec) {
       bf16x8 o;
 #pragma unroll
@@ -904,12 +910,23 @@ int cb200_ln_groups_per_frame(int L, int rows_per_cta) { return (L + rows_per_ct
 
 void cb200_ln_modulate_fwd(const void* x, const float* shift, const float* scale, void* y, float* mean, float* rstd,
                            long rows, int D, int L, long ld_shift, long ld_scale, float eps, cudaStream_t st) {
+  auto by_row = [&](auto kern, int threads, int per_cta) {
+    launch_pdl(kern, dim3((unsigned)((rows + per_cta - 1) / per_cta)), dim3(threads * per_cta), 0, st, (const bf16*)x, shift, scale, (bf16*)y, mean, rstd, rows,
+               D, L, ld_shift, ld_scale, eps);
+  };
+  // Many rows that a warp holds, where a walk over a frame's rows has little to walk over (frames of up to three rows) or few CTAs would walk
+  // (rows of 256: 8192 in frames of 16 4.1 us by warp and 4.8 in batches, 16,384 7.3 and 7.2): a warp for each.
+  if (D <= 512 && rows >= 2048 && (L < 4 || (D <= 256 && rows >= 3072 && rows < 12288))) {
+    if (D <= 256) by_row(ln_modulate_fwd_row_kernel<1, 32, 8>, 32, 8); else by_row(ln_modulate_fwd_row_kernel<2, 32, 8>, 32, 8);
+    return;
+  }
   // Few rows (or frames of fewer rows than a CTA takes at a time): a CTA for each. The line: 2048 rows of 2048 6.4 us that way and 6.2 us in
   // batches, 1024 rows 3.7 and 4.4; 1024 rows of 5120 8.6 and 6.9, 512 rows 4.9 and 6.3.
   if (rows < (D <= 2048 ? 2048 : 1024) || L < 4) {
-#define LAUNCH_ROW(NV, T) launch_pdl(ln_modulate_fwd_row_kernel<NV, T>, dim3((unsigned)rows), dim3(T), 0, st, (const bf16*)x, shift, scale, (bf16*)y, mean, rstd, D, L, ld_shift, ld_scale, eps)
-    if (D <= 1024) LAUNCH_ROW(1, 128); else if (D <= 2048) LAUNCH_ROW(2, 128); else if (D <= 4096) LAUNCH_ROW(2, 256); else LAUNCH_ROW(4, 256);
-#undef LAUNCH_ROW
+    if (D <= 1024) by_row(ln_modulate_fwd_row_kernel<1, 128, 1>, 128, 1);
+    else if (D <= 2048) by_row(ln_modulate_fwd_row_kernel<2, 128, 1>, 128, 1);
+    else if (D <= 4096) by_row(ln_modulate_fwd_row_kernel<2, 256, 1>, 256, 1);
+    else by_row(ln_modulate_fwd_row_kernel<4, 256, 1>, 256, 1);
     return;
   }
   // rows of a CTA: two waves of CTAs while they are few, at most 20 (longer walks leave the last wave emptier)

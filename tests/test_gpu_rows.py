@@ -36,10 +36,11 @@ def test_modulation_slices_are_read_in_place(D, L, T, offset):
     assert _max_rel(dg.view(1, T, D), (dout.double() * y.double()).sum(2)) < 1e-5
 
 
-# a CTA per row (few rows, short frames) and batches of rows per CTA: partial warps and partial last pieces of a row, frames that end
+# a CTA or a warp per row (few rows, short frames, narrow rows) and batches of rows per CTA: partial warps and partial last pieces of a row, frames that end
 # inside a batch, the row counts where the kernel changes, every instantiation
 @pytest.mark.parametrize("D,L,T", [(8, 700, 3), (520, 4, 520), (1024, 2047, 1), (2048, 2048, 1), (2040, 41, 53), (2048, 3, 700), (2056, 1023, 1),
-                                   (2056, 26, 41), (4104, 513, 2), (5120, 1041, 1), (5128, 130, 8), (8192, 7, 150), (8192, 5, 3)])
+                                   (2056, 26, 41), (4104, 513, 2), (5120, 1041, 1), (5128, 130, 8), (8192, 7, 150), (8192, 5, 3),
+                                   (256, 3, 691), (504, 1, 2051), (264, 2, 1024), (248, 769, 4), (8, 4097, 1), (256, 4096, 3)])
 def test_layernorm_row_counts_and_widths(D, L, T):
     torch.manual_seed(6)
     x = (torch.randn(T * L, D, device=DEV) * 2 + 3 * torch.randn(T * L, 1, device=DEV)).bfloat16()
