@@ -519,8 +519,9 @@ __global__ void __launch_bounds__(kThreads) gate_residual_bwd_kernel(
 // offset, so that the rotation partner of every element is in the lane itself and one cosine / sine vector serves both; reductions
 // stay inside the 16-lane half. Token and head of a row are counted along instead of divided out (64-bit divisions per row, a
 // shuffle per element and twice the table loads bound the first layout by instruction issue). Bound by memory and by the warps in flight:
-// the rows of later passes wait as bf16 (72 registers a thread before, 62 now: four CTAs on an SM for three) and the table's row is
-// loaded with the first ones and again only when the token changes. 46,800 tokens x 16 heads 88 us before, 68 now, without rotation
+// the rows of later passes wait as bf16 (72 registers a thread before, 62 now: four CTAs on an SM for three) and the table's rows are
+// loaded with them: one where a lane's rows are heads of one token (a multiple of eight heads), else one for each (loaded pass by pass behind
+// the sums, 512 x 2 tokens with one head of 64 took 2.7 us, now 2.1). 46,800 tokens x 16 heads 88 us before, 68 now, without rotation
 // 67 and 57 (the bytes take 59 us; part of them are in L2); 7040 tokens 10.4 and 8.0, 46,800 tokens x 40 heads 209 and 156.
 constexpr int kRmsPasses = 4;        // forward: passes (of two rows) whose loads a warp keeps in flight together
 
@@ -605,7 +606,8 @@ struct RmsTensors {
   float* rstd[2];
 };
 
-template <int HD, bool ROPE>
+// ROPE: 0 none; 1: all rows of a lane are heads of one token; 2: any tokens
+template <int HD, int ROPE>
 __global__ void __launch_bounds__(256) rmsnorm_rope_fwd_kernel(
     const __grid_constant__ RmsTensors tensors, const float* __restrict__ cosv, const float* __restrict__ sinv, long n_rows, int S, int H,
     float eps) {
@@ -635,12 +637,17 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_fwd_kernel(
   float2 wl[Q], wh[Q];
   load_weight_part<P>(w, w_bf16, sub * P, wl);
   load_weight_part<P>(w, w_bf16, HD / 2 + sub * P, wh);
-  RowCursor at(row0 < n_rows ? row0 : 0, S, H);
-  float2 c[Q], sn[Q];                         // of token `table_s`: a lane's rows are heads of one token as a rule
-  int table_s = at.s;
-  if (ROPE) {
-    load_f32_part<P>(cosv + (long)at.s * (HD / 2) + sub * P, c);
-    load_f32_part<P>(sinv + (long)at.s * (HD / 2) + sub * P, sn);
+  float2 c[ROPE == 2 ? U : 1][Q], sn[ROPE == 2 ? U : 1][Q];
+  if (ROPE != 0) {
+    RowCursor token(row0 < n_rows ? row0 : 0, S, H);
+#pragma unroll
+    for (int u = 0; u < (ROPE == 2 ? U : 1); ++u) {
+      if (row0 + 2 * u < n_rows) {
+        load_f32_part<P>(cosv + (long)token.s * (HD / 2) + sub * P, c[u]);
+        load_f32_part<P>(sinv + (long)token.s * (HD / 2) + sub * P, sn[u]);
+      }
+      token.advance(2, S, H);
+    }
   }
 #pragma unroll
   for (int u = 0; u < U; ++u) {
@@ -664,17 +671,15 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_fwd_kernel(
       lo[j] = mul2(mul2(lo[j], rs2), wl[j]);
       hi[j] = mul2(mul2(hi[j], rs2), wh[j]);
     }
-    if (ROPE && valid) {
-      if (at.s != table_s) {
-        load_f32_part<P>(cosv + (long)at.s * (HD / 2) + sub * P, c);
-        load_f32_part<P>(sinv + (long)at.s * (HD / 2) + sub * P, sn);
-        table_s = at.s;
-      }
+    if (ROPE != 0) {
+      constexpr int kTables = ROPE == 2 ? U : 1;
+      const float2(&cu)[Q] = c[u < kTables ? u : 0];
+      const float2(&su)[Q] = sn[u < kTables ? u : 0];
 #pragma unroll
       for (int j = 0; j < Q; ++j) {
-        const float2 a = lo[j], b = hi[j], ns = make_float2(-sn[j].x, -sn[j].y);
-        lo[j] = fma2(b, ns, mul2(a, c[j]));
-        hi[j] = fma2(a, sn[j], mul2(b, c[j]));
+        const float2 a = lo[j], b = hi[j], ns = make_float2(-su[j].x, -su[j].y);
+        lo[j] = fma2(b, ns, mul2(a, cu[j]));
+        hi[j] = fma2(a, su[j], mul2(b, cu[j]));
       }
     }
     if (valid) {
@@ -682,7 +687,6 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_fwd_kernel(
       store_part<P>(yr, lo);
       store_part<P>(yr + HD / 2, hi);
     }
-    at.advance(2, S, H);
   }
 }
 
@@ -975,8 +979,10 @@ static void launch_rmsnorm_rope_fwd(const RmsTensors& tensors, int n, const floa
                                     float eps, cudaStream_t st) {
   const dim3 blocks((unsigned)((n_rows + 16 * kRmsPasses - 1) / (16 * kRmsPasses)), n);   // 8 warps x 2 rows x passes per CTA
   auto launch = [&](auto kern) { launch_pdl(kern, blocks, dim3(256), 0, st, tensors, cosv, sinv, n_rows, S, H, eps); };
-  if (HD == 128) cosv != nullptr ? launch(rmsnorm_rope_fwd_kernel<128, true>) : launch(rmsnorm_rope_fwd_kernel<128, false>);
-  else cosv != nullptr ? launch(rmsnorm_rope_fwd_kernel<64, true>) : launch(rmsnorm_rope_fwd_kernel<64, false>);
+  const bool one_token = H % (2 * kRmsPasses) == 0;
+  if (cosv == nullptr) HD == 128 ? launch(rmsnorm_rope_fwd_kernel<128, 0>) : launch(rmsnorm_rope_fwd_kernel<64, 0>);
+  else if (one_token) HD == 128 ? launch(rmsnorm_rope_fwd_kernel<128, 1>) : launch(rmsnorm_rope_fwd_kernel<64, 1>);
+  else HD == 128 ? launch(rmsnorm_rope_fwd_kernel<128, 2>) : launch(rmsnorm_rope_fwd_kernel<64, 2>);
 }
 
 void cb200_rmsnorm_rope_fwd(const void* x, const void* w, int w_bf16, const float* cosv, const float* sinv, void* y, float* rstd,

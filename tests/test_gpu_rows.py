@@ -95,7 +95,8 @@ def test_row_operators_take_modulation_rows_of_any_shape():
     assert torch.equal(ops.gemm_bf16_gate_residual(h, w, x, flat, B * T * L), ops.gemm_bf16_gate_residual(h, w, x, flat[None], B * T * L))
 
 
-@pytest.mark.parametrize("HD,H,S,B", [(128, 5, 7, 2), (128, 16, 33, 1), (64, 3, 130, 2), (128, 40, 3, 1), (64, 1, 1, 1)])
+@pytest.mark.parametrize("HD,H,S,B", [(128, 5, 7, 2), (128, 16, 33, 1), (64, 3, 130, 2), (128, 40, 3, 1), (64, 1, 1, 1), (64, 8, 37, 1), (128, 12, 50, 2),
+                                          (128, 24, 5, 1)])
 @pytest.mark.parametrize("wdtype", [torch.bfloat16, torch.float32])
 def test_rmsnorm_rope_head_counts(HD, H, S, B, wdtype):
     torch.manual_seed(2)
