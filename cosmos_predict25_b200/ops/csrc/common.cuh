@@ -56,8 +56,9 @@ __device__ __forceinline__ float scrub(float x) {
 
 // Programmatic dependent launch: a kernel launched with `launch_pdl` may start before the kernel in front of it on the stream has
 // ended - its set-up (barriers, TMEM, descriptors) and its launch then overlap that kernel's tail. Every thread block of such a kernel
-// calls pdl_wait() before its first access to global memory; the call returns when the kernel in front is complete and its writes
-// are visible. pdl_trigger() lets the next kernel start; it comes after the block's own TMEM allocation, so that a waiting kernel
+// calls pdl_wait() before its first access to global memory (the device's error word apart, which the kernel reads again behind it); the
+// call returns when the kernel in front is complete and its writes are visible. Hints that ask a tile into L2 may come ahead of it: they read
+// nothing into the kernel, and L2 is where the writes of the kernel in front meet the loads behind the wait. pdl_trigger() lets the next kernel start; it comes after the block's own TMEM allocation, so that a waiting kernel
 // never holds what a block of this one still needs (the next kernel starts only when every block has triggered or ended).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
