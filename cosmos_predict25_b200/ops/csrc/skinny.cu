@@ -410,13 +410,14 @@ using namespace cb200;
 // padded to its warps (256, 512, 1024 or 2048), times the rows; the wide kernel takes about 9 us as soon as it splits, since the sums are a
 // launch more (from K = 256 on, up to 296 tiles of 256 columns), and 256 columns' time for few columns. us of the wide kernel and of this
 // one, launches back to back with the weights in L2 as far as they fit, and behind a flush of L2 (two layers of 28 blocks' modulation are
-// 84 x 256 x 2048 and 84 x 6144 x 256; a network's weights come from HBM):
+// 84 x 256 x 2048 and 84 x 6144 x 256; a network's weights come from HBM). The second of these with two rows stays here although it is slower by
+// itself: inside a denoising step of a 256 x 256 image the step takes 4,407 us with it and 4,413 with the wide kernel (spread below 2 us).
 //   rows                  1                         2                         4
 //   1 x 256 x 2048     9.9  3.6, 17.8 10.2      10.4  4.2, 19.5 10.2      11.2  5.1, 21.5 10.2
 //   1 x 4096 x 256     8.9  3.8, 17.4 10.2       9.2  4.6, 17.4 10.2      10.4  6.1, 19.4 12.3
 //   84 x 64 x 2048    32.1 10.8, 37.9 14.4      32.2  9.8, 39.8 16.4      32.6 14.1, 40.0 20.5
 //   84 x 256 x 2048   32.9 22.5, 46.0 28.7      33.7 30.2, 46.1 37.8      34.7 33.1, 48.1 39.9
-//   84 x 6144 x 256   68.6 54.7, 77.8 65.6      70.5 72.0, 79.9 84.0      74.3 90.3, 84.0 97.3     unsplit: one row only
+//   84 x 6144 x 256   68.6 54.7, 77.8 65.6      70.5 72.0, 79.9 84.0      74.3 90.3, 84.0 97.3     unsplit: one and two rows
 //   1 x 6144 x 2048   12.5 10.8, 21.5 14.4      13.0 10.4, 23.6 16.4      13.3 17.8, 25.6 20.5
 //   3 x 6144 x 1032   15.8 13.8, 25.7 20.5      16.4 20.2, 27.6 27.5      17.2 23.7, 29.7 30.7     half of the lanes idle
 //   84 x 768 x 64      5.3  8.4, 10.3 14.3       5.6 10.9, 12.3 18.4       6.4 14.9, 13.2 20.5     most of the lanes idle: to 4096 columns
@@ -430,8 +431,8 @@ extern "C" int cb200_skinny_rows(long a_k, long b_n, long b_k, int b_is_bf16, in
   if (R == 1 && (split || full || (K >= 256 && K * 3 >= padded * 2))) return 1;
   if (K < 256) return cols <= 16384;
   if (N <= 128 || E <= 6L << 20) return 1;
-  if (!split || R == 1) return 0;
-  return full || (R == 2 && E <= 14L << 20);
+  if (full) return split || R == 2;
+  return split && R == 2 && E <= 14L << 20;
 }
 
 // whether a call goes to the wide kernel (the split of long reductions counts its tiles): bf16 weights with one contiguous index and

@@ -101,13 +101,13 @@ def _few_rows(Z, R, N, K):
 
 
 def test_few_row_kernel_is_taken_where_it_is_faster():
-    """Measured slower there and back with the wide kernel: the second layer of 28 blocks' modulation from two rows on, weights of up to 64
+    """Measured slower there and back with the wide kernel: the second layer of 28 blocks' modulation from three rows on, weights of up to 64
     elements a row with many columns, half-empty lanes. Measured faster with the weights from HBM: the first layer, few columns, calls whose
     reduction the wide kernel splits."""
-    for Z, R, N, K in ((84, 2, 6144, 256), (84, 4, 6144, 256), (84, 2, 2048, 256), (84, 4, 256, 64), (84, 1, 768, 8), (84, 2, 6144, 64), (6, 2, 6144, 64),
-                       (84, 2, 2048, 512), (28, 2, 3072, 264), (3, 2, 6144, 1032), (28, 1, 6144, 264), (84, 3, 256, 128), (84, 1, 1024, 192)):
+    for Z, R, N, K in ((84, 3, 6144, 256), (84, 4, 6144, 256), (84, 4, 2048, 256), (84, 4, 256, 64), (84, 1, 768, 8), (84, 2, 6144, 64), (6, 2, 6144, 64),
+                       (84, 4, 2048, 512), (28, 2, 3072, 264), (3, 2, 6144, 1032), (28, 1, 6144, 264), (84, 3, 256, 128), (84, 1, 1024, 192)):
         assert not _few_rows(Z, R, N, K), (Z, R, N, K)
-    for Z, R, N, K in ((84, 1, 256, 2048), (84, 2, 256, 2048), (84, 4, 256, 2048), (84, 1, 6144, 256), (1, 1, 4096, 256), (1, 2, 4096, 256), (1, 4, 4096, 256),
+    for Z, R, N, K in ((84, 1, 256, 2048), (84, 2, 256, 2048), (84, 4, 256, 2048), (84, 1, 6144, 256), (84, 2, 6144, 256), (1, 1, 4096, 256), (1, 2, 4096, 256), (1, 4, 4096, 256),
                        (1, 4, 256, 2048), (1, 2, 6144, 2048), (84, 4, 64, 2048), (84, 4, 64, 256), (1, 4, 4096, 64), (1, 1, 1, 8), (12, 2, 1024, 520),
                        (84, 2, 768, 1024), (84, 1, 3072, 248), (12, 4, 3072, 2048), (84, 3, 768, 1024)):
         assert _few_rows(Z, R, N, K), (Z, R, N, K)
