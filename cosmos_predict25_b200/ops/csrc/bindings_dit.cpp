@@ -2,8 +2,8 @@
 // of all blocks for a prompt) as ONE operator each, which launches the package's kernels back to back. A block is 16 launches
 // (13 here: q, k and v are one GEMM over three weights, the norms of q and k one launch);
 // issued one by one through Python and the dispatcher they cost about 25 us of host time each, more than most of them take on the GPU
-// for an image of 256 x 256 (512 tokens with guidance): 12.9 ms a step, 8.0 ms with this loop when it was written, 6.1 ms with the
-// kernels of today (4.3 ms of it host time). The kernels are those of models/dit.py:
+// for an image of 256 x 256 (512 tokens with guidance): 12.9 ms a step, 8.0 ms with this loop when it was written, 4.4 ms with the
+// kernels of today (about 3 ms of host time beside them). The kernels are those of models/dit.py:
 // Block.forward and so are the sums, except where more tiles in a launch change how a contraction is split.
 
 #include <ATen/ATen.h>

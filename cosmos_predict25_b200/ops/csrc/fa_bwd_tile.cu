@@ -94,7 +94,7 @@ fa_bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint8_t* sQ = smem + 2 * kTile;                       // kQStages tiles
   uint8_t* sDO = sQ + kQStages * kTile;
   uint8_t* sDS = sDO + kTile;                           // dS^T [128 keys][128 queries] bf16, two 64-query halves
-  uint8_t* sRed = sDS + kTile;                          // [drain warp][2 stages] blocks on their way into the dQ buffer
+  uint8_t* sRed = sDS + kTile;                          // [drain warp][2 blocks] on their way into the dQ buffer, filled and emptied together
   float* sStat = reinterpret_cast<float*>(sRed + kRedBytes);  // [2 stages][256]
   uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(sStat) + 2 * kStatBytes);
   uint64_t* kv_full = bars;              // [1]

@@ -97,7 +97,8 @@ struct GemmEpilogue {
 
 // Exact GELU of a pair of values: x Phi(x) = (x + |x|) / 2 - |x| Phi(-|x|), and Phi(-a) = exp(-a^2 / 2) R(a), where R = erfcx(a / sqrt 2) / 2
 // falls smoothly from 1/2: a degree-11 polynomial in a scaled to [-1, 1] on [0, 5.5], fitted for the relative error (4.2e-6; a thousandth
-// of a bf16 rounding). a R(a) hardly changes beyond 5.5, where the product is below 1e-7: a is held there. The difference 1 + erff
+// of a bf16 rounding; 1 + erff is at 1.3e-7 for positive arguments, at 1.2e-5 for -3 and lost below. Behind the rounding to bf16, the only type
+// that leaves here, the 2-norm error is the same to eight digits for arguments of 0.25 to 4 in spread). a R(a) hardly changes beyond 5.5, where the product is below 1e-7: a is held there. The difference 1 + erff
 // that stood here loses its digits for x below -3, and took twice the instructions, which an epilogue has to itself when a CTA has one tile:
 // 512 x 8192 x 2048 with GELU 20.6 us before, now 18.6 (without GELU 16.1).
 // Coefficients are negated: the sum is a fused multiply-add. Infinities and NaN give what the product x Phi(x) gives.
