@@ -889,8 +889,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 // 1024 x 1024 read 1.6 GB instead of 0.4: 215 us.) Both operands K-major, N a multiple of 256.
 // ws: [slot][64 column quadruples][256 rows] float4; slots: pair turn * tiles + tile, then three for each pair of the tail.
 // From K = 100,352 to 1024 columns, before and now: 256 rows 125 and 72 us, 512 127 and 83, 768 133 and 115, 1024 174 and 154, 1536 251 and 206,
-// 3072 490 and 441; 2048 rows (32 tiles, two pairs each) would go from 282 to 332 and stay with clusters; 1024 rows from K = 32,768 80 and 72,
-// from K = 16,384 the same.
+// 3072 490 and 441; 2048 rows (32 tiles, two pairs each) would go from 282 to 332 and stay with clusters. Where the line lies: cb200_gemm_stream.
 struct StreamPlan {
   int tiles, tiles_n, k_all;
   int per_tile, extra, tail;     // pairs a tile, pairs of the tail, k-blocks of a tile that are theirs
